@@ -6,8 +6,7 @@
 // inside the same functor (force.h:18-21, 102-104, 145).  Because the j-list
 // is the caller's (an FDPS group superset), out-of-support j contribute zero
 // to sums but still enter v_sig_max in the hydro functor, exactly as on the
-// CPU.  One CTA per walk; the walk's j-list is staged through shared memory
-// in tiles and read by every thread (one thread per i).
+// CPU (kernels: sph_batch64.cu in FP64, sph_batch32.cu in mixed precision).
 //
 // Staging: the walks' payloads live in the caller's host memory, one array
 // per walk.  Where the GPU can read pageable host memory (GB300's
@@ -36,8 +35,6 @@ std::atomic<int> g_batch_prec{SPH_PREC_FP64};            // the arithmetic of th
 std::atomic<int> g_batch_staging{SPH_BATCH_STAGING_AUTO};   // who moves the payloads to the device
 
 constexpr int MAX_TAGS = 64;
-constexpr int WT = 128;
-
 thread_local std::string g_batch_err;
 
 int batch_fail(int code, const std::string &msg) {
@@ -140,8 +137,6 @@ int tag_state(int tag, TagState **out) {
 // ---------------------------------------------------------------------------
 // kernels: meta[w*6 + {0..5}] = i offset, n_i, j offset, n_j, spj offset, n_spj (element offsets)
 
-__device__ __forceinline__ double3 ld3(const double *p) { return make_double3(p[0], p[1], p[2]); }
-
 static_assert(sizeof(sph_epi_dens) % 8 == 0 && sizeof(sph_epj_dens) % 8 == 0 && sizeof(sph_epi_drvt) % 8 == 0 &&
                   sizeof(sph_epj_drvt) % 8 == 0 && sizeof(sph_epi_hydro) % 8 == 0 &&
                   sizeof(sph_epj_hydro) % 8 == 0 && sizeof(sph_epi_grav) % 8 == 0 &&
@@ -210,228 +205,10 @@ __global__ void __launch_bounds__(256) k_scatter_results(const int64_t *meta, co
                    (int64_t)s_res * m[1] / 8);
 }
 
-// CalcDensity, force.h:9-23
-__global__ void __launch_bounds__(WT) k_walk_dens(const int64_t *meta, const sph_epi_dens *epi, JSrc<sph_epj_dens> epj,
-                                                  sph_result_dens *res) {
-    __shared__ double4 tile[WT];
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        double3 pi = make_double3(0, 0, 0);
-        double hi = 1.0, mi = 1.0;
-        if (act) {
-            pi = ld3(epi[io + ii].pos);
-            hi = epi[io + ii].smth;
-            mi = epi[io + ii].mass;
-        }
-        const double H = SUPPORT * hi, invH = 1.0 / H, norm = kernel_norm(H);
-        double d = 0.0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_dens &q = epj[jo + t0 + threadIdx.x];
-                tile[threadIdx.x] = make_double4(q.pos[0], q.pos[1], q.pos[2], q.mass);
-            }
-            __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const double4 q = tile[t];
-                const double dx = q.x - pi.x, dy = q.y - pi.y, dz = q.z - pi.z;
-                double w, g;
-                wendland_poly(sqrt(dx * dx + dy * dy + dz * dz) * invH, w, g);
-                d += q.w * (w * norm);
-            }
-            __syncthreads();
-        }
-        if (act) {
-            d = fmax(DENS_FLOOR, d);
-            res[io + ii].dens = d;
-            res[io + ii].smth = SMTH_COEF * pow(mi / d, 1.0 / 3.0);
-        }
-    }
-}
-
-// CalcDerivative, force.h:89-106
-__global__ void __launch_bounds__(WT) k_walk_drvt(const int64_t *meta, const sph_epi_drvt *epi, JSrc<sph_epj_drvt> epj,
-                                                  sph_result_drvt *res) {
-    __shared__ double4 tp[WT];
-    __shared__ double4 tv[WT];
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        double3 pi = make_double3(0, 0, 0), vi = make_double3(0, 0, 0);
-        double hi = 1.0, rhoi = 1.0;
-        if (act) {
-            pi = ld3(epi[io + ii].pos);
-            vi = ld3(epi[io + ii].vel);
-            hi = epi[io + ii].smth;
-            rhoi = epi[io + ii].dens;
-        }
-        const double H = SUPPORT * hi, invH = 1.0 / H, norm = kernel_norm(H), ceps = 1.0e-6 * hi;
-        double dv = 0, r0 = 0, r1 = 0, r2 = 0, gs = 0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_drvt &q = epj[jo + t0 + threadIdx.x];
-                tp[threadIdx.x] = make_double4(q.pos[0], q.pos[1], q.pos[2], q.mass);
-                tv[threadIdx.x] = make_double4(q.vel[0], q.vel[1], q.vel[2], 0.0);
-            }
-            __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const double4 q = tp[t], u = tv[t];
-                const double dx = pi.x - q.x, dy = pi.y - q.y, dz = pi.z - q.z;
-                const double ax = -q.w * (vi.x - u.x), ay = -q.w * (vi.y - u.y), az = -q.w * (vi.z - u.z);
-                const double rr2 = dx * dx + dy * dy + dz * dz;
-                const double r = sqrt(rr2);
-                double w, g;
-                wendland_poly(r * invH, w, g);
-                const double gf = norm * g / (r * H + ceps);
-                dv += gf * (ax * dx + ay * dy + az * dz);
-                r0 += gf * (ay * dz - az * dy);
-                r1 += gf * (az * dx - ax * dz);
-                r2 += gf * (ax * dy - ay * dx);
-                gs -= q.w / hi * (3.0 * norm * w + gf * rr2);
-            }
-            __syncthreads();
-        }
-        if (act) {
-            sph_result_drvt &o = res[io + ii];
-            o.grad_smth = 1.0 / (1.0 + hi * gs / (3.0 * rhoi));
-            o.div_v = dv / rhoi;
-            o.rot_v[0] = r0 / rhoi;
-            o.rot_v[1] = r1 / rhoi;
-            o.rot_v[2] = r2 / rhoi;
-        }
-    }
-}
-
-// CalcHydroForce, force.h:113-147
-__global__ void __launch_bounds__(WT) k_walk_hydro(const int64_t *meta, const sph_epi_hydro *epi,
-                                                   JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
-    __shared__ double4 tp[WT];   // pos, mass
-    __shared__ double4 tv[WT];   // vel, smth
-    __shared__ double4 tq[WT];   // dens, pres, snds, grad_smth
-    __shared__ double tb[WT];    // Bal
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        sph_epi_hydro I;
-        if (act) I = epi[io + ii];
-        else std::memset(&I, 0, sizeof(I)), I.smth = 1.0, I.dens = 1.0;
-        const double Hi = SUPPORT * I.smth, invHi = 1.0 / Hi, normi = kernel_norm(Hi), cepsi = 1.0e-6 * I.smth;
-        const double Ai = I.grad_smth * I.pres / (I.dens * I.dens);
-        double a0 = 0, a1 = 0, a2 = 0, e = 0, vmax = 0.0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_hydro &q = epj[jo + t0 + threadIdx.x];
-                tp[threadIdx.x] = make_double4(q.pos[0], q.pos[1], q.pos[2], q.mass);
-                tv[threadIdx.x] = make_double4(q.vel[0], q.vel[1], q.vel[2], q.smth);
-                tq[threadIdx.x] = make_double4(q.dens, q.pres, q.snds, q.grad_smth);
-                tb[threadIdx.x] = q.Bal;
-            }
-            __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const double4 p = tp[t], v = tv[t], q = tq[t];
-                const double dx = I.pos[0] - p.x, dy = I.pos[1] - p.y, dz = I.pos[2] - p.z;
-                const double wx = I.vel[0] - v.x, wy = I.vel[1] - v.y, wz = I.vel[2] - v.z;
-                const double rr2 = dx * dx + dy * dy + dz * dz;
-                const double r = sqrt(rr2);
-                const double dvdr = wx * dx + wy * dy + wz * dz;
-                const double w = (dvdr < 0) ? dvdr / r : 0.0;
-                const double vsig = I.snds + q.z - 3.0 * w;
-                vmax = fmax(vmax, vsig);
-                const double AV = -AV_STRENGTH * 0.5 * vsig * w / (0.5 * (I.dens + q.x)) * 0.5 * (I.Bal + tb[t]);
-                const double Hj = SUPPORT * v.w;
-                double wi_, gi_, wj_, gj_;
-                wendland_poly(r * invHi, wi_, gi_);
-                wendland_poly(r / Hj, wj_, gj_);
-                const double gfi = normi * gi_ / (r * Hi + cepsi);
-                const double gfj = kernel_norm(Hj) * gj_ / (r * Hj + 1.0e-6 * v.w);
-                const double gws = 0.5 * (gfi * I.grad_smth + gfj * q.w);
-                const double Aj = q.w * q.y / (q.x * q.x);
-                const double coef = p.w * (Ai * gfi + Aj * gfj + AV * gws);
-                a0 -= coef * dx;
-                a1 -= coef * dy;
-                a2 -= coef * dz;
-                e += p.w * (Ai + 0.5 * AV) * gws * dvdr;
-            }
-            __syncthreads();
-        }
-        if (act) {
-            sph_result_hydro &o = res[io + ii];
-            o.acc[0] = a0;
-            o.acc[1] = a1;
-            o.acc[2] = a2;
-            o.eng_dot = e;
-            o.dt = C_CFL * 2.0 * I.smth / vmax;
-        }
-    }
-}
-
-// CalcGravityForce<EPJ::Grav> then CalcGravityForce<SPJMonopole>, force.h:154-168
-__global__ void __launch_bounds__(WT) k_walk_grav(const int64_t *meta, const sph_epi_grav *epi, JSrc<sph_epj_grav> epj,
-                                                  JSrc<sph_spj_monopole> spj, sph_result_grav *res) {
-    __shared__ double4 tile[WT];
-    const double G = 6.67e-11;   // force.h:171-172
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3], so = M[4], ns = M[5];
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        double3 pi = make_double3(0, 0, 0);
-        double eps2 = 1.0;
-        if (act) {
-            pi = ld3(epi[io + ii].pos);
-            eps2 = epi[io + ii].eps2;
-        }
-        double a0 = 0, a1 = 0, a2 = 0, p = 0;
-        for (int pass = 0; pass < 2; ++pass) {
-            const int64_t nl = pass == 0 ? nj : ns;
-            for (int64_t t0 = 0; t0 < nl; t0 += WT) {
-                if (t0 + threadIdx.x < nl) {
-                    if (pass == 0) {
-                        const sph_epj_grav &q = epj[jo + t0 + threadIdx.x];
-                        tile[threadIdx.x] = make_double4(q.pos[0], q.pos[1], q.pos[2], q.mass);
-                    } else {
-                        const sph_spj_monopole &q = spj[so + t0 + threadIdx.x];
-                        tile[threadIdx.x] = make_double4(q.pos[0], q.pos[1], q.pos[2], q.mass);
-                    }
-                }
-                __syncthreads();
-                const int tn = (int)min((int64_t)WT, nl - t0);
-                for (int t = 0; t < tn; ++t) {
-                    const double4 q = tile[t];
-                    const double dx = pi.x - q.x, dy = pi.y - q.y, dz = pi.z - q.z;
-                    const double dri = 1.0 / sqrt(dx * dx + dy * dy + dz * dz + eps2);
-                    const double mdr3 = q.w * (dri * dri * dri);
-                    a0 -= G * mdr3 * dx;
-                    a1 -= G * mdr3 * dy;
-                    a2 -= G * mdr3 * dz;
-                    p -= G * q.w * dri;
-                }
-                __syncthreads();
-            }
-        }
-        if (act) {
-            sph_result_grav &o = res[io + ii];
-            o.acc[0] = a0;
-            o.acc[1] = a1;
-            o.acc[2] = a2;
-            o.pot = p;
-            o.dt = 1.0e30;   // RESULT::Grav::clear(), dt untouched by the functor
-        }
-    }
-}
-
 // where a dispatch's sections sit in the tag's staging (bytes, 16-byte aligned sections)
 struct Layout {
     int64_t ni = 0, nj = 0, ns = 0;
+    int max_i = 0;   // i-particles of the largest walk
     size_t o_epj = 0, o_spj = 0, end = 0;
 };
 
@@ -457,6 +234,7 @@ int stage(int tag, int kind, int n_walk, const EPI **epi, const int *n_epi, cons
             return batch_fail(SPH_ERR_ARG, "negative walk size");
         if ((n_epi[w] > 0 && !epi[w]) || (n_epj[w] > 0 && !jw[w])) return batch_fail(SPH_ERR_ARG, "null walk");
         L.ni += n_epi[w];
+        L.max_i = std::max(L.max_i, n_epi[w]);
         L.nj += n_epj[w];
         if (sw && n_spj) L.ns += n_spj[w];
     }
@@ -791,7 +569,7 @@ int dispatch_walks(int tag, int kind, int n_walk, const EPI **epi, const int *n_
     if (n_walk > 0) {
         JSrc<EPJ> js{(const EPJ *)(ts->d_in + L.o_epj), nullptr, 0, nullptr};
         if (index) js = JSrc<EPJ>{rj.base, (const int *)(ts->d_in + L.o_epj), rj.n, ts->d_err};
-        launch(ts, (const EPI *)ts->d_in, js, (RES *)ts->d_out, g_batch_prec.load() == SPH_PREC_MIXED);
+        launch(ts, L, (const EPI *)ts->d_in, js, (RES *)ts->d_out, g_batch_prec.load() == SPH_PREC_MIXED);
     }
     return finish_dispatch(ts);
 }
@@ -818,26 +596,26 @@ int dispatch_grav(int tag, int n_walk, const sph_epi_grav **epi, const int *n_ep
         const sph_epi_grav *ei = (const sph_epi_grav *)ts->d_in;
         sph_result_grav *res = (sph_result_grav *)ts->d_out;
         if (g_batch_prec.load() == SPH_PREC_MIXED) batch32_grav(n_walk, ts->stream, ts->d_meta, ei, js, ss, res);
-        else k_walk_grav<<<n_walk, WT, 0, ts->stream>>>(ts->d_meta, ei, js, ss, res);
+        else batch64_grav(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, ss, res);
     }
     return finish_dispatch(ts);
 }
 
-auto launch_dens = [](TagState *ts, const sph_epi_dens *ei, JSrc<sph_epj_dens> js, sph_result_dens *res, bool mixed) {
+auto launch_dens = [](TagState *ts, const Layout &L, const sph_epi_dens *ei, JSrc<sph_epj_dens> js, sph_result_dens *res, bool mixed) {
     const int n_walk = ts->pending_walks;
     if (mixed) batch32_dens(n_walk, ts->stream, ts->d_meta, ei, js, res);
-    else k_walk_dens<<<n_walk, WT, 0, ts->stream>>>(ts->d_meta, ei, js, res);
+    else batch64_dens(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
-auto launch_drvt = [](TagState *ts, const sph_epi_drvt *ei, JSrc<sph_epj_drvt> js, sph_result_drvt *res, bool mixed) {
+auto launch_drvt = [](TagState *ts, const Layout &L, const sph_epi_drvt *ei, JSrc<sph_epj_drvt> js, sph_result_drvt *res, bool mixed) {
     const int n_walk = ts->pending_walks;
     if (mixed) batch32_drvt(n_walk, ts->stream, ts->d_meta, ei, js, res);
-    else k_walk_drvt<<<n_walk, WT, 0, ts->stream>>>(ts->d_meta, ei, js, res);
+    else batch64_drvt(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
-auto launch_hydro = [](TagState *ts, const sph_epi_hydro *ei, JSrc<sph_epj_hydro> js, sph_result_hydro *res,
+auto launch_hydro = [](TagState *ts, const Layout &L, const sph_epi_hydro *ei, JSrc<sph_epj_hydro> js, sph_result_hydro *res,
                        bool mixed) {
     const int n_walk = ts->pending_walks;
     if (mixed) batch32_hydro(n_walk, ts->stream, ts->d_meta, ei, js, res);
-    else k_walk_hydro<<<n_walk, WT, 0, ts->stream>>>(ts->d_meta, ei, js, res);
+    else batch64_hydro(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
 
 }  // namespace

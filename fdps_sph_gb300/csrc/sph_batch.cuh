@@ -1,5 +1,5 @@
-// Shared by the batch entry points (sph_batch.cu) and their mixed-precision kernels
-// (sph_batch32.cu).
+// Shared by the batch entry points (sph_batch.cu) and their FP64 (sph_batch64.cu) and mixed-precision
+// (sph_batch32.cu) kernels.
 #pragma once
 
 #include "sph_physics.cuh"
@@ -38,5 +38,16 @@ void batch32_hydro(int n_walk, cudaStream_t st, const int64_t *meta, const sph_e
                    JSrc<sph_epj_hydro> epj, sph_result_hydro *res);
 void batch32_grav(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi, JSrc<sph_epj_grav> epj,
                   JSrc<sph_spj_monopole> spj, sph_result_grav *res);
+
+// the FP64 functor kernels (sph_batch64.cu): blocks of up to 32 i-particles of a walk; n_i: i-particles of all
+// walks, max_i: of the largest
+void batch64_dens(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi,
+                  JSrc<sph_epj_dens> epj, sph_result_dens *res);
+void batch64_drvt(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi,
+                  JSrc<sph_epj_drvt> epj, sph_result_drvt *res);
+void batch64_hydro(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
+                   JSrc<sph_epj_hydro> epj, sph_result_hydro *res);
+void batch64_grav(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi,
+                  JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj, sph_result_grav *res);
 
 }  // namespace sph
