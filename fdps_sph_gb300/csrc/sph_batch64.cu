@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_dens64(const int64_t *meta, int
                                                         JSrc<sph_epj_dens> epj, sph_result_dens *res) {
     __shared__ float4 s_j[TJ];          // x, y, z relative to the walk's first i-particle, slack
     __shared__ int s_q[W][64];
-    __shared__ double s_i[IC_MAX][4];   // x, y, z, 1 / H
+    __shared__ double s_i[IC_MAX][5];   // x, y, z, 1 / H (hi, lo)
     __shared__ float4 s_f[IC_MAX];      // the same in FP32: x, y, z, reach + slack
     __shared__ double s_sum[IC_MAX];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -104,7 +104,9 @@ __global__ void __launch_bounds__(W * 32) k_walk_dens64(const int64_t *meta, int
             s_i[t][0] = p.pos[0];
             s_i[t][1] = p.pos[1];
             s_i[t][2] = p.pos[2];
-            s_i[t][3] = 1.0 / (SUPPORT * p.smth);
+            const Inv64 iH = inv64(SUPPORT * p.smth);
+            s_i[t][3] = iH.hi;
+            s_i[t][4] = iH.lo;
             const float x = (float)(p.pos[0] - cx), y = (float)(p.pos[1] - cy), z = (float)(p.pos[2] - cz);
             s_f[t] = make_float4(x, y, z, reach(p.smth) + slack1(x, y, z));
             s_sum[t] = 0.0;
@@ -120,7 +122,8 @@ __global__ void __launch_bounds__(W * 32) k_walk_dens64(const int64_t *meta, int
             __syncthreads();
             for (int i = warp; i < S.ni; i += W) {
                 const float4 f = s_f[i];
-                const double xi = s_i[i][0], yi = s_i[i][1], zi = s_i[i][2], invH = s_i[i][3];
+                const double xi = s_i[i][0], yi = s_i[i][1], zi = s_i[i][2];
+                const Inv64 invH{s_i[i][3], s_i[i][4]};
                 Queue Q{s_q[warp], 0};
                 double sum = 0.0;
                 auto eval = [&]() {
@@ -163,7 +166,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_drvt64(const int64_t *meta, int
                                                         JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
     __shared__ float4 s_j[TJ];
     __shared__ int s_q[W][64];
-    __shared__ double s_i[IC_MAX][9];   // x, v, 1 / H, H, 1e-6 h
+    __shared__ double s_i[IC_MAX][10];   // x, v, 1 / H (hi, lo), H, 1e-6 h
     __shared__ float4 s_f[IC_MAX];
     __shared__ double s_sum[IC_MAX][6];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -177,9 +180,11 @@ __global__ void __launch_bounds__(W * 32) k_walk_drvt64(const int64_t *meta, int
                 s_i[t][d] = p.pos[d];
                 s_i[t][3 + d] = p.vel[d];
             }
-            s_i[t][6] = 1.0 / (SUPPORT * p.smth);
-            s_i[t][7] = SUPPORT * p.smth;
-            s_i[t][8] = 1.0e-6 * p.smth;
+            const Inv64 iH = inv64(SUPPORT * p.smth);
+            s_i[t][6] = iH.hi;
+            s_i[t][7] = iH.lo;
+            s_i[t][8] = SUPPORT * p.smth;
+            s_i[t][9] = 1.0e-6 * p.smth;
             const float x = (float)(p.pos[0] - cx), y = (float)(p.pos[1] - cy), z = (float)(p.pos[2] - cz);
             const bool ok = fin(p.vel[0]) && fin(p.vel[1]) && fin(p.vel[2]);
             s_f[t] = make_float4(x, y, z, ok ? reach(p.smth) + slack1(x, y, z) : __int_as_float(0x7fffffff));
@@ -205,7 +210,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_drvt64(const int64_t *meta, int
                     if (j >= 0) {
                         const sph_epj_drvt &q = epj[S.jo + t0 + j];
                         drvt_pair64(I[0] - q.pos[0], I[1] - q.pos[1], I[2] - q.pos[2], I[3] - q.vel[0], I[4] - q.vel[1],
-                                    I[5] - q.vel[2], q.mass, I[6], I[7], I[8], D);
+                                    I[5] - q.vel[2], q.mass, Inv64{I[6], I[7]}, I[8], I[9], D);
                     }
                 };
                 for (int k = lane; k < TJ && k - lane < tn; k += 32) {

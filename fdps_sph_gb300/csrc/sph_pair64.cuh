@@ -5,7 +5,7 @@
 // cycles, about 1/40 of the FP32 rate, and an FP64 divide or square root costs 7.5 of them (measured with an
 // operation loop: sqrt 150, divide 148, rsqrt 97 against 20 for a fused multiply-add).  So the pair terms are
 // written for few FP64 instructions: square roots and reciprocals start from the hardware's approximate
-// seeds (an MUFU instruction, off the FP64 pipe) and take one third-order Newton / Householder step
+// seeds (an MUFU instruction, off the FP64 pipe) and take one or two Newton / Householder steps
 // (error below 2^-53 before the last rounding), constants are folded out of the sums, tests and clamps run on
 // the integer pipe.
 #pragma once
@@ -29,8 +29,9 @@ __device__ __forceinline__ double rcp64(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
-// r = sqrt(x) and y = 1 / sqrt(x) (y = 0 at x = 0): seed y0, e = 1 - x y0^2, both times (1 + e / 2 + 3 e^2 / 8)
-__device__ __forceinline__ void sqrt64(double x, double &r, double &y) {
+// r = sqrt(x) and y = 1 / sqrt(x) (y = 0 at x = 0), within 2 units of 2^-53 each: seed y0, e = 1 - x y0^2,
+// both times (1 + e / 2 + 3 e^2 / 8)
+__device__ __forceinline__ void sqrt_rsqrt64(double x, double &r, double &y) {
     const bool zero = (__double2hiint(x) | __double2loint(x)) == 0;
     if (!zero && !mid_range(x)) {
         r = sqrt(x);
@@ -47,6 +48,33 @@ __device__ __forceinline__ void sqrt64(double x, double &r, double &y) {
     y = fma(y0, ec, y0);
 }
 
+// sqrt(x) with the last step on the exact residual x - r^2, so the result is the rounded root but for rare
+// ties: the density's and the derivative's weights amplify its error
+__device__ __forceinline__ double sqrt64(double x) {
+    const bool zero = (__double2hiint(x) | __double2loint(x)) == 0;
+    if (!zero && !mid_range(x)) return sqrt(x);
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(x));
+    double h0 = __hiloint2double(__double2hiint(y0) - 0x00100000, __double2loint(y0));   // y0 / 2
+    if (zero) y0 = h0 = 0.0;
+    const double t = x * y0;
+    const double e = fma(-t, h0, 0.5);
+    const double r = fma(t, e, t), h = fma(h0, e, h0);
+    return fma(fma(-r, r, x), h, r);
+}
+
+// 1 / H as hi + lo (lo: the remainder of hi): r hi alone would carry hi's rounding into every weight of the
+// particle with the same sign
+struct Inv64 {
+    double hi, lo;
+};
+__device__ __forceinline__ Inv64 inv64(double H) {
+    Inv64 v;
+    v.hi = 1.0 / H;
+    v.lo = fma(-H, v.hi, 1.0) * v.hi;
+    return v;
+}
+
 // max(1 - s, 0) without an FP64 compare (a NaN stays a NaN or becomes 0; its product with the polynomial is a
 // NaN either way, as with fmax)
 __device__ __forceinline__ double kernel_q(double s) {
@@ -55,10 +83,9 @@ __device__ __forceinline__ double kernel_q(double s) {
 }
 
 // CalcDensity's pair (force.h:9-23): m_j W / norm added to sum
-__device__ __forceinline__ void dens_pair64(double dx, double dy, double dz, double mj, double invH, double &sum) {
-    double r, y;
-    sqrt64(fma(dx, dx, fma(dy, dy, dz * dz)), r, y);
-    const double s = r * invH, q = kernel_q(s);
+__device__ __forceinline__ void dens_pair64(double dx, double dy, double dz, double mj, Inv64 invH, double &sum) {
+    const double r = sqrt64(fma(dx, dx, fma(dy, dy, dz * dz)));
+    const double s = fma(r, invH.hi, r * invH.lo), q = kernel_q(s);
     const double q2 = q * q, q4 = q2 * q2;
     sum = fma(mj, fma(s, fma(s, fma(s, 32.0, 25.0), 8.0), 1.0) * (q4 * q4), sum);
 }
@@ -67,11 +94,10 @@ __device__ __forceinline__ void dens_pair64(double dx, double dy, double dz, dou
 // (r H + 1e-6 h) (gradW = -22 norm / H g dr, kernel.h:22-34), D[0] += m g v.dr, D[1..3] += m g (v x dr),
 // D[4] += m w, D[5] += m g r^2 with v = v_i - v_j
 __device__ __forceinline__ void drvt_pair64(double dx, double dy, double dz, double vx, double vy, double vz, double mj,
-                                            double invH, double H, double ceps, double D[6]) {
+                                            Inv64 invH, double H, double ceps, double D[6]) {
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    double r, y;
-    sqrt64(r2, r, y);
-    const double s = r * invH, q = kernel_q(s);
+    const double r = sqrt64(r2);
+    const double s = fma(r, invH.hi, r * invH.lo), q = kernel_q(s);
     const double q2 = q * q, q4 = q2 * q2, q7 = q4 * (q2 * q);
     const double w = fma(s, fma(s, fma(s, 32.0, 25.0), 8.0), 1.0) * (q7 * q);
     const double mg = mj * ((r * fma(s, fma(s, 16.0, 7.0), 1.0)) * (q7 * rcp64(fma(r, H, ceps))));
@@ -116,7 +142,7 @@ __device__ __forceinline__ double hydro_gf64(double r, double qn, double H, doub
 __device__ __forceinline__ void hydro_pair64(double dx, double dy, double dz, double vx, double vy, double vz, double mj,
                                              const Hydro64 &I, const Hydro64 &J, double D[4], double &vmax) {
     double r, y;
-    sqrt64(fma(dx, dx, fma(dy, dy, dz * dz)), r, y);
+    sqrt_rsqrt64(fma(dx, dx, fma(dy, dy, dz * dz)), r, y);
     const double dvdr = fma(vx, dx, fma(vy, dy, vz * dz));
     const double w = dvdr < 0 ? dvdr * y : 0.0;
     const double vsig = fma(-3.0, w, I.c + J.c);
