@@ -261,15 +261,17 @@ int sph_runs_layout(sph_ctx *ctx) {
     std::vector<int4> info(R.R), tiles;
     int64_t o = 0;
     int T = 0;
+    R.max_tiles = 0;
     for (int r = 0; r < R.R; ++r) {
         R.off[r] = o;
         const int nt = (int)((R.n[r] + RUN_TILE - 1) / RUN_TILE);
         info[r] = make_int4((int)o, (int)R.n[r], T, nt);
         for (int k = 0; k < nt; ++k)
             tiles.push_back(make_int4((int)(o + (int64_t)k * RUN_TILE), (int)std::min<int64_t>(RUN_TILE, R.n[r] - (int64_t)k * RUN_TILE),
-                                      256 * T + k, nt));
+                                      T, nt));
         o += R.n[r];
         T += nt;
+        R.max_tiles = std::max(R.max_tiles, nt);
     }
     R.T = T;
     if (R.R > R.cap_R) {

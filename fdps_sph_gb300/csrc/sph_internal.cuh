@@ -198,8 +198,8 @@ struct Sort {
     int64_t cap = 0;
     uint64_t *k0 = nullptr, *k1 = nullptr;
     uint32_t *v0 = nullptr, *v1 = nullptr;
-    uint32_t *hist = nullptr;   // [256 * nblocks]
-    uint32_t *hoff = nullptr;
+    uint32_t *hist = nullptr;   // digit counts [RS_HISTS][tile][256]
+    uint32_t *hoff = nullptr;   // offsets [tile][256], totals [first tile of a run][256]
     int nblocks_cap = 0;
 };
 
@@ -288,8 +288,9 @@ struct Runs {
     std::vector<double> mmax;               // the run's largest particle mass
     bool fix_split = true;                  // every run's largest mass x its own scale <= 15
     int T = 0;                              // tiles over all runs
+    int max_tiles = 0;                      // of the largest run
     int cap_R = 0, cap_T = 0;
-    int4 *tiles = nullptr;                  // device [T]: start, length, histogram base, tiles of its run
+    int4 *tiles = nullptr;                  // device [T]: start, length, first tile of its run, tiles of its run
     int4 *info = nullptr;                   // device [R]: first particle, particles, first tile, tiles
     double *dt_dev = nullptr;               // device [R]: dt of the coming step
     double *part = nullptr;                 // device [T * 8]: per-tile partials
@@ -303,7 +304,7 @@ struct Runs {
 }  // namespace sph
 
 namespace sph {
-constexpr int GRAPH_KEY_N = 21;
+constexpr int GRAPH_KEY_N = 22;
 // a captured sort + octree build and what it was captured for
 struct TreeGraph {
     cudaGraphExec_t exec = nullptr;
@@ -473,20 +474,22 @@ struct LenArg {
 };
 
 // Key-and-sort kernels of sph_tree.cu that sph_noalloc.cu also launches.
-constexpr int RS_THREADS = 256;          // threads of k_rs_hist / k_rs_scatter (one per digit)
-constexpr int RS_ITEMS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;   // keys per radix-sort tile
-__global__ void k_scan_reduce(const int *in, LenArg len, int *part);
-__global__ void k_scan_part(int *part, int nb, int *total);
-__global__ void k_scan_down(const int *in, int *out, LenArg len, const int *part);
-__global__ void k_bbox_partial(const double *x, const double *y, const double *z, int n, double *part);
-__global__ void k_bbox_final(const double *part, int nb, double theta, double *rb);
-__global__ void k_keys(const double *x, const double *y, const double *z, int n, const double *rb, uint64_t *keys,
-                       uint32_t *vals, int *err);
-__global__ void k_rs_hist(const uint64_t *keys, int n, int shift, uint32_t *hist, int nb, const int4 *tiles);
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
-                                                           uint32_t *vout, int n, int shift, const uint32_t *off,
-                                                           int nb, const int4 *tiles);
+constexpr int RS_THREADS = 512;
+constexpr int RS_TILE = 2048;            // keys per radix-sort tile
+constexpr int RS_SUB = RS_TILE / RS_THREADS;   // blocks of the key kernel per tile
+constexpr int RS_PASSES = 8;             // of 8 bits
+constexpr int RS_HISTS = 3;              // digit-count arrays: this pass's, the next one's, the one being cleared
+constexpr int RS_DIRECT = 64;            // most tiles of a run whose counts every block adds up itself
+__global__ void k_bbox_partial(const double *x, const double *y, const double *z, int n, long long *part,
+                               uint32_t *clear, int n_clear);
+__global__ void k_bbox_final(const long long *part, int nb, double theta, double *rb);
+__global__ void __launch_bounds__(RS_THREADS) k_keys_hist(const double *x, const double *y, const double *z, int n,
+                                                          const double *rb, const int *prun, const int4 *tiles, int nb,
+                                                          uint64_t *keys, uint32_t *hist, int *err);
+__global__ void __launch_bounds__(RS_THREADS, 4) k_rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
+                                                           uint32_t *vout, int n, int shift, const uint32_t *hist,
+                                                           uint32_t *next, uint32_t *clear, const uint32_t *off,
+                                                           const uint32_t *tot, int nb, const int4 *tiles);
 
 }  // namespace sph
 

@@ -21,6 +21,7 @@
 // `stream` is being captured into a CUDA graph, it only records its work (the
 // memset, the launches and the device-to-device copies are all capturable)
 // and returns at once: a replay reports no status.
+#include <algorithm>
 #include <mutex>
 
 #include "sph_internal.cuh"
@@ -35,20 +36,17 @@ constexpr int NA_MAX = SPH_NOALLOC_MAX_N;
 constexpr int NA_TILE = RS_TILE;                  // radix-sort tile (k_rs_scatter)
 constexpr int NA_NB = (NA_MAX + NA_TILE - 1) / NA_TILE;
 constexpr int NA_BOX = 304;                       // blocks of k_bbox_partial
-constexpr int NA_SCAN = 256;                      // blocks of the scan kernels
 
 // byte offsets inside the scratch array (each 256-byte aligned)
 constexpr size_t al(size_t b) { return (b + 255) & ~size_t(255); }
-constexpr size_t OFF_BOX = 0;                                           // double [NA_BOX * 6]
+constexpr size_t OFF_BOX = 0;                                           // int64 [NA_BOX * 6]
 constexpr size_t OFF_RB = OFF_BOX + al(sizeof(double) * NA_BOX * 6);    // double [8 + 22]
 constexpr size_t OFF_K0 = OFF_RB + al(sizeof(double) * 32);             // uint64 [NA_MAX]
 constexpr size_t OFF_K1 = OFF_K0 + al(sizeof(uint64_t) * NA_MAX);
 constexpr size_t OFF_V0 = OFF_K1 + al(sizeof(uint64_t) * NA_MAX);       // uint32 [NA_MAX]
 constexpr size_t OFF_V1 = OFF_V0 + al(sizeof(uint32_t) * NA_MAX);
-constexpr size_t OFF_HIST = OFF_V1 + al(sizeof(uint32_t) * NA_MAX);     // uint32 [256 * NA_NB]
-constexpr size_t OFF_HOFF = OFF_HIST + al(sizeof(uint32_t) * 256 * NA_NB);
-constexpr size_t OFF_PART = OFF_HOFF + al(sizeof(uint32_t) * 256 * NA_NB);   // int [NA_SCAN + 1]
-constexpr size_t OFF_ERR = OFF_PART + al(sizeof(int) * (NA_SCAN + 1));       // int
+constexpr size_t OFF_HIST = OFF_V1 + al(sizeof(uint32_t) * NA_MAX);     // uint32 [RS_HISTS][NA_NB][256]
+constexpr size_t OFF_ERR = OFF_HIST + al(sizeof(uint32_t) * 256 * RS_HISTS * NA_NB);   // int
 constexpr size_t NA_BYTES = OFF_ERR + 256;
 
 }  // namespace
@@ -112,47 +110,36 @@ extern "C" int sph_morton_order_noalloc(const double *x, const double *y, const 
     unsigned char *base = nullptr;
     const int rc = noalloc_setup(dev, &base);
     if (rc != SPH_OK) return rc;
-    double *box = reinterpret_cast<double *>(base + OFF_BOX);
+    long long *box = reinterpret_cast<long long *>(base + OFF_BOX);
     double *rb = reinterpret_cast<double *>(base + OFF_RB);
     uint64_t *ka = reinterpret_cast<uint64_t *>(base + OFF_K0), *kb = reinterpret_cast<uint64_t *>(base + OFF_K1);
     uint32_t *va = reinterpret_cast<uint32_t *>(base + OFF_V0), *vb = reinterpret_cast<uint32_t *>(base + OFF_V1);
-    uint32_t *hist = reinterpret_cast<uint32_t *>(base + OFF_HIST), *hoff = reinterpret_cast<uint32_t *>(base + OFF_HOFF);
-    int *part = reinterpret_cast<int *>(base + OFF_PART);
+    uint32_t *hist = reinterpret_cast<uint32_t *>(base + OFF_HIST);
     int *err = reinterpret_cast<int *>(base + OFF_ERR);
     const int nn = (int)n;
+    const int nb = (nn + NA_TILE - 1) / NA_TILE;
+    static_assert(NA_NB <= RS_DIRECT, "every block adds up the tiles' counts itself");
     // the error word is the one part of the array that must start at zero
     if (cudaMemsetAsync(err, 0, sizeof(int), st) != cudaSuccess) {
         cudaGetLastError();
         return SPH_ERR_CUDA;
     }
     // root cube and keys exactly as the octree build does (theta does not enter the keys)
-    k_bbox_partial<<<NA_BOX, 256, 0, st>>>(x, y, z, nn, box);
-    k_bbox_final<<<1, 256, 0, st>>>(box, NA_BOX, 0.5, rb);
-    k_keys<<<(nn + 255) / 256, 256, 0, st>>>(x, y, z, nn, rb, ka, va, err);
-    // stable LSD radix sort, 8 passes of 8 bits
-    const int nb = (nn + NA_TILE - 1) / NA_TILE;
-    const LenArg L{nullptr, 256 * nb, 0};
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = pass * 8;
-        k_rs_hist<<<nb, 256, 0, st>>>(ka, nn, shift, hist, nb, nullptr);
-        k_scan_reduce<<<NA_SCAN, 256, 0, st>>>(reinterpret_cast<const int *>(hist), L, part);
-        k_scan_part<<<1, NA_SCAN, 0, st>>>(part, NA_SCAN, nullptr);
-        k_scan_down<<<NA_SCAN, 256, 0, st>>>(reinterpret_cast<const int *>(hist), reinterpret_cast<int *>(hoff), L,
-                                             part);
-        k_rs_scatter<<<nb, 256, 0, st>>>(ka, va, kb, vb, nn, shift, hoff, nb, nullptr);
-        uint64_t *tk = ka;
-        ka = kb;
-        kb = tk;
-        uint32_t *tv = va;
-        va = vb;
-        vb = tv;
+    const int box_blocks = std::min(NA_BOX, (nn + 255) / 256);
+    const int64_t row = 256 * (int64_t)nb;   // digit counts of one pass
+    k_bbox_partial<<<box_blocks, 256, 0, st>>>(x, y, z, nn, box, hist, (int)(2 * row));
+    k_bbox_final<<<1, 256, 0, st>>>(box, box_blocks, 0.5, rb);
+    k_keys_hist<<<nb * RS_SUB, RS_THREADS, 0, st>>>(x, y, z, nn, rb, nullptr, nullptr, nb, ka, hist, err);
+    // stable LSD radix sort, 8 passes of 8 bits, the last one into the caller's buffers
+    for (int pass = 0; pass < RS_PASSES; ++pass) {
+        const bool odd = pass & 1, last = pass == RS_PASSES - 1;
+        k_rs_scatter<<<nb, RS_THREADS, 0, st>>>(
+            odd ? kb : ka, pass == 0 ? nullptr : (odd ? vb : va), last ? keys_out : (odd ? ka : kb),
+            last ? reinterpret_cast<uint32_t *>(order_out) : (odd ? va : vb), nn, 8 * pass,
+            hist + pass % RS_HISTS * row, last ? nullptr : hist + (pass + 1) % RS_HISTS * row,
+            last ? nullptr : hist + (pass + 2) % RS_HISTS * row, nullptr, nullptr, nb, nullptr);
     }
     if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
-    if (cudaMemcpyAsync(keys_out, ka, sizeof(uint64_t) * nn, cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(order_out, va, sizeof(uint32_t) * nn, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
-        cudaGetLastError();
-        return SPH_ERR_CUDA;
-    }
     if (capturing) return SPH_OK;   // recorded; a replay's status is not read back
     int herr = 0;
     if (cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -51,6 +51,11 @@ __device__ __forceinline__ long long dorder_key(double d) {
     return b >= 0 ? b : -(b & 0x7fffffffffffffffLL);
 }
 
+// the double of a key (a NaN's key gives a NaN)
+__device__ __forceinline__ double dorder_value(long long k) {
+    return __longlong_as_double(k >= 0 ? k : (-k | (long long)0x8000000000000000ull));
+}
+
 // std::lower_bound over an ascending axis (no NaN in it).  The comparisons run on the integer
 // pipe through dorder_key, with the same outcome as the FP64 comparisons (a NaN v compares false
 // with everything: index 0); on this GPU the FP64 pipe is the bound of the EoS kernel.

@@ -16,8 +16,9 @@
 //     (no fused multiply-add), so that centres of mass and hence the gravity
 //     opening decisions are bit-identical to the oracle's.
 #include <algorithm>
+#include <climits>
 
-#include "sph_internal.cuh"
+#include "sph_physics.cuh"
 
 namespace sph {
 
@@ -109,42 +110,68 @@ namespace sph {
 // ---------------------------------------------------------------------------
 // root box and keys
 
-constexpr int BOX_BLOCKS = 304;
-
-__global__ void k_bbox_partial(const double *x, const double *y, const double *z, int n, double *part) {
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double p[3] = {x[i], y[i], z[i]};
-#pragma unroll
+// The boxes are reduced on order-preserving integer images of the doubles (dorder_key), so the minima and maxima
+// run on the integer pipe: the FP64 pipe takes 16 cycles a warp instruction.  (-0 counts as +0; a NaN is left out, as by
+// fmin and fmax.)
+struct Box {
+    long long lo[3], hi[3];
+    __device__ __forceinline__ void empty() {
         for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], p[d]);
-            hi[d] = fmax(hi[d], p[d]);
+            lo[d] = LLONG_MAX;
+            hi[d] = LLONG_MIN;
         }
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-        }
+    __device__ __forceinline__ void add(int d, long long a, long long b) {
+        lo[d] = min(lo[d], a);
+        hi[d] = max(hi[d], b);
     }
-    __shared__ double s[32][6];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int d = 0; d < 3; ++d) { s[wid][d] = lo[d]; s[wid][3 + d] = hi[d]; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
+    __device__ __forceinline__ void add(double px, double py, double pz) {
+        const long long k[3] = {dorder_key(px), dorder_key(py), dorder_key(pz)};
+        for (int d = 0; d < 3; ++d)
+            if (llabs(k[d]) <= 0x7ff0000000000000LL) add(d, k[d], k[d]);
+    }
+    // of the whole block, valid in thread 0
+    __device__ void reduce() {
+        __shared__ long long s[6][32];
+        for (int d = 0; d < 3; ++d)
+            for (int o = 16; o > 0; o >>= 1)
+                add(d, __shfl_xor_sync(0xffffffffu, lo[d], o), __shfl_xor_sync(0xffffffffu, hi[d], o));
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        if (lane == 0)
             for (int d = 0; d < 3; ++d) {
-                lo[d] = fmin(lo[d], s[w][d]);
-                hi[d] = fmax(hi[d], s[w][3 + d]);
+                s[d][wid] = lo[d];
+                s[3 + d][wid] = hi[d];
             }
-        for (int d = 0; d < 3; ++d) { part[blockIdx.x * 6 + d] = lo[d]; part[blockIdx.x * 6 + 3 + d] = hi[d]; }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
+                for (int d = 0; d < 3; ++d) add(d, s[d][w], s[3 + d][w]);
     }
+};
+
+// block b: the box of every gridDim.x-th 256 positions; also clears the counts the key kernel and the sort's first
+// pass add to (n_clear words)
+__global__ void k_bbox_partial(const double *x, const double *y, const double *z, int n, long long *part,
+                               uint32_t *clear, int n_clear) {
+    Box b;
+    b.empty();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b.add(x[i], y[i], z[i]);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_clear; i += gridDim.x * blockDim.x) clear[i] = 0;
+    b.reduce();
+    if (threadIdx.x == 0)
+        for (int d = 0; d < 3; ++d) {
+            part[blockIdx.x * 6 + d] = b.lo[d];
+            part[blockIdx.x * 6 + 3 + d] = b.hi[d];
+        }
 }
 
 // the root cube from the particle box exactly as or_root_box, and the opening-radius table
-__device__ void root_cube(const double lo[3], const double hi[3], double theta, double *rb) {
+__device__ void root_cube(const Box &x, double theta, double *rb) {
+    double lo[3], hi[3];
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = dorder_value(x.lo[d]);
+        hi[d] = dorder_value(x.hi[d]);
+    }
     double L = 0.0;
     for (int d = 0; d < 3; ++d) {
         const double e = __dsub_rn(hi[d], lo[d]);
@@ -164,88 +191,56 @@ __device__ void root_cube(const double lo[3], const double hi[3], double theta, 
     }
 }
 
-// one block reduces the partial boxes (min / max are exact in any order), then
-// one thread forms the root cube
-__global__ void k_bbox_final(const double *part, int nb, double theta, double *rb) {
-    __shared__ double s[6][32];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+// one block reduces the partial boxes (min / max are exact in any order), then one thread forms the root cube
+__global__ void k_bbox_final(const long long *part, int nb, double theta, double *rb) {
+    Box x;
+    x.empty();
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], part[b * 6 + d]);
-            hi[d] = fmax(hi[d], part[b * 6 + 3 + d]);
-        }
-    for (int d = 0; d < 3; ++d)
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-        }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int d = 0; d < 3; ++d) {
-            s[d][wid] = lo[d];
-            s[3 + d][wid] = hi[d];
-        }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], s[d][w]);
-            hi[d] = fmax(hi[d], s[3 + d][w]);
-        }
-    root_cube(lo, hi, theta, rb);
+        for (int d = 0; d < 3; ++d) x.add(d, part[b * 6 + d], part[b * 6 + 3 + d]);
+    x.reduce();
+    if (threadIdx.x == 0) root_cube(x, theta, rb);
 }
 
-// per run: one block per tile reduces its particles' box, one block per run the tiles of the run
-__device__ void block_box(double lo[3], double hi[3]) {
-    __shared__ double s[6][32];
-    for (int d = 0; d < 3; ++d)
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-        }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-        for (int d = 0; d < 3; ++d) {
-            s[d][wid] = lo[d];
-            s[3 + d][wid] = hi[d];
-        }
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            for (int d = 0; d < 3; ++d) {
-                lo[d] = fmin(lo[d], s[d][w]);
-                hi[d] = fmax(hi[d], s[3 + d][w]);
-            }
-}
-
-__global__ void k_bbox_tiles(const double *x, const double *y, const double *z, const int4 *tiles, double *part) {
+// per run: one block per tile reduces its particles' box and clears its digit counts (the key kernel's and the
+// first pass's), one block per run the tiles of the run
+__global__ void k_bbox_tiles(const double *x, const double *y, const double *z, const int4 *tiles, long long *part,
+                             uint32_t *hist, uint32_t *next) {
     const int4 t = tiles[blockIdx.x];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = t.x + threadIdx.x; i < t.x + t.y; i += blockDim.x) {
-        const double p[3] = {x[i], y[i], z[i]};
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], p[d]);
-            hi[d] = fmax(hi[d], p[d]);
-        }
+    Box b;
+    b.empty();
+    for (int i = t.x + threadIdx.x; i < t.x + t.y; i += blockDim.x) b.add(x[i], y[i], z[i]);
+    if (threadIdx.x < 256) {
+        hist[(int64_t)blockIdx.x * 256 + threadIdx.x] = 0;
+        next[(int64_t)blockIdx.x * 256 + threadIdx.x] = 0;
     }
-    block_box(lo, hi);
+    b.reduce();
     if (threadIdx.x == 0)
         for (int d = 0; d < 3; ++d) {
-            part[blockIdx.x * 8 + d] = lo[d];
-            part[blockIdx.x * 8 + 3 + d] = hi[d];
+            part[blockIdx.x * 8 + d] = b.lo[d];
+            part[blockIdx.x * 8 + 3 + d] = b.hi[d];
         }
 }
 
-__global__ void k_bbox_runs(const double *part, const int4 *info, double theta, double *rb) {
+// also the run's octree root (level 0: cell r = run r) and, from block 0, an empty meta block
+__global__ void k_bbox_runs(const long long *part, const int4 *info, double theta, double *rb, int *meta, int *start,
+                            int *count, int *level, int *parent, int *first_child, int *n_child) {
     const int4 r = info[blockIdx.x];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    Box x;
+    x.empty();
     for (int b = r.z + threadIdx.x; b < r.z + r.w; b += blockDim.x)
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = fmin(lo[d], part[b * 8 + d]);
-            hi[d] = fmax(hi[d], part[b * 8 + 3 + d]);
-        }
-    block_box(lo, hi);
-    if (threadIdx.x == 0) root_cube(lo, hi, theta, rb + (int64_t)blockIdx.x * RB_STRIDE);
+        for (int d = 0; d < 3; ++d) x.add(d, part[b * 8 + d], part[b * 8 + 3 + d]);
+    if (blockIdx.x == 0 && threadIdx.x < META_N) meta[threadIdx.x] = threadIdx.x == 1 ? (int)gridDim.x : 0;
+    x.reduce();
+    if (threadIdx.x == 0) {
+        const int c = blockIdx.x;
+        root_cube(x, theta, rb + (int64_t)c * RB_STRIDE);
+        start[c] = r.x;
+        count[c] = r.y;
+        level[c] = 0;
+        parent[c] = -1;
+        first_child[c] = -1;
+        n_child[c] = 0;
+    }
 }
 
 __device__ __forceinline__ uint64_t spread3(uint64_t v) {
@@ -265,145 +260,216 @@ __device__ __forceinline__ uint64_t cell_coord(double v, double lo, double scale
     return (uint64_t)t;
 }
 
-__global__ void k_keys(const double *x, const double *y, const double *z, int n, const double *rb, uint64_t *keys,
-                       uint32_t *vals, int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double px = x[i], py = y[i], pz = z[i];
-    if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) atomicOr(err, ERR_NONFINITE);
-    const uint64_t qx = cell_coord(px, rb[0], rb[4]);
-    const uint64_t qy = cell_coord(py, rb[1], rb[4]);
-    const uint64_t qz = cell_coord(pz, rb[2], rb[4]);
-    keys[i] = (spread3(qx) << 2) | (spread3(qy) << 1) | spread3(qz);
-    vals[i] = (uint32_t)i;
-}
-
-// keys against the particle's own run's root cube
-__global__ void k_keys_runs(const double *x, const double *y, const double *z, int n, const double *rb,
-                            const int *prun, uint64_t *keys, uint32_t *vals, int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double *q = rb + (int64_t)prun[i] * RB_STRIDE;
-    const double px = x[i], py = y[i], pz = z[i];
-    if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) atomicOr(err, ERR_NONFINITE);
-    const uint64_t qx = cell_coord(px, q[0], q[4]);
-    const uint64_t qy = cell_coord(py, q[1], q[4]);
-    const uint64_t qz = cell_coord(pz, q[2], q[4]);
-    keys[i] = (spread3(qx) << 2) | (spread3(qy) << 1) | spread3(qz);
-    vals[i] = (uint32_t)i;
-}
-
 // ---------------------------------------------------------------------------
-// LSD radix sort of (key, value), 8 passes of 8 bits.  Each pass: per-tile
-// digit histogram, one exclusive scan over (digit, tile), then a stable
-// in-tile ranking and a scatter.  With a tile table (tiles aligned to run
-// starts; each entry: start, length, histogram base, tiles of its run) the
-// histogram is laid out run by run, digit-major within a run, so the one scan
-// yields offsets that keep every run in its own range: a segmented sort.
-// Without one, tile b covers [b * RS_TILE, ...) and the layout is digit-major.
+// LSD radix sort of (key, value), 8 passes of 8 bits over tiles of RS_TILE keys, stable.  With a tile table (tiles
+// aligned to run starts; each entry: start, length, first tile of its run, tiles of its run) every run is sorted
+// inside its own range; without one the tiles cover [0, n).
+//
+// What bounds it is latency: a pass moves 24 bytes per key, but it is a chain of dependent launches, and a
+// small run's tiles do not fill the chip.  So a pass is one launch where a run has at most RS_DIRECT tiles: the
+// digit counts of every tile are in place when the pass starts (the key kernel counts the first digit, each
+// pass counts the next digit of its outputs with one atomic per key into the counts of the tile they land
+// in; three count arrays rotate, each cleared a pass before it is added to), and every block adds up the counts of
+// its run's tiles itself.  Above RS_DIRECT tiles one more launch
+// per pass (k_rs_scan) prepares the offsets, since the blocks' own sums grow with the square of the tiles.  Before: a
+// histogram, three scan launches and a scatter of 256 threads per pass; keys, sort and permutation of 1M particles
+// 0.52 -> 0.38 ms, of 5,003 particles 0.27 -> 0.10 ms.
 
-// RS_THREADS, RS_ITEMS, RS_TILE: sph_internal.cuh
+constexpr int RS_WARPS = RS_THREADS / 32;
+constexpr int RS_WKEYS = RS_TILE / RS_WARPS;
+constexpr int RS_ROUNDS = RS_WKEYS / 32;
+
+// the lanes with this lane's digit (0..255; 256: none): nine votes (about 100 cycles a warp; __match_any_sync took
+// 1,000 with 16 warps on the SM)
+__device__ __forceinline__ unsigned same_digit(int d) {
+    unsigned m = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 9; ++b) {
+        const unsigned v = __ballot_sync(0xffffffffu, (d >> b) & 1);
+        m &= (d >> b) & 1 ? v : ~v;
+    }
+    return m;
+}
 
 __device__ __forceinline__ int4 rs_tile(const int4 *tiles, int n, int nb) {
     if (tiles) return tiles[blockIdx.x];
     const int s = blockIdx.x * RS_TILE;
-    return make_int4(s, min(RS_TILE, n - s), blockIdx.x, nb);
+    return make_int4(s, min(RS_TILE, n - s), 0, nb);
 }
 
-__global__ void k_rs_hist(const uint64_t *keys, int n, int shift, uint32_t *hist, int nb, const int4 *tiles) {
+// keys against the particle's run's root cube, and the counts of their lowest digit added to the tile's (zero on
+// entry).  Four blocks per tile, one key per thread: bound by the FP64 pipe (about 21 instructions a key), so a
+// small run's keys should spread over the SMs; 100,000 keys with one block per tile 16 us.
+__global__ void __launch_bounds__(RS_THREADS) k_keys_hist(const double *x, const double *y, const double *z, int n,
+                                                          const double *rb, const int *prun, const int4 *tiles, int nb,
+                                                          uint64_t *keys, uint32_t *hist, int *err) {
     __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
+    const int t = threadIdx.x, tile = blockIdx.x / RS_SUB, p = blockIdx.x % RS_SUB * RS_THREADS + t;
+    if (t < 256) h[t] = 0;
     __syncthreads();
-    const int4 tl = rs_tile(tiles, n, nb);
-#pragma unroll
-    for (int k = 0; k < RS_ITEMS; ++k) {
-        const int p = k * RS_THREADS + threadIdx.x;
-        if (p < tl.y) atomicAdd(&h[(keys[tl.x + p] >> shift) & 255u], 1u);
+    const int4 tl = tiles ? tiles[tile] : make_int4(tile * RS_TILE, min(RS_TILE, n - tile * RS_TILE), 0, nb);
+    if (p < tl.y) {
+        const double *q = rb + (prun ? (int64_t)prun[tl.x] * RB_STRIDE : 0);
+        const int i = tl.x + p;
+        const double px = x[i], py = y[i], pz = z[i];
+        if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) atomicOr(err, ERR_NONFINITE);
+        const uint64_t key = (spread3(cell_coord(px, q[0], q[4])) << 2) | (spread3(cell_coord(py, q[1], q[4])) << 1) |
+                             spread3(cell_coord(pz, q[2], q[4]));
+        keys[i] = key;
+        atomicAdd(&h[key & 255u], 1u);
     }
     __syncthreads();
-    hist[tl.z + threadIdx.x * tl.w] = h[threadIdx.x];
+    if (t < 256 && h[t]) atomicAdd(&hist[(int64_t)tile * 256 + t], h[t]);
 }
 
-// Stable in-tile ranking by warp multisplit: each warp ranks its 256 keys
-// (eight rounds of 32 consecutive keys) with __match_any_sync against
-// per-warp digit counters; the counters of the eight warps are then turned
-// into per-digit offsets, the tile is reordered by digit in shared memory and
-// written out in runs of equal digit.
-constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_WKEYS = RS_TILE / RS_WARPS;
-static_assert(RS_THREADS == 256, "one thread per digit in the offset step");
+// per run (blockIdx.y) and 32 digits (blockIdx.x): off[tile][digit] = keys of the digit in the run's earlier tiles,
+// tot[first tile][digit] = in all of them.  Warp w sums the w-th 32nd of the tiles, a digit per lane.
+__global__ void __launch_bounds__(1024) k_rs_scan(const uint32_t *hist, const int4 *info, uint32_t *off,
+                                                  uint32_t *tot) {
+    __shared__ uint32_t s[32][32];
+    const int4 r = info[blockIdx.y];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
+    const int per = (r.w + 31) / 32, t0 = r.z + w * per, t1 = min(r.z + r.w, t0 + per);
+    uint32_t v = 0;
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) v += hist[(int64_t)t * 256 + d];
+    s[w][lane] = v;
+    __syncthreads();
+    uint32_t base = 0;
+    for (int k = 0; k < w; ++k) base += s[k][lane];
+    if (w == 31) tot[(int64_t)r.z * 256 + d] = base + v;
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) {
+        off[(int64_t)t * 256 + d] = base;
+        base += hist[(int64_t)t * 256 + d];
+    }
+}
 
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
-                                                           uint32_t *vout, int n, int shift, const uint32_t *off,
-                                                           int nb, const int4 *tiles) {
-    __shared__ uint64_t sk[RS_TILE];
-    __shared__ uint32_t sv[RS_TILE];
-    __shared__ uint32_t wc[RS_WARPS][256];   // per-warp digit counts, then per-warp offsets within a digit
+// One pass over a tile: stable in-tile ranking by warp multisplit (each warp ranks its 128 keys, four rounds of 32
+// consecutive keys, by votes against per-warp digit counters, which then become per-digit
+// offsets), the tile reordered by digit in shared memory and written out in runs of equal digit.  16 warps of 128
+// keys instead of 8 of 256: the rounds of a warp are a serial chain.
+__global__ void __launch_bounds__(RS_THREADS, 4) k_rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
+                                                           uint32_t *vout, int n, int shift, const uint32_t *hist,
+                                                           uint32_t *next, uint32_t *clear, const uint32_t *off,
+                                                           const uint32_t *tot, int nb, const int4 *tiles) {
+    // per-warp digit counts, then per-warp offsets within a digit; then the reordered tile
+    __shared__ __align__(8) unsigned char s_buf[RS_TILE * (sizeof(uint64_t) + sizeof(uint32_t))];
+    static_assert(sizeof(s_buf) >= RS_WARPS * 256 * sizeof(uint32_t), "the counters fit the tile's buffer");
+    uint32_t(*wc)[256] = reinterpret_cast<uint32_t(*)[256]>(s_buf);
+    uint64_t *sk = reinterpret_cast<uint64_t *>(s_buf);
+    uint32_t *sv = reinterpret_cast<uint32_t *>(sk + RS_TILE);
     __shared__ uint32_t dstart[256];         // first tile position of each digit
+    __shared__ uint32_t gofs[256];           // a digit's first output minus its first tile position
+    __shared__ uint32_t s_pre[2][256], s_tot[2][256];
+    __shared__ uint64_t s_scan[8];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const int4 tl = rs_tile(tiles, n, nb);
     const int base = tl.x;
     const int cnt = tl.y;
+    const int run0 = tiles ? tiles[tl.z].x : 0;   // the run's first particle
     for (int k = t; k < RS_WARPS * 256; k += RS_THREADS) (&wc[0][0])[k] = 0u;
-    __syncthreads();
-    uint64_t key[RS_ITEMS];
-    uint32_t val[RS_ITEMS], rk[RS_ITEMS];
-    int dg[RS_ITEMS];
+    if (clear && t < 256) clear[(int64_t)blockIdx.x * 256 + t] = 0;   // what the next pass counts into
+    uint64_t key[RS_ROUNDS];
+    uint32_t val[RS_ROUNDS], rk[RS_ROUNDS];
+    const int p0 = w * RS_WKEYS + lane;   // tile position of the thread's first key
 #pragma unroll
-    for (int r = 0; r < RS_ITEMS; ++r) {
-        const int p = w * RS_WKEYS + r * 32 + lane;
-        const bool ok = p < cnt;
-        key[r] = ok ? kin[base + p] : 0ULL;
-        val[r] = ok ? vin[base + p] : 0u;
-        const int d = ok ? (int)((key[r] >> shift) & 255u) : 256;   // 256: no item
-        dg[r] = d;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
+    for (int r = 0; r < RS_ROUNDS; ++r) {
+        const bool ok = p0 + r * 32 < cnt;
+        const int i = base + p0 + r * 32;
+        key[r] = ok ? kin[i] : 0ULL;
+        val[r] = ok ? (vin ? vin[i] : (uint32_t)i) : 0u;   // the first pass's values are the indices
+    }
+    auto digit = [&](int r) { return p0 + r * 32 < cnt ? (int)((key[r] >> shift) & 255u) : 256; };   // 256: no item
+    {   // the digit's keys in the run's earlier tiles, and in all of them
+        const int d = t & 255, half = t >> 8;
+        uint32_t pre = 0, all = 0;
+        if (off) {
+            if (half == 0) {
+                pre = off[(int64_t)blockIdx.x * 256 + d];
+                all = tot[(int64_t)tl.z * 256 + d];
+            }
+        } else {
+            const int own = blockIdx.x - tl.z;
+            const uint32_t *h = hist + (int64_t)tl.z * 256 + d;
+#pragma unroll 16
+            for (int k = half; k < tl.w; k += 2) {
+                const uint32_t v = h[k * 256];
+                all += v;
+                pre += k < own ? v : 0u;
+            }
+        }
+        s_pre[half][d] = pre;
+        s_tot[half][d] = all;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; ++r) {
+        const int d = digit(r);
+        const unsigned peers = same_digit(d);
         uint32_t b0 = 0;
-        if (ok) b0 = wc[w][d];
+        if (d < 256) b0 = wc[w][d];
         rk[r] = b0 + (uint32_t)__popc(peers & lt);
         __syncwarp();
-        if (ok && lane == __ffs(peers) - 1) wc[w][d] = b0 + (uint32_t)__popc(peers);
+        if (d < 256 && lane == __ffs(peers) - 1) wc[w][d] = b0 + (uint32_t)__popc(peers);
         __syncwarp();
     }
     __syncthreads();
     {
-        uint32_t c = 0;
-        for (int ww = 0; ww < RS_WARPS; ++ww) {
-            const uint32_t v = wc[ww][t];
-            wc[ww][t] = c;
-            c += v;
+        uint32_t c = 0, all = 0;
+        if (t < 256) {
+            uint32_t v[RS_WARPS];   // all read before the first is written: one trip, not a chain
+#pragma unroll
+            for (int ww = 0; ww < RS_WARPS; ++ww) v[ww] = wc[ww][t];
+#pragma unroll
+            for (int ww = 0; ww < RS_WARPS; ++ww) {
+                wc[ww][t] = c;
+                c += v[ww];
+            }
+            all = s_tot[0][t] + s_tot[1][t];
         }
-        int tot;
-        const int incl = block_incl_scan((int)c, &tot);
-        dstart[t] = (uint32_t)incl - c;
+        // the digits' starts in the tile and in the run, one scan for both (digits 0..255: warps 0..7)
+        uint64_t x = c | (uint64_t)all << 32;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (t < 256 && lane == 31) s_scan[w] = x;
+        __syncthreads();
+        if (t < 256) {
+            for (int k = 0; k < w; ++k) x += s_scan[k];
+            const uint32_t ds = (uint32_t)x - c;
+            dstart[t] = ds;
+            gofs[t] = (uint32_t)run0 + (uint32_t)(x >> 32) - all + s_pre[0][t] + s_pre[1][t] - ds;
+        }
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RS_ITEMS; ++r) {
-        const int d = dg[r];
-        if (d < 256) {
-            const uint32_t p = dstart[d] + wc[w][d] + rk[r];
-            sk[p] = key[r];
-            sv[p] = val[r];
+    for (int r = 0; r < RS_ROUNDS; ++r)
+        if (digit(r) < 256) rk[r] += dstart[digit(r)] + wc[w][digit(r)];
+    __syncthreads();   // the counters have been read: the tile goes over them
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; ++r)
+        if (digit(r) < 256) {
+            sk[rk[r]] = key[r];
+            sv[rk[r]] = val[r];
         }
-    }
     __syncthreads();
-    for (int k = 0; k < RS_ITEMS; ++k) {
+#pragma unroll
+    for (int k = 0; k < RS_TILE / RS_THREADS; ++k) {
         const int p = k * RS_THREADS + t;
         if (p < cnt) {
             const uint64_t kk = sk[p];
-            const int d = (int)((kk >> shift) & 255u);
-            const uint32_t g = off[tl.z + d * tl.w] + (uint32_t)p - dstart[d];
+            const uint32_t g = gofs[(kk >> shift) & 255u] + (uint32_t)p;
             kout[g] = kk;
             vout[g] = sv[p];
+            if (next)
+                atomicAdd(&next[(int64_t)(tl.z + (int)(g - (uint32_t)run0) / RS_TILE) * 256 +
+                                ((kk >> (shift + 8)) & 255u)], 1u);
         }
     }
-}
-
-__global__ void k_u32_to_i32_copy(const uint32_t *a, int *b, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = (int)a[i];
 }
 
 // gather all particle arrays through the permutation
@@ -423,25 +489,6 @@ __global__ void k_permute(const double *F, double *F2, int64_t cap, int n, const
 
 // ---------------------------------------------------------------------------
 // octree
-
-// level 0: one root per run (cell r = run r)
-__global__ void k_tree_init(int R, const int4 *info, int *meta, int *start, int *count, int *level, int *parent,
-                            int *first_child, int *n_child) {
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
-        const int4 q = info[r];
-        start[r] = q.x;
-        count[r] = q.y;
-        level[r] = 0;
-        parent[r] = -1;
-        first_child[r] = -1;
-        n_child[r] = 0;
-    }
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < META_N; ++k) meta[k] = 0;
-        meta[0] = 0;
-        meta[1] = R;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // The octree in one pass over the sorted keys.
@@ -752,8 +799,8 @@ int sph_tree_reserve(sph_ctx *ctx, int64_t n) {
         s.cap = c;
     }
     if (s.nblocks_cap < ctx->runs.cap_T) {   // tiles of all runs (each run starts a tile)
-        SPH_TRY(dalloc(ctx, &s.hist, 256 * (int64_t)ctx->runs.cap_T));
-        SPH_TRY(dalloc(ctx, &s.hoff, 256 * (int64_t)ctx->runs.cap_T));
+        SPH_TRY(dalloc(ctx, &s.hist, RS_HISTS * 256 * (int64_t)ctx->runs.cap_T));
+        SPH_TRY(dalloc(ctx, &s.hoff, 2 * 256 * (int64_t)ctx->runs.cap_T));
         s.nblocks_cap = ctx->runs.cap_T;
     }
     if (!ctx->scan.part) {
@@ -763,23 +810,29 @@ int sph_tree_reserve(sph_ctx *ctx, int64_t n) {
     return SPH_OK;
 }
 
+// sorts the keys in sort.k0 (their first digit counted in sort.hist) into ctx->keys, the order into sort.v0
 static int radix_sort(sph_ctx *ctx, int n) {
     Sort &s = ctx->sort;
     const int nb = ctx->runs.T;
     const int4 *tiles = ctx->runs.tiles;
     static_assert(RS_TILE == RUN_TILE, "run tiles are radix tiles");
-    uint64_t *ka = s.k0, *kb = s.k1;
-    uint32_t *va = s.v0, *vb = s.v1;
-    for (int pass = 0; pass < 8; ++pass) {
-        const int shift = pass * 8;
-        k_rs_hist<<<nb, RS_THREADS, 0, ctx->stream>>>(ka, n, shift, s.hist, nb, tiles); ++ctx->launches;
-        SPH_TRY(sph_scan_exclusive(ctx, (const int *)s.hist, (int *)s.hoff, nullptr, 256 * nb, nullptr));
-        k_rs_scatter<<<nb, RS_THREADS, 0, ctx->stream>>>(ka, va, kb, vb, n, shift, s.hoff, nb, tiles); ++ctx->launches;
-        std::swap(ka, kb);
-        std::swap(va, vb);
+    const bool scan = ctx->runs.max_tiles > RS_DIRECT;
+    const int64_t row = 256 * (int64_t)nb;   // digit counts of one pass
+    for (int pass = 0; pass < RS_PASSES; ++pass) {
+        const bool odd = pass & 1, last = pass == RS_PASSES - 1;
+        uint32_t *hist = s.hist + pass % RS_HISTS * row;
+        uint32_t *next = last ? nullptr : s.hist + (pass + 1) % RS_HISTS * row;
+        uint32_t *clear = last ? nullptr : s.hist + (pass + 2) % RS_HISTS * row;
+        if (scan) {
+            k_rs_scan<<<dim3(8, ctx->runs.R), 1024, 0, ctx->stream>>>(hist, ctx->runs.info, s.hoff, s.hoff + row);
+            ++ctx->launches;
+        }
+        k_rs_scatter<<<nb, RS_THREADS, 0, ctx->stream>>>(odd ? s.k1 : s.k0, pass == 0 ? nullptr : (odd ? s.v1 : s.v0),
+                                                         last ? ctx->keys : (odd ? s.k0 : s.k1), odd ? s.v0 : s.v1, n,
+                                                         8 * pass, hist, next, clear, scan ? s.hoff : nullptr,
+                                                         s.hoff + row, nb, tiles); ++ctx->launches;
     }
     SPH_CUDA(ctx, cudaGetLastError());
-    // 8 passes: the result is back in k0 / v0
     return SPH_OK;
 }
 
@@ -825,12 +878,12 @@ static int enqueue_sort_tree(sph_ctx *ctx) {
     cudaStream_t st = ctx->stream;
     // root cube of every run (one block per tile, then one per run)
     const Runs &R = ctx->runs;
-    k_bbox_tiles<<<R.T, 256, 0, st>>>(x, y, z, R.tiles, R.part); ++ctx->launches;
-    k_bbox_runs<<<R.R, 256, 0, st>>>(R.part, R.info, ctx->cfg.theta, t.rb); ++ctx->launches;
-    k_tree_init<<<1, 256, 0, st>>>(R.R, R.info, t.meta, t.start, t.count, t.level, t.parent, t.first_child,
-                                   t.n_child); ++ctx->launches;
-    k_keys_runs<<<sph_div_up(n, 256), 256, 0, st>>>(x, y, z, n, t.rb, R.prun, ctx->sort.k0, ctx->sort.v0,
-                                                    t.meta + META_ERR); ++ctx->launches;
+    k_bbox_tiles<<<R.T, 512, 0, st>>>(x, y, z, R.tiles, (long long *)R.part, ctx->sort.hist,
+                                      ctx->sort.hist + 256 * (int64_t)R.T); ++ctx->launches;
+    k_bbox_runs<<<R.R, 256, 0, st>>>((const long long *)R.part, R.info, ctx->cfg.theta, t.rb, t.meta, t.start, t.count, t.level,
+                                     t.parent, t.first_child, t.n_child); ++ctx->launches;
+    k_keys_hist<<<R.T * RS_SUB, RS_THREADS, 0, st>>>(x, y, z, n, t.rb, R.prun, R.tiles, R.T, ctx->sort.k0,
+                                                     ctx->sort.hist, t.meta + META_ERR); ++ctx->launches;
     SPH_TRY(radix_sort(ctx, n));
     // permute the particle state into key order
     k_permute<<<sph_div_up(n, 256), 256, 0, st>>>(ctx->F, ctx->F2, cap, n, ctx->sort.v0, ctx->id, ctx->id2,
@@ -841,7 +894,6 @@ static int enqueue_sort_tree(sph_ctx *ctx) {
     std::swap(ctx->id, ctx->id2);
     std::swap(ctx->slot, ctx->slot2);
     std::swap(ctx->mat, ctx->mat2);
-    SPH_CUDA(ctx, cudaMemcpyAsync(ctx->keys, ctx->sort.k0, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, st));
     SPH_TRY(time_mark(ctx, SEG_SORT));
     return enqueue_tree(ctx);
 }
@@ -856,7 +908,7 @@ static void graph_key(const sph_ctx *ctx, uintptr_t key[GRAPH_KEY_N]) {
         (uintptr_t)ctx->mat,       (uintptr_t)ctx->runs.prun,  (uintptr_t)ctx->keys,     (uintptr_t)ctx->sort.k0,
         (uintptr_t)ctx->sort.hist, (uintptr_t)t.start,         (uintptr_t)t.rb,          (uintptr_t)t.cap,
         (uintptr_t)ctx->runs.tiles, (uintptr_t)ctx->runs.part, (uintptr_t)ctx->scan.part, (uintptr_t)t.cinfo,
-        (uintptr_t)ctx->cfg.n_leaf};
+        (uintptr_t)ctx->cfg.n_leaf, (uintptr_t)(ctx->runs.max_tiles > RS_DIRECT)};
     for (int i = 0; i < GRAPH_KEY_N; ++i) key[i] = k[i];
 }
 
