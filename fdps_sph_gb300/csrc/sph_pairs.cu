@@ -375,9 +375,14 @@ struct DrvtArgs32 {
     float kscale;   // (1365/64) / (pi mscale)
 };
 
-__device__ __forceinline__ void drvt_pair32(const float4 pih, const float4 pil, const float4 vih, const float4 vil,
-                                            const float4 qh, const float4 ql, const float4 uh, const float4 ul,
-                                            float invH, float Hf, float ceps, float P[5]) {
+// the pair's terms: mg times x[0..3] (divergence, curl), m times y (grad-h)
+struct DrvtT32 {
+    float mg, m, x[4], y;
+};
+
+__device__ __forceinline__ DrvtT32 drvt_terms32(const float4 pih, const float4 pil, const float4 vih, const float4 vil,
+                                                const float4 qh, const float4 ql, const float4 uh, const float4 ul,
+                                                float invH, float Hf, float ceps) {
     const float dx = df_diff(pih.x, pil.x, qh.x, ql.x);
     const float dy = df_diff(pih.y, pil.y, qh.y, ql.y);
     const float dz = df_diff(pih.z, pil.z, qh.z, ql.z);
@@ -389,16 +394,28 @@ __device__ __forceinline__ void drvt_pair32(const float4 pih, const float4 pil, 
     float w, g;
     wendland_poly_f(r * invH, w, g);
     const float gf = g * rcp_a(r * Hf + ceps);
-    const float mg = -qh.w * gf;
-    P[0] = fmaf(mg, wx * dx + wy * dy + wz * dz, P[0]);
-    P[1] = fmaf(mg, wy * dz - wz * dy, P[1]);
-    P[2] = fmaf(mg, wz * dx - wx * dz, P[2]);
-    P[3] = fmaf(mg, wx * dy - wy * dx, P[3]);
-    P[4] = fmaf(qh.w, 3.0f * w + gf * rr2, P[4]);
+    DrvtT32 t;
+    t.mg = -qh.w * gf;
+    t.m = qh.w;
+    t.x[0] = wx * dx + wy * dy + wz * dz;
+    t.x[1] = wy * dz - wz * dy;
+    t.x[2] = wz * dx - wx * dz;
+    t.x[3] = wx * dy - wy * dx;
+    t.y = 3.0f * w + gf * rr2;
+    return t;
 }
 
-// TPI threads share one i-particle: thread `sub` takes the neighbour pairs 2 sub, 2 sub + 2 TPI, ...
-// and the compensated partial sums are combined by shuffles (TPI = 1: one thread per particle)
+__device__ __forceinline__ void drvt_pair32(const float4 pih, const float4 pil, const float4 vih, const float4 vil,
+                                            const float4 qh, const float4 ql, const float4 uh, const float4 ul,
+                                            float invH, float Hf, float ceps, float P[5]) {
+    const DrvtT32 t = drvt_terms32(pih, pil, vih, vil, qh, ql, uh, ul, invH, Hf, ceps);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) P[q] = fmaf(t.mg, t.x[q], P[q]);
+    P[4] = fmaf(t.m, t.y, P[4]);
+}
+
+// TPI (2 or 4) threads share one i-particle: thread `sub` takes the neighbour pairs 2 sub, 2 sub + 2 TPI, ...
+// and the compensated partial sums are combined by shuffles
 template <int TPI>
 __device__ __forceinline__ void df_group_sum(float &hi, float &lo) {
     const unsigned m = __activemask();
@@ -408,6 +425,96 @@ __device__ __forceinline__ void df_group_sum(float &hi, float &lo) {
         df_add(hi, lo, oh);
         lo += ol;
     }
+}
+
+// per-particle tail of force.h:70-76 in FP32, from the sums times the kernel's normalisation
+__device__ __forceinline__ void drvt_tail32(const DrvtArgs32 &a, int i, double hi, const float D[5]) {
+    const float rho = (float)a.dens[i], hf = (float)hi;
+    const float gs = 1.0f / (1.0f + hf * (-D[4] / hf) / (3.0f * rho));
+    const float dv = D[0] / rho, r0 = D[1] / rho, r1 = D[2] / rho, r2 = D[3] / rho;
+    a.divv[i] = dv;
+    a.rx[i] = r0;
+    a.ry[i] = r1;
+    a.rz[i] = r2;
+    a.gradh[i] = gs;
+    a.bal[i] = fabsf(dv) / (fabsf(dv) + sqrtf(r0 * r0 + r1 * r1 + r2 * r2) + 1.0e-4f * (float)a.snds[i] / hf);
+}
+
+// Not tuned (threads per i-particle 1), a row's FP32 partial sums run over blocks of 32 entries in list order and
+// go into the compensated pair block by block.  One thread doing that is bound by the latency of its 106
+// gathers in a row.  Here four lanes share the particle, lane sub evaluates entries 2 sub, 2 sub + 1 of every eight
+// (neighbours in the list are neighbours in memory, so the lanes' gathers stay together), then the lanes swap their
+// terms so that lane q holds component q of all eight entries (a 4 x 4 transpose: four shuffles) and adds them in
+// list order: the bits are one thread's.  Derivative / hydro of 1M particles 0.88 / 1.12 -> 0.76 / 0.83 ms, of
+// 5,003 particles 59 / 64 -> 27 / 29 us.  Lanes that take whole blocks of 32 instead spread a particle's gathers over
+// its row: 0.96 / 1.20 ms at 1M, and no faster at any size from 3,000 particles on.
+__device__ __forceinline__ void transpose4(unsigned mask, int sub, float v[4]) {
+    const bool o1 = sub & 1, o2 = sub & 2;
+    float s0 = __shfl_xor_sync(mask, o1 ? v[0] : v[1], 1, 4), s1 = __shfl_xor_sync(mask, o1 ? v[2] : v[3], 1, 4);
+    if (o1) {
+        v[0] = s0;
+        v[2] = s1;
+    } else {
+        v[1] = s0;
+        v[3] = s1;
+    }
+    s0 = __shfl_xor_sync(mask, o2 ? v[0] : v[2], 2, 4);
+    s1 = __shfl_xor_sync(mask, o2 ? v[1] : v[3], 2, 4);
+    if (o2) {
+        v[0] = s0;
+        v[1] = s1;
+    } else {
+        v[2] = s0;
+        v[3] = s1;
+    }
+}
+
+
+__global__ void __launch_bounds__(PT) k_drvt32_lanes(int n, DrvtArgs32 a) {
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = gt / 4, sub = gt % 4;
+    if (i >= n) return;   // whole groups of four lanes leave together
+    const unsigned mask = 0xfu << (threadIdx.x & 28);
+    const float4 pih = a.xh[i], pil = a.xl[i], vih = a.vh[i], vil = a.vl[i];
+    const double hi = a.h[i];
+    const float Hf = (float)(SUPPORT * hi), invH = 1.0f / Hf, ceps = (float)(1.0e-6 * hi);
+    // component `sub`, and the fifth (grad-h) in every lane
+    float Dh = 0.0f, Dl = 0.0f, P = 0.0f, Eh = 0.0f, El = 0.0f, Q = 0.0f;
+    const RowView row = row_view(a.nbr, a.rm, i, a.cnt[i]);
+    const int c = row.c;
+    for (int k = 0; k < c; k += 8) {
+        const int kk = k + 2 * sub;
+        DrvtT32 t0{}, t1{};
+        if (kk < c) {
+            const int2 jp = *reinterpret_cast<const int2 *>(row.at(kk));
+            t0 = drvt_terms32(pih, pil, vih, vil, a.xh[jp.x], a.xl[jp.x], a.vh[jp.x], a.vl[jp.x], invH, Hf, ceps);
+            if (kk + 1 < c)
+                t1 = drvt_terms32(pih, pil, vih, vil, a.xh[jp.y], a.xl[jp.y], a.vh[jp.y], a.vl[jp.y], invH, Hf, ceps);
+        }
+        transpose4(mask, sub, t0.x);
+        transpose4(mask, sub, t1.x);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            P = fmaf(__shfl_sync(mask, t0.mg, l, 4), t0.x[l], P);
+            P = fmaf(__shfl_sync(mask, t1.mg, l, 4), t1.x[l], P);
+            Q = fmaf(__shfl_sync(mask, t0.m, l, 4), __shfl_sync(mask, t0.y, l, 4), Q);
+            Q = fmaf(__shfl_sync(mask, t1.m, l, 4), __shfl_sync(mask, t1.y, l, 4), Q);
+        }
+        if ((k & 31) == 24 && k + 8 <= c) {   // 32 entries summed
+            df_add(Dh, Dl, P);
+            df_add(Eh, El, Q);
+            P = Q = 0.0f;
+        }
+    }
+    df_add(Dh, Dl, P);
+    df_add(Eh, El, Q);
+    const float sc = a.kscale * (invH * invH * invH);
+    const float d = (Dh + Dl) * sc;
+    float D[5];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) D[q] = __shfl_sync(mask, d, q, 4);
+    D[4] = (Eh + El) * sc;
+    if (sub == 0) drvt_tail32(a, i, hi, D);
 }
 
 template <int TPI>
@@ -443,25 +550,15 @@ __global__ void __launch_bounds__(PT) k_drvt32(int n, DrvtArgs32 a) {
         const int j = *row.at(k);
         drvt_pair32(pih, pil, vih, vil, a.xh[j], a.xl[j], a.vh[j], a.vl[j], invH, Hf, ceps, P);
     }
-    // per-particle tail of force.h:70-76 in FP32
     const float sc = a.kscale * (invH * invH * invH);
     float D[5];
 #pragma unroll
     for (int q = 0; q < 5; ++q) {
         df_add(Dh[q], Dl[q], P[q]);
-        if (TPI > 1) df_group_sum<TPI>(Dh[q], Dl[q]);
+        df_group_sum<TPI>(Dh[q], Dl[q]);
         D[q] = (Dh[q] + Dl[q]) * sc;
     }
-    if (sub != 0) return;
-    const float rho = (float)a.dens[i], hf = (float)hi;
-    const float gs = 1.0f / (1.0f + hf * (-D[4] / hf) / (3.0f * rho));
-    const float dv = D[0] / rho, r0 = D[1] / rho, r1 = D[2] / rho, r2 = D[3] / rho;
-    a.divv[i] = dv;
-    a.rx[i] = r0;
-    a.ry[i] = r1;
-    a.rz[i] = r2;
-    a.gradh[i] = gs;
-    a.bal[i] = fabsf(dv) / (fabsf(dv) + sqrtf(r0 * r0 + r1 * r1 + r2 * r2) + 1.0e-4f * (float)a.snds[i] / hf);
+    if (sub == 0) drvt_tail32(a, i, hi, D);
 }
 
 // mixed hydro: per-particle FP32 pack hA = (f P / rho^2, c_s, f, Bal), and rho, 1/H and h in the
@@ -499,9 +596,14 @@ struct HydroJ32 {
     float4 qh, ql, uh, ul, A, B;
 };
 
-__device__ __forceinline__ void hydro_pair32(const float4 pih, const float4 pil, const float4 vih, const float4 vil,
-                                             const float4 Ai, const float4 Bi, const HydroJ32 &J, float P[4],
-                                             float &vmax) {
+// the pair's terms: acceleration c (dx, dy, dz) and energy e dvdr
+struct HydroT32 {
+    float c, e, dx, dy, dz, dvdr;
+};
+
+__device__ __forceinline__ HydroT32 hydro_terms32(const float4 pih, const float4 pil, const float4 vih,
+                                                  const float4 vil, const float4 Ai, const float4 Bi,
+                                                  const HydroJ32 &J, float &vmax) {
     const float dx = df_diff(pih.x, pil.x, J.qh.x, J.ql.x);
     const float dy = df_diff(pih.y, pil.y, J.qh.y, J.ql.y);
     const float dz = df_diff(pih.z, pil.z, J.qh.z, J.ql.z);
@@ -523,10 +625,17 @@ __device__ __forceinline__ void hydro_pair32(const float4 pih, const float4 pil,
     const float gfj = (nr * nr * nr) * gj_ * rcp_a(r * J.B.z + J.B.w);
     const float gws = 0.5f * (gfi * Ai.z + gfj * J.A.z);
     const float coef = J.qh.w * (Ai.x * gfi + J.A.x * gfj + AV * gws);
-    P[0] = fmaf(-coef, dx, P[0]);
-    P[1] = fmaf(-coef, dy, P[1]);
-    P[2] = fmaf(-coef, dz, P[2]);
-    P[3] = fmaf(J.qh.w * (Ai.x + 0.5f * AV) * gws, dvdr, P[3]);
+    return HydroT32{-coef, J.qh.w * (Ai.x + 0.5f * AV) * gws, dx, dy, dz, dvdr};
+}
+
+__device__ __forceinline__ void hydro_pair32(const float4 pih, const float4 pil, const float4 vih, const float4 vil,
+                                             const float4 Ai, const float4 Bi, const HydroJ32 &J, float P[4],
+                                             float &vmax) {
+    const HydroT32 t = hydro_terms32(pih, pil, vih, vil, Ai, Bi, J, vmax);
+    P[0] = fmaf(t.c, t.dx, P[0]);
+    P[1] = fmaf(t.c, t.dy, P[1]);
+    P[2] = fmaf(t.c, t.dz, P[2]);
+    P[3] = fmaf(t.e, t.dvdr, P[3]);
 }
 
 __device__ __forceinline__ HydroJ32 load_hydro_j(const HydroArgs32 &a, int j) {
@@ -538,6 +647,56 @@ __device__ __forceinline__ HydroJ32 load_hydro_j(const HydroArgs32 &a, int j) {
     J.A = a.hA[j];
     J.B = hydro_b(J.ql, J.uh, J.ul);
     return J;
+}
+
+// one thread's order on four lanes, as k_drvt32_lanes: lane q keeps component q
+__global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = gt / 4, sub = gt % 4;
+    if (i >= n) return;   // whole groups of four lanes leave together
+    const unsigned mask = 0xfu << (threadIdx.x & 28);
+    const float4 pih = a.xh[i], pil = a.xl[i], vih = a.vh[i], vil = a.vl[i];
+    const float4 Ai = a.hA[i], Bi = hydro_b(pil, vih, vil);
+    float Dh = 0.0f, Dl = 0.0f, P = 0.0f, vmax = 0.0f;   // component `sub`
+    const RowView row = row_view(a.nbr, a.rm, i, a.cnt[i]);
+    const int c = row.c;
+    int2 jn = 2 * sub < c ? *reinterpret_cast<const int2 *>(row.at(2 * sub)) : make_int2(i, i);
+    for (int k = 0; k < c; k += 8) {
+        const int kk = k + 2 * sub;
+        const int2 jp = jn;
+        if (kk + 8 < c) jn = *reinterpret_cast<const int2 *>(row.at(kk + 8));   // (past the row's end: padding, unused)
+        float u0[4] = {0, 0, 0, 0}, x0[4] = {0, 0, 0, 0}, u1[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0};
+        if (kk < c) {
+            const HydroT32 t = hydro_terms32(pih, pil, vih, vil, Ai, Bi, load_hydro_j(a, jp.x), vmax);
+            u0[0] = u0[1] = u0[2] = t.c;
+            u0[3] = t.e;
+            x0[0] = t.dx, x0[1] = t.dy, x0[2] = t.dz, x0[3] = t.dvdr;
+        }
+        if (kk + 1 < c) {
+            const HydroT32 t = hydro_terms32(pih, pil, vih, vil, Ai, Bi, load_hydro_j(a, jp.y), vmax);
+            u1[0] = u1[1] = u1[2] = t.c;
+            u1[3] = t.e;
+            x1[0] = t.dx, x1[1] = t.dy, x1[2] = t.dz, x1[3] = t.dvdr;
+        }
+        transpose4(mask, sub, u0);
+        transpose4(mask, sub, x0);
+        transpose4(mask, sub, u1);
+        transpose4(mask, sub, x1);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            P = fmaf(u0[l], x0[l], P);
+            P = fmaf(u1[l], x1[l], P);
+        }
+        if ((k & 31) == 24 && k + 8 <= c) {   // 32 entries summed
+            df_add(Dh, Dl, P);
+            P = 0.0f;
+        }
+    }
+    df_add(Dh, Dl, P);
+    for (int off = 2; off > 0; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(mask, vmax, off, 4));
+    double *out = sub == 0 ? a.ax : (sub == 1 ? a.ay : (sub == 2 ? a.az : a.edot));
+    out[i] = (Dh + Dl) * (a.kscale * (Bi.y * Bi.y * Bi.y));
+    if (sub == 0) a.dt[i] = (float)(2.0 * C_CFL) * (float)a.h[i] / vmax;   // force.h:126
 }
 
 // six blocks per SM, 80 registers (measured at 1M: 0.91 ms against 0.97 at the 86 registers of
@@ -584,13 +743,11 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32(int n, HydroArgs32 a) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         df_add(Dh[q], Dl[q], P[q]);
-        if (TPI > 1) df_group_sum<TPI>(Dh[q], Dl[q]);
+        df_group_sum<TPI>(Dh[q], Dl[q]);
         D[q] = (Dh[q] + Dl[q]) * sc;
     }
-    if (TPI > 1) {
-        const unsigned m = __activemask();
-        for (int off = TPI / 2; off > 0; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(m, vmax, off, TPI));
-    }
+    const unsigned m = __activemask();
+    for (int off = TPI / 2; off > 0; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(m, vmax, off, TPI));
     if (sub != 0) return;
     a.ax[i] = D[0];
     a.ay[i] = D[1];
@@ -1404,10 +1561,10 @@ int sph_pass_derivative(sph_ctx *ctx, int build_lists) {
                      CF(SPH_SNDS), CF(SPH_DIVV), CF(SPH_ROTX), CF(SPH_ROTY),  CF(SPH_ROTZ), CF(SPH_GRADH),
                      CF(SPH_BAL),  L.nbr,        L.cnt,        ctx->sup.map(),
                      (float)(WNORM / (PI_D * ctx->mscale))};
-        // threads per i-particle: chosen by sph_autotune (1 unless tuned)
+        // threads per i-particle in the sums' order: chosen by sph_autotune (1 unless tuned)
         const int tpi = ctx->tune.drvt_tpi;
-        auto kd = tpi == 4 ? k_drvt32<4> : (tpi == 2 ? k_drvt32<2> : k_drvt32<1>);
-        kd<<<sph_div_up((int64_t)n * tpi, PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        auto kd = tpi == 4 ? k_drvt32<4> : (tpi == 2 ? k_drvt32<2> : k_drvt32_lanes);
+        kd<<<sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
     } else {
         const Pack64 P = pack64<2>(ctx);
         DrvtArgs a{P.x,          P.v,          CF(SPH_SMTH),  CF(SPH_DENS), CF(SPH_SNDS), CF(SPH_DIVV), CF(SPH_ROTX),
@@ -1432,8 +1589,8 @@ int sph_pass_hydro(sph_ctx *ctx, int build_lists) {
                       CF(SPH_AX), CF(SPH_AY), CF(SPH_AZ), CF(SPH_ENGDOT), CF(SPH_DT), L.nbr, L.cnt,
                       ctx->sup.map(),    (float)(WNORM / (PI_D * ctx->mscale))};
         const int tpi = ctx->tune.hydro_tpi;
-        auto kh = tpi == 4 ? k_hydro32<4> : (tpi == 2 ? k_hydro32<2> : k_hydro32<1>);
-        kh<<<sph_div_up((int64_t)n * tpi, PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        auto kh = tpi == 4 ? k_hydro32<4> : (tpi == 2 ? k_hydro32<2> : k_hydro32_lanes);
+        kh<<<sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
     } else {
         HydroArgs a{pack64<4>(ctx), CF(SPH_SMTH), CF(SPH_AX), CF(SPH_AY), CF(SPH_AZ), CF(SPH_ENGDOT), CF(SPH_DT),
                     L.nbr,          L.cnt,        ctx->sup.map()};
