@@ -595,7 +595,7 @@ int dispatch_grav(int tag, int n_walk, const sph_epi_grav **epi, const int *n_ep
         }
         const sph_epi_grav *ei = (const sph_epi_grav *)ts->d_in;
         sph_result_grav *res = (sph_result_grav *)ts->d_out;
-        if (g_batch_prec.load() == SPH_PREC_MIXED) batch32_grav(n_walk, ts->stream, ts->d_meta, ei, js, ss, res);
+        if (g_batch_prec.load() == SPH_PREC_MIXED) batch32_grav(n_walk, L.max_i, ts->stream, ts->d_meta, ei, js, ss, res);
         else batch64_grav(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, ss, res);
     }
     return finish_dispatch(ts);
@@ -603,18 +603,18 @@ int dispatch_grav(int tag, int n_walk, const sph_epi_grav **epi, const int *n_ep
 
 auto launch_dens = [](TagState *ts, const Layout &L, const sph_epi_dens *ei, JSrc<sph_epj_dens> js, sph_result_dens *res, bool mixed) {
     const int n_walk = ts->pending_walks;
-    if (mixed) batch32_dens(n_walk, ts->stream, ts->d_meta, ei, js, res);
+    if (mixed) batch32_dens(n_walk, L.max_i, ts->stream, ts->d_meta, ei, js, res);
     else batch64_dens(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
 auto launch_drvt = [](TagState *ts, const Layout &L, const sph_epi_drvt *ei, JSrc<sph_epj_drvt> js, sph_result_drvt *res, bool mixed) {
     const int n_walk = ts->pending_walks;
-    if (mixed) batch32_drvt(n_walk, ts->stream, ts->d_meta, ei, js, res);
+    if (mixed) batch32_drvt(n_walk, L.max_i, ts->stream, ts->d_meta, ei, js, res);
     else batch64_drvt(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
 auto launch_hydro = [](TagState *ts, const Layout &L, const sph_epi_hydro *ei, JSrc<sph_epj_hydro> js, sph_result_hydro *res,
                        bool mixed) {
     const int n_walk = ts->pending_walks;
-    if (mixed) batch32_hydro(n_walk, ts->stream, ts->d_meta, ei, js, res);
+    if (mixed) batch32_hydro(n_walk, L.max_i, ts->stream, ts->d_meta, ei, js, res);
     else batch64_hydro(n_walk, L.ni, L.max_i, ts->stream, ts->d_meta, ei, js, res);
 };
 

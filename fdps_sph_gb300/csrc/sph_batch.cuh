@@ -29,14 +29,15 @@ struct JSrc {
     }
 };
 
-// the mixed-precision functor kernels (sph_batch32.cu): one block per walk on the tag's stream
-void batch32_dens(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi, JSrc<sph_epj_dens> epj,
+// the mixed-precision functor kernels (sph_batch32.cu): on the tag's stream; max_i: i-particles of the
+// largest walk
+void batch32_dens(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi, JSrc<sph_epj_dens> epj,
                   sph_result_dens *res);
-void batch32_drvt(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi, JSrc<sph_epj_drvt> epj,
+void batch32_drvt(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi, JSrc<sph_epj_drvt> epj,
                   sph_result_drvt *res);
-void batch32_hydro(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
+void batch32_hydro(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
                    JSrc<sph_epj_hydro> epj, sph_result_hydro *res);
-void batch32_grav(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi, JSrc<sph_epj_grav> epj,
+void batch32_grav(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi, JSrc<sph_epj_grav> epj,
                   JSrc<sph_spj_monopole> spj, sph_result_grav *res);
 
 // the FP64 functor kernels (sph_batch64.cu): blocks of up to 32 i-particles of a walk; n_i: i-particles of all

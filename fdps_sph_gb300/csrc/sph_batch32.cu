@@ -1,387 +1,451 @@
 // Mixed-precision functor kernels for the batch entry points (sph_dispatch_* after
 // sph_batch_set_precision(SPH_PREC_MIXED)).
 //
-// The same walks and results as the FP64 kernels of sph_batch.cu (the reference functors,
+// The same walks and results as the FP64 kernels of sph_batch64.cu (the reference functors,
 // force.h:9-23, 89-106, 113-147, 154-168), with the pair arithmetic of the device-resident mixed
 // path: positions and velocities relative to the walk's first i-particle as double-floats (hi + lo
 // FP32 pairs formed from the FP64 payload once per particle), pair terms in FP32 with the
 // approximate root / reciprocal instructions, masses in units of one mass of the walk and the
 // kernel normalisation of the i-particle factored out of the sums, FP32 partial sums of 32 terms
-// added into compensated FP32 accumulators, and the per-particle epilogue (density floor and h, grad-h factor, dt, the normalisation) in FP64.  One
-// block per walk, one thread per i-particle, the walk's j-list staged through shared memory.
+// added into compensated FP32 accumulators, and the per-particle epilogue (density floor and h, grad-h
+// factor, dt, the normalisation) in FP64.
 #include "sph_batch.cuh"
 
 using namespace sph;
 
 namespace {
 
-constexpr int WT = 128;
+// A block takes the walk's i-particles blockDim / 4 at a time, four lanes per i-particle, and the j-list (gravity:
+// EPJ, then SPJ) in tiles of 128 entries.  The sums' order is that of one thread over the list: FP32 partial sums
+// of 32 consecutive entries, added block by block into the compensated pair.  Lane q sums the tile's q-th block of
+// 32, then every lane adds the four partial sums in block order, so the bits are one thread's.  One thread per
+// i-particle in a block per walk had five warps on an SM (a dispatch of 256 walks, 93 i-particles each), bound by
+// latency, read each j as scalars and did the FP64 preparation of every i-particle in idle lanes too.  Four
+// blocks per SM (60 to 64 registers; three: 2.48 ms).  A pass of every functor over 100,003 particles, index
+// form: 3.12 -> 2.35 ms, host link and calls included.
+constexpr int LQ = 4;                  // lanes per i-particle
+constexpr int BT = 256;                // most threads per block
+constexpr int BI = BT / LQ;            // most i-particles per block
+constexpr int TJ = 32 * LQ;            // entries per tile
+constexpr int TP = 33 * LQ;            // its shared-memory slots: a slot of padding per 32 entries, so that the four
+                                       // lanes' float4 reads fall into different banks
+__device__ __forceinline__ int slot(int t) { return t + (t >> 5); }
 
-struct DF3 {   // a double-float 3-vector relative to the walk origin
-    float hx, hy, hz, lx, ly, lz;
-};
+__device__ __forceinline__ float4 hi4(const double *p, const double3 o, float w, float4 *lo, float lw) {
+    float a, b, c, d, e, f;
+    split_df(p[0] - o.x, a, d);
+    split_df(p[1] - o.y, b, e);
+    split_df(p[2] - o.z, c, f);
+    *lo = make_float4(d, e, f, lw);
+    return make_float4(a, b, c, w);
+}
 
-__device__ __forceinline__ DF3 rel3(const double *p, const double3 o) {
-    DF3 r;
-    float a, b;
-    split_df(p[0] - o.x, a, b);
-    r.hx = a;
-    r.lx = b;
-    split_df(p[1] - o.y, a, b);
-    r.hy = a;
-    r.ly = b;
-    split_df(p[2] - o.z, a, b);
-    r.hz = a;
-    r.lz = b;
-    return r;
+// m / m0, without the division (7.5 FP64 instructions) for the equal masses of most runs
+__device__ __forceinline__ float in_units(double m, double m0) {
+    return __double_as_longlong(m) == __double_as_longlong(m0) ? 1.0f : (float)(m / m0);
 }
 
 __device__ __forceinline__ float dfd(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
 
-// CalcDensity: rho = max(5, norm sum m_j W), h = 1.2 (m / rho)^(1/3)
-__global__ void __launch_bounds__(WT) k_walk_dens32(const int64_t *meta, const sph_epi_dens *epi,
-                                                    JSrc<sph_epj_dens> epj, sph_result_dens *res) {
-    __shared__ DF3 sp[WT];
-    __shared__ float sm[WT];
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    if (ni <= 0) return;
-    const double3 o = make_double3(epi[io].pos[0], epi[io].pos[1], epi[io].pos[2]);
-    const double m0 = epi[io].mass > 0.0 ? epi[io].mass : 1.0;   // the walk's mass unit (FP32 range)
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        DF3 pi{};
-        double hi = 1.0, mi = 1.0;
-        if (act) {
-            pi = rel3(epi[io + ii].pos, o);
-            hi = epi[io + ii].smth;
-            mi = epi[io + ii].mass;
+template <int Q>
+struct Sums {
+    float Dh[Q], Dl[Q], P[Q], rest[Q];   // compensated sums; this lane's block; the list's last, partial block
+    __device__ __forceinline__ Sums() {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) Dh[q] = Dl[q] = P[q] = rest[q] = 0.0f;
+    }
+    // the lanes' blocks b0 .. b0 + 3 of a list with n_full whole blocks, in order
+    __device__ __forceinline__ void add(int64_t b0, int64_t n_full) {
+        const unsigned mask = 0xfu << (threadIdx.x & 28);
+#pragma unroll
+        for (int l = 0; l < LQ; ++l)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const float v = __shfl_sync(mask, P[q], l, LQ);
+                if (b0 + l < n_full) df_add(Dh[q], Dl[q], v);
+                else if (b0 + l == n_full) rest[q] = v;
+            }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) P[q] = 0.0f;
+    }
+    // the sums of this i-particle to shared memory (the lanes hold the same)
+    __device__ __forceinline__ void store(float2 *out) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            df_add(Dh[q], Dl[q], rest[q]);
+            if (q % LQ == threadIdx.x % LQ) out[q] = make_float2(Dh[q], Dl[q]);
         }
-        const double Hd = SUPPORT * hi;
-        const float invH = (float)(1.0 / Hd);
-        float sh = 0.0f, sl = 0.0f, part = 0.0f;
-        int cnt = 0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_dens &q = epj[jo + t0 + threadIdx.x];
-                sp[threadIdx.x] = rel3(q.pos, o);
-                sm[threadIdx.x] = (float)(q.mass / m0);
+    }
+};
+
+__device__ __forceinline__ double total(float2 d) { return (double)d.x + (double)d.y; }
+
+// the block's walk and the loop over its i-particles
+struct Walk {
+    int64_t io, ni, jo, nj, so, ns;
+    int ipb, sub;   // i-particles per block, lane of the i-particle
+    __device__ __forceinline__ explicit Walk(const int64_t *meta) {
+        const int64_t *M = meta + 6 * blockIdx.x;
+        io = M[0];
+        ni = M[1];
+        jo = M[2];
+        nj = M[3];
+        so = M[4];
+        ns = M[5];
+        ipb = blockDim.x / LQ;
+        sub = threadIdx.x % LQ;
+    }
+    // entries of this lane's block of a tile of tn entries
+    __device__ __forceinline__ int count(int tn) const { return max(0, min(32, tn - 32 * sub)); }
+};
+
+// CalcDensity: rho = max(5, norm sum m_j W), h = 1.2 (m / rho)^(1/3)
+__global__ void __launch_bounds__(BT, 4) k_walk_dens32(const int64_t *meta, const sph_epi_dens *epi,
+                                                     JSrc<sph_epj_dens> epj, sph_result_dens *res) {
+    __shared__ float4 sp[TP], sl[TP];   // position hi, mass; lo
+    __shared__ float4 ip[BI], il[BI];   // of the i-particles: position hi, 1 / H; lo
+    __shared__ float2 is[BI];
+    const Walk W(meta);
+    if (W.ni <= 0) return;
+    const double3 o = make_double3(epi[W.io].pos[0], epi[W.io].pos[1], epi[W.io].pos[2]);
+    const double m0 = epi[W.io].mass > 0.0 ? epi[W.io].mass : 1.0;   // the walk's mass unit (FP32 range)
+    for (int64_t i0 = (int64_t)blockIdx.y * W.ipb; i0 < W.ni; i0 += (int64_t)gridDim.y * W.ipb) {
+        const int g = threadIdx.x / LQ;   // this lane's i-particle of the block's
+        const bool act = i0 + g < W.ni;
+        const int64_t im = i0 + threadIdx.x;   // the i-particle this thread prepares and finishes
+        const bool mine = threadIdx.x < W.ipb && im < W.ni;
+        const int s0 = 33 * W.sub;   // the first slot of this lane's block
+        if (mine) {
+            const sph_epi_dens &I = epi[W.io + im];
+            ip[threadIdx.x] = hi4(I.pos, o, (float)(1.0 / (SUPPORT * I.smth)), &il[threadIdx.x], 0.0f);
+        }
+        __syncthreads();
+        const float4 ph = ip[g], pl = il[g];
+        const float invH = ph.w;
+        Sums<1> S;
+        for (int64_t t0 = 0; t0 < W.nj; t0 += TJ) {
+            const int tn = (int)min((int64_t)TJ, W.nj - t0);
+            for (int k = threadIdx.x; k < tn; k += blockDim.x) {
+                const sph_epj_dens &q = epj[W.jo + t0 + k];
+                sp[slot(k)] = hi4(q.pos, o, in_units(q.mass, m0), &sl[slot(k)], 0.0f);
             }
             __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const DF3 q = sp[t];
-                const float dx = dfd(q.hx, q.lx, pi.hx, pi.lx), dy = dfd(q.hy, q.ly, pi.hy, pi.ly),
-                            dz = dfd(q.hz, q.lz, pi.hz, pi.lz);
+            const int tc = act ? W.count(tn) : 0;
+#pragma unroll 2
+            for (int t = 0; t < tc; ++t) {
+                const float4 qh = sp[s0 + t], ql = sl[s0 + t];
+                const float dx = dfd(qh.x, ql.x, ph.x, pl.x), dy = dfd(qh.y, ql.y, ph.y, pl.y),
+                            dz = dfd(qh.z, ql.z, ph.z, pl.z);
                 const float s = sqrt_a(dx * dx + dy * dy + dz * dz) * invH;
                 const float p = fmaxf(1.0f - s, 0.0f), p2 = p * p, p4 = p2 * p2;
-                part = fmaf(sm[t], (1.0f + s * (8.0f + s * (25.0f + s * 32.0f))) * (p4 * p4), part);
-                if (++cnt == 32) {
-                    df_add(sh, sl, part);
-                    part = 0.0f;
-                    cnt = 0;
-                }
+                S.P[0] = fmaf(qh.w, (1.0f + s * (8.0f + s * (25.0f + s * 32.0f))) * (p4 * p4), S.P[0]);
             }
+            if (act) S.add(t0 / 32, W.nj / 32);
             __syncthreads();
         }
-        df_add(sh, sl, part);
-        if (act) {
-            const double d = fmax(DENS_FLOOR, ((double)sh + (double)sl) * m0 * kernel_norm(Hd));
-            res[io + ii].dens = d;
-            res[io + ii].smth = SMTH_COEF * cbrt(mi / d);
+        S.store(&is[g]);
+        __syncthreads();
+        if (mine) {
+            const sph_epi_dens &I = epi[W.io + im];
+            const double d = fmax(DENS_FLOOR, total(is[threadIdx.x]) * m0 * kernel_norm(SUPPORT * I.smth));
+            res[W.io + im].dens = d;
+            res[W.io + im].smth = SMTH_COEF * cbrt(I.mass / d);
         }
+        __syncthreads();
     }
 }
 
 // CalcDerivative + grad-h factor: div v, rot v, grad_smth (force.h:89-106)
-__global__ void __launch_bounds__(WT) k_walk_drvt32(const int64_t *meta, const sph_epi_drvt *epi,
-                                                    JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
-    __shared__ DF3 sp[WT], sv[WT];
-    __shared__ float sm[WT];
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    if (ni <= 0) return;
-    const double3 o = make_double3(epi[io].pos[0], epi[io].pos[1], epi[io].pos[2]);
-    const double3 ov = make_double3(epi[io].vel[0], epi[io].vel[1], epi[io].vel[2]);
-    const double m0 = (nj > 0 && epj[jo].mass > 0.0) ? epj[jo].mass : 1.0;   // the walk's mass unit
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        DF3 pi{}, vi{};
-        double hi = 1.0, rhoi = 1.0;
-        if (act) {
-            pi = rel3(epi[io + ii].pos, o);
-            vi = rel3(epi[io + ii].vel, ov);
-            hi = epi[io + ii].smth;
-            rhoi = epi[io + ii].dens;
+__global__ void __launch_bounds__(BT, 4) k_walk_drvt32(const int64_t *meta, const sph_epi_drvt *epi,
+                                                     JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
+    __shared__ float4 sp[TP], sl[TP], sv[TP], su[TP];   // position hi, mass; lo; velocity hi; lo
+    // of the i-particles: position hi, 1 / H; lo, H; velocity hi, 1e-6 h; lo
+    __shared__ float4 ip[BI], il[BI], iv[BI], iu[BI];
+    __shared__ float2 is[BI][5];
+    const Walk W(meta);
+    if (W.ni <= 0) return;
+    const double3 o = make_double3(epi[W.io].pos[0], epi[W.io].pos[1], epi[W.io].pos[2]);
+    const double3 ov = make_double3(epi[W.io].vel[0], epi[W.io].vel[1], epi[W.io].vel[2]);
+    const double m0 = (W.nj > 0 && epj[W.jo].mass > 0.0) ? epj[W.jo].mass : 1.0;   // the walk's mass unit
+    for (int64_t i0 = (int64_t)blockIdx.y * W.ipb; i0 < W.ni; i0 += (int64_t)gridDim.y * W.ipb) {
+        const int g = threadIdx.x / LQ;   // this lane's i-particle of the block's
+        const bool act = i0 + g < W.ni;
+        const int64_t im = i0 + threadIdx.x;   // the i-particle this thread prepares and finishes
+        const bool mine = threadIdx.x < W.ipb && im < W.ni;
+        const int s0 = 33 * W.sub;   // the first slot of this lane's block
+        if (mine) {
+            const sph_epi_drvt &I = epi[W.io + im];
+            const double H = SUPPORT * I.smth;
+            ip[threadIdx.x] = hi4(I.pos, o, (float)(1.0 / H), &il[threadIdx.x], (float)H);
+            iv[threadIdx.x] = hi4(I.vel, ov, (float)(1.0e-6 * I.smth), &iu[threadIdx.x], 0.0f);
         }
-        const double Hd = SUPPORT * hi;
-        const float Hf = (float)Hd, invH = (float)(1.0 / Hd), ceps = (float)(1.0e-6 * hi);
-        float Dh[5] = {0, 0, 0, 0, 0}, Dl[5] = {0, 0, 0, 0, 0}, P[5] = {0, 0, 0, 0, 0};
-        int cnt = 0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_drvt &q = epj[jo + t0 + threadIdx.x];
-                sp[threadIdx.x] = rel3(q.pos, o);
-                sv[threadIdx.x] = rel3(q.vel, ov);
-                sm[threadIdx.x] = (float)(q.mass / m0);
+        __syncthreads();
+        const float4 ph = ip[g], pl = il[g], vh = iv[g], vl = iu[g];
+        const float invH = ph.w, Hf = pl.w, ceps = vh.w;
+        Sums<5> S;
+        for (int64_t t0 = 0; t0 < W.nj; t0 += TJ) {
+            const int tn = (int)min((int64_t)TJ, W.nj - t0);
+            for (int k = threadIdx.x; k < tn; k += blockDim.x) {
+                const sph_epj_drvt &q = epj[W.jo + t0 + k];
+                sp[slot(k)] = hi4(q.pos, o, in_units(q.mass, m0), &sl[slot(k)], 0.0f);
+                sv[slot(k)] = hi4(q.vel, ov, 0.0f, &su[slot(k)], 0.0f);
             }
             __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const DF3 q = sp[t], u = sv[t];
-                const float dx = dfd(pi.hx, pi.lx, q.hx, q.lx), dy = dfd(pi.hy, pi.ly, q.hy, q.ly),
-                            dz = dfd(pi.hz, pi.lz, q.hz, q.lz);
-                const float wx = dfd(u.hx, u.lx, vi.hx, vi.lx), wy = dfd(u.hy, u.ly, vi.hy, vi.ly),
-                            wz = dfd(u.hz, u.lz, vi.hz, vi.lz);   // v_j - v_i
+            const int tc = act ? W.count(tn) : 0;
+#pragma unroll 2
+            for (int t = 0; t < tc; ++t) {
+                const float4 qh = sp[s0 + t], ql = sl[s0 + t], uh = sv[s0 + t], ul = su[s0 + t];
+                const float dx = dfd(ph.x, pl.x, qh.x, ql.x), dy = dfd(ph.y, pl.y, qh.y, ql.y),
+                            dz = dfd(ph.z, pl.z, qh.z, ql.z);
+                const float wx = dfd(uh.x, ul.x, vh.x, vl.x), wy = dfd(uh.y, ul.y, vh.y, vl.y),
+                            wz = dfd(uh.z, ul.z, vh.z, vl.z);   // v_j - v_i
                 const float rr2 = dx * dx + dy * dy + dz * dz;
                 const float r = sqrt_a(rr2);
                 float w, g;
                 wendland_poly_f(r * invH, w, g);
                 const float gf = g * rcp_a(r * Hf + ceps);
-                const float m = sm[t];
-                P[0] = fmaf(m * gf, wx * dx + wy * dy + wz * dz, P[0]);
-                P[1] = fmaf(m * gf, wy * dz - wz * dy, P[1]);
-                P[2] = fmaf(m * gf, wz * dx - wx * dz, P[2]);
-                P[3] = fmaf(m * gf, wx * dy - wy * dx, P[3]);
-                P[4] = fmaf(m, 3.0f * w + gf * rr2, P[4]);
-                if (++cnt == 32) {
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) {
-                        df_add(Dh[k], Dl[k], P[k]);
-                        P[k] = 0.0f;
-                    }
-                    cnt = 0;
-                }
+                const float m = qh.w;
+                S.P[0] = fmaf(m * gf, wx * dx + wy * dy + wz * dz, S.P[0]);
+                S.P[1] = fmaf(m * gf, wy * dz - wz * dy, S.P[1]);
+                S.P[2] = fmaf(m * gf, wz * dx - wx * dz, S.P[2]);
+                S.P[3] = fmaf(m * gf, wx * dy - wy * dx, S.P[3]);
+                S.P[4] = fmaf(m, 3.0f * w + gf * rr2, S.P[4]);
             }
+            if (act) S.add(t0 / 32, W.nj / 32);
             __syncthreads();
         }
-        if (act) {
+        S.store(is[g]);
+        __syncthreads();
+        if (mine) {
+            const sph_epi_drvt &I = epi[W.io + im];
+            const double hi = I.smth, rhoi = I.dens, norm = m0 * kernel_norm(SUPPORT * hi);
             double D[5];
-            const double norm = m0 * kernel_norm(Hd);
 #pragma unroll
-            for (int k = 0; k < 5; ++k) {
-                df_add(Dh[k], Dl[k], P[k]);
-                D[k] = ((double)Dh[k] + (double)Dl[k]) * norm;
-            }
+            for (int k = 0; k < 5; ++k) D[k] = total(is[threadIdx.x][k]) * norm;
             const double gs = -D[4] / hi;
-            sph_result_drvt &out = res[io + ii];
+            sph_result_drvt &out = res[W.io + im];
             out.grad_smth = 1.0 / (1.0 + hi * gs / (3.0 * rhoi));
             out.div_v = D[0] / rhoi;
             out.rot_v[0] = D[1] / rhoi;
             out.rot_v[1] = D[2] / rhoi;
             out.rot_v[2] = D[3] / rhoi;
         }
+        __syncthreads();
     }
 }
 
 // CalcHydroForce: acceleration, du/dt, dt (force.h:113-147)
-struct HJ {
-    DF3 p, v;
-    float m, H, invH, rho, A, cs, f, bal;
-};
-
-__global__ void __launch_bounds__(WT) k_walk_hydro32(const int64_t *meta, const sph_epi_hydro *epi,
-                                                     JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
-    __shared__ HJ sj[WT];
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3];
-    if (ni <= 0) return;
-    const double3 o = make_double3(epi[io].pos[0], epi[io].pos[1], epi[io].pos[2]);
-    const double3 ov = make_double3(epi[io].vel[0], epi[io].vel[1], epi[io].vel[2]);
-    const double m0 = (nj > 0 && epj[jo].mass > 0.0) ? epj[jo].mass : 1.0;   // the walk's mass unit
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        DF3 pi{}, vi{};
-        double hi = 1.0, rhoi = 1.0, Pi = 0.0, ci = 0.0, fi = 1.0, bi = 0.0;
-        if (act) {
-            const sph_epi_hydro &I = epi[io + ii];
-            pi = rel3(I.pos, o);
-            vi = rel3(I.vel, ov);
-            hi = I.smth;
-            rhoi = I.dens;
-            Pi = I.pres;
-            ci = I.snds;
-            fi = I.grad_smth;
-            bi = I.Bal;
+__global__ void __launch_bounds__(BT, 4) k_walk_hydro32(const int64_t *meta, const sph_epi_hydro *epi,
+                                                      JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
+    // position hi, mass; lo, H; velocity hi, 1 / H; lo, rho; f P / rho^2, c_s, f, Bal
+    __shared__ float4 sp[TP], sl[TP], sv[TP], su[TP], sa[TP];
+    // of the i-particles: position hi, 1 / H; lo, H; velocity hi, 1e-6 h; lo, rho; f P / rho^2, c_s, f, Bal
+    __shared__ float4 ip[BI], il[BI], iv[BI], iu[BI], ia[BI];
+    __shared__ float2 is[BI][4];
+    __shared__ float iw[BI];   // v_sig_max
+    const Walk W(meta);
+    if (W.ni <= 0) return;
+    const double3 o = make_double3(epi[W.io].pos[0], epi[W.io].pos[1], epi[W.io].pos[2]);
+    const double3 ov = make_double3(epi[W.io].vel[0], epi[W.io].vel[1], epi[W.io].vel[2]);
+    const double m0 = (W.nj > 0 && epj[W.jo].mass > 0.0) ? epj[W.jo].mass : 1.0;   // the walk's mass unit
+    for (int64_t i0 = (int64_t)blockIdx.y * W.ipb; i0 < W.ni; i0 += (int64_t)gridDim.y * W.ipb) {
+        const int g = threadIdx.x / LQ;   // this lane's i-particle of the block's
+        const bool act = i0 + g < W.ni;
+        const int64_t im = i0 + threadIdx.x;   // the i-particle this thread prepares and finishes
+        const bool mine = threadIdx.x < W.ipb && im < W.ni;
+        const int s0 = 33 * W.sub;   // the first slot of this lane's block
+        if (mine) {
+            const sph_epi_hydro &I = epi[W.io + im];
+            const double H = SUPPORT * I.smth;
+            ip[threadIdx.x] = hi4(I.pos, o, (float)(1.0 / H), &il[threadIdx.x], (float)H);
+            iv[threadIdx.x] = hi4(I.vel, ov, (float)(1.0e-6 * I.smth), &iu[threadIdx.x], (float)I.dens);
+            ia[threadIdx.x] = make_float4((float)(I.grad_smth * I.pres / (I.dens * I.dens)), (float)I.snds,
+                                          (float)I.grad_smth, (float)I.Bal);
         }
-        const double Hd = SUPPORT * hi;
-        const float Hi = (float)Hd, invHi = (float)(1.0 / Hd), cepsi = (float)(1.0e-6 * hi);
-        const float Ai = (float)(fi * Pi / (rhoi * rhoi)), rhof = (float)rhoi, cf = (float)ci, ff = (float)fi,
-                    bf = (float)bi;
-        float Dh[4] = {0, 0, 0, 0}, Dl[4] = {0, 0, 0, 0}, P[4] = {0, 0, 0, 0};
+        __syncthreads();
+        const float4 ph = ip[g], pl = il[g], vh = iv[g], vl = iu[g], I4 = ia[g];
+        const float invHi = ph.w, Hi = pl.w, cepsi = vh.w, rhof = vl.w, Ai = I4.x, cf = I4.y, ff = I4.z, bf = I4.w;
+        Sums<4> S;
         float vmax = 0.0f;
-        int cnt = 0;
-        for (int64_t t0 = 0; t0 < nj; t0 += WT) {
-            if (t0 + threadIdx.x < nj) {
-                const sph_epj_hydro &q = epj[jo + t0 + threadIdx.x];
-                HJ h;
-                h.p = rel3(q.pos, o);
-                h.v = rel3(q.vel, ov);
+        for (int64_t t0 = 0; t0 < W.nj; t0 += TJ) {
+            const int tn = (int)min((int64_t)TJ, W.nj - t0);
+            for (int k = threadIdx.x; k < tn; k += blockDim.x) {
+                const sph_epj_hydro &q = epj[W.jo + t0 + k];
                 const double Hj = SUPPORT * q.smth;
-                h.m = (float)(q.mass / m0);
-                h.H = (float)Hj;
-                h.invH = (float)(1.0 / Hj);
-                h.rho = (float)q.dens;
-                h.A = (float)(q.grad_smth * q.pres / (q.dens * q.dens));
-                h.cs = (float)q.snds;
-                h.f = (float)q.grad_smth;
-                h.bal = (float)q.Bal;
-                sj[threadIdx.x] = h;
+                sp[slot(k)] = hi4(q.pos, o, in_units(q.mass, m0), &sl[slot(k)], (float)Hj);
+                sv[slot(k)] = hi4(q.vel, ov, (float)(1.0 / Hj), &su[slot(k)], (float)q.dens);
+                sa[slot(k)] = make_float4((float)(q.grad_smth * q.pres / (q.dens * q.dens)), (float)q.snds,
+                                          (float)q.grad_smth, (float)q.Bal);
             }
             __syncthreads();
-            const int tn = (int)min((int64_t)WT, nj - t0);
-            for (int t = 0; t < tn; ++t) {
-                const HJ &J = sj[t];
-                const float dx = dfd(pi.hx, pi.lx, J.p.hx, J.p.lx), dy = dfd(pi.hy, pi.ly, J.p.hy, J.p.ly),
-                            dz = dfd(pi.hz, pi.lz, J.p.hz, J.p.lz);
-                const float wx = dfd(vi.hx, vi.lx, J.v.hx, J.v.lx), wy = dfd(vi.hy, vi.ly, J.v.hy, J.v.ly),
-                            wz = dfd(vi.hz, vi.lz, J.v.hz, J.v.lz);
+            const int tc = act ? W.count(tn) : 0;
+#pragma unroll 2
+            for (int t = 0; t < tc; ++t) {
+                const float4 qh = sp[s0 + t], ql = sl[s0 + t], uh = sv[s0 + t], ul = su[s0 + t], J = sa[s0 + t];
+                const float jH = ql.w, jinvH = uh.w;
+                const float dx = dfd(ph.x, pl.x, qh.x, ql.x), dy = dfd(ph.y, pl.y, qh.y, ql.y),
+                            dz = dfd(ph.z, pl.z, qh.z, ql.z);
+                const float wx = dfd(vh.x, vl.x, uh.x, ul.x), wy = dfd(vh.y, vl.y, uh.y, ul.y),
+                            wz = dfd(vh.z, vl.z, uh.z, ul.z);
                 const float rr2 = dx * dx + dy * dy + dz * dz;
                 const float r = sqrt_a(rr2);
                 const float dvdr = wx * dx + wy * dy + wz * dz;
                 const float w = (dvdr < 0.0f) ? dvdr * rcp_a(r) : 0.0f;
-                const float vsig = cf + J.cs - 3.0f * w;
+                const float vsig = cf + J.y - 3.0f * w;
                 vmax = fmaxf(vmax, vsig);
-                const float AV = -0.5f * vsig * w * rcp_a(0.5f * (rhof + J.rho)) * 0.5f * (bf + J.bal);
+                const float AV = -0.5f * vsig * w * rcp_a(0.5f * (rhof + ul.w)) * 0.5f * (bf + J.w);
                 float wi_, gi_, wj_, gj_;
                 wendland_poly_f(r * invHi, wi_, gi_);
-                wendland_poly_f(r * J.invH, wj_, gj_);
-                const float nr = Hi * J.invH;   // the j kernel's normalisation relative to the i kernel's
+                wendland_poly_f(r * jinvH, wj_, gj_);
+                const float nr = Hi * jinvH;   // the j kernel's normalisation relative to the i kernel's
                 const float gfi = gi_ * rcp_a(r * Hi + cepsi);
-                const float gfj = (nr * nr * nr) * gj_ * rcp_a(r * J.H + 4.0e-7f * J.H);
-                const float gws = 0.5f * (gfi * ff + gfj * J.f);
-                const float coef = J.m * (Ai * gfi + J.A * gfj + AV * gws);
-                P[0] = fmaf(-coef, dx, P[0]);
-                P[1] = fmaf(-coef, dy, P[1]);
-                P[2] = fmaf(-coef, dz, P[2]);
-                P[3] = fmaf(J.m * (Ai + 0.5f * AV) * gws, dvdr, P[3]);
-                if (++cnt == 32) {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        df_add(Dh[k], Dl[k], P[k]);
-                        P[k] = 0.0f;
-                    }
-                    cnt = 0;
-                }
+                const float gfj = (nr * nr * nr) * gj_ * rcp_a(fmaf(r, jH, 4.0e-7f * jH));
+                const float gws = 0.5f * (gfi * ff + gfj * J.z);
+                const float coef = qh.w * (Ai * gfi + J.x * gfj + AV * gws);
+                S.P[0] = fmaf(-coef, dx, S.P[0]);
+                S.P[1] = fmaf(-coef, dy, S.P[1]);
+                S.P[2] = fmaf(-coef, dz, S.P[2]);
+                S.P[3] = fmaf(qh.w * (Ai + 0.5f * AV) * gws, dvdr, S.P[3]);
             }
+            if (act) S.add(t0 / 32, W.nj / 32);
             __syncthreads();
         }
-        if (act) {
-            const double norm = m0 * kernel_norm(Hd);
+        const unsigned mask = 0xfu << (threadIdx.x & 28);
+        for (int off = LQ / 2; off > 0; off >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(mask, vmax, off, LQ));
+        S.store(is[g]);
+        if (W.sub == 0) iw[g] = vmax;
+        __syncthreads();
+        if (mine) {
+            const double hi = epi[W.io + im].smth, norm = m0 * kernel_norm(SUPPORT * hi);
             double D[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                df_add(Dh[k], Dl[k], P[k]);
-                D[k] = ((double)Dh[k] + (double)Dl[k]) * norm;
-            }
-            sph_result_hydro &out = res[io + ii];
+            for (int k = 0; k < 4; ++k) D[k] = total(is[threadIdx.x][k]) * norm;
+            sph_result_hydro &out = res[W.io + im];
             out.acc[0] = D[0];
             out.acc[1] = D[1];
             out.acc[2] = D[2];
             out.eng_dot = D[3];
-            out.dt = C_CFL * 2.0 * hi / (double)vmax;
+            out.dt = C_CFL * 2.0 * hi / (double)iw[threadIdx.x];
         }
+        __syncthreads();
     }
 }
 
 // CalcGravityForce<EPJ::Grav> then <SPJMonopole> (force.h:154-168): G m folded into the tile
-__global__ void __launch_bounds__(WT) k_walk_grav32(const int64_t *meta, const sph_epi_grav *epi,
-                                                    JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj,
-                                                    sph_result_grav *res) {
-    __shared__ DF3 sp[WT];
-    __shared__ float sg[WT];
+__global__ void __launch_bounds__(BT, 4) k_walk_grav32(const int64_t *meta, const sph_epi_grav *epi,
+                                                     JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj,
+                                                     sph_result_grav *res) {
+    __shared__ float4 sp[TP], sl[TP];   // position hi, G m; lo
+    __shared__ float4 ip[BI], il[BI];   // of the i-particles: position hi, eps^2; lo
+    __shared__ float2 is[BI][4];
     const double G = 6.67e-11;   // force.h:171-172
-    const int64_t *M = meta + 6 * blockIdx.x;
-    const int64_t io = M[0], ni = M[1], jo = M[2], nj = M[3], so = M[4], ns = M[5];
-    if (ni <= 0) return;
-    const double3 o = make_double3(epi[io].pos[0], epi[io].pos[1], epi[io].pos[2]);
+    const Walk W(meta);
+    if (W.ni <= 0) return;
+    const double3 o = make_double3(epi[W.io].pos[0], epi[W.io].pos[1], epi[W.io].pos[2]);
     // G m in units of the walk's first EPJ mass (or SPJ mass) keeps the FP32 products in range
-    const double gscale = nj > 0 ? G * epj[jo].mass : (ns > 0 ? G * spj[so].mass : G);
-    for (int64_t i0 = 0; i0 < ni; i0 += WT) {
-        const int64_t ii = i0 + threadIdx.x;
-        const bool act = ii < ni;
-        DF3 pi{};
-        float e2 = 1.0f;
-        if (act) {
-            pi = rel3(epi[io + ii].pos, o);
-            e2 = (float)epi[io + ii].eps2;
-        }
-        float Dh[4] = {0, 0, 0, 0}, Dl[4] = {0, 0, 0, 0}, P[4] = {0, 0, 0, 0};
-        int cnt = 0;
-        for (int pass = 0; pass < 2; ++pass) {
-            const int64_t nl = pass == 0 ? nj : ns;
-            for (int64_t t0 = 0; t0 < nl; t0 += WT) {
-                if (t0 + threadIdx.x < nl) {
-                    const double *pp = pass == 0 ? epj[jo + t0 + threadIdx.x].pos : spj[so + t0 + threadIdx.x].pos;
-                    const double mm = pass == 0 ? epj[jo + t0 + threadIdx.x].mass : spj[so + t0 + threadIdx.x].mass;
-                    sp[threadIdx.x] = rel3(pp, o);
-                    sg[threadIdx.x] = (float)(G * mm / gscale);
+    const double gscale = W.nj > 0 ? G * epj[W.jo].mass : (W.ns > 0 ? G * spj[W.so].mass : G);
+    const int64_t nl = W.nj + W.ns;
+    for (int64_t i0 = (int64_t)blockIdx.y * W.ipb; i0 < W.ni; i0 += (int64_t)gridDim.y * W.ipb) {
+        const int g = threadIdx.x / LQ;   // this lane's i-particle of the block's
+        const bool act = i0 + g < W.ni;
+        const int64_t im = i0 + threadIdx.x;   // the i-particle this thread prepares and finishes
+        const bool mine = threadIdx.x < W.ipb && im < W.ni;
+        const int s0 = 33 * W.sub;   // the first slot of this lane's block
+        if (mine)
+            ip[threadIdx.x] = hi4(epi[W.io + im].pos, o, (float)epi[W.io + im].eps2, &il[threadIdx.x], 0.0f);
+        __syncthreads();
+        const float4 ph = ip[g], pl = il[g];
+        const float e2 = ph.w;
+        Sums<4> S;
+        for (int64_t t0 = 0; t0 < nl; t0 += TJ) {
+            const int tn = (int)min((int64_t)TJ, nl - t0);
+            for (int k = threadIdx.x; k < tn; k += blockDim.x) {
+                const int64_t e = t0 + k;
+                const double *pp;
+                double mm;
+                if (e < W.nj) {
+                    const sph_epj_grav &q = epj[W.jo + e];
+                    pp = q.pos;
+                    mm = q.mass;
+                } else {
+                    const sph_spj_monopole &q = spj[W.so + e - W.nj];
+                    pp = q.pos;
+                    mm = q.mass;
                 }
-                __syncthreads();
-                const int tn = (int)min((int64_t)WT, nl - t0);
-                for (int t = 0; t < tn; ++t) {
-                    const DF3 q = sp[t];
-                    const float dx = dfd(pi.hx, pi.lx, q.hx, q.lx), dy = dfd(pi.hy, pi.ly, q.hy, q.ly),
-                                dz = dfd(pi.hz, pi.lz, q.hz, q.lz);
-                    const float ri = rsqrt_a(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, e2))));
-                    const float mri = sg[t] * ri;
-                    const float mr3 = mri * ri * ri;
-                    P[0] = fmaf(-mr3, dx, P[0]);
-                    P[1] = fmaf(-mr3, dy, P[1]);
-                    P[2] = fmaf(-mr3, dz, P[2]);
-                    P[3] -= mri;
-                    if (++cnt == 32) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            df_add(Dh[k], Dl[k], P[k]);
-                            P[k] = 0.0f;
-                        }
-                        cnt = 0;
-                    }
-                }
-                __syncthreads();
+                sp[slot(k)] = hi4(pp, o, (float)(G * mm / gscale), &sl[slot(k)], 0.0f);
             }
+            __syncthreads();
+            const int tc = act ? W.count(tn) : 0;
+#pragma unroll 2
+            for (int t = 0; t < tc; ++t) {
+                const float4 qh = sp[s0 + t], ql = sl[s0 + t];
+                const float dx = dfd(ph.x, pl.x, qh.x, ql.x), dy = dfd(ph.y, pl.y, qh.y, ql.y),
+                            dz = dfd(ph.z, pl.z, qh.z, ql.z);
+                const float ri = rsqrt_a(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, e2))));
+                const float mri = qh.w * ri;
+                const float mr3 = mri * ri * ri;
+                S.P[0] = fmaf(-mr3, dx, S.P[0]);
+                S.P[1] = fmaf(-mr3, dy, S.P[1]);
+                S.P[2] = fmaf(-mr3, dz, S.P[2]);
+                S.P[3] -= mri;
+            }
+            if (act) S.add(t0 / 32, nl / 32);
+            __syncthreads();
         }
-        if (act) {
-            sph_result_grav &out = res[io + ii];
+        S.store(is[g]);
+        __syncthreads();
+        if (mine) {
             double D[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                df_add(Dh[k], Dl[k], P[k]);
-                D[k] = ((double)Dh[k] + (double)Dl[k]) * gscale;
-            }
+            for (int k = 0; k < 4; ++k) D[k] = total(is[threadIdx.x][k]) * gscale;
+            sph_result_grav &out = res[W.io + im];
             out.acc[0] = D[0];
             out.acc[1] = D[1];
             out.acc[2] = D[2];
             out.pot = D[3];
             out.dt = 1.0e30;   // RESULT::Grav::clear(), dt untouched by the functor
         }
+        __syncthreads();
     }
 }
+
+// 64 i-particles (256 threads) per block; with fewer walks than SMs (152) blocks of 32 i-particles, so that the few
+// walks spread over the chip
+struct Shape {
+    dim3 grid;
+    int threads;
+    Shape(int n_walk, int max_i) {
+        const int ipb = n_walk < 152 ? 32 : BT / LQ;
+        const int chunks = (max_i + ipb - 1) / ipb;
+        grid = dim3((unsigned)n_walk, (unsigned)(chunks < 1 ? 1 : (chunks > 4096 ? 4096 : chunks)));
+        threads = ipb * LQ;
+    }
+};
 
 }  // namespace
 
 namespace sph {
 
-// launchers for sph_batch.cu: one block per walk on the tag's stream
-void batch32_dens(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi, JSrc<sph_epj_dens> epj,
-                  sph_result_dens *res) {
-    k_walk_dens32<<<n_walk, WT, 0, st>>>(meta, epi, epj, res);
+// launchers for sph_batch.cu, on the tag's stream; max_i: i-particles of the largest walk
+void batch32_dens(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi,
+                  JSrc<sph_epj_dens> epj, sph_result_dens *res) {
+    const Shape s(n_walk, max_i);
+    k_walk_dens32<<<s.grid, s.threads, 0, st>>>(meta, epi, epj, res);
 }
-void batch32_drvt(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi, JSrc<sph_epj_drvt> epj,
-                  sph_result_drvt *res) {
-    k_walk_drvt32<<<n_walk, WT, 0, st>>>(meta, epi, epj, res);
+void batch32_drvt(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi,
+                  JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
+    const Shape s(n_walk, max_i);
+    k_walk_drvt32<<<s.grid, s.threads, 0, st>>>(meta, epi, epj, res);
 }
-void batch32_hydro(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
+void batch32_hydro(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
                    JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
-    k_walk_hydro32<<<n_walk, WT, 0, st>>>(meta, epi, epj, res);
+    const Shape s(n_walk, max_i);
+    k_walk_hydro32<<<s.grid, s.threads, 0, st>>>(meta, epi, epj, res);
 }
-void batch32_grav(int n_walk, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi, JSrc<sph_epj_grav> epj,
-                  JSrc<sph_spj_monopole> spj, sph_result_grav *res) {
-    k_walk_grav32<<<n_walk, WT, 0, st>>>(meta, epi, epj, spj, res);
+void batch32_grav(int n_walk, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi,
+                  JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj, sph_result_grav *res) {
+    const Shape s(n_walk, max_i);
+    k_walk_grav32<<<s.grid, s.threads, 0, st>>>(meta, epi, epj, spj, res);
 }
 
 }  // namespace sph

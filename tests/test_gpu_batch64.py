@@ -186,3 +186,33 @@ def test_fp64_functors_carry_non_finite_j_out_of_support(kind, field, value):
         assert np.array_equal(np.isnan(r["dens"]) | (r["dens"] == 5.0), np.isnan(ref["dens"][0]))
     else:
         assert np.array_equal(np.isfinite(r[got[1]]), np.isfinite(ref[got[0]][0]))
+
+
+@pytest.mark.parametrize("kind", ["dens", "drvt", "hydro", "grav"])
+def test_mixed_functors_give_the_same_bits_in_every_block_shape(kind):
+    """one walk alone and ten walks (blocks of 32 i-particles), 160 walks (blocks of 64), payload and index form"""
+    from fdps_sph_gb300 import lib
+    walks = [_walk(kind, ni, nj, 10 * ni + nj) for ni, nj in SIZES]
+    spj = [np.zeros((0, 1, 33)[k % 3], T.SPJ_MONO) for k in range(len(walks))]
+    for k, s in enumerate(spj):
+        s["pos"], s["mass"] = np.random.default_rng(k).normal(0, 5e7, (len(s), 3)), 1e20
+    I, J = [w[0] for w in walks], [w[1] for w in walks]
+    g = kind == "grav"
+    lib.batch_precision("mixed")
+    try:
+        ten = lib.run_walks(kind, I, J, spj if g else None)
+        many = lib.run_walks(kind, 16 * I, 16 * J, 16 * spj if g else None)
+        at = np.concatenate([[0], np.cumsum([len(j) for j in J])])
+        ats = np.concatenate([[0], np.cumsum([len(s) for s in spj])])
+        ids = [np.arange(at[k], at[k + 1], dtype=np.int32) for k in range(len(J))]
+        sids = [np.arange(ats[k], ats[k + 1], dtype=np.int32) for k in range(len(J))]
+        n = lib.dispatch_index(kind, 0, I, ids, np.concatenate(J), sids if g else None,
+                               np.concatenate(spj) if g else None, send=True)
+        index = lib.retrieve(kind, 0, n)
+        for k in range(len(walks)):
+            alone = lib.run_walks(kind, [I[k]], [J[k]], [spj[k]] if g else None)[0]
+            assert alone.tobytes() == ten[k].tobytes() == index[k].tobytes()
+            for r in range(16):
+                assert many[r * len(walks) + k].tobytes() == alone.tobytes()
+    finally:
+        lib.batch_precision("fp64")
