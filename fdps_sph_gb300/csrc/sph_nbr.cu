@@ -35,6 +35,8 @@ constexpr float KAPPA = 1.06f;   // measured at 1M: 1.15 -> 13.7 ms, 1.10 -> 12.
 // units' walks differ in length); 1M walk: 1.95 ms with four warps per block, 1.97 with two,
 // 1.92 with one (about 30 blocks per SM, limited by shared memory)
 constexpr int NB_WARPS = 1;
+constexpr int WALK_SMALL = 100, WALK_MID = 330;   // particles per SM below which 4 / 2 warps walk a unit
+constexpr int DENS_SMALL = 200;   // particles per SM below which the density takes 8 threads per particle
 constexpr int ROW_K_MAX = 512;   // widest row block; longer rows continue in spill ranges (RowMap)
 constexpr int NB_CAND = 256;   // raw candidate indices per warp (flushes half as often as with 128: -0.02 ms at 1M)
 constexpr int NB_SURV = 64;    // culled candidates staged for the pair test
@@ -124,7 +126,7 @@ __device__ __forceinline__ float gap2_rd(float4 a_lo, float4 a_hi, float3 glo, f
 // the hot loop carries no spill code (a row longer than K only raises the overflow flag)
 template <bool SPILL>
 __global__ void __launch_bounds__(NB_WARPS * 32, 32 / NB_WARPS)
-k_sup_walk(int n_units, const int2 *__restrict__ units, const int *__restrict__ uidx, const double *__restrict__ x,
+k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__restrict__ uidx, const double *__restrict__ x,
            const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ h,
            double *__restrict__ hsup, const float4 *__restrict__ xh,
            const float4 *__restrict__ xl, const float *__restrict__ H2f, const int *__restrict__ prun, WalkTree T,
@@ -142,9 +144,15 @@ k_sup_walk(int n_units, const int2 *__restrict__ units, const int *__restrict__ 
     __shared__ float4 s_pih[NB_WARPS][32], s_pil[NB_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int w = blockIdx.x * NB_WARPS + warp;
-    if (w >= n_units) return;   // warp-uniform
-    const int uid = uidx ? uidx[w] : w;
-    const int2 U = units[uid];
+    if (w >= n_units * split) return;   // warp-uniform
+    const int uid = uidx ? uidx[w / split] : w / split;
+    // this warp's part of the unit
+    int2 U = units[uid];
+    const int part = w % split, part_n = (U.y + split - 1) / split;
+    const int parts = (U.y + part_n - 1) / part_n;   // non-empty parts
+    U.x += part * part_n;
+    U.y = min(U.y - part * part_n, part_n);
+    if (U.y <= 0) return;   // warp-uniform
     const int K = rm.K;
     const bool valid = lane < U.y;
     const int i = U.x + (valid ? lane : 0);
@@ -399,7 +407,11 @@ k_sup_walk(int n_units, const int2 *__restrict__ units, const int *__restrict__ 
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(FULLM, m, o));
     if (lane == 0) {
         atomicMax(maxcnt, m);
-        uover[uid] = m > K ? 1 : 0;   // the unit holds rows that need a spill range
+        // the unit holds rows that need a spill range: one bit per part
+        if (split == 1) uover[uid] = m > K ? 1 : 0;
+        else if (m > K) atomicOr(&uover[uid], 1 << part);
+        else atomicAnd(&uover[uid], ~(1 << part));
+        if (part == 0) atomicAnd(&uover[uid], (1 << parts) - 1);   // bits of parts this unit does not have
     }
 }
 
@@ -517,13 +529,18 @@ k_unit_mark(int n_units, const int2 *__restrict__ units, const float4 *__restric
     if (lane == 0) umark[u] = hit ? 1 : 0;
 }
 
+__global__ void k_unit_flag(int n_units, const int *uover, int *umark) {
+    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x)
+        umark[u] = uover[u] != 0;
+}
+
 __global__ void k_unit_compact(int n_units, const int *umark, const int *off, int *uidx) {
     for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x)
         if (umark[u]) uidx[off[u]] = u;
 }
 
 // ---------------------------------------------------------------------------
-// exact filter: one thread per particle
+// exact filter
 
 constexpr int ERR_SKIN = 16;
 
@@ -546,6 +563,16 @@ __device__ __forceinline__ bool exact_in(float r2, float thr, int j, double xi, 
     return false;
 }
 
+// the same with the i-particle's doubles loaded only inside the band
+__device__ __forceinline__ bool exact_in(float r2, float thr, int j, int i, const double *__restrict__ x,
+                                         const double *__restrict__ y, const double *__restrict__ z,
+                                         const double *__restrict__ h, bool sym) {
+    if (r2 < thr * (1.0f - 1.9073486328125e-06f)) return true;
+    if (r2 > thr * (1.0f + 1.9073486328125e-06f)) return false;
+    const double Hi = __dmul_rn(SUPPORT, h[i]);
+    return exact_in(r2, thr, j, x[i], y[i], z[i], __dmul_rn(Hi, Hi), x, y, z, h, sym);
+}
+
 // exact_in behind a call: a loop that decides several entries before summing them would
 // otherwise have the FP64 test if-converted, issuing its FP64 instructions for every entry
 __device__ __noinline__ bool exact_in_call(float r2, float thr, int j, double xi, double yi, double zi, double H2,
@@ -554,131 +581,98 @@ __device__ __noinline__ bool exact_in_call(float r2, float thr, int j, double xi
     return exact_in(r2, thr, j, xi, yi, zi, H2, x, y, z, h, false);
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(128)
-k_filter(int n, const int *__restrict__ sup, const float *__restrict__ sup_r2, const int *__restrict__ scnt,
-         RowMap rm, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-         const double *__restrict__ h, const double *__restrict__ hsup, const float *__restrict__ H2f,
-         int *__restrict__ out, int *__restrict__ ocnt, int *err) {
-    __shared__ int s_buf[8][128];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double hi = h[i];
-    const double Hi = __dmul_rn(SUPPORT, hi);
-    const double H2 = __dmul_rn(Hi, Hi);
-    const float H2i = (float)H2;
-    const double xi = x[i], yi = y[i], zi = z[i];
-    const int c = scnt[i];
-    const int K = rm.K;
-    int *orow = out + (int64_t)i * K;
-    // the exact list is a subset of the superset row: it fits the row and the same spill range
-    int *ospill = (c > K && rm.soff) ? out + rm.main + rm.soff[i] - K : nullptr;   // entry k >= K at ospill + k
-    const int t = threadIdx.x;
-    int k2 = 0;
-    for (int seg = 0; seg < 2; ++seg) {
-        int cs;
-        const int64_t b = row_seg(rm, i, seg, c, &cs);
-        if (cs <= 0) break;
-        const int *row = sup + b;
-        const float *rrow = sup_r2 + b;
-        for (int k = 0; k < cs; k += 8) {
-            const int4 j0 = reinterpret_cast<const int4 *>(row + k)[0], j1 = reinterpret_cast<const int4 *>(row + k)[1];
-            const float4 r0 = reinterpret_cast<const float4 *>(rrow + k)[0],
-                         r1 = reinterpret_cast<const float4 *>(rrow + k)[1];
-            const int jj[8] = {j0.x, j0.y, j0.z, j0.w, j1.x, j1.y, j1.z, j1.w};
-            const float rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-            const int m = min(8, cs - k);
-            float thr[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) thr[u] = (MODE == 1 && u < m) ? fmaxf(H2i, H2f[jj[u]]) : H2i;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (u < m && exact_in(rr[u], thr[u], jj[u], xi, yi, zi, H2, x, y, z, h, MODE == 1)) {
-                    s_buf[k2 & 7][t] = jj[u];
-                    ++k2;
-                    if ((k2 & 7) == 0) {
-                        int4 *dst = reinterpret_cast<int4 *>((k2 - 8 < K ? orow : ospill) + k2 - 8);
-                        dst[0] = make_int4(s_buf[0][t], s_buf[1][t], s_buf[2][t], s_buf[3][t]);
-                        dst[1] = make_int4(s_buf[4][t], s_buf[5][t], s_buf[6][t], s_buf[7][t]);
-                    }
-                }
-            }
-        }
-    }
-    for (int q = 0; q < (k2 & 7); ++q) {
-        const int k = (k2 & ~7) + q;
-        (k < K ? orow : ospill)[k] = s_buf[q][t];
-    }
-    ocnt[i] = k2;
+// MODE 0: gather list, 1: symmetric list, 2: both (the gather set is a subset of the symmetric set, so its test runs
+// only on symmetric members).  Bound by the latency of the dependent loads (entry, then h of its particle) and by the
+// bytes of the superset rows.  A warp per row: 32 entries at a time, loads and compacted stores contiguous, entries
+// loaded two chunks and h one chunk ahead, 16 blocks per SM at 32 registers (12 blocks: 0.64 ms at 1M, 10:
+// 0.73); outside the edge band nothing touches the FP64 pipe, (2.5 h_i)^2 coming from the rounded-up float copy
+// (within the band the exact test decides, whatever the copy's rounding).  One thread per row, eight entries at a time, took 0.87 ms at 1M and 84 us at 5,003 particles; a warp takes 0.57 ms and 27 us.
+constexpr int FW = 4;   // rows (warps) per block
+constexpr float BAND_LO = 1.0f - 1.9073486328125e-06f, BAND_HI = 1.0f + 1.9073486328125e-06f;   // exact_in's band
+
+// entry k of a row: in the row block, or (SPILL rows, k >= K) in its spill range, base + k
+template <bool SPILL, class T>
+__device__ __forceinline__ T *entry(T *blk, T *spill, int K, int k) {
+    return (SPILL && k >= K ? spill : blk) + k;
 }
 
-// Both exact lists in one pass over the superset (the gather set is a subset of the symmetric
-// set, so the gather test runs only on symmetric members); same decisions and order as
-// k_filter<0> and k_filter<1>.
-__global__ void __launch_bounds__(128)
-k_filter2(int n, const int *__restrict__ sup, const float *__restrict__ sup_r2, const int *__restrict__ scnt,
-          RowMap rm, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-          const double *__restrict__ h, const float *__restrict__ H2f, int *__restrict__ out0,
-          int *__restrict__ ocnt0, int *__restrict__ out1, int *__restrict__ ocnt1) {
-    __shared__ int s_b0[8][128], s_b1[8][128];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double hi = h[i];
-    const double Hi = __dmul_rn(SUPPORT, hi);
-    const double H2 = __dmul_rn(Hi, Hi);
-    const float H2i = (float)H2;
-    const double xi = x[i], yi = y[i], zi = z[i];
-    const int c = scnt[i];
-    const int K = rm.K;
-    int *orow0 = out0 + (int64_t)i * K, *orow1 = out1 + (int64_t)i * K;
-    const bool sp = c > K && rm.soff;
-    int *osp0 = sp ? out0 + rm.main + rm.soff[i] - K : nullptr, *osp1 = sp ? out1 + rm.main + rm.soff[i] - K : nullptr;
-    const int t = threadIdx.x;
+template <int MODE, bool SPILL>
+__device__ __forceinline__ void filter_row(int i, int lane, int c, int K, int64_t spill, const int *__restrict__ sup,
+                                           const float *__restrict__ sup_r2, const double *__restrict__ x,
+                                           const double *__restrict__ y, const double *__restrict__ z,
+                                           const double *__restrict__ h, const float *__restrict__ H2f, int *out0,
+                                           int *out1, int &k0, int &k1) {
+    const int64_t blk = (int64_t)i * K;
+    const int *row = sup + blk, *row_s = sup + spill;
+    const float *rrow = sup_r2 + blk, *rrow_s = sup_r2 + spill;
+    int *o0 = out0 + blk, *o0_s = out0 + spill, *o1 = out1 + blk, *o1_s = out1 + spill;
+    const unsigned lt = (1u << lane) - 1u;
+    const float H2i = H2f[i], lo0 = H2i * BAND_LO, hi0 = H2i * BAND_HI;
+    // two chunks ahead: entries; one chunk ahead: the h of their particles
+    int jn = i, jm = i;
+    float rn = INFINITY, rm = INFINITY;   // past the end: no member of anything
+    if (lane < c) {
+        jn = *entry<SPILL>(row, row_s, K, lane);
+        rn = *entry<SPILL>(rrow, rrow_s, K, lane);
+    }
+    if (lane + 32 < c) {
+        jm = *entry<SPILL>(row, row_s, K, lane + 32);
+        rm = *entry<SPILL>(rrow, rrow_s, K, lane + 32);
+    }
+    float hn = MODE != 0 ? H2f[jn] : 0.0f;
+    for (int b = 0; b < c; b += 32) {
+        const int j = jn, kn = b + 64 + lane;
+        const float r2 = rn, hj = hn;
+        jn = jm;
+        rn = rm;
+        if (MODE != 0) hn = H2f[jn];
+        rm = INFINITY;
+        if (kn < c) {
+            jm = *entry<SPILL>(row, row_s, K, kn);
+            rm = *entry<SPILL>(rrow, rrow_s, K, kn);
+        }
+        bool in0 = r2 < lo0, edge0 = !in0 && r2 <= hi0, in1 = false, edge1 = false;
+        if (MODE != 0) {
+            const float t = fmaxf(H2i, hj);
+            in1 = r2 < t * BAND_LO;
+            edge1 = !in1 && r2 <= t * BAND_HI;
+        }
+        if (__any_sync(FULLM, (MODE != 1 && edge0) || edge1)) {   // rare: the exact test decides
+            if (edge1) in1 = exact_in(r2, fmaxf(H2i, hj), j, i, x, y, z, h, true);
+            if (MODE != 1 && edge0) in0 = exact_in(r2, H2i, j, i, x, y, z, h, false);
+        }
+        if (MODE != 1) {
+            const unsigned m = __ballot_sync(FULLM, in0);
+            if (in0) *entry<SPILL>(o0, o0_s, K, k0 + __popc(m & lt)) = j;
+            k0 += __popc(m);
+        }
+        if (MODE != 0) {
+            const unsigned m = __ballot_sync(FULLM, in1);
+            if (in1) *entry<SPILL>(o1, o1_s, K, k1 + __popc(m & lt)) = j;
+            k1 += __popc(m);
+        }
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(FW * 32, 16)
+k_filter(int n, const int *__restrict__ sup, const float *__restrict__ sup_r2, const int *__restrict__ scnt,
+         RowMap rm, const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
+         const double *__restrict__ h, const float *__restrict__ H2f, int *__restrict__ out0, int *__restrict__ ocnt0,
+         int *__restrict__ out1, int *__restrict__ ocnt1) {
+    const int lane = threadIdx.x & 31, i = blockIdx.x * FW + (threadIdx.x >> 5);
+    if (i >= n) return;   // warp-uniform
+    const int c = scnt[i], K = rm.K;
     int k0 = 0, k1 = 0;
-    auto put = [&](int (*buf)[128], int &kk, int *orow, int *osp, int j) {
-        buf[kk & 7][t] = j;
-        ++kk;
-        if ((kk & 7) == 0) {
-            int4 *dst = reinterpret_cast<int4 *>((kk - 8 < K ? orow : osp) + kk - 8);
-            dst[0] = make_int4(buf[0][t], buf[1][t], buf[2][t], buf[3][t]);
-            dst[1] = make_int4(buf[4][t], buf[5][t], buf[6][t], buf[7][t]);
-        }
-    };
-    for (int seg = 0; seg < 2; ++seg) {
-        int cs;
-        const int64_t b = row_seg(rm, i, seg, c, &cs);
-        if (cs <= 0) break;
-        const int *row = sup + b;
-        const float *rrow = sup_r2 + b;
-        for (int k = 0; k < cs; k += 8) {
-            const int4 j0 = reinterpret_cast<const int4 *>(row + k)[0], j1 = reinterpret_cast<const int4 *>(row + k)[1];
-            const float4 r0 = reinterpret_cast<const float4 *>(rrow + k)[0],
-                         r1 = reinterpret_cast<const float4 *>(rrow + k)[1];
-            const int jj[8] = {j0.x, j0.y, j0.z, j0.w, j1.x, j1.y, j1.z, j1.w};
-            const float rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-            const int m = min(8, cs - k);
-            float thr[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) thr[u] = u < m ? fmaxf(H2i, H2f[jj[u]]) : H2i;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (u < m && exact_in(rr[u], thr[u], jj[u], xi, yi, zi, H2, x, y, z, h, true)) {
-                    put(s_b1, k1, orow1, osp1, jj[u]);
-                    if (exact_in(rr[u], H2i, jj[u], xi, yi, zi, H2, x, y, z, h, false)) put(s_b0, k0, orow0, osp0, jj[u]);
-                }
-            }
-        }
+    if (c <= K)
+        filter_row<MODE, false>(i, lane, c, K, 0, sup, sup_r2, x, y, z, h, H2f, out0, out1, k0, k1);
+    else
+        filter_row<MODE, true>(i, lane, c, K, rm.main + rm.soff[i] - K, sup, sup_r2, x, y, z, h, H2f, out0, out1, k0,
+                               k1);
+    if (lane == 0) {
+        if (MODE != 1) ocnt0[i] = k0;
+        if (MODE != 0) ocnt1[i] = k1;
     }
-    for (int q = 0; q < (k0 & 7); ++q) {
-        const int k = (k0 & ~7) + q;
-        (k < K ? orow0 : osp0)[k] = s_b0[q][t];
-    }
-    for (int q = 0; q < (k1 & 7); ++q) {
-        const int k = (k1 & ~7) + q;
-        (k < K ? orow1 : osp1)[k] = s_b1[q][t];
-    }
-    ocnt0[i] = k0;
-    ocnt1[i] = k1;
 }
 
 // Mixed-precision density straight from the superset: the gather-set
@@ -745,7 +739,8 @@ k_density_sup32(int n, const int *__restrict__ sup, const float *__restrict__ su
 // Every density pass of a step (CalcDensity, force.h:9-23, main.cpp:138-139) for a particle
 // in one go: the passes only use the particle's own h, and its row holds its gather set as
 // long as h <= KAPPA h_sup.  DT threads share a particle (entries 4 sub .. 4 sub + 3 in steps
-// of 4 DT; measured at 1M: DT 1 1.07 ms, 2 0.98, 4 0.97 for the four passes before the loop
+// of 4 DT; 8 for small runs, whose passes are the latency of
+// one thread's chain: 5,000 particles 36 -> 19 us, 20,000 41 -> 34, equal at 40,000; measured at 1M: DT 1 1.07 ms, 2 0.98, 4 0.97 for the four passes before the loop
 // below was made branch-free); a particle whose new h leaves the skin stops after that pass, to
 // go on once its row is walked again.  The four entries of a chunk are decided first (the rare
 // FP64 edge test behind a call), then summed without branches, two at a time in paired FP32
@@ -757,8 +752,7 @@ k_density_sup32(int n, const int *__restrict__ sup, const float *__restrict__ su
 // every run's masses on its own scale are at most 15, so each term is at most 16 and takes
 // sph_fix40_add (FP32 / integer pipes) instead of __float2ll_rn (FP64 pipe); both give the same
 // integers.  Blocks of 64 threads (32 particles): 0.67 -> 0.65 ms at 1M against 128.
-constexpr int DT = 2;
-template <bool SPLIT>
+template <bool SPLIT, int DT>
 __global__ void __launch_bounds__(64)
 k_density_fused32(int n, int n_pass, const int *__restrict__ sup, const float *__restrict__ sup_r2,
                   const float *__restrict__ sup_m, const int *__restrict__ scnt, RowMap rm,
@@ -1050,12 +1044,19 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         }
         SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR, 0, sizeof(int), ctx->stream));
         SPH_CUDA(ctx, cudaMemsetAsync(meta + META_MAXCNT, 0, sizeof(int), ctx->stream));
-        const int blocks = (n_walk + NB_WARPS - 1) / NB_WARPS;
+        // A warp walks a unit, or two or four share it: the walk of a small run is the latency of one warp's chain
+        // (depth-first steps, candidates, accepted entries), and more and shorter chains fill the chip.  Rows do not
+        // depend on the split, and units stay the units of the skin repairs.  Walk of 5,000 / 10,000 particles by
+        // one warp per unit 181 / 236 us, two 146 / 174, four 130 / 158; of 20,000 223, 173, 179; of 40,000 239, 219,
+        // 248; 70,000 particles and more are fastest with one.
+        const int64_t per_sm = n / ctx->num_sms;
+        const int split = per_sm < WALK_SMALL ? 4 : (per_sm < WALK_MID ? 2 : 1);
+        const int blocks = (n_walk * split + NB_WARPS - 1) / NB_WARPS;
         WalkTree T{t.cinfo, t.blo, t.bhi};
         if (blocks > 0) {
             auto walk = S.spill_on ? k_sup_walk<true> : k_sup_walk<false>;
             walk<<<blocks, NB_WARPS * 32, 0, ctx->stream>>>(
-                n_walk, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
+                n_walk, split, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
                 FLD(ctx->F, SPH_SMTH, cap), S.hsup, walk_xh(ctx), walk_xl(ctx), S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
                 S.cnt, S.map(), S.uover, meta + META_ERR, meta + META_MAXCNT);
             ++ctx->launches;
@@ -1103,8 +1104,10 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
                 continue;
             }
             const int grid = 2 * ctx->num_sms;
-            SPH_TRY(sph_scan_exclusive(ctx, S.uover, S.uoff, nullptr, S.n_units, ctx->scan.total));
-            k_unit_compact<<<grid, 256, 0, ctx->stream>>>(S.n_units, S.uover, S.uoff, S.uidx);
+            k_unit_flag<<<grid, 256, 0, ctx->stream>>>(S.n_units, S.uover, S.umark);
+            ++ctx->launches;
+            SPH_TRY(sph_scan_exclusive(ctx, S.umark, S.uoff, nullptr, S.n_units, ctx->scan.total));
+            k_unit_compact<<<grid, 256, 0, ctx->stream>>>(S.n_units, S.umark, S.uoff, S.uidx);
             ++ctx->launches;
             SPH_CUDA(ctx, cudaMemcpyAsync(hs, ctx->scan.total, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
             SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1172,30 +1175,16 @@ int sph_build_sph_lists(sph_ctx *ctx, int mode) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
     const int64_t cap = ctx->cap;
-    int *meta = ctx->tree.meta;
     SPH_TRY(ensure_superset(ctx));
-    if (mode == 2) {   // both lists in one pass
-        SphLists &L0 = ctx->lists[0], &L1 = ctx->lists[1];
-        k_filter2<<<sph_div_up(n, 128), 128, 0, ctx->stream>>>(
-            n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
-            FLD(ctx->F, SPH_SMTH, cap), S.H2f, L0.nbr, L0.cnt, L1.nbr, L1.cnt);
-        ++ctx->launches;
-        SPH_CUDA(ctx, cudaGetLastError());
-        L0.valid = L1.valid = true;
-        return SPH_OK;
-    }
-    SphLists &L = ctx->lists[mode];
-    if (mode == 0)
-        k_filter<0><<<sph_div_up(n, 128), 128, 0, ctx->stream>>>(
-            n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
-            FLD(ctx->F, SPH_SMTH, cap), S.hsup, S.H2f, L.nbr, L.cnt, meta + META_ERR);
-    else
-        k_filter<1><<<sph_div_up(n, 128), 128, 0, ctx->stream>>>(
-            n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
-            FLD(ctx->F, SPH_SMTH, cap), S.hsup, S.H2f, L.nbr, L.cnt, meta + META_ERR);
+    SphLists &L0 = ctx->lists[0], &L1 = ctx->lists[1];
+    auto filter = mode == 0 ? k_filter<0> : (mode == 1 ? k_filter<1> : k_filter<2>);
+    filter<<<sph_div_up(n, FW), FW * 32, 0, ctx->stream>>>(
+        n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
+        FLD(ctx->F, SPH_SMTH, cap), S.H2f, L0.nbr, L0.cnt, L1.nbr, L1.cnt);
     ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
-    L.valid = true;
+    if (mode != 1) L0.valid = true;
+    if (mode != 0) L1.valid = true;
     return SPH_OK;
 }
 
@@ -1233,8 +1222,10 @@ int sph_density_fused(sph_ctx *ctx) {
         SPH_TRY(ensure_superset(ctx));
         SPH_TRY(time_mark(ctx, SEG_DENS_LIST));
         SPH_CUDA(ctx, cudaMemsetAsync(stopped, 0, sizeof(int), ctx->stream));
-        auto kd = ctx->runs.fix_split ? k_density_fused32<true> : k_density_fused32<false>;
-        kd<<<sph_div_up((int64_t)n * DT, 64), 64, 0, ctx->stream>>>(
+        const int dt = (int64_t)n < (int64_t)ctx->num_sms * DENS_SMALL ? 8 : 2;
+        auto kd = ctx->runs.fix_split ? (dt == 8 ? k_density_fused32<true, 8> : k_density_fused32<true, 2>)
+                                      : (dt == 8 ? k_density_fused32<false, 8> : k_density_fused32<false, 2>);
+        kd<<<sph_div_up((int64_t)n * dt, 64), 64, 0, ctx->stream>>>(
             n, np, S.nbr, S.r2, S.m, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
             FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap), FLD(ctx->F, SPH_SMTH, cap), S.hsup,
             FLD(ctx->F, SPH_DENS, cap), (float)(1365.0 / 64.0 / (3.141592653589793 * ctx->mscale)), S.npass,
