@@ -38,14 +38,14 @@ __global__ void k_iota32(int32_t *a, int n) {
 }
 
 // back to upload order: particle k of run r goes to base + slot[k], base = the run's first particle
-// (all runs) or 0 (one run, k in [k0, k0 + n))
-__global__ void k_unpermute(const double *F, double *F2, int64_t cap, int k0, int n, const int32_t *slot,
+// (all runs) or 0 (one run, k in [k0, k0 + n)); the first n_field fields (the others' copies come from k_gather_rows)
+__global__ void k_unpermute(const double *F, double *F2, int n_field, int64_t cap, int k0, int n, const int32_t *slot,
                             const int *prun, const int4 *info, const int64_t *id, int64_t *id2, const int32_t *mat,
                             int32_t *mat2) {
     const int k = k0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= k0 + n) return;
     const int dst = (info ? info[prun[k]].x : 0) + slot[k];
-    for (int f = 0; f < SPH_NFIELD; ++f) F2[(int64_t)f * cap + dst] = F[(int64_t)f * cap + k];
+    for (int f = 0; f < n_field; ++f) F2[(int64_t)f * cap + dst] = F[(int64_t)f * cap + k];
     id2[dst] = id[k];
     mat2[dst] = mat[k];
 }
@@ -123,6 +123,105 @@ __global__ void k_remove_run(const double *F, double *F2, int64_t cap, int n_new
     mat2[k] = mat[src];
     const int q = prun[src];
     prun2[k] = q > r ? q - 1 : q;
+}
+
+// ---- copies between a pinned host block and the state, by kernels
+//
+// The GPU reads and writes pinned host memory at the rate of the copy engine (4M particles, all fields: 5.2 ms up, 5.6
+// ms down, the engine's 5.1 and 5.6), and keeps that rate where the block's pages are scattered, as they are on a host
+// that has run for a while: there the engine took 6 to 29 ms up and up to 50 ms down for the same block.  Downloads
+// also save the pass that puts the fields into upload order first.  A row (field) per blockIdx.y.
+
+// the k-th field of a mask
+__device__ __forceinline__ int mask_field(uint64_t mask, int k) {
+    for (; k > 0; --k) mask &= mask - 1;
+    return __ffsll((long long)mask) - 1;
+}
+
+// rows of the fields in `mask`, n doubles each: dst + f * dst_ld <- src + f * src_ld
+__global__ void __launch_bounds__(512) k_copy_rows(uint64_t mask, int64_t n, const double *src, int64_t src_ld,
+                                                   double *dst, int64_t dst_ld) {
+    const int f = mask_field(mask, blockIdx.y);
+    src += f * src_ld;
+    dst += f * dst_ld;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t done = 0;   // elements the 16-byte copies cover, after `head`
+    const int64_t head = ((uintptr_t)src & 8) ? 1 : 0;
+    if ((((uintptr_t)src ^ (uintptr_t)dst) & 8) == 0 && n > head) {
+        const ulonglong2 *a = reinterpret_cast<const ulonglong2 *>(src + head);
+        ulonglong2 *b = reinterpret_cast<ulonglong2 *>(dst + head);
+        const int64_t m = (n - head) / 2;
+        int64_t k = t;
+        for (; k + 3 * stride < m; k += 4 * stride) {   // four loads in flight: the link's latency
+            const ulonglong2 p = a[k], q = a[k + stride], r = a[k + 2 * stride], w = a[k + 3 * stride];
+            b[k] = p;
+            b[k + stride] = q;
+            b[k + 2 * stride] = r;
+            b[k + 3 * stride] = w;
+        }
+        for (; k < m; k += stride) b[k] = a[k];
+        if (t == 0 && head) dst[0] = src[0];
+        done = head + 2 * m;
+    }
+    for (int64_t k = done + t; k < n; k += stride) dst[k] = src[k];
+}
+
+// the sorted index of every particle of [k0, k0 + n) in upload order (k_unpermute's order)
+__global__ void k_inverse_slots(int k0, int n, const int32_t *slot, const int *prun, const int4 *info, uint32_t *inv) {
+    const int k = k0 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < k0 + n) inv[(info ? info[prun[k]].x : 0) + slot[k]] = (uint32_t)k;
+}
+
+// the fields in `mask` to the host block in upload order
+__global__ void __launch_bounds__(512) k_gather_rows(uint64_t mask, int n, const double *F, int64_t cap,
+                                                     const uint32_t *inv, double *out, int64_t ld) {
+    const int f = mask_field(mask, blockIdx.y);
+    F += f * cap;
+    out += f * ld;
+    const int stride = gridDim.x * blockDim.x;
+    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    for (; k + 3 * (int64_t)stride < n; k += 4 * stride) {
+        const double a = F[inv[k]], b = F[inv[k + stride]], c = F[inv[k + 2 * stride]], d = F[inv[k + 3 * stride]];
+        out[k] = a;
+        out[k + stride] = b;
+        out[k + 2 * stride] = c;
+        out[k + 3 * stride] = d;
+    }
+    for (; k < n; k += stride) out[k] = F[inv[k]];
+}
+
+// the device's address of a host block of doubles that is pinned from its first to its last byte, else null
+double *pinned_block(const double *p, size_t doubles) {
+    cudaPointerAttributes a, b;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + doubles - 1) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || ((uintptr_t)p & 7))
+        return nullptr;
+    // one mapping: the device addresses are as far apart as the host's
+    if ((const char *)b.devicePointer - (const char *)a.devicePointer != (const char *)(p + doubles - 1) - (const char *)p)
+        return nullptr;
+    return (double *)a.devicePointer;
+}
+
+// blocks per row: about two 512-thread blocks per SM over all rows saturate the link
+dim3 row_grid(const sph_ctx *ctx, uint64_t mask, int64_t n) {
+    const int rows = __builtin_popcountll(mask);
+    const int64_t want = (2 * ctx->num_sms + rows - 1) / rows, most = (n + 1023) / 1024;
+    return dim3((unsigned)std::max<int64_t>(1, std::min(want, most)), (unsigned)rows);
+}
+
+// the fields in `mask` of the particles [k0, k0 + n) to a pinned host block in upload order (info: of all runs,
+// null: of one run)
+int gather_to_host(sph_ctx *ctx, uint64_t mask, int k0, int n, const int4 *info, double *out, int64_t ld) {
+    if (!mask) return SPH_OK;
+    uint32_t *inv = ctx->sort.v1;   // free between sorts
+    k_inverse_slots<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(k0, n, ctx->slot, ctx->runs.prun, info, inv);
+    k_gather_rows<<<row_grid(ctx, mask, n), 512, 0, ctx->stream>>>(mask, n, ctx->F, ctx->cap, inv, out, ld);
+    ctx->launches += 2;
+    SPH_CUDA(ctx, cudaGetLastError());
+    return SPH_OK;
 }
 
 template <class T>
@@ -375,17 +474,24 @@ int append_run(sph_ctx *ctx, int64_t n, const double *fields, int64_t ld, const 
     SPH_TRY(grow_particles(ctx, o + n));
     const int64_t c = ctx->cap;
     // field rows: all of them, or (SPH_UPLOAD_STEP_INPUTS) the ones a step reads or carries, the
-    // others zeroed; consecutive rows go in one 2D copy
-    const uint64_t want = (flags & SPH_UPLOAD_STEP_INPUTS) ? (uint64_t)SPH_STEP_INPUT_FIELDS : ~0ull;
+    // others zeroed; from a pinned block by one kernel, else consecutive rows in one 2D copy
+    const uint64_t all = (1ull << SPH_NFIELD) - 1;
+    const uint64_t want = (flags & SPH_UPLOAD_STEP_INPUTS) ? (uint64_t)SPH_STEP_INPUT_FIELDS : all;
+    const double *pinned = pinned_block(fields, (size_t)ld * (SPH_NFIELD - 1) + n);
+    if (pinned) {
+        k_copy_rows<<<row_grid(ctx, want, n), 512, 0, ctx->stream>>>(want, n, pinned, ld, ctx->F + o, c);
+        ++ctx->launches;
+        SPH_CUDA(ctx, cudaGetLastError());
+    }
     for (int f = 0; f < SPH_NFIELD;) {
         const bool in = (want >> f) & 1;
         int g = f;
         while (g < SPH_NFIELD && (((want >> g) & 1) != 0) == in) ++g;
-        if (in)
+        if (in && !pinned)
             SPH_CUDA(ctx, cudaMemcpy2DAsync(ctx->F + (int64_t)f * c + o, sizeof(double) * c, fields + (int64_t)f * ld,
                                             sizeof(double) * ld, sizeof(double) * n, g - f, cudaMemcpyHostToDevice,
                                             ctx->stream));
-        else
+        else if (!in)
             SPH_CUDA(ctx, cudaMemset2DAsync(ctx->F + (int64_t)f * c + o, sizeof(double) * c, 0, sizeof(double) * n,
                                             g - f, ctx->stream));
         f = g;
@@ -898,12 +1004,16 @@ int sph_download_run(sph_ctx *ctx, int64_t handle, double *fields, int64_t ld, i
     const int n = (int)R.n[r];
     if (!fields || ld < n) return sph_fail(ctx, SPH_ERR_ARG, "bad output block");
     cudaSetDevice(ctx->device);
-    k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, ctx->cap, (int)R.off[r], n, ctx->slot,
-                                                             R.prun, nullptr, ctx->id, ctx->id2, ctx->mat,
-                                                             ctx->mat2); ++ctx->launches;
+    const uint64_t all = (1ull << SPH_NFIELD) - 1;
+    double *pinned = ctx->sort.cap >= n ? pinned_block(fields, (size_t)ld * (SPH_NFIELD - 1) + n) : nullptr;
+    if (pinned) SPH_TRY(gather_to_host(ctx, all, (int)R.off[r], n, nullptr, pinned, ld));
+    k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, pinned ? 0 : SPH_NFIELD, ctx->cap,
+                                                             (int)R.off[r], n, ctx->slot, R.prun, nullptr, ctx->id,
+                                                             ctx->id2, ctx->mat, ctx->mat2); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
-    SPH_CUDA(ctx, cudaMemcpy2DAsync(fields, sizeof(double) * ld, ctx->F2, sizeof(double) * ctx->cap,
-                                    sizeof(double) * n, SPH_NFIELD, cudaMemcpyDeviceToHost, ctx->stream));
+    if (!pinned)
+        SPH_CUDA(ctx, cudaMemcpy2DAsync(fields, sizeof(double) * ld, ctx->F2, sizeof(double) * ctx->cap,
+                                        sizeof(double) * n, SPH_NFIELD, cudaMemcpyDeviceToHost, ctx->stream));
     if (id) SPH_CUDA(ctx, cudaMemcpyAsync(id, ctx->id2, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
     if (material)
         SPH_CUDA(ctx, cudaMemcpyAsync(material, ctx->mat2, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -929,12 +1039,19 @@ int sph_download_fields(sph_ctx *ctx, double *fields, int64_t ld, uint64_t field
     if ((field_mask && !fields) || ld < ctx->n) return sph_fail(ctx, SPH_ERR_ARG, "bad output block");
     cudaSetDevice(ctx->device);
     const int n = (int)ctx->n;
-    k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, ctx->cap, 0, n, ctx->slot,
-                                                             ctx->runs.prun, ctx->runs.info, ctx->id, ctx->id2,
-                                                             ctx->mat, ctx->mat2); ++ctx->launches;
+    field_mask &= (1ull << SPH_NFIELD) - 1;
+    double *pinned = nullptr;
+    if (field_mask && ctx->sort.cap >= n)   // (the scratch of the order: as many particles as were ever sorted)
+        pinned = pinned_block(fields, (size_t)ld * (63 - __builtin_clzll(field_mask)) + n);
+    if (pinned) SPH_TRY(gather_to_host(ctx, field_mask, 0, n, ctx->runs.info, pinned, ld));
+    if (!pinned || id || material) {
+        k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, pinned ? 0 : SPH_NFIELD, ctx->cap, 0,
+                                                                 n, ctx->slot, ctx->runs.prun, ctx->runs.info, ctx->id,
+                                                                 ctx->id2, ctx->mat, ctx->mat2); ++ctx->launches;
+    }
     SPH_CUDA(ctx, cudaGetLastError());
     // rows of consecutive requested fields in one 2D copy each
-    for (int f = 0; f < SPH_NFIELD;) {
+    for (int f = pinned ? SPH_NFIELD : 0; f < SPH_NFIELD;) {
         if (!((field_mask >> f) & 1)) {
             ++f;
             continue;
