@@ -50,9 +50,9 @@ struct TagState {
     size_t cap_out = 0;
     int64_t *h_meta = nullptr, *d_meta = nullptr;   // per walk: i offset, n_i, j offset, n_j, s offset, n_s
     size_t cap_meta = 0;
-    uint64_t *h_src = nullptr, *d_src = nullptr;    // per walk: the caller's EPI, EPJ, SPJ addresses
+    uint64_t *h_src = nullptr;                      // per walk: the caller's EPI, EPJ, SPJ addresses
     size_t cap_src = 0;
-    uint64_t *h_dst = nullptr, *d_dst = nullptr;    // per walk: the caller's RESULT address (retrieve)
+    uint64_t *h_dst = nullptr;                      // per walk: the caller's RESULT address (retrieve)
     size_t cap_dst = 0;
     cudaEvent_t gathered = nullptr;                 // the device gather of the pending dispatch is done
     bool gather_pending = false;
@@ -78,15 +78,16 @@ std::mutex *tag_mutex(int tag) { return (tag >= 0 && tag < MAX_TAGS) ? &g_tags[t
     if (!tm_) return batch_fail(SPH_ERR_ARG, "tag out of range [0, 64)");                   \
     std::lock_guard<std::mutex> lk(*tm_)
 
+// a pinned host buffer, and (d) its device counterpart
 int grow(char **h, char **d, size_t *cap, size_t need) {
     if (need <= *cap) return SPH_OK;
     size_t c = std::max(need, *cap * 2);
     if (*h) cudaFreeHost(*h);
-    if (*d) cudaFree(*d);
+    if (d && *d) cudaFree(*d);
     *h = nullptr;
-    *d = nullptr;
+    if (d) *d = nullptr;
     *cap = 0;
-    if (cudaMallocHost((void **)h, c) != cudaSuccess || cudaMalloc((void **)d, c) != cudaSuccess) {
+    if (cudaMallocHost((void **)h, c) != cudaSuccess || (d && cudaMalloc((void **)d, c) != cudaSuccess)) {
         cudaGetLastError();
         return batch_fail(SPH_ERR_OOM, "batch staging allocation failed");
     }
@@ -106,15 +107,14 @@ int tag_state(int tag, TagState **out) {
             for (char **h : {&t.h_in, &t.h_out, (char **)&t.h_meta, (char **)&t.h_src, (char **)&t.h_dst,
                              (char **)&t.h_err})
                 if (*h) cudaFreeHost(*h);
-            for (char **d : {&t.d_in, &t.d_out, (char **)&t.d_meta, (char **)&t.d_src, (char **)&t.d_dst,
-                             (char **)&t.d_err})
+            for (char **d : {&t.d_in, &t.d_out, (char **)&t.d_meta, (char **)&t.d_err})
                 if (*d) cudaFree(*d);
             cudaStreamDestroy(t.stream);
             if (t.gathered) cudaEventDestroy(t.gathered);
             cudaSetDevice(dev);
             t.h_in = t.h_out = t.d_in = t.d_out = nullptr;
             t.h_meta = t.d_meta = nullptr;
-            t.h_src = t.d_src = t.h_dst = t.d_dst = nullptr;
+            t.h_src = t.h_dst = nullptr;
             t.h_err = t.d_err = nullptr;
             t.cap_in = t.cap_out = t.cap_meta = t.cap_src = t.cap_dst = 0;
             t.stream = nullptr;
@@ -147,11 +147,11 @@ static_assert(sizeof(sph_result_dens) % 8 == 0 && sizeof(sph_result_drvt) % 8 ==
                   sizeof(sph_result_hydro) % 8 == 0 && sizeof(sph_result_grav) % 8 == 0,
               "results move as 8-byte words");
 
-// a block copies n 8-byte words, four independent loads per thread in flight (the source may be
-// host memory across the host link, where the latency wants many loads outstanding)
+// the walk's blocks (blockIdx.y of gridDim.y) copy n 8-byte words, four independent loads per thread in
+// flight (the source may be host memory across the host link, where the latency wants many loads outstanding)
 __device__ __forceinline__ void copy_words(const unsigned long long *src, unsigned long long *dst, int64_t n) {
-    const int64_t bd = blockDim.x;
-    int64_t k = threadIdx.x;
+    const int64_t bd = (int64_t)blockDim.x * gridDim.y;
+    int64_t k = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
     for (; k + 3 * bd < n; k += 4 * bd) {
         const unsigned long long a = src[k], b = src[k + bd], c = src[k + 2 * bd], d = src[k + 3 * bd];
         dst[k] = a;
@@ -164,8 +164,8 @@ __device__ __forceinline__ void copy_words(const unsigned long long *src, unsign
 
 // the same in 4-byte words (the index form's int32 index arrays)
 __device__ __forceinline__ void copy_words4(const unsigned *src, unsigned *dst, int64_t n) {
-    const int64_t bd = blockDim.x;
-    int64_t k = threadIdx.x;
+    const int64_t bd = (int64_t)blockDim.x * gridDim.y;
+    int64_t k = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
     for (; k + 3 * bd < n; k += 4 * bd) {
         const unsigned a = src[k], b = src[k + bd], c = src[k + 2 * bd], d = src[k + 3 * bd];
         dst[k] = a;
@@ -183,27 +183,44 @@ __device__ __forceinline__ void copy_run(const void *src, void *dst, int64_t byt
     else copy_words4((const unsigned *)src, (unsigned *)dst, bytes / 4);
 }
 
-// block w copies walk w's EPI, EPJ and SPJ runs (payloads, or index arrays in the index form) from
+// Blocks (w, *) copy walk w's EPI, EPJ and SPJ runs (payloads, or index arrays in the index form) from
 // the caller's arrays (host memory, read over the host link) to their places in the tag's device
-// staging; s_* are the element sizes in bytes
-__global__ void __launch_bounds__(256) k_gather_walks(const int64_t *meta, const uint64_t *src, char *dst,
-                                                      int64_t o_epj, int64_t o_spj, int s_epi, int s_epj,
+// staging; s_* are the element sizes in bytes.  The walk's sizes and addresses are read from the pinned host tables
+// directly, and the sizes left on the device for the kernels that follow: copies of the tables ahead of the kernels
+// were three more calls per dispatch and retrieve (one walk of 180 particles, every functor 225 -> 168 us, with a few
+// walks' copies spread over eight blocks each).
+__global__ void __launch_bounds__(256) k_gather_walks(const int64_t *h_meta, const uint64_t *h_src, int64_t *meta,
+                                                      char *dst, int64_t o_epj, int64_t o_spj, int s_epi, int s_epj,
                                                       int s_spj) {
-    const int64_t *m = meta + 6 * blockIdx.x;
-    const uint64_t *p = src + 3 * blockIdx.x;
+    __shared__ int64_t m[6];
+    __shared__ uint64_t p[3];
+    const int t = threadIdx.x, w = blockIdx.x;
+    if (t < 6) {
+        m[t] = h_meta[6 * (int64_t)w + t];
+        if (blockIdx.y == 0) meta[6 * (int64_t)w + t] = m[t];
+    } else if (t < 9) {
+        p[t - 6] = h_src[3 * (int64_t)w + t - 6];
+    }
+    __syncthreads();
     if (m[1] > 0) copy_run((const void *)p[0], dst + (int64_t)s_epi * m[0], (int64_t)s_epi * m[1], s_epi);
     if (m[3] > 0) copy_run((const void *)p[1], dst + o_epj + (int64_t)s_epj * m[2], (int64_t)s_epj * m[3], s_epj);
     if (m[5] > 0) copy_run((const void *)p[2], dst + o_spj + (int64_t)s_spj * m[4], (int64_t)s_spj * m[5], s_spj);
 }
 
-// block w copies walk w's results from the tag's device buffer to the caller's RESULT array
-__global__ void __launch_bounds__(256) k_scatter_results(const int64_t *meta, const uint64_t *dst, const char *src,
+// blocks (w, *) copy walk w's results from the tag's device buffer to the caller's RESULT array
+__global__ void __launch_bounds__(256) k_scatter_results(const int64_t *meta, const uint64_t *h_dst, const char *src,
                                                          int s_res) {
-    const int64_t *m = meta + 6 * blockIdx.x;
+    __shared__ uint64_t dst;
+    const int64_t *m = meta + 6 * (int64_t)blockIdx.x;
+    if (threadIdx.x == 0) dst = h_dst[blockIdx.x];
+    __syncthreads();
     if (m[1] > 0)
-        copy_words((const unsigned long long *)(src + (int64_t)s_res * m[0]), (unsigned long long *)dst[blockIdx.x],
+        copy_words((const unsigned long long *)(src + (int64_t)s_res * m[0]), (unsigned long long *)dst,
                    (int64_t)s_res * m[1] / 8);
 }
+
+// blocks per walk of the two copies: eight where the walks alone would leave SMs (152) idle
+dim3 copy_grid(int n_walk) { return dim3((unsigned)n_walk, n_walk < 152 ? 8 : 1); }
 
 // where a dispatch's sections sit in the tag's staging (bytes, 16-byte aligned sections)
 struct Layout {
@@ -297,22 +314,16 @@ int stage(int tag, int kind, int n_walk, const EPI **epi, const int *n_epi, cons
         return batch_fail(SPH_ERR_CUDA, "cannot clear the batch error word");
     }
     if (gather) {
-        SPH_TRY(grow((char **)&ts->h_src, (char **)&ts->d_src, &ts->cap_src, sizeof(uint64_t) * 3 * (n_walk + 1)));
+        SPH_TRY(grow((char **)&ts->h_src, nullptr, &ts->cap_src, sizeof(uint64_t) * 3 * (n_walk + 1)));
         for (int w = 0; w < n_walk; ++w) {
             const int64_t *m = ts->h_meta + 6 * w;
             ts->h_src[3 * w] = m[1] ? (uint64_t)(uintptr_t)epi[w] : 0;
             ts->h_src[3 * w + 1] = m[3] ? (uint64_t)(uintptr_t)jw[w] : 0;
             ts->h_src[3 * w + 2] = m[5] ? (uint64_t)(uintptr_t)sw[w] : 0;
         }
-        if (cudaMemcpyAsync(ts->d_meta, ts->h_meta, sizeof(int64_t) * 6 * n_walk, cudaMemcpyHostToDevice,
-                            ts->stream) != cudaSuccess ||
-            cudaMemcpyAsync(ts->d_src, ts->h_src, sizeof(uint64_t) * 3 * n_walk, cudaMemcpyHostToDevice,
-                            ts->stream) != cudaSuccess) {
-            cudaGetLastError();
-            return batch_fail(SPH_ERR_CUDA, "host-to-device copy failed");
-        }
-        k_gather_walks<<<n_walk, 256, 0, ts->stream>>>(ts->d_meta, ts->d_src, ts->d_in, (int64_t)L.o_epj,
-                                                       (int64_t)L.o_spj, (int)sizeof(EPI), (int)s_j, (int)s_s);
+        k_gather_walks<<<copy_grid(n_walk), 256, 0, ts->stream>>>(ts->h_meta, ts->h_src, ts->d_meta, ts->d_in,
+                                                                  (int64_t)L.o_epj, (int64_t)L.o_spj,
+                                                                  (int)sizeof(EPI), (int)s_j, (int)s_s);
         if (cudaGetLastError() != cudaSuccess || cudaEventRecord(ts->gathered, ts->stream) != cudaSuccess) {
             cudaGetLastError();
             return batch_fail(SPH_ERR_CUDA, "walk gather launch failed");
@@ -521,16 +532,14 @@ int retrieve(int tag, int kind, int n_walk, const int *n_epi, RES **result) {
     };
     if (ts.direct_out && aligned && n_walk > 0) {
         // the scatter kernel writes every walk's results into the caller's arrays
-        const int rc = grow((char **)&ts.h_dst, (char **)&ts.d_dst, &ts.cap_dst, sizeof(uint64_t) * (n_walk + 1));
+        const int rc = grow((char **)&ts.h_dst, nullptr, &ts.cap_dst, sizeof(uint64_t) * (n_walk + 1));
         if (rc != SPH_OK) {
             cudaStreamSynchronize(ts.stream);
             ts.pending_kind = -1;
             return rc;
         }
         for (int w = 0; w < n_walk; ++w) ts.h_dst[w] = n_epi[w] > 0 ? (uint64_t)(uintptr_t)result[w] : 0;
-        if (cudaMemcpyAsync(ts.d_dst, ts.h_dst, sizeof(uint64_t) * n_walk, cudaMemcpyHostToDevice, ts.stream) ==
-            cudaSuccess)
-            k_scatter_results<<<n_walk, 256, 0, ts.stream>>>(ts.d_meta, ts.d_dst, ts.d_out, (int)sizeof(RES));
+        k_scatter_results<<<copy_grid(n_walk), 256, 0, ts.stream>>>(ts.d_meta, ts.h_dst, ts.d_out, (int)sizeof(RES));
         const cudaError_t e = cudaStreamSynchronize(ts.stream);
         ts.pending_kind = -1;
         const cudaError_t l = cudaGetLastError();

@@ -14,7 +14,7 @@
 // epilogues (divisions, the pow of the smoothing length) run once per block with one i-particle per lane.
 //
 // Against one thread per i-particle over the whole list in FP64, one 128-thread block per walk, a call of every
-// functor: 180 particles in one walk 4,506 -> 229 us, 30,011 particles 63.7 -> 4.28 ms, staging, results and
+// functor: 180 particles in one walk 4,506 -> 152 us, 30,011 particles 63.7 -> 4.4 ms, staging, results and
 // host included.
 #include "sph_batch.cuh"
 #include "sph_pair64.cuh"
@@ -23,7 +23,7 @@ namespace sph {
 
 namespace {
 
-constexpr int W = 8;            // warps per block
+constexpr int W = 8;            // most warps per block
 constexpr int TJ = 512;         // j entries per tile
 constexpr int IC_MAX = 32;      // i-particles per block
 constexpr unsigned FULLW = 0xffffffffu;
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_dens64(const int64_t *meta, int
     __shared__ double s_i[IC_MAX][5];   // x, y, z, 1 / H (hi, lo)
     __shared__ float4 s_f[IC_MAX];      // the same in FP32: x, y, z, reach + slack
     __shared__ double s_sum[IC_MAX];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
     for (int64_t i0 = (int64_t)blockIdx.y * ic; i0 < meta[6 * blockIdx.x + 1]; i0 += (int64_t)gridDim.y * ic) {
         const Span S = span(meta, i0, ic);
         __syncthreads();   // the last chunk's epilogue has read the shared sums
@@ -114,13 +114,13 @@ __global__ void __launch_bounds__(W * 32) k_walk_dens64(const int64_t *meta, int
         for (int64_t t0 = 0; t0 < S.nj; t0 += TJ) {
             const int tn = (int)min((int64_t)TJ, S.nj - t0);
             __syncthreads();
-            for (int k = t; k < tn; k += W * 32) {
+            for (int k = t; k < tn; k += blockDim.x) {
                 const sph_epj_dens &q = epj[S.jo + t0 + k];
                 const float x = (float)(q.pos[0] - cx), y = (float)(q.pos[1] - cy), z = (float)(q.pos[2] - cz);
                 s_j[k] = make_float4(x, y, z, fin(q.mass) ? slack1(x, y, z) : __int_as_float(0x7fffffff));
             }
             __syncthreads();
-            for (int i = warp; i < S.ni; i += W) {
+            for (int i = warp; i < S.ni; i += nw) {
                 const float4 f = s_f[i];
                 const double xi = s_i[i][0], yi = s_i[i][1], zi = s_i[i][2];
                 const Inv64 invH{s_i[i][3], s_i[i][4]};
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_drvt64(const int64_t *meta, int
     __shared__ double s_i[IC_MAX][10];   // x, v, 1 / H (hi, lo), H, 1e-6 h
     __shared__ float4 s_f[IC_MAX];
     __shared__ double s_sum[IC_MAX][6];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
     for (int64_t i0 = (int64_t)blockIdx.y * ic; i0 < meta[6 * blockIdx.x + 1]; i0 += (int64_t)gridDim.y * ic) {
         const Span S = span(meta, i0, ic);
         __syncthreads();   // the last chunk's epilogue has read the shared sums
@@ -193,14 +193,14 @@ __global__ void __launch_bounds__(W * 32) k_walk_drvt64(const int64_t *meta, int
         for (int64_t t0 = 0; t0 < S.nj; t0 += TJ) {
             const int tn = (int)min((int64_t)TJ, S.nj - t0);
             __syncthreads();
-            for (int k = t; k < tn; k += W * 32) {
+            for (int k = t; k < tn; k += blockDim.x) {
                 const sph_epj_drvt &q = epj[S.jo + t0 + k];
                 const float x = (float)(q.pos[0] - cx), y = (float)(q.pos[1] - cy), z = (float)(q.pos[2] - cz);
                 const bool ok = fin(q.mass) && fin(q.vel[0]) && fin(q.vel[1]) && fin(q.vel[2]);
                 s_j[k] = make_float4(x, y, z, ok ? slack1(x, y, z) : __int_as_float(0x7fffffff));
             }
             __syncthreads();
-            for (int i = warp; i < S.ni; i += W) {
+            for (int i = warp; i < S.ni; i += nw) {
                 const float4 f = s_f[i];
                 const double *I = s_i[i];
                 Queue Q{s_q[warp], 0};
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_hydro64(const int64_t *meta, in
     __shared__ Hydro64 s_k[IC_MAX];
     __shared__ float4 s_f[IC_MAX], s_g[IC_MAX];   // x, y, z, reach; v, c_s
     __shared__ double s_sum[IC_MAX][5];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
     for (int64_t i0 = (int64_t)blockIdx.y * ic; i0 < meta[6 * blockIdx.x + 1]; i0 += (int64_t)gridDim.y * ic) {
         const Span S = span(meta, i0, ic);
         __syncthreads();   // the last chunk's epilogue has read the shared sums
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_hydro64(const int64_t *meta, in
         for (int64_t t0 = 0; t0 < S.nj; t0 += TJ) {
             const int tn = (int)min((int64_t)TJ, S.nj - t0);
             __syncthreads();
-            for (int k = t; k < tn; k += W * 32) {
+            for (int k = t; k < tn; k += blockDim.x) {
                 const sph_epj_hydro &q = epj[S.jo + t0 + k];
                 const float x = (float)(q.pos[0] - cx), y = (float)(q.pos[1] - cy), z = (float)(q.pos[2] - cz);
                 const bool ok = fin(q.mass) && fin(q.dens) && fin(q.pres) && fin(q.snds) && fin(q.grad_smth) &&
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_hydro64(const int64_t *meta, in
                 s_h[k] = ok ? reach(q.smth) : __int_as_float(0x7fffffff);
             }
             __syncthreads();
-            for (int i = warp; i < S.ni; i += W) {
+            for (int i = warp; i < S.ni; i += nw) {
                 const float4 f = s_f[i], g = s_g[i];
                 const float sl_i = slack1(f.x, f.y, f.z), ev_i = fabsf(g.x) + fabsf(g.y) + fabsf(g.z);
                 const double *I = s_i[i];
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_grav64(const int64_t *meta, int
     __shared__ double s_i[IC_MAX][4];
     __shared__ double s_sum[IC_MAX][4];
     const double G = 6.67e-11;   // force.h:171-172
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
     for (int64_t i0 = (int64_t)blockIdx.y * ic; i0 < meta[6 * blockIdx.x + 1]; i0 += (int64_t)gridDim.y * ic) {
         const Span S = span(meta, i0, ic);
         __syncthreads();   // the last chunk's epilogue has read the shared sums
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_grav64(const int64_t *meta, int
         for (int64_t t0 = 0; t0 < nl; t0 += TG) {
             const int tn = (int)min((int64_t)TG, nl - t0);
             __syncthreads();
-            for (int k = t; k < tn; k += W * 32) {
+            for (int k = t; k < tn; k += blockDim.x) {
                 const int64_t e = t0 + k;
                 const double *pos;
                 double m;
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(W * 32) k_walk_grav64(const int64_t *meta, int
                 s_x[3][k] = G * m;
             }
             __syncthreads();
-            for (int i = warp; i < S.ni; i += W) {
+            for (int i = warp; i < S.ni; i += nw) {
                 const double xi = s_i[i][0], yi = s_i[i][1], zi = s_i[i][2], e2 = s_i[i][3];
                 double A[4] = {0, 0, 0, 0};
     #pragma unroll 2
@@ -429,36 +429,42 @@ __global__ void __launch_bounds__(W * 32) k_walk_grav64(const int64_t *meta, int
     }
 }
 
-// i-particles per block: 32 (four per warp, one staging of the j-list for them) where that still
-// gives every SM two blocks (152 SMs), else 8 (one per warp), so that a few walks spread over the chip
-int block_i(int64_t n_i) { return n_i >= 152 * 64 ? IC_MAX : W; }
-
-dim3 walk_grid(int n_walk, int max_i, int ic) {
-    const int chunks = (max_i + ic - 1) / ic;
-    return dim3((unsigned)n_walk, (unsigned)(chunks > 0 ? (chunks < 4096 ? chunks : 4096) : 1));
-}
+// Blocks of 8 warps with 32 i-particles (four per warp, one staging of the j-list for them) where that still
+// gives every SM two blocks (152 SMs), else with 8 (one per warp), so that a few walks spread over the chip, and for
+// the smallest dispatches 4 warps with one i-particle each, so that every warp has an FP64 pipe (one per SM quarter)
+// to itself: a call of every functor on one walk of 180 particles 168 -> 152 us.
+struct Shape {
+    int ic, threads;
+    dim3 grid;
+    Shape(int n_walk, int64_t n_i, int max_i) {
+        ic = n_i >= 152 * 64 ? IC_MAX : (n_i > 152 * 4 ? W : 4);
+        threads = ic == 4 ? 128 : W * 32;
+        const int chunks = (max_i + ic - 1) / ic;
+        grid = dim3((unsigned)n_walk, (unsigned)(chunks > 0 ? (chunks < 4096 ? chunks : 4096) : 1));
+    }
+};
 
 }  // namespace
 
 void batch64_dens(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_dens *epi,
                   JSrc<sph_epj_dens> epj, sph_result_dens *res) {
-    const int ic = block_i(n_i);
-    k_walk_dens64<<<walk_grid(n_walk, max_i, ic), W * 32, 0, st>>>(meta, ic, epi, epj, res);
+    const Shape s(n_walk, n_i, max_i);
+    k_walk_dens64<<<s.grid, s.threads, 0, st>>>(meta, s.ic, epi, epj, res);
 }
 void batch64_drvt(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_drvt *epi,
                   JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
-    const int ic = block_i(n_i);
-    k_walk_drvt64<<<walk_grid(n_walk, max_i, ic), W * 32, 0, st>>>(meta, ic, epi, epj, res);
+    const Shape s(n_walk, n_i, max_i);
+    k_walk_drvt64<<<s.grid, s.threads, 0, st>>>(meta, s.ic, epi, epj, res);
 }
 void batch64_hydro(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_hydro *epi,
                    JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
-    const int ic = block_i(n_i);
-    k_walk_hydro64<<<walk_grid(n_walk, max_i, ic), W * 32, 0, st>>>(meta, ic, epi, epj, res);
+    const Shape s(n_walk, n_i, max_i);
+    k_walk_hydro64<<<s.grid, s.threads, 0, st>>>(meta, s.ic, epi, epj, res);
 }
 void batch64_grav(int n_walk, int64_t n_i, int max_i, cudaStream_t st, const int64_t *meta, const sph_epi_grav *epi,
                   JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj, sph_result_grav *res) {
-    const int ic = block_i(n_i);
-    k_walk_grav64<<<walk_grid(n_walk, max_i, ic), W * 32, 0, st>>>(meta, ic, epi, epj, spj, res);
+    const Shape s(n_walk, n_i, max_i);
+    k_walk_grav64<<<s.grid, s.threads, 0, st>>>(meta, s.ic, epi, epj, spj, res);
 }
 
 }  // namespace sph
