@@ -882,6 +882,7 @@ __global__ void __launch_bounds__(GT) k_grav32(const int *__restrict__ group_cel
 // and tiles of 256 1.96 ms, 1,024 and 1,024 2.09 ms, 2,048 and 1,024 at three
 // blocks per SM 2.00 ms).  More independent blocks let one block's walk
 // overlap another's sums.
+constexpr int GRAV_ONE = 8;   // groups per SM below which a block takes one of a thread's two i-particles
 template <int T>
 struct GravShape;
 template <>
@@ -933,7 +934,12 @@ __device__ __forceinline__ void grav_acc2(f32x2 nx, f32x2 ny, f32x2 nz, f32x2 e2
     a3 = f2_add(a3, mri);
 }
 
-template <int GF_T>
+// NU: of a thread's two i-particles, both, or (small runs, whose groups do not fill the chip) one, the block's
+// blockIdx.y saying which: the partitions and so the bits are the same, the sums take half as long and the walk is done
+// twice.  Lists and sums, both against one: 137 -> 109 us at 3,000 particles, 152 -> 116 at 5,000, 189 -> 141 at 10,000,
+// 193 -> 175 at 40,000; 370 -> 339 at 100,000, but 278 -> 282 at 70,000 and from 150,000 on a loss (405 -> 432, 447 -> 514
+// at 200,000).  The line of 8 groups per SM (1,216; near 50,000 particles) lies where the gain ends for good or ill.
+template <int GF_T, int NU>
 __global__ void __launch_bounds__(GF_T, GravShape<GF_T>::MIN_BLOCKS)
 k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinfo, const double4 *__restrict__ com,
                const double *__restrict__ rb_all, const int *__restrict__ prun, const double *__restrict__ x,
@@ -1004,6 +1010,7 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
     // (octants k and k + 4); appends go cell by cell, first children before second children
     const int q = tid >> 2, k = tid & 3, qw = lane >> 2;
     const unsigned cellm = 0xFu << (qw * 4), before = (1u << (qw * 4)) - 1u;
+    const int u0 = NU == 1 ? blockIdx.y : 0;
     int tot_e = 0, tot_s = 0;
     for (int i_base = 0; i_base < cnt_all; i_base += 2 * GF_T) {
         const int cnt = min(2 * GF_T, cnt_all - i_base);
@@ -1015,9 +1022,9 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
         const int TE = GF_TILE / (4 * P) * (4 * P);   // tile entries: a multiple of every partition's stride
         const int part = tid / Wt, ii = tid - part * Wt;
         const bool slot = part < P;
-        float px[2], py[2], pz[2], e2[2];
-        for (int u = 0; u < 2; ++u) {
-            const int iu = ii + u * Wt;
+        float px[NU], py[NU], pz[NU], e2[NU];
+        for (int u = 0; u < NU; ++u) {
+            const int iu = ii + (u0 + u) * Wt;
             px[u] = py[u] = pz[u] = 0.f;
             e2[u] = 1.f;
             if (slot && iu < cnt) {
@@ -1030,7 +1037,9 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
                 e2[u] = (float)(hh * hh);
             }
         }
-        float Dh[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, Dl[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+        float Dh[NU][4], Dl[NU][4];
+        for (int u = 0; u < NU; ++u)
+            for (int c4 = 0; c4 < 4; ++c4) Dh[u][c4] = Dl[u][c4] = 0.0f;
         int head = 0, tail = 1, it = 0;
         if (tid == 0) s_q[0] = cinfo[root];   // the run's root, level 0
         __syncthreads();
@@ -1198,14 +1207,16 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
                     if (slot) {
                         const int step = 4 * P;
                         const int tnr = (min(TE, nl - t0) + step - 1) / step * step;   // <= TE: step divides it
-                        f32x2 A[2][4] = {{0ull, 0ull, 0ull, 0ull}, {0ull, 0ull, 0ull, 0ull}};
+                        f32x2 A[NU][4];
+                        for (int u = 0; u < NU; ++u)
+                            for (int c4 = 0; c4 < 4; ++c4) A[u][c4] = 0ull;
                         for (int t = 4 * part; t < tnr; t += step) {
                             const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(s_tx + t);
                             const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(s_ty + t);
                             const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(s_tz + t);
                             const ulonglong2 M = *reinterpret_cast<const ulonglong2 *>(s_tm + t);
 #pragma unroll
-                            for (int u = 0; u < 2; ++u) {
+                            for (int u = 0; u < NU; ++u) {
                                 const f32x2 nx = f2_pack(-px[u], -px[u]), ny = f2_pack(-py[u], -py[u]),
                                             nz = f2_pack(-pz[u], -pz[u]), ee = f2_pack(e2[u], e2[u]);
                                 grav_acc2(nx, ny, nz, ee, X.x, Y.x, Z.x, M.x, A[u][0], A[u][1], A[u][2], A[u][3]);
@@ -1213,7 +1224,7 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
                             }
                         }
 #pragma unroll
-                        for (int u = 0; u < 2; ++u)
+                        for (int u = 0; u < NU; ++u)
                             for (int c4 = 0; c4 < 4; ++c4) {
                                 float lo, hi;
                                 f2_unpack(A[u][c4], lo, hi);
@@ -1229,10 +1240,10 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
         // GF_T x 4 doubles, in the tile or the EPJ buffer (whichever holds them; both are free here)
         double *red = 4 * GF_TILE * 4 >= GF_T * 4 * 8 ? reinterpret_cast<double *>(&s_tile[0][0])
                                                        : reinterpret_cast<double *>(s_e);
-        for (int u = 0; u < 2; ++u) {
+        for (int u = 0; u < NU; ++u) {
             for (int c4 = 0; c4 < 4; ++c4) red[c4 * GF_T + tid] = (double)Dh[u][c4] + (double)Dl[u][c4];
             __syncthreads();
-            const int iu = ii + u * Wt;
+            const int iu = ii + (u0 + u) * Wt;
             if (slot && part == 0 && iu < cnt) {
                 double r[4] = {0, 0, 0, 0};
                 for (int p2 = 0; p2 < P; ++p2)
@@ -1246,7 +1257,7 @@ k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinf
             __syncthreads();
         }
     }
-    if (tid == 0) {
+    if (tid == 0 && u0 == 0) {
         n_epj[blockIdx.x] = tot_e;   // of the first chunk of i when a group has more than 512 particles
         n_spj[blockIdx.x] = tot_s;
     }
@@ -1767,11 +1778,12 @@ int sph_gravity_fused(sph_ctx *ctx) {
     // group's forces and counts
     for (int wide = 0; wide < 2; ++wide) {
         SPH_CUDA(ctx, cudaMemsetAsync(t.meta + META_ERR, 0, sizeof(int), ctx->stream));
-        auto kern = wide ? k_grav_fused32<256> : k_grav_fused32<128>;
-        kern<<<G.ng, wide ? 256 : 128, 0, ctx->stream>>>(G.group_cell, t.cinfo, t.com, t.rb, ctx->runs.prun, CF(SPH_X),
-                                                         CF(SPH_Y), CF(SPH_Z), ctx->xh, ctx->xl, CF(SPH_SMTH), chp, clp,
-                                                         gms, CF(SPH_GX), CF(SPH_GY), CF(SPH_GZ), CF(SPH_POT), G.n_epj,
-                                                         G.n_spj, t.meta + META_ERR);
+        const bool one = !wide && G.ng < ctx->num_sms * GRAV_ONE;
+        auto kern = wide ? k_grav_fused32<256, 2> : (one ? k_grav_fused32<128, 1> : k_grav_fused32<128, 2>);
+        kern<<<dim3(G.ng, one ? 2 : 1), wide ? 256 : 128, 0, ctx->stream>>>(
+            G.group_cell, t.cinfo, t.com, t.rb, ctx->runs.prun, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), ctx->xh, ctx->xl,
+            CF(SPH_SMTH), chp, clp, gms, CF(SPH_GX), CF(SPH_GY), CF(SPH_GZ), CF(SPH_POT), G.n_epj, G.n_spj,
+            t.meta + META_ERR);
         ++ctx->launches;
         SPH_CUDA(ctx, cudaGetLastError());
         SPH_CUDA(ctx, cudaMemcpyAsync(hs, t.meta + META_ERR, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
