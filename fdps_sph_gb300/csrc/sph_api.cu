@@ -307,7 +307,6 @@ int compute_forces(sph_ctx *ctx) {
     // final from here on: positions, half-step velocities and energies (kick-drift, then sorted)
     SPH_TRY(dl_milestone(ctx, FB(SPH_X) | FB(SPH_Y) | FB(SPH_Z) | FB(SPH_VHX) | FB(SPH_VHY) | FB(SPH_VHZ) |
                                   FB(SPH_ENGHALF)));
-    if (ctx->cfg.precision == SPH_PREC_MIXED) SPH_TRY(sph_pack_mixed(ctx));
     SPH_TRY(time_mark(ctx, SEG_NBR_PREP));
     if (ctx->cfg.precision == SPH_PREC_MIXED) {
         // all passes straight from the superset, with the same neighbour decisions as the exact list
@@ -631,6 +630,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
     for (int k = 0; k < 64; ++k) cudaEventCreate(&ctx->ev[k]);
     for (int k = 0; k < 8; ++k) cudaEventCreateWithFlags(&ctx->dl_ev[k], cudaEventDisableTiming);
     cudaEventCreate(&ctx->ev_begin);
+    cudaEventCreateWithFlags(&ctx->tree_done, cudaEventDisableTiming);
     cudaEventCreate(&ctx->ev_end);
     if (cudaMalloc((void **)&ctx->mats_dev, sizeof(ctx->mats_host)) != cudaSuccess ||
         cudaMalloc((void **)&ctx->scratch_d, sizeof(double) * 8192) != cudaSuccess ||
@@ -659,7 +659,7 @@ int sph_ctx_destroy(sph_ctx *ctx) {
                     ctx->tree.tmp_cnt, ctx->tree.tmp_off, ctx->tree.tmp_b, ctx->tree.meta, ctx->tree.rb,
                     ctx->sort.k0, ctx->sort.k1, ctx->sort.v0, ctx->sort.v1, ctx->sort.hist, ctx->sort.hoff,
                     ctx->lists[0].nbr, ctx->lists[0].cnt, ctx->lists[1].nbr, ctx->lists[1].cnt,
-                    ctx->grav.group_cell, ctx->grav.is_group, ctx->grav.n_epj, ctx->grav.n_spj, ctx->grav.off_epj,
+                    ctx->grav.group_cell, ctx->grav.n_epj, ctx->grav.n_spj, ctx->grav.off_epj,
                     ctx->grav.off_spj, ctx->grav.epj, ctx->grav.spj, ctx->scan.part, ctx->scan.total,
                     ctx->sup.nbr, ctx->sup.cnt, ctx->sup.hsup, ctx->sup.pxh, ctx->sup.pxl, ctx->sup.H2f,
                     ctx->sup.units, ctx->tree.cinfo, ctx->sup.r2, ctx->sup.m, ctx->sup.vR, ctx->sup.cvR,
@@ -676,6 +676,7 @@ int sph_ctx_destroy(sph_ctx *ctx) {
     for (int k = 0; k < 64; ++k)
         if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
     if (ctx->ev_begin) cudaEventDestroy(ctx->ev_begin);
+    if (ctx->tree_done) cudaEventDestroy(ctx->tree_done);
     if (ctx->ev_end) cudaEventDestroy(ctx->ev_end);
     for (int k = 0; k < 8; ++k)
         if (ctx->dl_ev[k]) cudaEventDestroy(ctx->dl_ev[k]);
@@ -1193,7 +1194,6 @@ int sph_run_pass(sph_ctx *ctx, int pass) {
     switch (pass) {
         case 0:
             SPH_TRY(sph_sort_and_build(ctx));
-            if (ctx->cfg.precision == SPH_PREC_MIXED) SPH_TRY(sph_pack_mixed(ctx));
             break;
         case 1: SPH_TRY(sph_pass_density(ctx, 1)); break;
         case 2: SPH_TRY(sph_pass_eos(ctx)); break;

@@ -172,10 +172,11 @@ struct DevMaterial {
 // meta[MAX_LEVELS] = total cells, META_ERR = error bits.
 constexpr int META_N = 64;
 constexpr int META_ERR = 40;
-constexpr int META_NGROUP = 41;
-constexpr int META_MAXCNT = 42;   // max SPH neighbour count seen by the last list build
+constexpr int META_MAXCNT = 41;   // max SPH neighbour count seen by the last list build
 constexpr int META_NEPJ = 43;     // total gravity EPJ entries
 constexpr int META_NSPJ = 44;     // total gravity SPJ entries
+constexpr int META_ROLES = 46;    // (an aligned pair) walk units, gravity groups of the tree
+constexpr int UNIT = 32;          // particles of a walk unit at most
 
 struct Tree {
     int64_t cap = 0;
@@ -215,7 +216,6 @@ struct SphLists {
 struct GravLists {
     int64_t cap_groups = 0, cap_epj = 0, cap_spj = 0;
     int *group_cell = nullptr;   // [ng]
-    int *is_group = nullptr;     // [cell cap] scratch
     int *n_epj = nullptr, *n_spj = nullptr;          // [ng]
     int *off_epj = nullptr, *off_spj = nullptr;      // [ng]
     int *epj = nullptr, *spj = nullptr;
@@ -268,7 +268,7 @@ struct SphSuper {
 };
 
 struct Scan {
-    int *part = nullptr;   // [SCAN_BLOCKS + 1]
+    int *part = nullptr;   // [2 SCAN_BLOCKS]: parts of 32 or 64 bits
     int *total = nullptr;  // device int
 };
 
@@ -304,7 +304,7 @@ struct Runs {
 }  // namespace sph
 
 namespace sph {
-constexpr int GRAPH_KEY_N = 22;
+constexpr int GRAPH_KEY_N = 25;
 // a captured sort + octree build and what it was captured for
 struct TreeGraph {
     cudaGraphExec_t exec = nullptr;
@@ -370,6 +370,7 @@ struct sph_ctx {
     int64_t seg_calls[16] = {0};
     bool timing = false;
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
+    cudaEvent_t tree_done = nullptr;   // the tree's counts are on the host
 
     int64_t launches = 0;   // kernels launched by this context
 
@@ -422,7 +423,7 @@ int sph_tree_refresh_hmax(sph_ctx *ctx);       // cell hmax after h changed
 int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev, int len_host, int *total_dev);
 
 // lists (sph_nbr.cu, sph_lists.cu)
-int sph_nbr_prepare(sph_ctx *ctx);       // after the sort
+int sph_nbr_prepare(sph_ctx *ctx);       // after the sort (also packs the mixed path's records)
 int sph_nbr_refresh_h(sph_ctx *ctx);     // after h changed
 int sph_build_sph_lists(sph_ctx *ctx, int mode);
 int sph_density_from_superset(sph_ctx *ctx);
@@ -433,7 +434,6 @@ int dl_milestone(sph_ctx *ctx, uint64_t final_fields);   // sph_step_download: s
 int sph_runs_layout(sph_ctx *ctx);        // offsets and tiles of the runs after a change of the run set
 int sph_run_reduce_dt(sph_ctx *ctx);      // per-run min dt into runs.dt_dev and runs.dt
 int sph_run_diag(sph_ctx *ctx, double *out);   // per-run conserved quantities, out[R * 8]
-int sph_build_grav_groups(sph_ctx *ctx);   // gravity i-groups (cells with <= n_group particles)
 int sph_build_grav_lists(sph_ctx *ctx);
 int sph_gravity_fused(sph_ctx *ctx);       // mixed precision: walk + force in one kernel
 

@@ -19,30 +19,7 @@ constexpr unsigned FULL = 0xffffffffu;
 
 
 // --------------------------------------------------------------------------
-// gravity i-groups and interaction lists
-
-__global__ void k_mark_groups(const int *meta, const int *count, const int *parent, int n_group, int *is_group) {
-    const int nc = meta[MAX_LEVELS];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int p = parent[c];
-        is_group[c] = (count[c] <= n_group && (p < 0 || count[p] > n_group)) ? 1 : 0;
-    }
-    // cells that are leaves but still above n_group (only possible at the deepest level) are groups too
-}
-
-__global__ void k_mark_groups_fix(const int *meta, const int *count, const int *parent, const int *n_child,
-                                  int n_group, int *is_group) {
-    const int nc = meta[MAX_LEVELS];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        if (n_child[c] == 0 && count[c] > n_group) is_group[c] = 1;
-    }
-}
-
-__global__ void k_compact_groups(const int *meta, const int *is_group, const int *off, int *group_cell) {
-    const int nc = meta[MAX_LEVELS];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
-        if (is_group[c]) group_cell[off[c]] = c;
-}
+// interaction lists of the gravity i-groups (found with the tree)
 
 constexpr int GL_T = 128;      // threads per block: one i-group
 constexpr int GLCAP = 2048;    // ring buffer of opened cells (power of two)
@@ -226,35 +203,7 @@ static int dalloc_l(sph_ctx *ctx, T **p, int64_t n) {
     return SPH_OK;
 }
 
-int sph_build_grav_groups(sph_ctx *ctx) {
-    GravLists &G = ctx->grav;
-    Tree &t = ctx->tree;
-    const int nc = t.n_cell_host;
-    const int grid = 2 * ctx->num_sms;
-    cudaStream_t st = ctx->stream;
-    k_mark_groups<<<grid, 256, 0, st>>>(t.meta, t.count, t.parent, ctx->cfg.n_group, G.is_group); ++ctx->launches;
-    k_mark_groups_fix<<<grid, 256, 0, st>>>(t.meta, t.count, t.parent, t.n_child, ctx->cfg.n_group, G.is_group); ++ctx->launches;
-    SPH_TRY(sph_scan_exclusive(ctx, G.is_group, t.tmp_off, nullptr, nc, t.meta + META_NGROUP));
-    if (G.cap_groups < nc) {
-        const int64_t c = nc + nc / 4 + 64;
-        SPH_TRY(dalloc_l(ctx, &G.group_cell, c));
-        SPH_TRY(dalloc_l(ctx, &G.n_epj, c + 1));
-        SPH_TRY(dalloc_l(ctx, &G.n_spj, c + 1));
-        SPH_TRY(dalloc_l(ctx, &G.off_epj, c + 1));
-        SPH_TRY(dalloc_l(ctx, &G.off_spj, c + 1));
-        G.cap_groups = c;
-    }
-    k_compact_groups<<<grid, 256, 0, st>>>(t.meta, G.is_group, t.tmp_off, G.group_cell); ++ctx->launches;
-    int *hs = (int *)ctx->host_scalars;
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs, t.meta + META_NGROUP, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaStreamSynchronize(st));
-    const int ng = hs[0];
-    G.ng = ng;
-    return SPH_OK;
-}
-
 int sph_build_grav_lists(sph_ctx *ctx) {
-    SPH_TRY(sph_build_grav_groups(ctx));
     GravLists &G = ctx->grav;
     Tree &t = ctx->tree;
     cudaStream_t st = ctx->stream;

@@ -29,7 +29,6 @@
 
 namespace sph {
 
-constexpr int UNIT = 32;
 constexpr float KAPPA = 1.06f;   // measured at 1M: 1.15 -> 13.7 ms, 1.10 -> 12.9, 1.06 -> 12.6, 1.03 -> 13.0 (repairs)
 // walk warps per block: one, so a block's SM slot is freed as soon as its walk unit is done (the
 // units' walks differ in length); 1M walk: 1.95 ms with four warps per block, 1.97 with two,
@@ -45,67 +44,6 @@ constexpr int NB_MULTI = 116;   // the stack may reach this with several cells e
 constexpr unsigned FULLM = 0xffffffffu;
 
 __device__ __forceinline__ float df_sub(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
-
-// ---------------------------------------------------------------------------
-// units
-
-// number of units contributed by cell c (see file comment); EMIT writes them at off[c]
-template <bool EMIT>
-__global__ void k_units(const int *meta, const int *start, const int *count, const int *first_child,
-                        const int *n_child, int *nunits, const int *off, int2 *units) {
-    const int nc = meta[MAX_LEVELS], n_roots = meta[1];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int cnt = count[c], nch = n_child[c];
-        const bool root = c < n_roots;   // level 0: one root per run
-        int k = 0;
-        int2 *out = EMIT ? units + off[c] : nullptr;
-        if (root && cnt <= UNIT) {
-            if (EMIT) out[k] = make_int2(start[c], cnt);
-            ++k;
-        } else if (root && nch == 0) {
-            for (int s = 0; s < cnt; s += UNIT) {
-                if (EMIT) out[k] = make_int2(start[c] + s, min(UNIT, cnt - s));
-                ++k;
-            }
-        } else if (cnt > UNIT && nch > 0) {
-            const int f = first_child[c];
-            int us = -1, un = 0;
-            for (int q = 0; q < nch; ++q) {
-                const int ch = f + q, cc = count[ch];
-                if (cc <= UNIT) {
-                    if (us >= 0 && un + cc <= UNIT) {
-                        un += cc;
-                    } else {
-                        if (us >= 0) {
-                            if (EMIT) out[k] = make_int2(us, un);
-                            ++k;
-                        }
-                        us = start[ch];
-                        un = cc;
-                    }
-                } else {
-                    if (us >= 0) {
-                        if (EMIT) out[k] = make_int2(us, un);
-                        ++k;
-                    }
-                    us = -1;
-                    un = 0;
-                    if (n_child[ch] == 0) {   // a leaf above the unit size (only at the deepest level)
-                        for (int s = 0; s < cc; s += UNIT) {
-                            if (EMIT) out[k] = make_int2(start[ch] + s, min(UNIT, cc - s));
-                            ++k;
-                        }
-                    }
-                }
-            }
-            if (us >= 0) {
-                if (EMIT) out[k] = make_int2(us, un);
-                ++k;
-            }
-        }
-        if (!EMIT) nunits[c] = k;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // superset walk: one warp per unit
@@ -945,7 +883,7 @@ int sph_nbr_refresh_h(sph_ctx *ctx) {
     return SPH_OK;
 }
 
-// after the sort: positions as double-float, units, and the superset marked stale
+// after the sort: positions as double-float, h as float, and the superset marked stale
 int sph_nbr_prepare(sph_ctx *ctx) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
@@ -960,43 +898,20 @@ int sph_nbr_prepare(sph_ctx *ctx) {
         SPH_TRY(dalloc_n(ctx, &S.npass, pitch));
         S.cap_particles = pitch;
     }
+    if (S.cap_cells < ctx->tree.cap) {
+        S.cap_cells = ctx->tree.cap;
+        SPH_TRY(dalloc_n(ctx, &S.cvR, S.cap_cells));
+    }
     const int64_t cap = ctx->cap;
-    if (ctx->cfg.precision != SPH_PREC_MIXED) {   // the mixed path walks on sph_pack_mixed's packs
+    if (ctx->cfg.precision == SPH_PREC_MIXED) {   // the mixed path walks on its own packs
+        SPH_TRY(sph_pack_mixed(ctx));
+    } else {
         k_pack_pos<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
                                                                 FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap),
                                                                 ctx->mscale, S.pxh, S.pxl);
         ++ctx->launches;
     }
     SPH_TRY(sph_nbr_refresh_h(ctx));
-    // units
-    Tree &t = ctx->tree;
-    const int nc = t.n_cell_host;
-    const int grid = 2 * ctx->num_sms;
-    k_units<false><<<grid, 256, 0, ctx->stream>>>(t.meta, t.start, t.count, t.first_child, t.n_child, t.tmp_cnt,
-                                                  nullptr, nullptr);
-    ++ctx->launches;
-    SPH_TRY(sph_scan_exclusive(ctx, t.tmp_cnt, t.tmp_off, nullptr, nc, ctx->scan.total));
-    int tot = 0;
-    SPH_CUDA(ctx, cudaMemcpyAsync(&ctx->host_scalars[0], ctx->scan.total, sizeof(int), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
-    SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    std::memcpy(&tot, &ctx->host_scalars[0], sizeof(int));
-    if (S.cap_units < tot) {
-        S.cap_units = tot + tot / 4 + 64;
-        SPH_TRY(dalloc_n(ctx, &S.units, S.cap_units));
-        SPH_TRY(dalloc_n(ctx, &S.umark, S.cap_units));
-        SPH_TRY(dalloc_n(ctx, &S.uoff, S.cap_units));
-        SPH_TRY(dalloc_n(ctx, &S.uidx, S.cap_units));
-    }
-    if (S.cap_cells < t.cap) {
-        S.cap_cells = t.cap;
-        SPH_TRY(dalloc_n(ctx, &S.cvR, S.cap_cells));
-    }
-    k_units<true><<<grid, 256, 0, ctx->stream>>>(t.meta, t.start, t.count, t.first_child, t.n_child, nullptr,
-                                                 t.tmp_off, S.units);
-    ++ctx->launches;
-    SPH_CUDA(ctx, cudaGetLastError());
-    S.n_units = tot;
     S.valid = false;
     S.rebuilds_step = 0;
     ctx->lists[0].valid = ctx->lists[1].valid = false;
@@ -1042,8 +957,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
             S.K_alloc = S.K;
             S.spill_alloc = S.spill_cap;
         }
-        SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR, 0, sizeof(int), ctx->stream));
-        SPH_CUDA(ctx, cudaMemsetAsync(meta + META_MAXCNT, 0, sizeof(int), ctx->stream));
+        static_assert(META_MAXCNT == META_ERR + 1, "cleared together");
+        SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR, 0, 2 * sizeof(int), ctx->stream));
         // A warp walks a unit, or two or four share it: the walk of a small run is the latency of one warp's chain
         // (depth-first steps, candidates, accepted entries), and more and shorter chains fill the chip.  Rows do not
         // depend on the split, and units stay the units of the skin repairs.  Walk of 5,000 / 10,000 particles by

@@ -1762,7 +1762,6 @@ int sph_work_counts(sph_ctx *ctx, int64_t out[8]) {
 
 // mixed-precision gravity with the walk fused into the force kernel
 int sph_gravity_fused(sph_ctx *ctx) {
-    SPH_TRY(sph_build_grav_groups(ctx));
     GravLists &G = ctx->grav;
     Tree &t = ctx->tree;
     if (G.ng == 0) return SPH_OK;

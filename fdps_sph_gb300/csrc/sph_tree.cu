@@ -25,25 +25,27 @@ namespace sph {
 constexpr int SCAN_BLOCKS = 256;
 constexpr int SCAN_THREADS = 256;
 
-__device__ __forceinline__ int warp_incl_scan(int v) {
+template <class T>
+__device__ __forceinline__ T warp_incl_scan(T v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        const T t = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += t;
     }
     return v;
 }
 
 // inclusive block scan for blockDim.x <= 1024; returns inclusive value, *total = block sum
-__device__ int block_incl_scan(int v, int *total) {
-    __shared__ int ws[32];
+template <class T>
+__device__ T block_incl_scan(T v, T *total) {
+    __shared__ T ws[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    int x = warp_incl_scan(v);
+    T x = warp_incl_scan(v);
     if (lane == 31) ws[wid] = x;
     __syncthreads();
     if (wid == 0) {
-        int y = (lane < nw) ? ws[lane] : 0;
+        T y = (lane < nw) ? ws[lane] : 0;
         y = warp_incl_scan(y);
         if (lane < nw) ws[lane] = y;
     }
@@ -52,6 +54,17 @@ __device__ int block_incl_scan(int v, int *total) {
     *total = ws[nw - 1];
     __syncthreads();
     return x;
+}
+
+// the sum of the blocks' parts before this block's, the sum of all in *total (SCAN_BLOCKS == SCAN_THREADS)
+template <class T>
+__device__ T parts_before(const T *part, T *total) {
+    __shared__ T mine;
+    const T v = part[threadIdx.x];
+    const T x = block_incl_scan(v, total);
+    if (threadIdx.x == blockIdx.x) mine = x - v;
+    __syncthreads();
+    return mine;
 }
 
 __global__ void k_scan_reduce(const int *in, LenArg len, int *part) {
@@ -66,21 +79,14 @@ __global__ void k_scan_reduce(const int *in, LenArg len, int *part) {
     if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_part(int *part, int nb, int *total) {
-    const int t = threadIdx.x;
-    const int v = (t < nb) ? part[t] : 0;
-    int tot;
-    const int x = block_incl_scan(v, &tot);
-    if (t < nb) part[t] = x - v;
-    if (t == 0 && total) *total = tot;
-}
-
-__global__ void k_scan_down(const int *in, int *out, LenArg len, const int *part) {
+__global__ void k_scan_down(const int *in, int *out, LenArg len, const int *part, int *total) {
     const int n = len.get();
     const int chunk = (n + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * chunk;
     const int b1 = min(n, b0 + chunk);
-    int base = part[blockIdx.x];
+    int all;
+    int base = parts_before(part, &all);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && total) *total = all;
     for (int t0 = b0; t0 < b1; t0 += blockDim.x) {
         const int i = t0 + threadIdx.x;
         const int v = (i < b1) ? in[i] : 0;
@@ -95,12 +101,12 @@ __global__ void k_scan_down(const int *in, int *out, LenArg len, const int *part
 
 using namespace sph;
 
-// exclusive scan of int32; length from device (len_dev, if non-null) or host
+// exclusive scan of int32 in two launches (every block of the second sums the first's parts itself); length from
+// device (len_dev, if non-null) or host
 int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev, int len_host, int *total_dev) {
     LenArg L{len_dev, len_host, 0};
     k_scan_reduce<<<SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream>>>(in, L, ctx->scan.part); ++ctx->launches;
-    k_scan_part<<<1, SCAN_BLOCKS, 0, ctx->stream>>>(ctx->scan.part, SCAN_BLOCKS, total_dev); ++ctx->launches;
-    k_scan_down<<<SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream>>>(in, out, L, ctx->scan.part); ++ctx->launches;
+    k_scan_down<<<SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream>>>(in, out, L, ctx->scan.part, total_dev); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -720,11 +726,108 @@ __global__ void k_moments_up(const int *meta, const double *x, const double *y, 
     }
 }
 
-__global__ void k_pack_cinfo(const int *meta, const int *first_child, const int *n_child, const int *start,
-                             const int *count, int4 *cinfo) {
-    const int nc = meta[MAX_LEVELS];
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
-        cinfo[c] = make_int4(first_child[c], n_child[c], start[c], count[c]);
+// ---------------------------------------------------------------------------
+// What a cell of the finished tree is to the passes: its packed record, the walk units it contributes (sph_nbr.cu) and
+// whether it is a gravity i-group: at most n_group particles under a parent (or as a root) with more, or a leaf of the
+// deepest level with more.  Counts and places come from one scan of both numbers in 64 bits (units low, groups high),
+// in the launch sequence of the tree and with its one read of totals.  Latency-bound like the whole tree of a small
+// run: as two passes of their own after the tree, with six launches and a read back to the host each, a step of 5,000
+// particles took 580 us, this way 523.
+
+// the walk units contributed by cell c; EMIT writes them to out
+template <bool EMIT>
+__device__ int cell_units(int c, int n_roots, int first, const int *start, int cnt, const int *count,
+                          const int *n_child, int nch, int2 *out) {
+    const bool root = c < n_roots;   // level 0: one root per run
+    int k = 0;
+    if (root && cnt <= UNIT) {
+        if (EMIT) out[k] = make_int2(start[c], cnt);
+        ++k;
+    } else if (root && nch == 0) {
+        for (int s = 0; s < cnt; s += UNIT) {
+            if (EMIT) out[k] = make_int2(start[c] + s, min(UNIT, cnt - s));
+            ++k;
+        }
+    } else if (cnt > UNIT && nch > 0) {
+        int us = -1, un = 0;
+        for (int q = 0; q < nch; ++q) {
+            const int ch = first + q, cc = count[ch];
+            if (cc <= UNIT) {
+                if (us >= 0 && un + cc <= UNIT) {
+                    un += cc;
+                } else {
+                    if (us >= 0) {
+                        if (EMIT) out[k] = make_int2(us, un);
+                        ++k;
+                    }
+                    us = start[ch];
+                    un = cc;
+                }
+            } else {
+                if (us >= 0) {
+                    if (EMIT) out[k] = make_int2(us, un);
+                    ++k;
+                }
+                us = -1;
+                un = 0;
+                if (n_child[ch] == 0) {   // a leaf above the unit size (only at the deepest level)
+                    for (int s = 0; s < cc; s += UNIT) {
+                        if (EMIT) out[k] = make_int2(start[ch] + s, min(UNIT, cc - s));
+                        ++k;
+                    }
+                }
+            }
+        }
+        if (us >= 0) {
+            if (EMIT) out[k] = make_int2(us, un);
+            ++k;
+        }
+    }
+    return k;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_cell_roles(const int *meta, int n_group, const int *start, const int *count, const int *first_child,
+             const int *n_child, const int *parent, int4 *cinfo, long long *role, long long *part) {
+    const int nc = meta[MAX_LEVELS], n_roots = meta[1];
+    const int chunk = (nc + gridDim.x - 1) / gridDim.x;
+    const int b1 = min(nc, (int)(blockIdx.x + 1) * chunk);
+    long long sum = 0;
+    for (int c = blockIdx.x * chunk + threadIdx.x; c < b1; c += blockDim.x) {
+        const int cnt = count[c], nch = n_child[c], f = first_child[c], p = parent[c];
+        cinfo[c] = make_int4(f, nch, start[c], cnt);
+        const bool group = cnt <= n_group ? (p < 0 || count[p] > n_group) : nch == 0;
+        const int k = cell_units<false>(c, n_roots, f, start, cnt, count, n_child, nch, nullptr);
+        const long long v = (long long)k | (long long)group << 32;
+        role[c] = v;
+        sum += v;
+    }
+    long long tot;
+    block_incl_scan(sum, &tot);
+    if (threadIdx.x == 0) part[blockIdx.x] = tot;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_role_emit(const int *meta, const int4 *cinfo, const int *start, const int *count, const int *n_child,
+            const long long *role, const long long *part, int2 *units, int *group_cell, long long *total) {
+    const int nc = meta[MAX_LEVELS], n_roots = meta[1];
+    const int chunk = (nc + gridDim.x - 1) / gridDim.x;
+    const int b0 = blockIdx.x * chunk, b1 = min(nc, b0 + chunk);
+    long long all;
+    long long base = parts_before(part, &all);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *total = all;
+    for (int t0 = b0; t0 < b1; t0 += blockDim.x) {
+        const int c = t0 + threadIdx.x;
+        const long long v = c < b1 ? role[c] : 0;
+        long long tot;
+        const long long at = base + block_incl_scan(v, &tot) - v;
+        if ((int)v) {
+            const int4 ci = cinfo[c];
+            cell_units<true>(c, n_roots, ci.x, start, ci.w, count, n_child, ci.y, units + (int)at);
+        }
+        if (v >> 32) group_cell[at >> 32] = c;
+        base += tot;
+    }
 }
 
 __global__ void k_hmax(int l, const int *meta, const double *h, const int *start, const int *count,
@@ -781,8 +884,26 @@ int sph_tree_reserve(sph_ctx *ctx, int64_t n) {
         SPH_TRY(dalloc(ctx, &t.tmp_off, c));
         SPH_TRY(dalloc(ctx, &t.tmp_b, 9 * c));
         SPH_TRY(dalloc(ctx, &t.cinfo, c));
-        SPH_TRY(dalloc(ctx, &ctx->grav.is_group, c));
         t.cap = c;
+    }
+    SphSuper &S = ctx->sup;
+    if (S.cap_units < n) {   // units and groups hold one particle or more each, and no particle twice
+        const int64_t c = n + n / 8 + 64;
+        SPH_TRY(dalloc(ctx, &S.units, c));
+        SPH_TRY(dalloc(ctx, &S.umark, c));
+        SPH_TRY(dalloc(ctx, &S.uoff, c));
+        SPH_TRY(dalloc(ctx, &S.uidx, c));
+        S.cap_units = c;
+    }
+    GravLists &G = ctx->grav;
+    if (G.cap_groups < n) {
+        const int64_t c = n + n / 8 + 64;
+        SPH_TRY(dalloc(ctx, &G.group_cell, c));
+        SPH_TRY(dalloc(ctx, &G.n_epj, c + 1));
+        SPH_TRY(dalloc(ctx, &G.n_spj, c + 1));
+        SPH_TRY(dalloc(ctx, &G.off_epj, c + 1));
+        SPH_TRY(dalloc(ctx, &G.off_spj, c + 1));
+        G.cap_groups = c;
     }
     if (!t.meta) SPH_TRY(dalloc(ctx, &t.meta, META_N));
     if (t.rb_cap < ctx->runs.cap_R) {
@@ -804,7 +925,7 @@ int sph_tree_reserve(sph_ctx *ctx, int64_t n) {
         s.nblocks_cap = ctx->runs.cap_T;
     }
     if (!ctx->scan.part) {
-        SPH_TRY(dalloc(ctx, &ctx->scan.part, SCAN_BLOCKS + 1));
+        SPH_TRY(dalloc(ctx, &ctx->scan.part, 2 * SCAN_BLOCKS));   // 32- or 64-bit parts
         SPH_TRY(dalloc(ctx, &ctx->scan.total, 16));
     }
     return SPH_OK;
@@ -837,7 +958,7 @@ static int radix_sort(sph_ctx *ctx, int n) {
 }
 
 // the octree over the sorted particles in one pass (k_cell_levels, a scan, k_cell_emit,
-// k_cell_link), then the moments bottom-up in one launch and the packed cell records
+// k_cell_link), then the cells' records and roles, then the moments bottom-up in one launch
 static int enqueue_tree(sph_ctx *ctx) {
     const int64_t cap = ctx->cap;
     const int n = (int)ctx->n;
@@ -855,14 +976,20 @@ static int enqueue_tree(sph_ctx *ctx) {
                                      t.tmp_b, t.meta, t.start, t.count, t.level); ++ctx->launches;
     k_cell_link<<<grid, 256, 0, st>>>(t.meta, t.start, t.count, t.level, t.parent, t.first_child, t.n_child);
     ++ctx->launches;
+    // packed records, walk units, gravity groups (tmp_b, free again, as 64-bit numbers)
+    static_assert(SCAN_BLOCKS == SCAN_THREADS, "parts_before");
+    long long *role = (long long *)t.tmp_b, *part = (long long *)ctx->scan.part;
+    k_cell_roles<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, ctx->cfg.n_group, t.start, t.count, t.first_child,
+                                                       t.n_child, t.parent, t.cinfo, role, part); ++ctx->launches;
+    k_role_emit<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, t.cinfo, t.start, t.count, t.n_child, role, part,
+                                                      ctx->sup.units, ctx->grav.group_cell,
+                                                      (long long *)(t.meta + META_ROLES)); ++ctx->launches;
     // moments bottom-up in one launch (tmp_cnt, free again, counts the arrivals)
     SPH_CUDA(ctx, cudaMemsetAsync(t.tmp_cnt, 0, sizeof(int) * t.cap, st));
     // one thread per cell: the leaves' fences and arrivals all in flight at once
     const int grid_up = (int)std::min<int64_t>((t.cap + 127) / 128, 1 << 16);
     k_moments_up<<<grid_up, 128, 0, st>>>(t.meta, x, y, z, m, h, t.start, t.count, t.first_child, t.n_child,
                                           t.parent, t.tmp_cnt, t.mom, t.com, t.blo, t.bhi); ++ctx->launches;
-    k_pack_cinfo<<<grid, 256, 0, st>>>(t.meta, t.first_child, t.n_child, t.start, t.count, t.cinfo);
-    ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -908,7 +1035,8 @@ static void graph_key(const sph_ctx *ctx, uintptr_t key[GRAPH_KEY_N]) {
         (uintptr_t)ctx->mat,       (uintptr_t)ctx->runs.prun,  (uintptr_t)ctx->keys,     (uintptr_t)ctx->sort.k0,
         (uintptr_t)ctx->sort.hist, (uintptr_t)t.start,         (uintptr_t)t.rb,          (uintptr_t)t.cap,
         (uintptr_t)ctx->runs.tiles, (uintptr_t)ctx->runs.part, (uintptr_t)ctx->scan.part, (uintptr_t)t.cinfo,
-        (uintptr_t)ctx->cfg.n_leaf, (uintptr_t)(ctx->runs.max_tiles > RS_DIRECT)};
+        (uintptr_t)ctx->cfg.n_leaf, (uintptr_t)(ctx->runs.max_tiles > RS_DIRECT), (uintptr_t)ctx->cfg.n_group,
+        (uintptr_t)ctx->sup.units, (uintptr_t)ctx->grav.group_cell};
     for (int i = 0; i < GRAPH_KEY_N; ++i) key[i] = k[i];
 }
 
@@ -970,10 +1098,13 @@ int sph_sort_and_build(sph_ctx *ctx) {
     // ~170 launches of the sort and the level loop replay as one CUDA graph.
     if (ctx->timing || !ctx->use_graphs) SPH_TRY(enqueue_sort_tree(ctx));
     else SPH_TRY(sort_tree_graph(ctx));
-    // bring back the cell count and the error word (one small synchronous read per tree)
+    SPH_TRY(time_mark(ctx, SEG_TREE));
+    // bring back the counts and the error word (one small synchronous read per tree); the packs run behind it
     int *hs = (int *)ctx->host_scalars;
     SPH_CUDA(ctx, cudaMemcpyAsync(hs, t.meta, sizeof(int) * META_N, cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaStreamSynchronize(st));
+    SPH_CUDA(ctx, cudaEventRecord(ctx->tree_done, st));
+    SPH_TRY(sph_nbr_prepare(ctx));
+    SPH_CUDA(ctx, cudaEventSynchronize(ctx->tree_done));
     if (hs[META_ERR] & ERR_NONFINITE) return sph_fail(ctx, SPH_ERR_NONFINITE, "non-finite particle position");
     if (hs[META_ERR] & ERR_CELL_OVERFLOW) return sph_fail(ctx, SPH_ERR_CAPACITY, "octree cell capacity exceeded");
     t.n_cell_host = hs[MAX_LEVELS];
@@ -981,10 +1112,11 @@ int sph_sort_and_build(sph_ctx *ctx) {
     for (int l = 0; l < MAX_LEVELS; ++l)
         if (hs[l + 1] > hs[l]) depth = l;
     t.depth = depth;
+    ctx->sup.n_units = hs[META_ROLES];
+    ctx->grav.ng = hs[META_ROLES + 1];
     ctx->grav.valid = false;
     ctx->grav.counts_valid = false;
-    SPH_TRY(time_mark(ctx, SEG_TREE));
-    return sph_nbr_prepare(ctx);
+    return SPH_OK;
 }
 
 int sph_tree_refresh_hmax(sph_ctx *ctx) {
