@@ -651,83 +651,99 @@ __global__ void k_cell_link(const int *meta, const int *start, const int *count,
     }
 }
 
-__device__ __forceinline__ double4 ldcg_d4(const double4 *p) {
-    const double2 *q = reinterpret_cast<const double2 *>(p);
-    const double2 a = __ldcg(q), b = __ldcg(q + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
-}
-
-// Moments, boxes and hmax of every cell in one launch, bottom-up.  A thread takes a leaf, then
-// climbs: after its cell is written it counts itself in at the parent (arrive[], zeroed before the
-// launch), and the child that arrives last sums the parent's children in octant order and climbs
-// on.  The sums and their order are those of a level-by-level pass (leaf particles ascending, then
-// children in octant order, one rounding per operation), independent of which thread arrives last;
-// no thread waits for another (a climb ends at the first parent with children still to come, or
-// at the root, after at most KEY_LEVELS steps).  Children written by other threads are read
+// Moments, boxes and hmax of every cell in one launch, bottom-up.  A thread takes a leaf; then the warp's lanes climb
+// together: after a cell is written its lane counts it in at the parent (arrive[], zeroed before the launch), and the
+// child that arrives last has its parent's children summed in octant order and climbs on.  The sums and their order are
+// those of a level-by-level pass (leaf particles ascending, then children in octant order, one rounding per operation),
+// independent of which lane arrives last; no lane waits for another warp (a climb ends at the first parent with
+// children still to come, or at the root, after at most KEY_LEVELS steps).  Children written by other threads are read
 // through L2 after the fence that orders them before their arrival.
-__global__ void k_moments_up(const int *meta, const double *x, const double *y, const double *z, const double *m,
-                             const double *h, const int *start, const int *count, const int *first_child,
-                             const int *n_child, const int *parent, int *arrive, double4 *mom, double4 *com,
-                             float4 *blo, float4 *bhi) {
-    const int nc = meta[MAX_LEVELS];
-    for (int c0 = blockIdx.x * blockDim.x + threadIdx.x; c0 < nc; c0 += gridDim.x * blockDim.x) {
-        if (n_child[c0] != 0) continue;
-        {
+//
+// Bound by the FP64 pipe (a warp instruction every 16 cycles and more per SM, however few lanes take part) and, in a
+// small run, by the chain of climbs.  So boxes and hmax are found on integer images and rounded once per leaf, not once
+// per particle; a climber's four sums run on four lanes, eight climbers at once (a quarter of the additions issued);
+// and the centres of mass are divided in k_cell_roles, by full warps.  The tree of 1M / 100,000 / 5,000
+// particles 437 / 123 / 90 -> 340 / 107 / 78 us.
+__global__ void __launch_bounds__(128)
+k_moments_up(const int *meta, const double *x, const double *y, const double *z, const double *m, const double *h,
+             const int *start, const int *count, const int *first_child, const int *n_child, const int *parent,
+             int *arrive, double4 *mom, float4 *blo, float4 *bhi) {
+    const int nc = meta[MAX_LEVELS], lane = threadIdx.x & 31, q = lane >> 2, comp = lane & 3;
+    for (int cw = blockIdx.x * blockDim.x + (threadIdx.x & ~31); cw < nc; cw += gridDim.x * blockDim.x) {
+        int c = cw + lane;
+        bool on = c < nc && n_child[c] == 0;
+        if (on) {
             double ms = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-            float hm = 0.0f;
-            const int s = start[c0], e = s + count[c0];
+            long long lo[3] = {LLONG_MAX, LLONG_MAX, LLONG_MAX}, hi[3] = {LLONG_MIN, LLONG_MIN, LLONG_MIN}, hm = 0;
+            const int s = start[c], e = s + count[c];
             for (int j = s; j < e; ++j) {
-                const double mj = m[j], xj = x[j], yj = y[j], zj = z[j];
+                const double mj = m[j], p[3] = {x[j], y[j], z[j]};
                 ms = __dadd_rn(ms, mj);
-                mx = __dadd_rn(mx, __dmul_rn(mj, xj));
-                my = __dadd_rn(my, __dmul_rn(mj, yj));
-                mz = __dadd_rn(mz, __dmul_rn(mj, zj));
-                lo[0] = fminf(lo[0], __double2float_rd(xj)); hi[0] = fmaxf(hi[0], __double2float_ru(xj));
-                lo[1] = fminf(lo[1], __double2float_rd(yj)); hi[1] = fmaxf(hi[1], __double2float_ru(yj));
-                lo[2] = fminf(lo[2], __double2float_rd(zj)); hi[2] = fmaxf(hi[2], __double2float_ru(zj));
-                hm = fmaxf(hm, __double2float_ru(h[j]));
+                mx = __dadd_rn(mx, __dmul_rn(mj, p[0]));
+                my = __dadd_rn(my, __dmul_rn(mj, p[1]));
+                mz = __dadd_rn(mz, __dmul_rn(mj, p[2]));
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const long long k = dorder_key(p[d]);
+                    lo[d] = min(lo[d], k);
+                    hi[d] = max(hi[d], k);
+                }
+                const long long hk = __double_as_longlong(h[j]);   // a positive double's order is its integer image's
+                if (hk <= __double_as_longlong((double)INFINITY)) hm = max(hm, hk);   // (as fmax: no NaN)
             }
-            mom[c0] = make_double4(mx, my, mz, ms);
-            com[c0] = make_double4(__ddiv_rn(mx, ms), __ddiv_rn(my, ms), __ddiv_rn(mz, ms), ms);
-            blo[c0] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-            bhi[c0] = make_float4(hi[0], hi[1], hi[2], hm);
+            mom[c] = make_double4(mx, my, mz, ms);
+            blo[c] = make_float4(__double2float_rd(dorder_value(lo[0])), __double2float_rd(dorder_value(lo[1])),
+                                 __double2float_rd(dorder_value(lo[2])), 0.0f);
+            bhi[c] = make_float4(__double2float_ru(dorder_value(hi[0])), __double2float_ru(dorder_value(hi[1])),
+                                 __double2float_ru(dorder_value(hi[2])), __double2float_ru(__longlong_as_double(hm)));
         }
-        int c = c0;
         for (int up = 0; up < KEY_LEVELS + 1; ++up) {
-            const int p = parent[c];
-            if (p < 0) break;
-            // release: this cell's moments before its arrival; acquire: every sibling's arrival (and
-            // so its moments) before the reads
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            if (atomicAdd(&arrive[p], 1) != n_child[p] - 1) break;
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            double ms = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
-            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-            float hm = 0.0f;
-            const int f = first_child[p], nch = n_child[p];
-            for (int k = 0; k < nch; ++k) {
-                const double4 q = ldcg_d4(mom + f + k);
-                ms = __dadd_rn(ms, q.w);
-                mx = __dadd_rn(mx, q.x);
-                my = __dadd_rn(my, q.y);
-                mz = __dadd_rn(mz, q.z);
-                const float4 a = __ldcg(blo + f + k), b = __ldcg(bhi + f + k);
-                lo[0] = fminf(lo[0], a.x); lo[1] = fminf(lo[1], a.y); lo[2] = fminf(lo[2], a.z);
-                hi[0] = fmaxf(hi[0], b.x); hi[1] = fmaxf(hi[1], b.y); hi[2] = fmaxf(hi[2], b.z);
-                hm = fmaxf(hm, b.w);
+            int p = -1, f = 0, nch = 0;
+            if (on) p = parent[c];
+            on = p >= 0;
+            if (on) {
+                f = first_child[p];
+                nch = n_child[p];
+                // release: this cell's moments (written by lanes of this warp, ordered by the barrier below) before its
+                // arrival; acquire: every sibling's arrival (and so its moments) before the reads
+                asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                on = atomicAdd(&arrive[p], 1) == nch - 1;
+                asm volatile("fence.acq_rel.gpu;" ::: "memory");
             }
-            mom[p] = make_double4(mx, my, mz, ms);
-            com[p] = make_double4(__ddiv_rn(mx, ms), __ddiv_rn(my, ms), __ddiv_rn(mz, ms), ms);
-            blo[p] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-            bhi[p] = make_float4(hi[0], hi[1], hi[2], hm);
+            unsigned left = __ballot_sync(0xffffffffu, on);
+            if (!left) break;
+            __syncwarp();   // the reads below follow the fences
             c = p;
+            while (left) {   // eight climbers at a time, four lanes each
+                unsigned rest = left;
+                for (int k = 0; k < q && rest; ++k) rest &= rest - 1;
+                const int src = rest ? __ffs(rest) - 1 : 0;
+                const int pp = __shfl_sync(0xffffffffu, p, src), ff = __shfl_sync(0xffffffffu, f, src),
+                          nn = __shfl_sync(0xffffffffu, nch, src);
+                if (rest) {
+                    const double *mq = reinterpret_cast<const double *>(mom + ff) + comp;
+                    double v = 0.0;
+                    for (int k = 0; k < nn; ++k) v = __dadd_rn(v, __ldcg(mq + 4 * k));
+                    reinterpret_cast<double *>(mom + pp)[comp] = v;
+                    float lo = INFINITY, hi = comp == 3 ? 0.0f : -INFINITY;
+                    const float *lq = reinterpret_cast<const float *>(blo + ff) + comp;
+                    const float *hq = reinterpret_cast<const float *>(bhi + ff) + comp;
+                    for (int k = 0; k < nn; ++k) {
+                        lo = fminf(lo, __ldcg(lq + 4 * k));
+                        hi = fmaxf(hi, __ldcg(hq + 4 * k));
+                    }
+                    reinterpret_cast<float *>(blo + pp)[comp] = comp == 3 ? 0.0f : lo;
+                    reinterpret_cast<float *>(bhi + pp)[comp] = hi;
+                }
+                for (int k = 0; k < 8 && left; ++k) left &= left - 1;
+            }
+            __syncwarp();
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// What a cell of the finished tree is to the passes: its packed record, the walk units it contributes (sph_nbr.cu) and
+// What a cell of the finished tree is to the passes: its packed record, its centre of mass, the walk units it contributes (sph_nbr.cu) and
 // whether it is a gravity i-group: at most n_group particles under a parent (or as a root) with more, or a leaf of the
 // deepest level with more.  Counts and places come from one scan of both numbers in 64 bits (units low, groups high),
 // in the launch sequence of the tree and with its one read of totals.  Latency-bound like the whole tree of a small
@@ -788,7 +804,8 @@ __device__ int cell_units(int c, int n_roots, int first, const int *start, int c
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_cell_roles(const int *meta, int n_group, const int *start, const int *count, const int *first_child,
-             const int *n_child, const int *parent, int4 *cinfo, long long *role, long long *part) {
+             const int *n_child, const int *parent, const double4 *mom, double4 *com, int4 *cinfo, long long *role,
+             long long *part) {
     const int nc = meta[MAX_LEVELS], n_roots = meta[1];
     const int chunk = (nc + gridDim.x - 1) / gridDim.x;
     const int b1 = min(nc, (int)(blockIdx.x + 1) * chunk);
@@ -796,6 +813,8 @@ k_cell_roles(const int *meta, int n_group, const int *start, const int *count, c
     for (int c = blockIdx.x * chunk + threadIdx.x; c < b1; c += blockDim.x) {
         const int cnt = count[c], nch = n_child[c], f = first_child[c], p = parent[c];
         cinfo[c] = make_int4(f, nch, start[c], cnt);
+        const double4 q = mom[c];
+        com[c] = make_double4(__ddiv_rn(q.x, q.w), __ddiv_rn(q.y, q.w), __ddiv_rn(q.z, q.w), q.w);
         const bool group = cnt <= n_group ? (p < 0 || count[p] > n_group) : nch == 0;
         const int k = cell_units<false>(c, n_roots, f, start, cnt, count, n_child, nch, nullptr);
         const long long v = (long long)k | (long long)group << 32;
@@ -958,7 +977,7 @@ static int radix_sort(sph_ctx *ctx, int n) {
 }
 
 // the octree over the sorted particles in one pass (k_cell_levels, a scan, k_cell_emit,
-// k_cell_link), then the cells' records and roles, then the moments bottom-up in one launch
+// k_cell_link), then the moments bottom-up in one launch, then the cells' records and roles
 static int enqueue_tree(sph_ctx *ctx) {
     const int64_t cap = ctx->cap;
     const int n = (int)ctx->n;
@@ -976,20 +995,21 @@ static int enqueue_tree(sph_ctx *ctx) {
                                      t.tmp_b, t.meta, t.start, t.count, t.level); ++ctx->launches;
     k_cell_link<<<grid, 256, 0, st>>>(t.meta, t.start, t.count, t.level, t.parent, t.first_child, t.n_child);
     ++ctx->launches;
-    // packed records, walk units, gravity groups (tmp_b, free again, as 64-bit numbers)
-    static_assert(SCAN_BLOCKS == SCAN_THREADS, "parts_before");
-    long long *role = (long long *)t.tmp_b, *part = (long long *)ctx->scan.part;
-    k_cell_roles<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, ctx->cfg.n_group, t.start, t.count, t.first_child,
-                                                       t.n_child, t.parent, t.cinfo, role, part); ++ctx->launches;
-    k_role_emit<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, t.cinfo, t.start, t.count, t.n_child, role, part,
-                                                      ctx->sup.units, ctx->grav.group_cell,
-                                                      (long long *)(t.meta + META_ROLES)); ++ctx->launches;
     // moments bottom-up in one launch (tmp_cnt, free again, counts the arrivals)
     SPH_CUDA(ctx, cudaMemsetAsync(t.tmp_cnt, 0, sizeof(int) * t.cap, st));
     // one thread per cell: the leaves' fences and arrivals all in flight at once
     const int grid_up = (int)std::min<int64_t>((t.cap + 127) / 128, 1 << 16);
     k_moments_up<<<grid_up, 128, 0, st>>>(t.meta, x, y, z, m, h, t.start, t.count, t.first_child, t.n_child,
-                                          t.parent, t.tmp_cnt, t.mom, t.com, t.blo, t.bhi); ++ctx->launches;
+                                          t.parent, t.tmp_cnt, t.mom, t.blo, t.bhi); ++ctx->launches;
+    // packed records, centres of mass, walk units, gravity groups (tmp_b, free again, as 64-bit numbers)
+    static_assert(SCAN_BLOCKS == SCAN_THREADS, "parts_before");
+    long long *role = (long long *)t.tmp_b, *part = (long long *)ctx->scan.part;
+    k_cell_roles<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, ctx->cfg.n_group, t.start, t.count, t.first_child,
+                                                       t.n_child, t.parent, t.mom, t.com, t.cinfo, role,
+                                                       part); ++ctx->launches;
+    k_role_emit<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, t.cinfo, t.start, t.count, t.n_child, role, part,
+                                                      ctx->sup.units, ctx->grav.group_cell,
+                                                      (long long *)(t.meta + META_ROLES)); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
