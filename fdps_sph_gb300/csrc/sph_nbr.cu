@@ -37,8 +37,8 @@ constexpr int NB_WARPS = 1;
 constexpr int WALK_SMALL = 100, WALK_MID = 330;   // particles per SM below which 4 / 2 warps walk a unit
 constexpr int DENS_SMALL = 200;   // particles per SM below which the density takes 8 threads per particle
 constexpr int ROW_K_MAX = 512;   // widest row block; longer rows continue in spill ranges (RowMap)
-constexpr int NB_CAND = 256;   // raw candidate indices per warp (flushes half as often as with 128: -0.02 ms at 1M)
-constexpr int NB_SURV = 64;    // culled candidates staged for the pair test
+constexpr int NB_SURV = 64;    // ring of culled candidates staged for the pair test
+constexpr int NB_FREE = 16;    // stack entries beyond NB_STACK: room for the accepted entries of a batch at any depth
 constexpr int NB_STACK = 264;   // depth-first from any stack of <= NB_MULTI entries: + 21 levels x 7 pending siblings + 1
 constexpr int NB_MULTI = 116;   // the stack may reach this with several cells expanded at once
 constexpr unsigned FULLM = 0xffffffffu;
@@ -60,6 +60,12 @@ __device__ __forceinline__ float gap2_rd(float4 a_lo, float4 a_hi, float3 glo, f
     return __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz));
 }
 
+// Bound by instruction issue (about three a cycle per SM with 32 one-warp blocks), so what is left is what the tests
+// need: a step of the walk takes up to 32 leaves or four inner cells from one read of the stack's top, a candidate's
+// place comes from a scan and a vote, pairs are tested two per instruction in full batches of 32 survivors, and an
+// accepted pair's owner and survivor are read from a list that the lanes wrote instead of searched for.  1M particles:
+// 1.71 -> 1.08 billion instructions, 1.92 -> 1.42 ms (the searches, leaves eight at a time by a loop, and tests one by
+// one before); 100,000 0.32 -> 0.25 ms, 5,000 124 -> 109 us.
 // SPILL: rows may continue in spill ranges (walks after this step's spill layout); without it
 // the hot loop carries no spill code (a row longer than K only raises the overflow flag)
 template <bool SPILL>
@@ -72,12 +78,10 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
            float *__restrict__ sup_r2, float *__restrict__ sup_m, int *__restrict__ cnt, RowMap rm, int *uover,
            int *err, int *maxcnt) {
     // cells to visit: (first_child, -n_child) for an internal cell, (start, count) for a leaf
-    __shared__ int2 s_stack[NB_WARPS][NB_STACK];
-    __shared__ int s_cand[NB_WARPS][NB_CAND];
-    // candidates that survived the per-particle cull: index, hi, lo (.w = (2.5 h_j)^2 rounded up)
+    __shared__ int2 s_stack[NB_WARPS][NB_STACK + NB_FREE];
+    // candidates that survived the per-particle cull: index; hi x, y, z, mass, lo x, y, z, kappa'^2 (2.5 h_j)^2
     __shared__ int s_sj[NB_WARPS][NB_SURV];
-    __shared__ float4 s_ph[NB_WARPS][NB_SURV];
-    __shared__ float4 s_pl[NB_WARPS][NB_SURV];
+    __shared__ __align__(16) float s_sv[NB_WARPS][8][NB_SURV];
     // every lane's double-float position, for the lanes that write another lane's entries
     __shared__ float4 s_pih[NB_WARPS][32], s_pil[NB_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -115,8 +119,11 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
     const float Rg2 = __fmul_ru(Rg, Rg);
     const unsigned lt = (1u << lane) - 1u;
     int2 *stack = s_stack[warp];
-    int *cand = s_cand[warp];
-    int count = 0, nc = 0;
+    int *sj = s_sj[warp];
+    float(*sv)[NB_SURV] = s_sv[warp];
+    int count = 0;         // accepted entries of this lane's row
+    int wr = 0, rd = 0;    // staged survivors, tested ones (a multiple of 32)
+    int sp = 0;            // cells on the stack
     // the spill range continues a row at entry K: entry k >= K of particle p at
     // rm.main + rm.soff[p] - K + k (computed on the rare paths that need it)
     auto spill_cap = [&]() { return valid ? row_spill_cap(rm, i) : 0; };
@@ -124,134 +131,125 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
     s_pil[warp][lane] = pil;
     __syncwarp();
 
-    // Candidates are culled 32 at a time, each against the unit's box grown by its own reach:
-    // a lower bound of the distance (the point's hi / lo interval, rounded down) against an
-    // upper bound of max(Rg, kappa' 2.5 h_j), so no pair the test below would accept is
-    // dropped.  Survivors are staged with their coordinates and tested against every lane.
-    auto flush = [&]() {
-        int ns = 0;
-        for (int b = 0; b < nc; b += 32) {
-            const int kk = b + lane;
-            bool keep = false;
-            int j = 0;
-            float4 qh = make_float4(0.f, 0.f, 0.f, 0.f), ql = qh;
-            if (kk < nc) {
-                j = cand[kk];
-                qh = xh[j];
-                ql = xl[j];
-                ql.w = H2f[j];
-                const float ex = fabsf(ql.x), ey = fabsf(ql.y), ez = fabsf(ql.z);
-                const float gx = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.x, ex), ghi.x),
-                                                   __fsub_rd(glo.x, __fadd_ru(qh.x, ex))));
-                const float gy = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.y, ey), ghi.y),
-                                                   __fsub_rd(glo.y, __fadd_ru(qh.y, ey))));
-                const float gz = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.z, ez), ghi.z),
-                                                   __fsub_rd(glo.z, __fadd_ru(qh.z, ez))));
-                const float g2 = __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz));
-                keep = g2 < fmaxf(Rg2, __fmul_ru(k2, ql.w));
-            }
-            const unsigned km = __ballot_sync(FULLM, keep);
-            if (keep) {
-                const int p = ns + __popc(km & lt);
-                s_sj[warp][p] = j;
-                s_ph[warp][p] = qh;
-                s_pl[warp][p] = ql;
-            }
-            ns += __popc(km);
-            __syncwarp();
-            if (ns >= 32 || b + 32 >= nc) {
-                // every lane tests every survivor without branching (bit t of `am`), then writes
-                // its accepted ones in survivor order; the warp diverges only over those
-                unsigned amw[2] = {0u, 0u};
+    // 32 staged survivors (the last batch: n of them) against every lane, without branching (bit t of `am`), two
+    // survivors per instruction.  The accepted entries, lane by lane and in survivor order within a lane, are
+    // numbered e = 0 .. total - 1, listed as (lane, survivor) in the free part of the stack's memory, and written by
+    // the whole warp, 32 at a time: a lane's run of entries lands contiguously in its row, so every store covers a
+    // few runs instead of 32 rows.
+    const f32x2 nxh = f2_pack(-pih.x, -pih.x), nyh = f2_pack(-pih.y, -pih.y), nzh = f2_pack(-pih.z, -pih.z),
+                nxl = f2_pack(-pil.x, -pil.x), nyl = f2_pack(-pil.y, -pil.y), nzl = f2_pack(-pil.z, -pil.z);
+    const float ti = k2 * H2i;
+    auto batch = [&](int n) {
+        const int s0 = rd & (NB_SURV - 1);
+        unsigned am = 0;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int t1 = min(ns, 32 * h + 32);
-#pragma unroll 4
-                    for (int t = 32 * h; t < t1; ++t) {
-                        const float4 ph = s_ph[warp][t], pl = s_pl[warp][t];
-                        const float dx = df_sub(ph.x, pl.x, pih.x, pil.x);
-                        const float dy = df_sub(ph.y, pl.y, pih.y, pil.y);
-                        const float dz = df_sub(ph.z, pl.z, pih.z, pil.z);
-                        const float r2 = dx * dx + dy * dy + dz * dz;
-                        amw[h] |= (unsigned)(r2 < k2 * fmaxf(H2i, pl.w)) << (t - 32 * h);
-                    }
-                }
-                unsigned long long am = ((unsigned long long)amw[1] << 32) | amw[0];
-                if (!valid) am = 0ull;
-                // The batch's accepted entries, lane by lane and in survivor order within a lane,
-                // are numbered e = 0 .. total - 1 and written by the whole warp, 32 at a time: a
-                // lane's run of entries lands contiguously in its row, so every store covers a few
-                // runs instead of 32 rows.  Entry e belongs to lane L (prefix[L] <= e < prefix[L]
-                // + nacc[L]) and is that lane's k-th accepted survivor, k = e - prefix[L].
-                const unsigned alo = (unsigned)am, ahi = (unsigned)(am >> 32);
-                const int nacc = __popc(alo) + __popc(ahi);
-                int incl = nacc;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(FULLM, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                const int total = __shfl_sync(FULLM, incl, 31);
-                for (int e0 = 0; e0 < total; e0 += 32) {
-                    const int e = e0 + lane;
-                    int L = 0;   // the owner: the number of lanes whose inclusive prefix is <= e
-                    for (int st = 16; st > 0; st >>= 1) {
-                        const int v = __shfl_sync(FULLM, incl, L + st - 1);
-                        if (v <= e) L += st;
-                    }
-                    L = min(L, 31);
-                    const int excl = __shfl_sync(FULLM, incl - nacc, L);
-                    const unsigned lo = __shfl_sync(FULLM, alo, L), hi = __shfl_sync(FULLM, ahi, L);
-                    const int base = __shfl_sync(FULLM, count, L);
-                    if (e < total) {
-                        // t = the position of the k-th set bit of the 64-bit mask hi:lo, by halving with
-                        // popc (__fns here cost 0.17 ms of the walk's 2.55 ms per 1M step)
-                        const int k = e - excl;
-                        int kk = k, t = 0;
-                        unsigned x = lo;
-                        const int plo = __popc(lo);
-                        if (kk >= plo) {
-                            kk -= plo;
-                            x = hi;
-                            t = 32;
-                        }
-#pragma unroll
-                        for (int w = 16; w >= 1; w >>= 1) {
-                            const int c = __popc(x & ((1u << w) - 1u));
-                            if (kk >= c) {
-                                kk -= c;
-                                x >>= w;
-                                t += w;
-                            }
-                        }
-                        const float4 ph = s_ph[warp][t], pl = s_pl[warp][t];
-                        const float4 qh = s_pih[warp][L], ql = s_pil[warp][L];
-                        const float dx = df_sub(ph.x, pl.x, qh.x, ql.x);
-                        const float dy = df_sub(ph.y, pl.y, qh.y, ql.y);
-                        const float dz = df_sub(ph.z, pl.z, qh.z, ql.z);
-                        const float r2 = dx * dx + dy * dy + dz * dz;
-                        const int iL = U.x + L, pos = base + k;
-                        if (pos < K) {
-                            const int64_t o = (int64_t)iL * K + pos;
-                            sup[o] = s_sj[warp][t];
-                            sup_r2[o] = r2;
-                            sup_m[o] = ph.w;
-                        } else if (SPILL && pos < K + row_spill_cap(rm, iL)) {
-                            const int64_t o = rm.main + rm.soff[iL] - K + pos;
-                            sup[o] = s_sj[warp][t];
-                            sup_r2[o] = r2;
-                            sup_m[o] = ph.w;
-                        }
-                    }
-                }
-                count += nacc;
-                ns = 0;
-                __syncwarp();
-            }
+        for (int g = 0; g < 8; ++g) {
+            if (4 * g >= n) break;
+            auto four = [&](int c) { return *reinterpret_cast<const ulonglong2 *>(&sv[c][s0 + 4 * g]); };
+            const ulonglong2 xh4 = four(0), yh4 = four(1), zh4 = four(2), xl4 = four(4), yl4 = four(5), zl4 = four(6);
+            const float4 tj = *reinterpret_cast<const float4 *>(&sv[7][s0 + 4 * g]);
+            auto r2_of = [&](f32x2 xh2, f32x2 yh2, f32x2 zh2, f32x2 xl2, f32x2 yl2, f32x2 zl2) {
+                const f32x2 dx = f2_add(f2_add(xh2, nxh), f2_add(xl2, nxl));
+                const f32x2 dy = f2_add(f2_add(yh2, nyh), f2_add(yl2, nyl));
+                const f32x2 dz = f2_add(f2_add(zh2, nzh), f2_add(zl2, nzl));
+                return f2_fma(dz, dz, f2_fma(dy, dy, f2_mul(dx, dx)));
+            };
+            float ra, rb, rc, rd4;
+            f2_unpack(r2_of(xh4.x, yh4.x, zh4.x, xl4.x, yl4.x, zl4.x), ra, rb);
+            f2_unpack(r2_of(xh4.y, yh4.y, zh4.y, xl4.y, yl4.y, zl4.y), rc, rd4);
+            if (ra < fmaxf(ti, tj.x)) am |= 1u << (4 * g);
+            if (rb < fmaxf(ti, tj.y)) am |= 2u << (4 * g);
+            if (rc < fmaxf(ti, tj.z)) am |= 4u << (4 * g);
+            if (rd4 < fmaxf(ti, tj.w)) am |= 8u << (4 * g);
         }
-        nc = 0;
+        if (n < 32) am &= (1u << n) - 1u;
+        if (!valid) am = 0u;
+        const int nacc = __popc(am);
+        int incl = nacc;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULLM, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int total = __shfl_sync(FULLM, incl, 31);
+        const int before = count - (incl - nacc);   // entry e of this lane is entry before + e of its row
+        unsigned short *ent = reinterpret_cast<unsigned short *>(stack + sp);
+        const int room = 4 * (NB_STACK + NB_FREE - sp);
+        for (int e0 = 0; e0 < total; e0 += room) {
+            int e = incl - nacc - e0;
+            for (unsigned x = am; x; x &= x - 1, ++e)
+                if ((unsigned)e < (unsigned)room) ent[e] = (unsigned short)(lane << 5 | (__ffs(x) - 1));
+            __syncwarp();
+            const int m = min(total - e0, room);
+            for (int q0 = 0; q0 < m; q0 += 32) {
+                const int q = q0 + lane;
+                const int le = q < m ? ent[q] : 0, L = le >> 5, t = s0 + (le & 31);
+                const int pos = __shfl_sync(FULLM, before, L) + e0 + q;
+                if (q < m) {
+                    const float4 qh = s_pih[warp][L], ql = s_pil[warp][L];
+                    const float dx = df_sub(sv[0][t], sv[4][t], qh.x, ql.x);
+                    const float dy = df_sub(sv[1][t], sv[5][t], qh.y, ql.y);
+                    const float dz = df_sub(sv[2][t], sv[6][t], qh.z, ql.z);
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    const int iL = U.x + L;
+                    if (pos < K) {
+                        const int64_t o = (int64_t)iL * K + pos;
+                        sup[o] = sj[t];
+                        sup_r2[o] = r2;
+                        sup_m[o] = sv[3][t];
+                    } else if (SPILL && pos < K + row_spill_cap(rm, iL)) {
+                        const int64_t o = rm.main + rm.soff[iL] - K + pos;
+                        sup[o] = sj[t];
+                        sup_r2[o] = r2;
+                        sup_m[o] = sv[3][t];
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        count += nacc;
     };
 
-    int sp = 0;
+    // Up to 32 candidates are culled, each against the unit's box grown by its own reach: a lower bound of the
+    // distance (the point's hi / lo interval, rounded down) against an upper bound of max(Rg, kappa' 2.5 h_j), so no
+    // pair the test above would accept is dropped.  Survivors are staged with their coordinates.
+    auto cull = [&](int j, bool act) {
+        bool keep = false;
+        float4 qh = make_float4(0.f, 0.f, 0.f, 0.f), ql = qh;
+        if (act) {
+            qh = xh[j];
+            ql = xl[j];
+            ql.w = H2f[j];
+            const float ex = fabsf(ql.x), ey = fabsf(ql.y), ez = fabsf(ql.z);
+            const float gx = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.x, ex), ghi.x),
+                                               __fsub_rd(glo.x, __fadd_ru(qh.x, ex))));
+            const float gy = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.y, ey), ghi.y),
+                                               __fsub_rd(glo.y, __fadd_ru(qh.y, ey))));
+            const float gz = fmaxf(0.0f, fmaxf(__fsub_rd(__fsub_rd(qh.z, ez), ghi.z),
+                                               __fsub_rd(glo.z, __fadd_ru(qh.z, ez))));
+            const float g2 = __fadd_rd(__fadd_rd(__fmul_rd(gx, gx), __fmul_rd(gy, gy)), __fmul_rd(gz, gz));
+            keep = g2 < fmaxf(Rg2, __fmul_ru(k2, ql.w));
+        }
+        const unsigned km = __ballot_sync(FULLM, keep);
+        if (keep) {
+            const int p = (wr + __popc(km & lt)) & (NB_SURV - 1);
+            sj[p] = j;
+            sv[0][p] = qh.x;
+            sv[1][p] = qh.y;
+            sv[2][p] = qh.z;
+            sv[3][p] = qh.w;
+            sv[4][p] = ql.x;
+            sv[5][p] = ql.y;
+            sv[6][p] = ql.z;
+            sv[7][p] = k2 * ql.w;
+        }
+        wr += __popc(km);
+        __syncwarp();
+        if (wr - rd >= 32) {
+            batch(32);
+            rd += 32;
+        }
+    };
+
     {
         const int root = prun[U.x];   // the unit's run's octree root
         const float4 a = T.blo[root], b = T.bhi[root];
@@ -266,39 +264,29 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
         __syncwarp();
     }
     while (sp > 0) {
-        const int2 ci = stack[sp - 1];
-        if (ci.y > 0) {   // a leaf: with the leaves right below it, while their particles fit 32 lanes
-            if (nc + 32 > NB_CAND) flush();
-            int k = 1, tot = ci.y;
-            while (k < 8 && sp - 1 - k >= 0) {
-                const int2 nx = stack[sp - 1 - k];
-                if (nx.y <= 0 || tot + nx.y > 32) break;
-                tot += nx.y;
-                ++k;
+        const int2 se = lane < sp ? stack[sp - 1 - lane] : make_int2(0, 0);   // lane 0: the top
+        const unsigned leaves = __ballot_sync(FULLM, se.y > 0);
+        if (leaves & 1u) {   // a leaf: with the leaves right below it, while their particles fit 32 lanes
+            const int run = leaves == FULLM ? 32 : __ffs(~leaves) - 1;
+            const int v = lane < run ? min(se.y, 33) : 0;
+            int incl = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(FULLM, incl, o);
+                if (lane >= o) incl += u;
             }
-            if (tot <= 32) {
+            const int k = __popc(__ballot_sync(FULLM, lane < run && incl <= 32));
+            if (k > 0) {
                 // lane -> (leaf, offset): leaves in stack order from the top, particles in order
-                int acc = 0, src = -1;
-                for (int g = 0; g < k; ++g) {
-                    const int2 lf = stack[sp - 1 - g];
-                    if (src < 0 && lane < acc + lf.y) src = lf.x + (lane - acc);
-                    acc += lf.y;
-                }
-                __syncwarp();
-                if (lane < tot) cand[nc + lane] = src;
-                nc += tot;
+                const unsigned first = __reduce_or_sync(FULLM, lane < k ? 1u << (incl - v) : 0u);
+                const int tot = __shfl_sync(FULLM, incl, k - 1);
+                const int g = __popc(first & ((2u << lane) - 1u)) - 1;
+                const int j = __shfl_sync(FULLM, se.x - (incl - v), g) + lane;
                 sp -= k;
-                __syncwarp();
+                cull(j, lane < tot);
             } else {   // a leaf above 32 particles (only at the deepest level)
+                const int s = __shfl_sync(FULLM, se.x, 0), ct = __shfl_sync(FULLM, se.y, 0);
                 --sp;
-                __syncwarp();
-                const int s = ci.x, ct = ci.y;
-                for (int b0 = 0; b0 < ct; b0 += 32) {
-                    if (nc + 32 > NB_CAND) flush();
-                    if (b0 + lane < ct) cand[nc + lane] = s + b0 + lane;
-                    nc += min(32, ct - b0);
-                    __syncwarp();
-                }
+                for (int b0 = 0; b0 < ct; b0 += 32) cull(s + b0 + lane, b0 + lane < ct);
             }
         } else {
             // up to four internal cells from the top of the stack expanded at once, eight lanes per
@@ -306,21 +294,18 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
             // expansion would visit them (the leaves, and so the rows, keep their order).  More
             // than one only while the stack stays below NB_MULTI, so a depth-first continuation
             // (at most 7 pending siblings per level below) still fits NB_STACK.
-            int k = 1;
-            while (k < 4 && sp - 1 - k >= 0 && stack[sp - 1 - k].y <= 0 && sp - (k + 1) + 8 * (k + 1) <= NB_MULTI) ++k;
+            const int inner = leaves ? __ffs(leaves) - 1 : 32;
+            const int k = min(min(4, sp), min(inner, max(1, (NB_MULTI - sp) / 7)));
             const int g = lane >> 3, q = lane & 7;
+            const int f = __shfl_sync(FULLM, se.x, g), nch = -__shfl_sync(FULLM, se.y, g);
             bool ok = false;
             int2 chi = make_int2(0, 0);
-            if (g < k) {
-                const int2 cg = stack[sp - 1 - g];
-                const int f = cg.x, nch = -cg.y;
-                if (q < nch) {
-                    const float4 a = T.blo[f + q], b = T.bhi[f + q];
-                    const int4 r = T.cinfo[f + q];   // independent of the box loads: one round trip
-                    chi = r.y == 0 ? make_int2(r.z, r.w) : make_int2(r.x, -r.y);
-                    const float R = fmaxf(Rg, __fmul_ru(2.5f * KAPPA * 1.00390625f, b.w));
-                    ok = gap2_rd(a, b, glo, ghi) < __fmul_ru(R, R);
-                }
+            if (g < k && q < nch) {
+                const float4 a = T.blo[f + q], b = T.bhi[f + q];
+                const int4 r = T.cinfo[f + q];   // independent of the box loads: one round trip
+                chi = r.y == 0 ? make_int2(r.z, r.w) : make_int2(r.x, -r.y);
+                const float R = fmaxf(Rg, __fmul_ru(2.5f * KAPPA * 1.00390625f, b.w));
+                ok = gap2_rd(a, b, glo, ghi) < __fmul_ru(R, R);
             }
             sp -= k;
             __syncwarp();
@@ -335,7 +320,7 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
             __syncwarp();
         }
     }
-    flush();
+    if (wr > rd) batch(wr - rd);
     if (valid) {
         const int scap = (SPILL && count > K) ? spill_cap() : 0;
         cnt[i] = count;   // the true count, also when the row had no room for all of it
@@ -962,8 +947,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         // A warp walks a unit, or two or four share it: the walk of a small run is the latency of one warp's chain
         // (depth-first steps, candidates, accepted entries), and more and shorter chains fill the chip.  Rows do not
         // depend on the split, and units stay the units of the skin repairs.  Walk of 5,000 / 10,000 particles by
-        // one warp per unit 181 / 236 us, two 146 / 174, four 130 / 158; of 20,000 223, 173, 179; of 40,000 239, 219,
-        // 248; 70,000 particles and more are fastest with one.
+        // one warp per unit 150 / 185 us, two 122 / 142, four 109 / 129; of 20,000 179, 141, 145; of 40,000 195, 172,
+        // 199; 70,000 particles and more are fastest with one (214, 251, 301).
         const int64_t per_sm = n / ctx->num_sms;
         const int split = per_sm < WALK_SMALL ? 4 : (per_sm < WALK_MID ? 2 : 1);
         const int blocks = (n_walk * split + NB_WARPS - 1) / NB_WARPS;
