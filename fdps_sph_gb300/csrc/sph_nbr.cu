@@ -809,11 +809,13 @@ __global__ void k_h2f(int n, const double *h, float *H2f) {
     H2f[i] = __double2float_ru(H * H);
 }
 
-// double-float positions (hi / lo floats); .w of xh carries the mass x mscale
+// double-float positions (hi / lo floats); .w of xh carries the mass x mscale; (2.5 h)^2 as k_h2f
 __global__ void k_pack_pos(int n, const double *x, const double *y, const double *z, const double *m, double mscale,
-                           float4 *xh, float4 *xl) {
+                           const double *h, float4 *xh, float4 *xl, float *H2f) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const double H = SUPPORT * h[i];
+    H2f[i] = __double2float_ru(H * H);
     const float ax = (float)x[i], ay = (float)y[i], az = (float)z[i];
     xh[i] = make_float4(ax, ay, az, (float)(m[i] * mscale));
     xl[i] = make_float4((float)(x[i] - (double)ax), (float)(y[i] - (double)ay), (float)(z[i] - (double)az), 0.0f);
@@ -858,7 +860,7 @@ static const float4 *walk_xl(const sph_ctx *ctx) {
     return ctx->cfg.precision == SPH_PREC_MIXED ? ctx->xl : ctx->sup.pxl;
 }
 
-// h-dependent float copies; called after every density pass and after the sort
+// h-dependent float copies; called after every density pass
 int sph_nbr_refresh_h(sph_ctx *ctx) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
@@ -893,10 +895,11 @@ int sph_nbr_prepare(sph_ctx *ctx) {
     } else {
         k_pack_pos<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
                                                                 FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap),
-                                                                ctx->mscale, S.pxh, S.pxl);
+                                                                ctx->mscale, FLD(ctx->F, SPH_SMTH, cap), S.pxh, S.pxl,
+                                                                S.H2f);
         ++ctx->launches;
     }
-    SPH_TRY(sph_nbr_refresh_h(ctx));
+    SPH_CUDA(ctx, cudaGetLastError());
     S.valid = false;
     S.rebuilds_step = 0;
     ctx->lists[0].valid = ctx->lists[1].valid = false;

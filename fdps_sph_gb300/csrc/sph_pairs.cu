@@ -311,10 +311,10 @@ k_grav64(const int *__restrict__ group_cell, const int4 *__restrict__ cinfo, int
 
 // split_df: sph_physics.cuh
 
-// positions + scaled mass, velocities + h; called after the sort (and h refresh)
+// positions + scaled mass, velocities + h, (2.5 h)^2 as k_h2f; called after the sort
 __global__ void k_pack_df(int n, const double *x, const double *y, const double *z, const double *vx,
                           const double *vy, const double *vz, const double *m, const double *h, double mscale,
-                          float4 *xh, float4 *xl, float4 *vh, float4 *vl) {
+                          float4 *xh, float4 *xl, float4 *vh, float4 *vl, float *H2f) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float a, b, c, d, e, f;
@@ -328,6 +328,8 @@ __global__ void k_pack_df(int n, const double *x, const double *y, const double 
     split_df(vz[i], c, f);
     vh[i] = make_float4(a, b, c, 0.0f);
     vl[i] = make_float4(d, e, f, 0.0f);
+    const double H = SUPPORT * h[i];
+    H2f[i] = __double2float_ru(H * H);
 }
 
 __device__ __forceinline__ float df_diff(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
@@ -1518,7 +1520,7 @@ int sph_pack_mixed(sph_ctx *ctx) {
     k_pack_df<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), CF(SPH_VX), CF(SPH_VY),
                                                            CF(SPH_VZ), CF(SPH_MASS), CF(SPH_SMTH),
                                                            ctx->mscale, ctx->xh, ctx->xl, ctx->vhf,
-                                                           ctx->vlf); ++ctx->launches;
+                                                           ctx->vlf, ctx->sup.H2f); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
