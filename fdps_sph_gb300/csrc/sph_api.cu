@@ -302,14 +302,15 @@ namespace {
 #define FB(f) (1ull << (f))
 
 // main.cpp:138-146 (positions fixed): sort + tree, density x n, EoS, derivative, hydro, gravity
-int compute_forces(sph_ctx *ctx) {
+// (later: gravity's outcome is asked for by the caller, sph_gravity_redo)
+int compute_forces(sph_ctx *ctx, bool later) {
     SPH_TRY(sph_sort_and_build(ctx));   // marks SEG_SORT and SEG_TREE
     // final from here on: positions, half-step velocities and energies (kick-drift, then sorted)
     SPH_TRY(dl_milestone(ctx, FB(SPH_X) | FB(SPH_Y) | FB(SPH_Z) | FB(SPH_VHX) | FB(SPH_VHY) | FB(SPH_VHZ) |
                                   FB(SPH_ENGHALF)));
     SPH_TRY(time_mark(ctx, SEG_NBR_PREP));
     if (ctx->cfg.precision == SPH_PREC_MIXED) {
-        // all passes straight from the superset, with the same neighbour decisions as the exact list
+        // density, EoS and the lists; density straight from the superset, with the exact list's neighbour decisions
         SPH_TRY(sph_density_fused(ctx));
     } else {
         for (int it = 0; it < ctx->cfg.n_dens_iter; ++it) {
@@ -318,11 +319,11 @@ int compute_forces(sph_ctx *ctx) {
             SPH_TRY(sph_pass_density(ctx, 0));
             SPH_TRY(time_mark(ctx, SEG_DENS));
         }
+        SPH_TRY(sph_pass_eos(ctx));
+        SPH_TRY(time_mark(ctx, SEG_EOS));
+        SPH_TRY(dl_milestone(ctx, FB(SPH_DENS) | FB(SPH_SMTH) | FB(SPH_PRES) | FB(SPH_SNDS)));
+        SPH_TRY(sph_build_sph_lists(ctx, 2));   // gather and symmetric lists of the final h, one pass
     }
-    SPH_TRY(sph_pass_eos(ctx));
-    SPH_TRY(time_mark(ctx, SEG_EOS));
-    SPH_TRY(dl_milestone(ctx, FB(SPH_DENS) | FB(SPH_SMTH) | FB(SPH_PRES) | FB(SPH_SNDS)));
-    SPH_TRY(sph_build_sph_lists(ctx, 2));   // gather and symmetric lists of the final h, one pass
     SPH_TRY(time_mark(ctx, SEG_DRVT_LIST));
     SPH_TRY(sph_pass_derivative(ctx, 0));
     SPH_TRY(time_mark(ctx, SEG_DRVT));
@@ -337,7 +338,7 @@ int compute_forces(sph_ctx *ctx) {
     if (ctx->cfg.self_gravity) {
         if (ctx->cfg.precision == SPH_PREC_MIXED) {
             SPH_TRY(time_mark(ctx, SEG_GRAV_LIST));   // no lists: the walk runs inside the force kernel
-            SPH_TRY(sph_gravity_fused(ctx));
+            SPH_TRY(sph_gravity_fused(ctx, later));
         } else {
             SPH_TRY(sph_build_grav_lists(ctx));
             SPH_TRY(time_mark(ctx, SEG_GRAV_LIST));
@@ -1083,7 +1084,7 @@ int sph_prologue(sph_ctx *ctx) {
     cudaSetDevice(ctx->device);
     ctx->n_ev = 0;
     SPH_TRY(time_mark(ctx, -1));
-    SPH_TRY(compute_forces(ctx));
+    SPH_TRY(compute_forces(ctx, false));
     SPH_TRY(sph_run_reduce_dt(ctx));           // main.cpp:103
     SPH_TRY(sph_ext_force(ctx));               // main.cpp:104
     SPH_TRY(time_mark(ctx, SEG_FINAL));
@@ -1118,7 +1119,12 @@ int sph_step(sph_ctx *ctx, int n_steps) {
         SPH_TRY(sph_kick_drift_predict(ctx));       // main.cpp:126-131
         SPH_TRY(time_mark(ctx, SEG_KDP));
         for (int r = 0; r < R.R; ++r) R.time[r] += dt_step[r];   // main.cpp:132
-        SPH_TRY(compute_forces(ctx));               // main.cpp:136-147
+        // Whether gravity needs its larger buffers (rare) is asked after the kick and the new dt are launched, where
+        // nothing between them and the answer adds to the state: the kick only reads what gravity wrote, and is
+        // repeated with the step's dt if gravity is.
+        const bool later = ctx->cfg.self_gravity && ctx->cfg.precision == SPH_PREC_MIXED && ctx->cfg.mode != 2 &&
+                           !ctx->cfg.ext_damp && !ctx->dl_host;
+        SPH_TRY(compute_forces(ctx, later));        // main.cpp:136-147
         SPH_TRY(sph_ext_force(ctx));                // main.cpp:148
         SPH_TRY(sph_final_kick(ctx));               // main.cpp:149-153
         if (ctx->cfg.mode == 2) {                   // main.cpp:155-158
@@ -1126,7 +1132,18 @@ int sph_step(sph_ctx *ctx, int n_steps) {
             SPH_TRY(sph_entropy_step(ctx));
             SPH_TRY(time_mark(ctx, SEG_ENTROPY));
         }
-        SPH_TRY(sph_run_reduce_dt(ctx));            // main.cpp:160
+        int rc = sph_run_reduce_dt(ctx);            // main.cpp:160
+        if (later) {
+            bool again;
+            SPH_TRY(sph_gravity_redo(ctx, &again));
+            if (again) {
+                SPH_CUDA(ctx, cudaMemcpyAsync(R.dt_dev, dt_step.data(), sizeof(double) * R.R, cudaMemcpyHostToDevice,
+                                              ctx->stream));
+                SPH_TRY(sph_final_kick(ctx));
+                rc = sph_run_reduce_dt(ctx);
+            }
+        }
+        SPH_TRY(rc);
         if (ctx->cfg.mode == 2) SPH_TRY(sph_entropy_check(ctx));
         SPH_TRY(time_mark(ctx, SEG_FINAL));
         SPH_TRY(collect_timings(ctx));

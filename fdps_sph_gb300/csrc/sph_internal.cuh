@@ -435,7 +435,8 @@ int sph_runs_layout(sph_ctx *ctx);        // offsets and tiles of the runs after
 int sph_run_reduce_dt(sph_ctx *ctx);      // per-run min dt into runs.dt_dev and runs.dt
 int sph_run_diag(sph_ctx *ctx, double *out);   // per-run conserved quantities, out[R * 8]
 int sph_build_grav_lists(sph_ctx *ctx);
-int sph_gravity_fused(sph_ctx *ctx);       // mixed precision: walk + force in one kernel
+int sph_gravity_fused(sph_ctx *ctx, bool later);   // mixed precision: walk + force in one kernel
+int sph_gravity_redo(sph_ctx *ctx, bool *again);    // after sph_gravity_fused(later)
 
 // passes (sph_pairs.cu)
 int sph_pass_density(sph_ctx *ctx, int build_lists);

@@ -358,6 +358,19 @@ __global__ void k_viol_mark(int n, const double *h, const double *hsup, float *v
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nviol, __popc(b));
 }
 
+// after a density round: (2.5 h)^2 of the new h as k_h2f, and the count of k_viol_mark
+__global__ void k_h2f_viol(int n, const double *h, const double *hsup, float *H2f, int *nviol) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool v = false;
+    if (i < n) {
+        const double H = SUPPORT * h[i];
+        H2f[i] = __double2float_ru(H * H);
+        v = h[i] > (double)KAPPA * hsup[i];
+    }
+    const unsigned b = __ballot_sync(FULLM, v);
+    if ((threadIdx.x & 31) == 0 && b) atomicAdd(nviol, __popc(b));
+}
+
 __global__ void k_cell_vmax(int l, const int *meta, const float *vR, const int4 *cinfo, float *cvR) {
     const int L0 = meta[l], L1 = meta[l + 1];
     for (int c = L0 + blockIdx.x * blockDim.x + threadIdx.x; c < L1; c += gridDim.x * blockDim.x) {
@@ -1074,11 +1087,11 @@ static int ensure_superset(sph_ctx *ctx) {
 }
 
 // exact list of `mode` (0 gather, 1 symmetric, 2 both) for the current h
-int sph_build_sph_lists(sph_ctx *ctx, int mode) {
+// the exact lists from a superset that is valid for the current h
+static int filter_lists(sph_ctx *ctx, int mode) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
     const int64_t cap = ctx->cap;
-    SPH_TRY(ensure_superset(ctx));
     SphLists &L0 = ctx->lists[0], &L1 = ctx->lists[1];
     auto filter = mode == 0 ? k_filter<0> : (mode == 1 ? k_filter<1> : k_filter<2>);
     filter<<<sph_div_up(n, FW), FW * 32, 0, ctx->stream>>>(
@@ -1089,6 +1102,11 @@ int sph_build_sph_lists(sph_ctx *ctx, int mode) {
     if (mode != 1) L0.valid = true;
     if (mode != 0) L1.valid = true;
     return SPH_OK;
+}
+
+int sph_build_sph_lists(sph_ctx *ctx, int mode) {
+    SPH_TRY(ensure_superset(ctx));
+    return filter_lists(ctx, mode);
 }
 
 // mixed-precision density pass straight from the superset (no exact list)
@@ -1110,21 +1128,26 @@ int sph_density_from_superset(sph_ctx *ctx) {
 
 int sph_nbr_ensure_superset(sph_ctx *ctx) { return ensure_superset(ctx); }
 
-// all density passes of the mixed path: rounds of k_density_fused32, the rows of the particles
-// that left their skin walked again between rounds (each round takes every unfinished particle
-// at least one pass further, so there are at most n_dens_iter rounds)
+// All density passes of the mixed path, the EoS and the exact lists of the final h: rounds of k_density_fused32, the
+// rows of the particles that left their skin walked again between rounds (each round takes every unfinished particle
+// at least one pass further, so there are at most n_dens_iter rounds).  The host has to know whether a particle
+// stopped (another round) or outgrew its skin in the last pass (a repair before the lists); both are rare, so the EoS
+// and the lists are launched behind the round before it knows, and run again where it was needed: they only read what
+// the round wrote.  The wait for the answer was a gap in a small run's step, and the lists had one of their own:
+// a step of 5,000 particles 473 -> 455 us, of 100,000 1.276 -> 1.239 ms.  While a download follows the step, the lists wait, so that what the EoS finished is sent first.
 int sph_density_fused(sph_ctx *ctx) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
     const int64_t cap = ctx->cap;
     const int np = ctx->cfg.n_dens_iter;
-    int *stopped = ctx->tree.meta + META_ERR + 9;
+    int *nviol = ctx->tree.meta + META_ERR + 8, *stopped = nviol + 1;
     int *hs = (int *)ctx->host_scalars;
+    const bool ahead = !ctx->dl_host;
     SPH_CUDA(ctx, cudaMemsetAsync(S.npass, 0, sizeof(int) * n, ctx->stream));
     for (int round = 0; round <= np; ++round) {
         SPH_TRY(ensure_superset(ctx));
         SPH_TRY(time_mark(ctx, SEG_DENS_LIST));
-        SPH_CUDA(ctx, cudaMemsetAsync(stopped, 0, sizeof(int), ctx->stream));
+        SPH_CUDA(ctx, cudaMemsetAsync(nviol, 0, 2 * sizeof(int), ctx->stream));
         const int dt = (int64_t)n < (int64_t)ctx->num_sms * DENS_SMALL ? 8 : 2;
         auto kd = ctx->runs.fix_split ? (dt == 8 ? k_density_fused32<true, 8> : k_density_fused32<true, 2>)
                                       : (dt == 8 ? k_density_fused32<false, 8> : k_density_fused32<false, 2>);
@@ -1134,14 +1157,23 @@ int sph_density_fused(sph_ctx *ctx) {
             FLD(ctx->F, SPH_DENS, cap), (float)(1365.0 / 64.0 / (3.141592653589793 * ctx->mscale)), S.npass,
             stopped, ctx->runs.prun, ctx->runs.fixd);
         ++ctx->launches;
+        k_h2f_viol<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_SMTH, cap), S.hsup, S.H2f, nviol);
+        ++ctx->launches;
         SPH_CUDA(ctx, cudaGetLastError());
         SPH_TRY(time_mark(ctx, SEG_DENS));
-        SPH_CUDA(ctx, cudaMemcpyAsync(hs, stopped, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        SPH_TRY(sph_nbr_refresh_h(ctx));   // H2f of the current h, for the walks and the filters
-        if (hs[0] == 0) break;
+        SPH_CUDA(ctx, cudaMemcpyAsync(hs, nviol, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        SPH_CUDA(ctx, cudaEventRecord(ctx->tree_done, ctx->stream));
+        SPH_TRY(sph_pass_eos(ctx));
+        SPH_TRY(time_mark(ctx, SEG_EOS));
+        if (ahead) SPH_TRY(filter_lists(ctx, 2));
+        SPH_CUDA(ctx, cudaEventSynchronize(ctx->tree_done));
+        if (hs[1] == 0) break;
+        ctx->lists[0].valid = ctx->lists[1].valid = false;
         if (round == np) return sph_fail(ctx, SPH_ERR_STATE, "density passes did not converge over the skin repairs");
     }
-    ctx->lists[0].valid = false;
-    return SPH_OK;
+    const bool outgrown = hs[0] > 0;
+    // final from here on
+    SPH_TRY(dl_milestone(ctx, 1ull << SPH_DENS | 1ull << SPH_SMTH | 1ull << SPH_PRES | 1ull << SPH_SNDS));
+    if (outgrown) SPH_TRY(ensure_superset(ctx));
+    return outgrown || !ahead ? filter_lists(ctx, 2) : SPH_OK;
 }
