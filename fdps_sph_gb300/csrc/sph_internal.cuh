@@ -420,6 +420,7 @@ int sph_fail(sph_ctx *ctx, int code, const char *fmt, ...);
 int sph_tree_reserve(sph_ctx *ctx, int64_t n);
 int sph_sort_and_build(sph_ctx *ctx);          // root box, keys, sort, permute, octree, moments
 int sph_tree_refresh_hmax(sph_ctx *ctx);       // cell hmax after h changed
+int sph_publish(sph_ctx *ctx, const int *src, int n);
 int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev, int len_host, int *total_dev);
 
 // lists (sph_nbr.cu, sph_lists.cu)

@@ -185,6 +185,13 @@ k_grav_lists(int ng, const int *__restrict__ group_cell, const double *__restric
     }
 }
 
+// the totals of the counting pass and its error word, for the host (pinned memory)
+__global__ void k_list_totals(const int *oe, const int *ne, const int *os, const int *ns, const int *err, int *host) {
+    const int *p[5] = {oe, ne, os, ns, err};
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 5; ++k) host[k] = *p[k];
+}
+
 }  // namespace sph
 
 using namespace sph;
@@ -216,11 +223,9 @@ int sph_build_grav_lists(sph_ctx *ctx) {
                                                          nullptr, nullptr, nullptr, t.meta + META_ERR); ++ctx->launches;
     SPH_TRY(sph_scan_exclusive(ctx, G.n_epj, G.off_epj, nullptr, ng, nullptr));
     SPH_TRY(sph_scan_exclusive(ctx, G.n_spj, G.off_spj, nullptr, ng, nullptr));
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs, G.off_epj + (ng - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs + 1, G.n_epj + (ng - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs + 2, G.off_spj + (ng - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs + 3, G.n_spj + (ng - 1), sizeof(int), cudaMemcpyDeviceToHost, st));
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs + 4, t.meta + META_ERR, sizeof(int), cudaMemcpyDeviceToHost, st));
+    k_list_totals<<<1, 32, 0, st>>>(G.off_epj + (ng - 1), G.n_epj + (ng - 1), G.off_spj + (ng - 1), G.n_spj + (ng - 1),
+                                    t.meta + META_ERR, hs); ++ctx->launches;
+    SPH_CUDA(ctx, cudaGetLastError());
     SPH_CUDA(ctx, cudaStreamSynchronize(st));
     if (hs[4] & ERR_GRAV_OVERFLOW) return sph_fail(ctx, SPH_ERR_CAPACITY, "gravity walk stack overflow");
     const int64_t tot_e = (int64_t)hs[0] + hs[1], tot_s = (int64_t)hs[2] + hs[3];

@@ -959,7 +959,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
             S.spill_alloc = S.spill_cap;
         }
         static_assert(META_MAXCNT == META_ERR + 1, "cleared together");
-        SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR, 0, 2 * sizeof(int), ctx->stream));
+        if (attempt > 0 || S.rebuilds_step > 1)   // the first walk after a sort finds them cleared
+            SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR, 0, 2 * sizeof(int), ctx->stream));
         // A warp walks a unit, or two or four share it: the walk of a small run is the latency of one warp's chain
         // (depth-first steps, candidates, accepted entries), and more and shorter chains fill the chip.  Rows do not
         // depend on the split, and units stay the units of the skin repairs.  Walk of 5,000 / 10,000 particles by
@@ -979,7 +980,7 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         }
         SPH_CUDA(ctx, cudaGetLastError());
         int *hs = (int *)ctx->host_scalars;
-        SPH_CUDA(ctx, cudaMemcpyAsync(hs, meta + META_ERR, 4 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        SPH_TRY(sph_publish(ctx, meta + META_ERR, 2));
         SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         const int errw = hs[0], maxc = hs[META_MAXCNT - META_ERR];
         if (errw & ERR_SPH_STACK) return sph_fail(ctx, SPH_ERR_CAPACITY, "SPH walk stack overflow");
@@ -1061,7 +1062,7 @@ static int ensure_superset(sph_ctx *ctx) {
                                                               meta + META_ERR + 8);
     ++ctx->launches;
     int *hs = (int *)ctx->host_scalars;
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs, meta + META_ERR + 8, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    SPH_TRY(sph_publish(ctx, meta + META_ERR + 8, 1));
     SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int nviol = hs[0];
     if (nviol == 0) return SPH_OK;
@@ -1080,14 +1081,13 @@ static int ensure_superset(sph_ctx *ctx) {
     SPH_TRY(sph_scan_exclusive(ctx, S.umark, S.uoff, nullptr, S.n_units, ctx->scan.total));
     k_unit_compact<<<grid, 256, 0, ctx->stream>>>(S.n_units, S.umark, S.uoff, S.uidx);
     ++ctx->launches;
-    SPH_CUDA(ctx, cudaMemcpyAsync(hs, ctx->scan.total, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    SPH_TRY(sph_publish(ctx, ctx->scan.total, 1));
     SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int nmark = hs[0];
     return walk_units(ctx, S.uidx, nmark);
 }
 
-// exact list of `mode` (0 gather, 1 symmetric, 2 both) for the current h
-// the exact lists from a superset that is valid for the current h
+// exact list of `mode` (0 gather, 1 symmetric, 2 both) from a superset that is valid for the current h
 static int filter_lists(sph_ctx *ctx, int mode) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
@@ -1104,6 +1104,7 @@ static int filter_lists(sph_ctx *ctx, int mode) {
     return SPH_OK;
 }
 
+// the same, with the superset made valid first
 int sph_build_sph_lists(sph_ctx *ctx, int mode) {
     SPH_TRY(ensure_superset(ctx));
     return filter_lists(ctx, mode);
@@ -1143,11 +1144,10 @@ int sph_density_fused(sph_ctx *ctx) {
     int *nviol = ctx->tree.meta + META_ERR + 8, *stopped = nviol + 1;
     int *hs = (int *)ctx->host_scalars;
     const bool ahead = !ctx->dl_host;
-    SPH_CUDA(ctx, cudaMemsetAsync(S.npass, 0, sizeof(int) * n, ctx->stream));
     for (int round = 0; round <= np; ++round) {
         SPH_TRY(ensure_superset(ctx));
         SPH_TRY(time_mark(ctx, SEG_DENS_LIST));
-        SPH_CUDA(ctx, cudaMemsetAsync(nviol, 0, 2 * sizeof(int), ctx->stream));
+        if (round > 0) SPH_CUDA(ctx, cudaMemsetAsync(nviol, 0, 2 * sizeof(int), ctx->stream));   // else cleared by the tree
         const int dt = (int64_t)n < (int64_t)ctx->num_sms * DENS_SMALL ? 8 : 2;
         auto kd = ctx->runs.fix_split ? (dt == 8 ? k_density_fused32<true, 8> : k_density_fused32<true, 2>)
                                       : (dt == 8 ? k_density_fused32<false, 8> : k_density_fused32<false, 2>);
@@ -1161,7 +1161,7 @@ int sph_density_fused(sph_ctx *ctx) {
         ++ctx->launches;
         SPH_CUDA(ctx, cudaGetLastError());
         SPH_TRY(time_mark(ctx, SEG_DENS));
-        SPH_CUDA(ctx, cudaMemcpyAsync(hs, nviol, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        SPH_TRY(sph_publish(ctx, nviol, 2));
         SPH_CUDA(ctx, cudaEventRecord(ctx->tree_done, ctx->stream));
         SPH_TRY(sph_pass_eos(ctx));
         SPH_TRY(time_mark(ctx, SEG_EOS));

@@ -311,10 +311,10 @@ k_grav64(const int *__restrict__ group_cell, const int4 *__restrict__ cinfo, int
 
 // split_df: sph_physics.cuh
 
-// positions + scaled mass, velocities + h, (2.5 h)^2 as k_h2f; called after the sort
+// positions + scaled mass, velocities + h, (2.5 h)^2 as k_h2f, no density pass done; called after the sort
 __global__ void k_pack_df(int n, const double *x, const double *y, const double *z, const double *vx,
                           const double *vy, const double *vz, const double *m, const double *h, double mscale,
-                          float4 *xh, float4 *xl, float4 *vh, float4 *vl, float *H2f) {
+                          float4 *xh, float4 *xl, float4 *vh, float4 *vl, float *H2f, int *npass) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float a, b, c, d, e, f;
@@ -330,6 +330,7 @@ __global__ void k_pack_df(int n, const double *x, const double *y, const double 
     vl[i] = make_float4(d, e, f, 0.0f);
     const double H = SUPPORT * h[i];
     H2f[i] = __double2float_ru(H * H);
+    npass[i] = 0;
 }
 
 __device__ __forceinline__ float df_diff(float ah, float al, float bh, float bl) { return (ah - bh) + (al - bl); }
@@ -759,7 +760,10 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32(int n, HydroArgs32 a) {
 }
 
 // cell monopoles as double-float with G folded into the mass
-__global__ void k_pack_cells32(const int *meta, const double4 *com, double G, double gscale, float4 *ch, float4 *cl) {
+// (err, if given, is cleared)
+__global__ void k_pack_cells32(const int *meta, const double4 *com, double G, double gscale, float4 *ch, float4 *cl,
+                               int *err) {
+    if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const int nc = meta[MAX_LEVELS];
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
         const double4 q = com[c];
@@ -1377,12 +1381,15 @@ __global__ void k_min_tiles(const double *v, const int4 *tiles, double *part) {
     if (threadIdx.x == 0) part[blockIdx.x] = r;
 }
 
-__global__ void k_min_runs(const double *part, const int4 *info, double *out) {
+__global__ void k_min_runs(const double *part, const int4 *info, double *out, double *host) {
     const int4 q = info[blockIdx.x];
     double r = 1.0e30;
     for (int b = q.z + threadIdx.x; b < q.z + q.w; b += blockDim.x) r = (part[b] < r || part[b] != part[b]) ? part[b] : r;
     r = block_min(r);
-    if (threadIdx.x == 0) out[blockIdx.x] = r;
+    if (threadIdx.x == 0) {
+        out[blockIdx.x] = r;
+        if (host) host[blockIdx.x] = r;
+    }
 }
 
 // conserved quantities, fixed-order two-stage reduction in FP64
@@ -1520,7 +1527,7 @@ int sph_pack_mixed(sph_ctx *ctx) {
     k_pack_df<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), CF(SPH_VX), CF(SPH_VY),
                                                            CF(SPH_VZ), CF(SPH_MASS), CF(SPH_SMTH),
                                                            ctx->mscale, ctx->xh, ctx->xl, ctx->vhf,
-                                                           ctx->vlf, ctx->sup.H2f); ++ctx->launches;
+                                                           ctx->vlf, ctx->sup.H2f, ctx->sup.npass); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -1631,7 +1638,8 @@ int sph_pass_gravity(sph_ctx *ctx, int build_lists) {
         if ((int64_t)t.n_cell_host * 2 > ctx->cap * 4) return sph_fail(ctx, SPH_ERR_CAPACITY, "cell pack scratch");
         float4 *ch = (float4 *)ctx->F2, *cl = ch + t.n_cell_host;
         const double gscale = 1.0;
-        k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, gscale, ch, cl); ++ctx->launches;
+        k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, gscale, ch, cl, nullptr);
+        ++ctx->launches;
         k_grav32<<<G.ng, GT, 0, ctx->stream>>>(G.group_cell, t.start, t.count, ctx->xh, ctx->xl, CF(SPH_MASS),
                                                CF(SPH_SMTH), ch, cl, G.n_epj, G.off_epj, G.epj, G.n_spj, G.off_spj,
                                                G.spj, ctx->cfg.G, gscale, 1.0 / gscale, CF(SPH_GX), CF(SPH_GY),
@@ -1686,9 +1694,17 @@ int sph_ext_force(sph_ctx *ctx) {
 int sph_run_reduce_dt(sph_ctx *ctx) {
     Runs &R = ctx->runs;
     k_min_tiles<<<R.T, 256, 0, ctx->stream>>>(CF(SPH_DT), R.tiles, R.part); ++ctx->launches;
-    k_min_runs<<<R.R, 256, 0, ctx->stream>>>(R.part, R.info, R.dt_dev); ++ctx->launches;
-    std::vector<double> h(R.R);
-    SPH_CUDA(ctx, cudaMemcpyAsync(h.data(), R.dt_dev, sizeof(double) * R.R, cudaMemcpyDeviceToHost, ctx->stream));
+    // the host's values straight into the pinned block (behind the words of sph_publish) where they fit it
+    double *h = ctx->host_scalars + 32;
+    const bool fits = R.R <= 480;
+    k_min_runs<<<R.R, 256, 0, ctx->stream>>>(R.part, R.info, R.dt_dev, fits ? h : nullptr); ++ctx->launches;
+    SPH_CUDA(ctx, cudaGetLastError());
+    std::vector<double> many;
+    if (!fits) {
+        many.resize(R.R);
+        h = many.data();
+        SPH_CUDA(ctx, cudaMemcpyAsync(h, R.dt_dev, sizeof(double) * R.R, cudaMemcpyDeviceToHost, ctx->stream));
+    }
     SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int r = 0; r < R.R; ++r) {
         const double d = h[r];
@@ -1769,7 +1785,7 @@ static int launch_grav_fused(sph_ctx *ctx, bool wide) {
     float4 *chp = (float4 *)ctx->F2, *clp = chp + t.n_cell_host;
     // xh.w holds m * mscale: G m = xh.w * (G / mscale)
     const float gms = (float)(ctx->cfg.G / ctx->mscale);
-    SPH_CUDA(ctx, cudaMemsetAsync(t.meta + META_ERR, 0, sizeof(int), ctx->stream));
+    if (wide) SPH_CUDA(ctx, cudaMemsetAsync(t.meta + META_ERR, 0, sizeof(int), ctx->stream));
     const bool one = !wide && G.ng < ctx->num_sms * GRAV_ONE;
     auto kern = wide ? k_grav_fused32<256, 2> : (one ? k_grav_fused32<128, 1> : k_grav_fused32<128, 2>);
     kern<<<dim3(G.ng, one ? 2 : 1), wide ? 256 : 128, 0, ctx->stream>>>(
@@ -1778,6 +1794,7 @@ static int launch_grav_fused(sph_ctx *ctx, bool wide) {
         t.meta + META_ERR);
     ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
+    if (!wide) return sph_publish(ctx, t.meta + META_ERR, 1);
     SPH_CUDA(ctx, cudaMemcpyAsync(ctx->host_scalars, t.meta + META_ERR, sizeof(int), cudaMemcpyDeviceToHost,
                                   ctx->stream));
     return SPH_OK;
@@ -1793,7 +1810,7 @@ int sph_gravity_fused(sph_ctx *ctx, bool later) {
     if (G.ng == 0) return SPH_OK;
     if ((int64_t)t.n_cell_host * 2 > ctx->cap * 4) return sph_fail(ctx, SPH_ERR_CAPACITY, "cell pack scratch");
     float4 *chp = (float4 *)ctx->F2, *clp = chp + t.n_cell_host;
-    k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, 1.0, chp, clp);
+    k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, 1.0, chp, clp, t.meta + META_ERR);
     ++ctx->launches;
     SPH_TRY(launch_grav_fused(ctx, false));
     G.counts_valid = true;
