@@ -445,11 +445,13 @@ __device__ __forceinline__ void drvt_tail32(const DrvtArgs32 &a, int i, double h
 
 // Not tuned (threads per i-particle 1), a row's FP32 partial sums run over blocks of 32 entries in list order and
 // go into the compensated pair block by block.  One thread doing that is bound by the latency of its 106
-// gathers in a row.  Here four lanes share the particle, lane sub evaluates entries 2 sub, 2 sub + 1 of every eight
+// gathers in a row.  Here four lanes share the particle, lane sub evaluates entries sub and sub + 4 of every eight
 // (neighbours in the list are neighbours in memory, so the lanes' gathers stay together), then the lanes swap their
 // terms so that lane q holds component q of all eight entries (a 4 x 4 transpose: four shuffles) and adds them in
-// list order: the bits are one thread's.  Derivative / hydro of 1M particles 0.88 / 1.12 -> 0.76 / 0.83 ms, of
-// 5,003 particles 59 / 64 -> 27 / 29 us.  Lanes that take whole blocks of 32 instead spread a particle's gathers over
+// list order: the bits are one thread's.  What bounds it then is the L1 data stage (95%), which the gathers share with
+// the shuffles; so the derivative's fifth sum goes from lane to lane instead of its terms to every lane.  Derivative /
+// hydro of 1M particles 0.88 / 1.12 -> 0.72 / 0.81 ms (entries 2 sub and 2 sub + 1, all terms sent: 0.76 / 0.83), of
+// 5,003 particles 59 / 64 -> 26 / 27 us.  Lanes that take whole blocks of 32 instead spread a particle's gathers over
 // its row: 0.96 / 1.20 ms at 1M, and no faster at any size from 3,000 particles on.
 __device__ __forceinline__ void transpose4(unsigned mask, int sub, float v[4]) {
     const bool o1 = sub & 1, o2 = sub & 2;
@@ -486,22 +488,27 @@ __global__ void __launch_bounds__(PT) k_drvt32_lanes(int n, DrvtArgs32 a) {
     const RowView row = row_view(a.nbr, a.rm, i, a.cnt[i]);
     const int c = row.c;
     for (int k = 0; k < c; k += 8) {
-        const int kk = k + 2 * sub;
+        const int kk = k + sub;
         DrvtT32 t0{}, t1{};
         if (kk < c) {
-            const int2 jp = *reinterpret_cast<const int2 *>(row.at(kk));
-            t0 = drvt_terms32(pih, pil, vih, vil, a.xh[jp.x], a.xl[jp.x], a.vh[jp.x], a.vl[jp.x], invH, Hf, ceps);
-            if (kk + 1 < c)
-                t1 = drvt_terms32(pih, pil, vih, vil, a.xh[jp.y], a.xl[jp.y], a.vh[jp.y], a.vl[jp.y], invH, Hf, ceps);
+            const int j0 = *row.at(kk);
+            if (kk + 4 < c) {
+                const int j1 = *row.at(kk + 4);
+                t1 = drvt_terms32(pih, pil, vih, vil, a.xh[j1], a.xl[j1], a.vh[j1], a.vl[j1], invH, Hf, ceps);
+            }
+            t0 = drvt_terms32(pih, pil, vih, vil, a.xh[j0], a.xl[j0], a.vh[j0], a.vl[j0], invH, Hf, ceps);
         }
         transpose4(mask, sub, t0.x);
         transpose4(mask, sub, t1.x);
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
             P = fmaf(__shfl_sync(mask, t0.mg, l, 4), t0.x[l], P);
+            Q = __shfl_sync(mask, fmaf(t0.m, t0.y, Q), l, 4);   // lane l's entry: the sum goes from lane to lane
+        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
             P = fmaf(__shfl_sync(mask, t1.mg, l, 4), t1.x[l], P);
-            Q = fmaf(__shfl_sync(mask, t0.m, l, 4), __shfl_sync(mask, t0.y, l, 4), Q);
-            Q = fmaf(__shfl_sync(mask, t1.m, l, 4), __shfl_sync(mask, t1.y, l, 4), Q);
+            Q = __shfl_sync(mask, fmaf(t1.m, t1.y, Q), l, 4);   // lane l's entry: the sum goes from lane to lane
         }
         if ((k & 31) == 24 && k + 8 <= c) {   // 32 entries summed
             df_add(Dh, Dl, P);
@@ -663,11 +670,12 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
     float Dh = 0.0f, Dl = 0.0f, P = 0.0f, vmax = 0.0f;   // component `sub`
     const RowView row = row_view(a.nbr, a.rm, i, a.cnt[i]);
     const int c = row.c;
-    int2 jn = 2 * sub < c ? *reinterpret_cast<const int2 *>(row.at(2 * sub)) : make_int2(i, i);
+    int2 jn = make_int2(sub < c ? *row.at(sub) : i, sub + 4 < c ? *row.at(sub + 4) : i);
     for (int k = 0; k < c; k += 8) {
-        const int kk = k + 2 * sub;
+        const int kk = k + sub;
         const int2 jp = jn;
-        if (kk + 8 < c) jn = *reinterpret_cast<const int2 *>(row.at(kk + 8));   // (past the row's end: padding, unused)
+        if (kk + 8 < c) jn.x = *row.at(kk + 8);
+        if (kk + 12 < c) jn.y = *row.at(kk + 12);
         float u0[4] = {0, 0, 0, 0}, x0[4] = {0, 0, 0, 0}, u1[4] = {0, 0, 0, 0}, x1[4] = {0, 0, 0, 0};
         if (kk < c) {
             const HydroT32 t = hydro_terms32(pih, pil, vih, vil, Ai, Bi, load_hydro_j(a, jp.x), vmax);
@@ -675,7 +683,7 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
             u0[3] = t.e;
             x0[0] = t.dx, x0[1] = t.dy, x0[2] = t.dz, x0[3] = t.dvdr;
         }
-        if (kk + 1 < c) {
+        if (kk + 4 < c) {
             const HydroT32 t = hydro_terms32(pih, pil, vih, vil, Ai, Bi, load_hydro_j(a, jp.y), vmax);
             u1[0] = u1[1] = u1[2] = t.c;
             u1[3] = t.e;
@@ -686,10 +694,9 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
         transpose4(mask, sub, u1);
         transpose4(mask, sub, x1);
 #pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            P = fmaf(u0[l], x0[l], P);
-            P = fmaf(u1[l], x1[l], P);
-        }
+        for (int l = 0; l < 4; ++l) P = fmaf(u0[l], x0[l], P);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) P = fmaf(u1[l], x1[l], P);
         if ((k & 31) == 24 && k + 8 <= c) {   // 32 entries summed
             df_add(Dh, Dl, P);
             P = 0.0f;
