@@ -25,7 +25,7 @@
 #include <cstring>
 
 #include "sph_fixpoint.cuh"
-#include "sph_internal.cuh"
+#include "sph_physics.cuh"
 
 namespace sph {
 
@@ -829,9 +829,12 @@ __global__ void k_pack_pos(int n, const double *x, const double *y, const double
     if (i >= n) return;
     const double H = SUPPORT * h[i];
     H2f[i] = __double2float_ru(H * H);
-    const float ax = (float)x[i], ay = (float)y[i], az = (float)z[i];
-    xh[i] = make_float4(ax, ay, az, (float)(m[i] * mscale));
-    xl[i] = make_float4((float)(x[i] - (double)ax), (float)(y[i] - (double)ay), (float)(z[i] - (double)az), 0.0f);
+    float a, b, c, d, e, f;
+    split_df(x[i], a, d);
+    split_df(y[i], b, e);
+    split_df(z[i], c, f);
+    xh[i] = make_float4(a, b, c, (float)(m[i] * mscale));
+    xl[i] = make_float4(d, e, f, 0.0f);
 }
 
 // spill range lengths: rows longer than K take round8(count - K) entries beyond the row block
