@@ -187,6 +187,7 @@ k_grav_lists(int ng, const int *__restrict__ group_cell, const double *__restric
 
 // the totals of the counting pass and its error word, for the host (pinned memory)
 __global__ void k_list_totals(const int *oe, const int *ne, const int *os, const int *ns, const int *err, int *host) {
+    after_previous();
     const int *p[5] = {oe, ne, os, ns, err};
     if (threadIdx.x == 0)
         for (int k = 0; k < 5; ++k) host[k] = *p[k];
@@ -217,14 +218,14 @@ int sph_build_grav_lists(sph_ctx *ctx) {
     const int ng = G.ng;
     int *hs = (int *)ctx->host_scalars;
     SPH_CUDA(ctx, cudaMemsetAsync(t.meta + META_ERR, 0, sizeof(int), st));
-    k_grav_lists<false><<<ng, GL_T, 0, st>>>(ng, G.group_cell, FLD(ctx->F, SPH_X, ctx->cap),
-                                                         FLD(ctx->F, SPH_Y, ctx->cap), FLD(ctx->F, SPH_Z, ctx->cap),
-                                                         t.cinfo, t.level, t.com, t.rb, ctx->runs.prun, G.n_epj, G.n_spj, nullptr,
-                                                         nullptr, nullptr, nullptr, t.meta + META_ERR); ++ctx->launches;
+    k_grav_lists<false><<<ng, GL_T, 0, st>>>(
+        ng, G.group_cell, FLD(ctx->F, SPH_X, ctx->cap), FLD(ctx->F, SPH_Y, ctx->cap), FLD(ctx->F, SPH_Z, ctx->cap),
+        t.cinfo, t.level, t.com, t.rb, ctx->runs.prun, G.n_epj, G.n_spj, nullptr, nullptr, nullptr, nullptr,
+        t.meta + META_ERR); ++ctx->launches;
     SPH_TRY(sph_scan_exclusive(ctx, G.n_epj, G.off_epj, nullptr, ng, nullptr));
     SPH_TRY(sph_scan_exclusive(ctx, G.n_spj, G.off_spj, nullptr, ng, nullptr));
-    k_list_totals<<<1, 32, 0, st>>>(G.off_epj + (ng - 1), G.n_epj + (ng - 1), G.off_spj + (ng - 1), G.n_spj + (ng - 1),
-                                    t.meta + META_ERR, hs); ++ctx->launches;
+    launch_after(true, k_list_totals, 1, 32, 0, st, G.off_epj + (ng - 1), G.n_epj + (ng - 1), G.off_spj + (ng - 1),
+                 G.n_spj + (ng - 1), t.meta + META_ERR, hs); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     SPH_CUDA(ctx, cudaStreamSynchronize(st));
     if (hs[4] & ERR_GRAV_OVERFLOW) return sph_fail(ctx, SPH_ERR_CAPACITY, "gravity walk stack overflow");
@@ -241,10 +242,10 @@ int sph_build_grav_lists(sph_ctx *ctx) {
     }
     G.tot_epj = tot_e;
     G.tot_spj = tot_s;
-    k_grav_lists<true><<<ng, GL_T, 0, st>>>(ng, G.group_cell, FLD(ctx->F, SPH_X, ctx->cap),
-                                                        FLD(ctx->F, SPH_Y, ctx->cap), FLD(ctx->F, SPH_Z, ctx->cap),
-                                                        t.cinfo, t.level, t.com, t.rb, ctx->runs.prun, G.n_epj, G.n_spj, G.off_epj,
-                                                        G.off_spj, G.epj, G.spj, t.meta + META_ERR); ++ctx->launches;
+    k_grav_lists<true><<<ng, GL_T, 0, st>>>(
+        ng, G.group_cell, FLD(ctx->F, SPH_X, ctx->cap), FLD(ctx->F, SPH_Y, ctx->cap), FLD(ctx->F, SPH_Z, ctx->cap),
+        t.cinfo, t.level, t.com, t.rb, ctx->runs.prun, G.n_epj, G.n_spj, G.off_epj, G.off_spj, G.epj, G.spj,
+        t.meta + META_ERR); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     G.valid = true;
     G.counts_valid = true;

@@ -360,6 +360,7 @@ __global__ void k_viol_mark(int n, const double *h, const double *hsup, float *v
 
 // after a density round: (2.5 h)^2 of the new h as k_h2f, and the count of k_viol_mark
 __global__ void k_h2f_viol(int n, const double *h, const double *hsup, float *H2f, int *nviol) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool v = false;
     if (i < n) {
@@ -825,6 +826,7 @@ __global__ void k_h2f(int n, const double *h, float *H2f) {
 // double-float positions (hi / lo floats); .w of xh carries the mass x mscale; (2.5 h)^2 as k_h2f
 __global__ void k_pack_pos(int n, const double *x, const double *y, const double *z, const double *m, double mscale,
                            const double *h, float4 *xh, float4 *xl, float *H2f) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double H = SUPPORT * h[i];
@@ -909,10 +911,9 @@ int sph_nbr_prepare(sph_ctx *ctx) {
     if (ctx->cfg.precision == SPH_PREC_MIXED) {   // the mixed path walks on its own packs
         SPH_TRY(sph_pack_mixed(ctx));
     } else {
-        k_pack_pos<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
-                                                                FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap),
-                                                                ctx->mscale, FLD(ctx->F, SPH_SMTH, cap), S.pxh, S.pxl,
-                                                                S.H2f);
+        launch_after(true, k_pack_pos, sph_div_up(n, 256), 256, 0, ctx->stream, n, FLD(ctx->F, SPH_X, cap),
+                     FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap), ctx->mscale,
+                     FLD(ctx->F, SPH_SMTH, cap), S.pxh, S.pxl, S.H2f);
         ++ctx->launches;
     }
     SPH_CUDA(ctx, cudaGetLastError());
@@ -975,8 +976,7 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         WalkTree T{t.cinfo, t.blo, t.bhi};
         if (blocks > 0) {
             auto walk = S.spill_on ? k_sup_walk<true> : k_sup_walk<false>;
-            walk<<<blocks, NB_WARPS * 32, 0, ctx->stream>>>(
-                n_walk, split, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
+            walk<<<blocks, NB_WARPS * 32, 0, ctx->stream>>>(n_walk, split, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
                 FLD(ctx->F, SPH_SMTH, cap), S.hsup, walk_xh(ctx), walk_xl(ctx), S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
                 S.cnt, S.map(), S.uover, meta + META_ERR, meta + META_MAXCNT);
             ++ctx->launches;
@@ -1097,8 +1097,7 @@ static int filter_lists(sph_ctx *ctx, int mode) {
     const int64_t cap = ctx->cap;
     SphLists &L0 = ctx->lists[0], &L1 = ctx->lists[1];
     auto filter = mode == 0 ? k_filter<0> : (mode == 1 ? k_filter<1> : k_filter<2>);
-    filter<<<sph_div_up(n, FW), FW * 32, 0, ctx->stream>>>(
-        n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
+    filter<<<sph_div_up(n, FW), FW * 32, 0, ctx->stream>>>(n, S.nbr, S.r2, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
         FLD(ctx->F, SPH_SMTH, cap), S.H2f, L0.nbr, L0.cnt, L1.nbr, L1.cnt);
     ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
@@ -1154,13 +1153,13 @@ int sph_density_fused(sph_ctx *ctx) {
         const int dt = (int64_t)n < (int64_t)ctx->num_sms * DENS_SMALL ? 8 : 2;
         auto kd = ctx->runs.fix_split ? (dt == 8 ? k_density_fused32<true, 8> : k_density_fused32<true, 2>)
                                       : (dt == 8 ? k_density_fused32<false, 8> : k_density_fused32<false, 2>);
-        kd<<<sph_div_up((int64_t)n * dt, 64), 64, 0, ctx->stream>>>(
-            n, np, S.nbr, S.r2, S.m, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
+        kd<<<sph_div_up((int64_t)n * dt, 64), 64, 0, ctx->stream>>>(n, np, S.nbr, S.r2, S.m, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
             FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap), FLD(ctx->F, SPH_SMTH, cap), S.hsup,
             FLD(ctx->F, SPH_DENS, cap), (float)(1365.0 / 64.0 / (3.141592653589793 * ctx->mscale)), S.npass,
             stopped, ctx->runs.prun, ctx->runs.fixd);
         ++ctx->launches;
-        k_h2f_viol<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_SMTH, cap), S.hsup, S.H2f, nviol);
+        launch_after(true, k_h2f_viol, sph_div_up(n, 256), 256, 0, ctx->stream, n, FLD(ctx->F, SPH_SMTH, cap), S.hsup,
+                     S.H2f, nviol);
         ++ctx->launches;
         SPH_CUDA(ctx, cudaGetLastError());
         SPH_TRY(time_mark(ctx, SEG_DENS));

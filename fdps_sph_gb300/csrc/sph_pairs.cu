@@ -60,6 +60,7 @@ template <int PARTS>   // 1: x; 2: x, v; 4: all
 __global__ void k_pack64(int n, const double *x, const double *y, const double *z, const double *m, const double *vx,
                          const double *vy, const double *vz, const double *h, const double *dens, const double *pres,
                          const double *snds, const double *gradh, const double *bal, Pack64 P) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     P.x[i] = make_double4(x[i], y[i], z[i], m[i]);
@@ -111,9 +112,10 @@ __global__ void __launch_bounds__(LB) k_density64(int n, const double4 *__restri
 // ---------------------------------------------------------------------------
 // EoS, CalcPressure (force.h:26-32)
 
-__global__ void k_eos(int n, const DevMaterial *__restrict__ mats, const int32_t *__restrict__ mat,
-                      const double *__restrict__ dens, const double *__restrict__ eng, double *__restrict__ pres,
-                      double *__restrict__ snds) {
+__global__ void k_eos(int n, const DevMaterial *mats, const int32_t *mat,
+                      const double *dens, const double *eng, double *pres,
+                      double *snds) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double P, cs;
@@ -134,6 +136,7 @@ struct DrvtArgs {
 };
 
 __global__ void __launch_bounds__(LB) k_drvt64(int n, DrvtArgs a) {
+    after_previous();
     __shared__ double s_sum[LI][6];
     const int t = threadIdx.x, sub = t % LT, g = t / LT;
     const int li = blockDim.x / LT, i = blockIdx.x * li + g;
@@ -201,6 +204,7 @@ __device__ __forceinline__ Hydro64 hydro64_of(const double4 &a, const double4 &b
 }
 
 __global__ void __launch_bounds__(LB) k_hydro64(int n, HydroArgs a) {
+    after_previous();
     const int t = threadIdx.x, sub = t % LT;
     const int i = blockIdx.x * (blockDim.x / LT) + t / LT;
     const bool act = i < n;
@@ -315,6 +319,7 @@ k_grav64(const int *__restrict__ group_cell, const int4 *__restrict__ cinfo, int
 __global__ void k_pack_df(int n, const double *x, const double *y, const double *z, const double *vx,
                           const double *vy, const double *vz, const double *m, const double *h, double mscale,
                           float4 *xh, float4 *xl, float4 *vh, float4 *vl, float *H2f, int *npass) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float a, b, c, d, e, f;
@@ -476,6 +481,7 @@ __device__ __forceinline__ void transpose4(unsigned mask, int sub, float v[4]) {
 
 
 __global__ void __launch_bounds__(PT) k_drvt32_lanes(int n, DrvtArgs32 a) {
+    after_previous();
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gt / 4, sub = gt % 4;
     if (i >= n) return;   // whole groups of four lanes leave together
@@ -529,6 +535,7 @@ __global__ void __launch_bounds__(PT) k_drvt32_lanes(int n, DrvtArgs32 a) {
 
 template <int TPI>
 __global__ void __launch_bounds__(PT) k_drvt32(int n, DrvtArgs32 a) {
+    after_previous();
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gt / TPI, sub = gt % TPI;
     if (i >= n) return;   // whole groups of TPI lanes leave together
@@ -579,6 +586,7 @@ __global__ void __launch_bounds__(PT) k_drvt32(int n, DrvtArgs32 a) {
 __global__ void k_hydro_pack32(int n, const double *h, const double *dens, const double *pres, const double *snds,
                                const double *gradh, const double *bal, float4 *hA, float4 *xl, float4 *vh,
                                float4 *vl) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float hi = (float)h[i], H = __fmul_rn((float)SUPPORT, hi), rho = (float)dens[i], f = (float)gradh[i];
@@ -661,6 +669,7 @@ __device__ __forceinline__ HydroJ32 load_hydro_j(const HydroArgs32 &a, int j) {
 
 // one thread's order on four lanes, as k_drvt32_lanes: lane q keeps component q
 __global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
+    after_previous();
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gt / 4, sub = gt % 4;
     if (i >= n) return;   // whole groups of four lanes leave together
@@ -714,6 +723,7 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32_lanes(int n, HydroArgs32 a) {
 // 72 registers and spills)
 template <int TPI>
 __global__ void __launch_bounds__(PT, 6) k_hydro32(int n, HydroArgs32 a) {
+    after_previous();
     const int gt = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gt / TPI, sub = gt % TPI;
     if (i >= n) return;   // whole groups of TPI lanes leave together
@@ -770,6 +780,7 @@ __global__ void __launch_bounds__(PT, 6) k_hydro32(int n, HydroArgs32 a) {
 // (err, if given, is cleared)
 __global__ void k_pack_cells32(const int *meta, const double4 *com, double G, double gscale, float4 *ch, float4 *cl,
                                int *err) {
+    after_previous();
     if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const int nc = meta[MAX_LEVELS];
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
@@ -1286,6 +1297,7 @@ struct IntegArgs {
 };
 
 __global__ void k_kick_drift_predict(int n, IntegArgs a) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double dt = a.run_dt[a.prun[i]];
@@ -1305,6 +1317,7 @@ __global__ void k_kick_drift_predict(int n, IntegArgs a) {
 }
 
 __global__ void k_final_kick(int n, IntegArgs a, double damp) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double dt = a.run_dt[a.prun[i]];
@@ -1377,6 +1390,7 @@ __device__ double block_min(double r) {
 }
 
 __global__ void k_min_tiles(const double *v, const int4 *tiles, double *part) {
+    after_previous();
     const int4 t = tiles[blockIdx.x];
     double r = 1.0e30;
     for (int i = t.x + threadIdx.x; i < t.x + t.y; i += blockDim.x) {
@@ -1389,6 +1403,7 @@ __global__ void k_min_tiles(const double *v, const int4 *tiles, double *part) {
 }
 
 __global__ void k_min_runs(const double *part, const int4 *info, double *out, double *host) {
+    after_previous();
     const int4 q = info[blockIdx.x];
     double r = 1.0e30;
     for (int b = q.z + threadIdx.x; b < q.z + q.w; b += blockDim.x) r = (part[b] < r || part[b] != part[b]) ? part[b] : r;
@@ -1531,10 +1546,9 @@ static int ensure_mixed_buffers(sph_ctx *ctx) {
 int sph_pack_mixed(sph_ctx *ctx) {
     SPH_TRY(ensure_mixed_buffers(ctx));
     const int n = (int)ctx->n;
-    k_pack_df<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), CF(SPH_VX), CF(SPH_VY),
-                                                           CF(SPH_VZ), CF(SPH_MASS), CF(SPH_SMTH),
-                                                           ctx->mscale, ctx->xh, ctx->xl, ctx->vhf,
-                                                           ctx->vlf, ctx->sup.H2f, ctx->sup.npass); ++ctx->launches;
+    launch_after(true, k_pack_df, sph_div_up(n, 256), 256, 0, ctx->stream, n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z),
+                 CF(SPH_VX), CF(SPH_VY), CF(SPH_VZ), CF(SPH_MASS), CF(SPH_SMTH), ctx->mscale, ctx->xh, ctx->xl,
+                 ctx->vhf, ctx->vlf, ctx->sup.H2f, ctx->sup.npass); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -1546,9 +1560,9 @@ static Pack64 pack64(sph_ctx *ctx) {
     const int n = (int)ctx->n;
     double4 *f = (double4 *)ctx->F2;
     const Pack64 P{f, f + ctx->cap, f + 2 * ctx->cap, f + 3 * ctx->cap};
-    k_pack64<PARTS><<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(
-        n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), CF(SPH_MASS), CF(SPH_VX), CF(SPH_VY), CF(SPH_VZ), CF(SPH_SMTH),
-        CF(SPH_DENS), CF(SPH_PRES), CF(SPH_SNDS), CF(SPH_GRADH), CF(SPH_BAL), P); ++ctx->launches;
+    launch_after(true, k_pack64<PARTS>, sph_div_up(n, 256), 256, 0, ctx->stream, n, CF(SPH_X), CF(SPH_Y), CF(SPH_Z),
+                 CF(SPH_MASS), CF(SPH_VX), CF(SPH_VY), CF(SPH_VZ), CF(SPH_SMTH), CF(SPH_DENS), CF(SPH_PRES),
+                 CF(SPH_SNDS), CF(SPH_GRADH), CF(SPH_BAL), P); ++ctx->launches;
     return P;
 }
 
@@ -1579,8 +1593,8 @@ int sph_pass_density(sph_ctx *ctx, int build_lists) {
 
 int sph_pass_eos(sph_ctx *ctx) {
     const int n = (int)ctx->n;
-    k_eos<<<sph_div_up(n, PT), PT, 0, ctx->stream>>>(n, ctx->mats_dev, ctx->mat, CF(SPH_DENS), CF(SPH_ENG),
-                                                    CF(SPH_PRES), CF(SPH_SNDS)); ++ctx->launches;
+    launch_after(true, k_eos, sph_div_up(n, PT), PT, 0, ctx->stream, n, ctx->mats_dev, ctx->mat, CF(SPH_DENS),
+                 CF(SPH_ENG), CF(SPH_PRES), CF(SPH_SNDS)); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -1597,13 +1611,14 @@ int sph_pass_derivative(sph_ctx *ctx, int build_lists) {
         // threads per i-particle in the sums' order: chosen by sph_autotune (1 unless tuned)
         const int tpi = ctx->tune.drvt_tpi;
         auto kd = tpi == 4 ? k_drvt32<4> : (tpi == 2 ? k_drvt32<2> : k_drvt32_lanes);
-        kd<<<sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        launch_after(true, kd, sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream, n, a);
+        ++ctx->launches;
     } else {
         const Pack64 P = pack64<2>(ctx);
         const int li = block_i64(ctx, 16);
         DrvtArgs a{P.x,          P.v,          CF(SPH_SMTH),  CF(SPH_DENS), CF(SPH_SNDS), CF(SPH_DIVV), CF(SPH_ROTX),
                    CF(SPH_ROTY), CF(SPH_ROTZ), CF(SPH_GRADH), CF(SPH_BAL),  L.nbr,        L.cnt,        ctx->sup.map()};
-        k_drvt64<<<sph_div_up(n, li), li * LT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        launch_after(true, k_drvt64, sph_div_up(n, li), li * LT, 0, ctx->stream, n, a); ++ctx->launches;
     }
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
@@ -1616,20 +1631,21 @@ int sph_pass_hydro(sph_ctx *ctx, int build_lists) {
     // scratch in the F2 ping-pong block (free between sorts)
     if (ctx->cfg.precision == SPH_PREC_MIXED) {
         float4 *hA = (float4 *)ctx->F2;
-        k_hydro_pack32<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, CF(SPH_SMTH), CF(SPH_DENS), CF(SPH_PRES),
-                                                                    CF(SPH_SNDS), CF(SPH_GRADH), CF(SPH_BAL), hA,
-                                                                    ctx->xl, ctx->vhf, ctx->vlf); ++ctx->launches;
+        launch_after(true, k_hydro_pack32, sph_div_up(n, 256), 256, 0, ctx->stream, n, CF(SPH_SMTH), CF(SPH_DENS),
+                     CF(SPH_PRES), CF(SPH_SNDS), CF(SPH_GRADH), CF(SPH_BAL), hA, ctx->xl, ctx->vhf, ctx->vlf);
+        ++ctx->launches;
         HydroArgs32 a{ctx->xh,    ctx->xl,    ctx->vhf,   ctx->vlf,       hA,    CF(SPH_SMTH),
                       CF(SPH_AX), CF(SPH_AY), CF(SPH_AZ), CF(SPH_ENGDOT), CF(SPH_DT), L.nbr, L.cnt,
                       ctx->sup.map(),    (float)(WNORM / (PI_D * ctx->mscale))};
         const int tpi = ctx->tune.hydro_tpi;
         auto kh = tpi == 4 ? k_hydro32<4> : (tpi == 2 ? k_hydro32<2> : k_hydro32_lanes);
-        kh<<<sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        launch_after(true, kh, sph_div_up((int64_t)n * (tpi == 1 ? 4 : tpi), PT), PT, 0, ctx->stream, n, a);
+        ++ctx->launches;
     } else {
         const int li = block_i64(ctx, 8);
         HydroArgs a{pack64<4>(ctx), CF(SPH_SMTH), CF(SPH_AX), CF(SPH_AY), CF(SPH_AZ), CF(SPH_ENGDOT), CF(SPH_DT),
                     L.nbr,          L.cnt,        ctx->sup.map()};
-        k_hydro64<<<sph_div_up(n, li), li * LT, 0, ctx->stream>>>(n, a); ++ctx->launches;
+        launch_after(true, k_hydro64, sph_div_up(n, li), li * LT, 0, ctx->stream, n, a); ++ctx->launches;
     }
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
@@ -1645,7 +1661,8 @@ int sph_pass_gravity(sph_ctx *ctx, int build_lists) {
         if ((int64_t)t.n_cell_host * 2 > ctx->cap * 4) return sph_fail(ctx, SPH_ERR_CAPACITY, "cell pack scratch");
         float4 *ch = (float4 *)ctx->F2, *cl = ch + t.n_cell_host;
         const double gscale = 1.0;
-        k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, gscale, ch, cl, nullptr);
+        launch_after(true, k_pack_cells32, 2 * ctx->num_sms, 256, 0, ctx->stream, t.meta, t.com, ctx->cfg.G, gscale, ch,
+                     cl, nullptr);
         ++ctx->launches;
         k_grav32<<<G.ng, GT, 0, ctx->stream>>>(G.group_cell, t.start, t.count, ctx->xh, ctx->xl, CF(SPH_MASS),
                                                CF(SPH_SMTH), ch, cl, G.n_epj, G.off_epj, G.epj, G.n_spj, G.off_spj,
@@ -1666,14 +1683,16 @@ int sph_pass_gravity(sph_ctx *ctx, int build_lists) {
 // the step's dt of every run is in runs.dt_dev (set by sph_run_reduce_dt or the host)
 int sph_kick_drift_predict(sph_ctx *ctx) {
     const int n = (int)ctx->n;
-    k_kick_drift_predict<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, integ_args(ctx)); ++ctx->launches;
+    launch_after(true, k_kick_drift_predict, sph_div_up(n, 256), 256, 0, ctx->stream, n, integ_args(ctx));
+    ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
 
 int sph_final_kick(sph_ctx *ctx) {
     const int n = (int)ctx->n;
-    k_final_kick<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, integ_args(ctx), ctx->cfg.damping); ++ctx->launches;
+    launch_after(true, k_final_kick, sph_div_up(n, 256), 256, 0, ctx->stream, n, integ_args(ctx), ctx->cfg.damping);
+    ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -1700,11 +1719,12 @@ int sph_ext_force(sph_ctx *ctx) {
 // getTimeStepGlobal (integral.h:4-20) for every run: min over the run's dt_i into runs.dt_dev and runs.dt
 int sph_run_reduce_dt(sph_ctx *ctx) {
     Runs &R = ctx->runs;
-    k_min_tiles<<<R.T, 256, 0, ctx->stream>>>(CF(SPH_DT), R.tiles, R.part); ++ctx->launches;
+    launch_after(true, k_min_tiles, R.T, 256, 0, ctx->stream, CF(SPH_DT), R.tiles, R.part); ++ctx->launches;
     // the host's values straight into the pinned block (behind the words of sph_publish) where they fit it
     double *h = ctx->host_scalars + 32;
     const bool fits = R.R <= 480;
-    k_min_runs<<<R.R, 256, 0, ctx->stream>>>(R.part, R.info, R.dt_dev, fits ? h : nullptr); ++ctx->launches;
+    launch_after(true, k_min_runs, R.R, 256, 0, ctx->stream, R.part, R.info, R.dt_dev, fits ? h : nullptr);
+    ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     std::vector<double> many;
     if (!fits) {
@@ -1795,8 +1815,7 @@ static int launch_grav_fused(sph_ctx *ctx, bool wide) {
     if (wide) SPH_CUDA(ctx, cudaMemsetAsync(t.meta + META_ERR, 0, sizeof(int), ctx->stream));
     const bool one = !wide && G.ng < ctx->num_sms * GRAV_ONE;
     auto kern = wide ? k_grav_fused32<256, 2> : (one ? k_grav_fused32<128, 1> : k_grav_fused32<128, 2>);
-    kern<<<dim3(G.ng, one ? 2 : 1), wide ? 256 : 128, 0, ctx->stream>>>(
-        G.group_cell, t.cinfo, t.com, t.rb, ctx->runs.prun, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), ctx->xh, ctx->xl,
+    kern<<<dim3(G.ng, one ? 2 : 1), wide ? 256 : 128, 0, ctx->stream>>>(G.group_cell, t.cinfo, t.com, t.rb, ctx->runs.prun, CF(SPH_X), CF(SPH_Y), CF(SPH_Z), ctx->xh, ctx->xl,
         CF(SPH_SMTH), chp, clp, gms, CF(SPH_GX), CF(SPH_GY), CF(SPH_GZ), CF(SPH_POT), G.n_epj, G.n_spj,
         t.meta + META_ERR);
     ++ctx->launches;
@@ -1817,7 +1836,8 @@ int sph_gravity_fused(sph_ctx *ctx, bool later) {
     if (G.ng == 0) return SPH_OK;
     if ((int64_t)t.n_cell_host * 2 > ctx->cap * 4) return sph_fail(ctx, SPH_ERR_CAPACITY, "cell pack scratch");
     float4 *chp = (float4 *)ctx->F2, *clp = chp + t.n_cell_host;
-    k_pack_cells32<<<2 * ctx->num_sms, 256, 0, ctx->stream>>>(t.meta, t.com, ctx->cfg.G, 1.0, chp, clp, t.meta + META_ERR);
+    launch_after(true, k_pack_cells32, 2 * ctx->num_sms, 256, 0, ctx->stream, t.meta, t.com, ctx->cfg.G, 1.0, chp, clp,
+                 t.meta + META_ERR);
     ++ctx->launches;
     SPH_TRY(launch_grav_fused(ctx, false));
     G.counts_valid = true;

@@ -68,6 +68,7 @@ __device__ T parts_before(const T *part, T *total) {
 }
 
 __global__ void k_scan_reduce(const int *in, LenArg len, int *part) {
+    after_previous();
     const int n = len.get();
     const int chunk = (n + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * chunk;
@@ -80,6 +81,7 @@ __global__ void k_scan_reduce(const int *in, LenArg len, int *part) {
 }
 
 __global__ void k_scan_down(const int *in, int *out, LenArg len, const int *part, int *total) {
+    after_previous();
     const int n = len.get();
     const int chunk = (n + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * chunk;
@@ -105,8 +107,10 @@ using namespace sph;
 // device (len_dev, if non-null) or host
 int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev, int len_host, int *total_dev) {
     LenArg L{len_dev, len_host, 0};
-    k_scan_reduce<<<SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream>>>(in, L, ctx->scan.part); ++ctx->launches;
-    k_scan_down<<<SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream>>>(in, out, L, ctx->scan.part, total_dev); ++ctx->launches;
+    launch_after(true, k_scan_reduce, SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream, in, L, ctx->scan.part);
+    ++ctx->launches;
+    launch_after(true, k_scan_down, SCAN_BLOCKS, SCAN_THREADS, 0, ctx->stream, in, out, L, ctx->scan.part, total_dev);
+    ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -117,6 +121,7 @@ namespace sph {
 // the copy engine is a detour of the stream.  With the words that need clearing cleared by kernels that run anyway, a
 // step of 5,000 particles 448 -> 427 us, of 100,000 1.247 -> 1.206 ms, of 10,000 in FP64 1.95 -> 1.90 ms.
 __global__ void k_publish(const int *src, int n, int *host) {
+    after_previous();
     if ((int)threadIdx.x < n) host[threadIdx.x] = src[threadIdx.x];
 }
 
@@ -124,7 +129,7 @@ __global__ void k_publish(const int *src, int n, int *host) {
 
 // src[0 .. n) (n <= 64 ints) into the first words of host_scalars, in stream order
 int sph_publish(sph_ctx *ctx, const int *src, int n) {
-    k_publish<<<1, 64, 0, ctx->stream>>>(src, n, (int *)ctx->host_scalars); ++ctx->launches;
+    launch_after(true, k_publish, 1, 64, 0, ctx->stream, src, n, (int *)ctx->host_scalars); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
 }
@@ -174,9 +179,11 @@ struct Box {
 };
 
 // block b: the box of every gridDim.x-th 256 positions; also clears the counts the key kernel and the sort's first
-// pass add to (n_clear words)
+// pass add to (n_clear words) and the error word
 __global__ void k_bbox_partial(const double *x, const double *y, const double *z, int n, long long *part,
-                               uint32_t *clear, int n_clear) {
+                               uint32_t *clear, int n_clear, int *err) {
+    after_previous();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     Box b;
     b.empty();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b.add(x[i], y[i], z[i]);
@@ -217,6 +224,7 @@ __device__ void root_cube(const Box &x, double theta, double *rb) {
 
 // one block reduces the partial boxes (min / max are exact in any order), then one thread forms the root cube
 __global__ void k_bbox_final(const long long *part, int nb, double theta, double *rb) {
+    after_previous();
     Box x;
     x.empty();
     for (int b = threadIdx.x; b < nb; b += blockDim.x)
@@ -229,6 +237,7 @@ __global__ void k_bbox_final(const long long *part, int nb, double theta, double
 // first pass's), one block per run the tiles of the run
 __global__ void k_bbox_tiles(const double *x, const double *y, const double *z, const int4 *tiles, long long *part,
                              uint32_t *hist, uint32_t *next) {
+    after_previous();
     const int4 t = tiles[blockIdx.x];
     Box b;
     b.empty();
@@ -248,6 +257,7 @@ __global__ void k_bbox_tiles(const double *x, const double *y, const double *z, 
 // also the run's octree root (level 0: cell r = run r) and, from block 0, an empty meta block
 __global__ void k_bbox_runs(const long long *part, const int4 *info, double theta, double *rb, int *meta, int *start,
                             int *count, int *level, int *parent, int *first_child, int *n_child) {
+    after_previous();
     const int4 r = info[blockIdx.x];
     Box x;
     x.empty();
@@ -327,6 +337,7 @@ __device__ __forceinline__ int4 rs_tile(const int4 *tiles, int n, int nb) {
 __global__ void __launch_bounds__(RS_THREADS) k_keys_hist(const double *x, const double *y, const double *z, int n,
                                                           const double *rb, const int *prun, const int4 *tiles, int nb,
                                                           uint64_t *keys, uint32_t *hist, int *err) {
+    after_previous();
     __shared__ uint32_t h[256];
     const int t = threadIdx.x, tile = blockIdx.x / RS_SUB, p = blockIdx.x % RS_SUB * RS_THREADS + t;
     if (t < 256) h[t] = 0;
@@ -350,6 +361,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_keys_hist(const double *x, const
 // tot[first tile][digit] = in all of them.  Warp w sums the w-th 32nd of the tiles, a digit per lane.
 __global__ void __launch_bounds__(1024) k_rs_scan(const uint32_t *hist, const int4 *info, uint32_t *off,
                                                   uint32_t *tot) {
+    after_previous();
     __shared__ uint32_t s[32][32];
     const int4 r = info[blockIdx.y];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
@@ -377,6 +389,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_scatter(const uint64_t *ki
                                                            uint32_t *vout, int n, int shift, const uint32_t *hist,
                                                            uint32_t *next, uint32_t *clear, const uint32_t *off,
                                                            const uint32_t *tot, int nb, const int4 *tiles) {
+    after_previous();
     // per-warp digit counts, then per-warp offsets within a digit; then the reordered tile
     __shared__ __align__(8) unsigned char s_buf[RS_TILE * (sizeof(uint64_t) + sizeof(uint32_t))];
     static_assert(sizeof(s_buf) >= RS_WARPS * 256 * sizeof(uint32_t), "the counters fit the tile's buffer");
@@ -505,6 +518,7 @@ constexpr int RB_T = 1024, RB_ITEMS = 8, RB_KEYS = RB_T * RB_ITEMS, RB_W = RB_T 
 constexpr size_t RB_SMEM = RB_KEYS * (sizeof(uint64_t) + sizeof(uint16_t)) + RB_W * 256 * sizeof(uint16_t);
 __global__ void __launch_bounds__(RB_T) k_rs_block(const uint64_t *kin, uint64_t *kout, uint32_t *vout,
                                                    const int4 *info) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char rb_smem[];
     uint64_t *sk = reinterpret_cast<uint64_t *>(rb_smem);
     uint16_t *sv = reinterpret_cast<uint16_t *>(sk + RB_KEYS);
@@ -601,6 +615,7 @@ __global__ void __launch_bounds__(RB_T) k_rs_block(const uint64_t *kin, uint64_t
 __global__ void k_permute(const double *F, double *F2, int64_t cap, int n, const uint32_t *perm, const int64_t *id,
                           int64_t *id2, const int32_t *slot, int32_t *slot2, const int32_t *mat, int32_t *mat2,
                           const int *prun, int *prun2) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int src = (int)perm[k];
@@ -641,9 +656,10 @@ __device__ __forceinline__ int key_common(uint64_t a, uint64_t b) {
 
 // per particle: the levels at which it starts a cell (lo | hi << 8, empty when hi < lo), and per
 // block and level the number of cells starting in the block (cnt[L * n_blocks + block])
-__global__ void __launch_bounds__(OT_B) k_cell_levels(int n, int n_leaf, const uint64_t *__restrict__ keys,
-                                                      const int *__restrict__ prun, const int4 *__restrict__ info,
-                                                      int *__restrict__ lev, int *__restrict__ cnt) {
+__global__ void __launch_bounds__(OT_B) k_cell_levels(int n, int n_leaf, const uint64_t *keys,
+                                                      const int *prun, const int4 *info,
+                                                      int *lev, int *cnt) {
+    after_previous();
     __shared__ uint64_t sk[OT_B + 2 * OT_HALO];
     __shared__ int sc[MAX_LEVELS];
     const int t = threadIdx.x, b0 = blockIdx.x * OT_B, i = b0 + t;
@@ -681,11 +697,12 @@ __global__ void __launch_bounds__(OT_B) k_cell_levels(int n, int n_leaf, const u
 // rank of the particle among its block's starts at that level; start, count (the end found by
 // a binary search over the run's keys), level.  Also the level offsets in meta; more cells than
 // the capacity sets ERR_CELL_OVERFLOW and leaves no cells.
-__global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const uint64_t *__restrict__ keys,
-                                                    const int *__restrict__ prun, const int4 *__restrict__ info,
-                                                    const int *__restrict__ lev, const int *__restrict__ cnt,
-                                                    const int *__restrict__ off, int *meta, int *start, int *count,
+__global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const uint64_t *keys,
+                                                    const int *prun, const int4 *info,
+                                                    const int *lev, const int *cnt,
+                                                    const int *off, int *meta, int *start, int *count,
                                                     int *level) {
+    after_previous();
     __shared__ int sw[MAX_LEVELS][OT_B / 32];
     const int nb = gridDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, i = blockIdx.x * OT_B + t;
     const int64_t last = (int64_t)(MAX_LEVELS - 1) * nb + nb - 1;
@@ -733,7 +750,8 @@ __global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const ui
 // parent, first child and child count of every cell, by binary searches over the starts of the
 // levels above and below (each level's cells are sorted by start)
 __global__ void k_cell_link(const int *meta, const int *start, const int *count, const int *level, int *parent,
-                            int *first_child, int *n_child) {
+                            int *first_child, int *n_child, int *arrive) {
+    after_previous();
     const int nc = meta[MAX_LEVELS];
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
         const int L = level[c], s = start[c], e = s + count[c];
@@ -769,6 +787,7 @@ __global__ void k_cell_link(const int *meta, const int *start, const int *count,
         parent[c] = p;
         first_child[c] = f;
         n_child[c] = nch;
+        arrive[c] = 0;
     }
 }
 
@@ -789,6 +808,7 @@ __global__ void __launch_bounds__(128)
 k_moments_up(const int *meta, const double *x, const double *y, const double *z, const double *m, const double *h,
              const int *start, const int *count, const int *first_child, const int *n_child, const int *parent,
              int *arrive, double4 *mom, float4 *blo, float4 *bhi) {
+    after_previous();
     const int nc = meta[MAX_LEVELS], lane = threadIdx.x & 31, q = lane >> 2, comp = lane & 3;
     for (int cw = blockIdx.x * blockDim.x + (threadIdx.x & ~31); cw < nc; cw += gridDim.x * blockDim.x) {
         int c = cw + lane;
@@ -927,6 +947,7 @@ __global__ void __launch_bounds__(SCAN_THREADS)
 k_cell_roles(const int *meta, int n_group, const int *start, const int *count, const int *first_child,
              const int *n_child, const int *parent, const double4 *mom, double4 *com, int4 *cinfo, long long *role,
              long long *part) {
+    after_previous();
     const int nc = meta[MAX_LEVELS], n_roots = meta[1];
     const int chunk = (nc + gridDim.x - 1) / gridDim.x;
     const int b1 = min(nc, (int)(blockIdx.x + 1) * chunk);
@@ -950,6 +971,7 @@ k_cell_roles(const int *meta, int n_group, const int *start, const int *count, c
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_role_emit(const int *meta, const int4 *cinfo, const int *start, const int *count, const int *n_child,
             const long long *role, const long long *part, int2 *units, int *group_cell, long long *total) {
+    after_previous();
     const int nc = meta[MAX_LEVELS], n_roots = meta[1];
     const int chunk = (nc + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * chunk, b1 = min(nc, b0 + chunk);
@@ -1080,7 +1102,8 @@ static int radix_sort(sph_ctx *ctx, int n) {
     if (ctx->runs.max_tiles <= RB_KEYS / RUN_TILE) {
         static_assert(RB_KEYS % RUN_TILE == 0, "whole tiles");
         SPH_CUDA(ctx, cudaFuncSetAttribute(k_rs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RB_SMEM));
-        k_rs_block<<<ctx->runs.R, RB_T, RB_SMEM, ctx->stream>>>(s.k0, ctx->keys, s.v0, ctx->runs.info); ++ctx->launches;
+        launch_after(true, k_rs_block, ctx->runs.R, RB_T, RB_SMEM, ctx->stream, s.k0, ctx->keys, s.v0, ctx->runs.info);
+        ++ctx->launches;
         SPH_CUDA(ctx, cudaGetLastError());
         return SPH_OK;
     }
@@ -1092,13 +1115,14 @@ static int radix_sort(sph_ctx *ctx, int n) {
         uint32_t *next = last ? nullptr : s.hist + (pass + 1) % RS_HISTS * row;
         uint32_t *clear = last ? nullptr : s.hist + (pass + 2) % RS_HISTS * row;
         if (scan) {
-            k_rs_scan<<<dim3(8, ctx->runs.R), 1024, 0, ctx->stream>>>(hist, ctx->runs.info, s.hoff, s.hoff + row);
+            launch_after(true, k_rs_scan, dim3(8, ctx->runs.R), 1024, 0, ctx->stream, hist, ctx->runs.info, s.hoff,
+                         s.hoff + row);
             ++ctx->launches;
         }
-        k_rs_scatter<<<nb, RS_THREADS, 0, ctx->stream>>>(odd ? s.k1 : s.k0, pass == 0 ? nullptr : (odd ? s.v1 : s.v0),
-                                                         last ? ctx->keys : (odd ? s.k0 : s.k1), odd ? s.v0 : s.v1, n,
-                                                         8 * pass, hist, next, clear, scan ? s.hoff : nullptr,
-                                                         s.hoff + row, nb, tiles); ++ctx->launches;
+        launch_after(true, k_rs_scatter, nb, RS_THREADS, 0, ctx->stream, odd ? s.k1 : s.k0,
+                     pass == 0 ? nullptr : (odd ? s.v1 : s.v0), last ? ctx->keys : (odd ? s.k0 : s.k1),
+                     odd ? s.v0 : s.v1, n, 8 * pass, hist, next, clear, scan ? s.hoff : nullptr, s.hoff + row, nb,
+                     tiles); ++ctx->launches;
     }
     SPH_CUDA(ctx, cudaGetLastError());
     return SPH_OK;
@@ -1116,28 +1140,26 @@ static int enqueue_tree(sph_ctx *ctx) {
     const int grid = 2 * ctx->num_sms;
     const int nb = sph_div_up(n, OT_B);
     // scratch: tmp_off the particles' cell levels, tmp_cnt the block-and-level counts, tmp_b their scan
-    k_cell_levels<<<nb, OT_B, 0, st>>>(n, ctx->cfg.n_leaf, ctx->keys, ctx->runs.prun, ctx->runs.info, t.tmp_off,
-                                       t.tmp_cnt); ++ctx->launches;
+    launch_after(true, k_cell_levels, nb, OT_B, 0, st, n, ctx->cfg.n_leaf, ctx->keys, ctx->runs.prun, ctx->runs.info,
+                 t.tmp_off, t.tmp_cnt); ++ctx->launches;
     SPH_TRY(sph_scan_exclusive(ctx, t.tmp_cnt, t.tmp_b, nullptr, MAX_LEVELS * nb, nullptr));
-    k_cell_emit<<<nb, OT_B, 0, st>>>(n, t.cap, ctx->keys, ctx->runs.prun, ctx->runs.info, t.tmp_off, t.tmp_cnt,
-                                     t.tmp_b, t.meta, t.start, t.count, t.level); ++ctx->launches;
-    k_cell_link<<<grid, 256, 0, st>>>(t.meta, t.start, t.count, t.level, t.parent, t.first_child, t.n_child);
+    launch_after(true, k_cell_emit, nb, OT_B, 0, st, n, t.cap, ctx->keys, ctx->runs.prun, ctx->runs.info, t.tmp_off,
+                 t.tmp_cnt, t.tmp_b, t.meta, t.start, t.count, t.level); ++ctx->launches;
+    launch_after(true, k_cell_link, grid, 256, 0, st, t.meta, t.start, t.count, t.level, t.parent, t.first_child,
+                 t.n_child, t.tmp_cnt);
     ++ctx->launches;
-    // moments bottom-up in one launch (tmp_cnt, free again, counts the arrivals)
-    SPH_CUDA(ctx, cudaMemsetAsync(t.tmp_cnt, 0, sizeof(int) * t.cap, st));
+    // moments bottom-up in one launch (tmp_cnt, free again and cleared, counts the arrivals)
     // one thread per cell: the leaves' fences and arrivals all in flight at once
     const int grid_up = (int)std::min<int64_t>((t.cap + 127) / 128, 1 << 16);
-    k_moments_up<<<grid_up, 128, 0, st>>>(t.meta, x, y, z, m, h, t.start, t.count, t.first_child, t.n_child,
-                                          t.parent, t.tmp_cnt, t.mom, t.blo, t.bhi); ++ctx->launches;
+    launch_after(true, k_moments_up, grid_up, 128, 0, st, t.meta, x, y, z, m, h, t.start, t.count, t.first_child,
+                 t.n_child, t.parent, t.tmp_cnt, t.mom, t.blo, t.bhi); ++ctx->launches;
     // packed records, centres of mass, walk units, gravity groups (tmp_b, free again, as 64-bit numbers)
     static_assert(SCAN_BLOCKS == SCAN_THREADS, "parts_before");
     long long *role = (long long *)t.tmp_b, *part = (long long *)ctx->scan.part;
-    k_cell_roles<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, ctx->cfg.n_group, t.start, t.count, t.first_child,
-                                                       t.n_child, t.parent, t.mom, t.com, t.cinfo, role,
-                                                       part); ++ctx->launches;
-    k_role_emit<<<SCAN_BLOCKS, SCAN_THREADS, 0, st>>>(t.meta, t.cinfo, t.start, t.count, t.n_child, role, part,
-                                                      ctx->sup.units, ctx->grav.group_cell,
-                                                      (long long *)(t.meta + META_ROLES)); ++ctx->launches;
+    launch_after(true, k_cell_roles, SCAN_BLOCKS, SCAN_THREADS, 0, st, t.meta, ctx->cfg.n_group, t.start, t.count,
+                 t.first_child, t.n_child, t.parent, t.mom, t.com, t.cinfo, role, part); ++ctx->launches;
+    launch_after(true, k_role_emit, SCAN_BLOCKS, SCAN_THREADS, 0, st, t.meta, t.cinfo, t.start, t.count, t.n_child,
+                 role, part, ctx->sup.units, ctx->grav.group_cell, (long long *)(t.meta + META_ROLES)); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return sph_publish(ctx, t.meta, META_N);
 }
@@ -1155,17 +1177,16 @@ static int enqueue_sort_tree(sph_ctx *ctx) {
     const Runs &R = ctx->runs;
     uint32_t *hist = ctx->sort.hist, *next = hist + 256 * (int64_t)R.T;
     k_bbox_tiles<<<R.T, 512, 0, st>>>(x, y, z, R.tiles, (long long *)R.part, hist, next); ++ctx->launches;
-    k_bbox_runs<<<R.R, 256, 0, st>>>((const long long *)R.part, R.info, ctx->cfg.theta, t.rb, t.meta, t.start, t.count,
-                                     t.level, t.parent, t.first_child, t.n_child); ++ctx->launches;
-    k_keys_hist<<<R.T * RS_SUB, RS_THREADS, 0, st>>>(x, y, z, n, t.rb, R.prun, R.tiles, R.T, ctx->sort.k0,
-                                                     ctx->sort.hist, t.meta + META_ERR); ++ctx->launches;
+    launch_after(true, k_bbox_runs, R.R, 256, 0, st, (const long long *)R.part, R.info, ctx->cfg.theta, t.rb, t.meta,
+                 t.start, t.count, t.level, t.parent, t.first_child, t.n_child); ++ctx->launches;
+    launch_after(true, k_keys_hist, R.T * RS_SUB, RS_THREADS, 0, st, x, y, z, n, t.rb, R.prun, R.tiles, R.T,
+                 ctx->sort.k0, ctx->sort.hist, t.meta + META_ERR); ++ctx->launches;
     SPH_TRY(radix_sort(ctx, n));
     // permute the particle state into key order
     const int pb = (int)sph_div_up(n, 256);
     const int py = pb < 8 * ctx->num_sms ? 9 : 1;
-    k_permute<<<dim3(pb, py), 256, 0, st>>>(ctx->F, ctx->F2, cap, n, ctx->sort.v0, ctx->id, ctx->id2,
-                                                  ctx->slot, ctx->slot2, ctx->mat, ctx->mat2, R.prun,
-                                                  ctx->runs.prun2); ++ctx->launches;
+    launch_after(true, k_permute, dim3(pb, py), 256, 0, st, ctx->F, ctx->F2, cap, n, ctx->sort.v0, ctx->id, ctx->id2,
+                 ctx->slot, ctx->slot2, ctx->mat, ctx->mat2, R.prun, ctx->runs.prun2); ++ctx->launches;
     std::swap(ctx->F, ctx->F2);
     std::swap(ctx->runs.prun, ctx->runs.prun2);
     std::swap(ctx->id, ctx->id2);
