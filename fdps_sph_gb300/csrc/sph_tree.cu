@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const ui
                                                     const int *off, int *meta, int *start, int *count,
                                                     int *level) {
     after_previous();
-    __shared__ int sw[MAX_LEVELS][OT_B / 32];
+    __shared__ unsigned sb[MAX_LEVELS][OT_B / 32];   // per level and warp: the lanes that start a cell
     const int nb = gridDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, i = blockIdx.x * OT_B + t;
     const int64_t last = (int64_t)(MAX_LEVELS - 1) * nb + nb - 1;
     const int64_t total = (int64_t)off[last] + cnt[last];
@@ -718,11 +718,10 @@ __global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const ui
         lo = v & 255;
         hi = v >> 8;
     }
-    unsigned bals[MAX_LEVELS];
 #pragma unroll
     for (int L = 0; L < MAX_LEVELS; ++L) {
-        bals[L] = __ballot_sync(0xffffffffu, L >= lo && L <= hi);
-        if (lane == 0) sw[L][warp] = __popc(bals[L]);
+        const unsigned v = __ballot_sync(0xffffffffu, L >= lo && L <= hi);
+        if (lane == 0) sb[L][warp] = v;
     }
     __syncthreads();
     if (overflow || i >= n || hi < lo) return;
@@ -730,12 +729,25 @@ __global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const ui
     const int re = ri.x + ri.y;
     const uint64_t ki = keys[i];
     const unsigned below = (1u << lane) - 1u;
-    for (int L = lo; L <= hi; ++L) {
-        int r = __popc(bals[L] & below);
-        for (int w = 0; w < warp; ++w) r += sw[L][w];
+    // The range's end: the first particle of the run past i whose key differs in the first L digits.  Deepest level
+    // first, every level from the end of the one below, in steps of 1, 8, 64, ..., then by halving: most cells hold a
+    // few particles.  Against a halving of the whole run for every level the tree of 1M particles takes 308 us instead
+    // of 328, and as long up to 200,000, where the few cells of the upper levels are the longest chain (steps of 1, 2,
+    // 4, ... are 4 us slower there).
+    int a = i + 1;
+    for (int L = hi; L >= lo; --L) {
+        int r = __popc(sb[L][warp] & below);
+        for (int w = 0; w < warp; ++w) r += __popc(sb[L][w]);
         const int id = off[(int64_t)L * nb + blockIdx.x] + r;
-        // the range's end: the first particle of the run past i whose key differs in the first L digits
-        int a = i + 1, b = re;
+        int b = re;
+        for (int step = 1; a + step - 1 < re; step <<= 3) {
+            const int p = a + step - 1;
+            if (key_common(keys[p], ki) < L) {
+                b = p;
+                break;
+            }
+            a = p + 1;
+        }
         while (a < b) {
             const int mid = (a + b) >> 1;
             if (key_common(keys[mid], ki) >= L) a = mid + 1;
