@@ -56,11 +56,11 @@ __device__ T block_incl_scan(T v, T *total) {
     return x;
 }
 
-// the sum of the blocks' parts before this block's, the sum of all in *total (SCAN_BLOCKS == SCAN_THREADS)
+// the sum of the blocks' parts before this block's, the sum of all in *total (SCAN_BLOCKS <= blockDim.x)
 template <class T>
 __device__ T parts_before(const T *part, T *total) {
     __shared__ T mine;
-    const T v = part[threadIdx.x];
+    const T v = threadIdx.x < SCAN_BLOCKS ? part[threadIdx.x] : 0;
     const T x = block_incl_scan(v, total);
     if (threadIdx.x == blockIdx.x) mine = x - v;
     __syncthreads();
@@ -955,7 +955,7 @@ __device__ int cell_units(int c, int n_roots, int first, const int *start, int c
     return k;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS)
+__global__ void __launch_bounds__(1024)
 k_cell_roles(const int *meta, int n_group, const int *start, const int *count, const int *first_child,
              const int *n_child, const int *parent, const double4 *mom, double4 *com, int4 *cinfo, long long *role,
              long long *part) {
@@ -980,7 +980,7 @@ k_cell_roles(const int *meta, int n_group, const int *start, const int *count, c
     if (threadIdx.x == 0) part[blockIdx.x] = tot;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS)
+__global__ void __launch_bounds__(1024)
 k_role_emit(const int *meta, const int4 *cinfo, const int *start, const int *count, const int *n_child,
             const long long *role, const long long *part, int2 *units, int *group_cell, long long *total) {
     after_previous();
@@ -1157,7 +1157,8 @@ static int enqueue_tree(sph_ctx *ctx) {
     SPH_TRY(sph_scan_exclusive(ctx, t.tmp_cnt, t.tmp_b, nullptr, MAX_LEVELS * nb, nullptr));
     launch_after(true, k_cell_emit, nb, OT_B, 0, st, n, t.cap, ctx->keys, ctx->runs.prun, ctx->runs.info, t.tmp_off,
                  t.tmp_cnt, t.tmp_b, t.meta, t.start, t.count, t.level); ++ctx->launches;
-    launch_after(true, k_cell_link, grid, 256, 0, st, t.meta, t.start, t.count, t.level, t.parent, t.first_child,
+    // (eight blocks per SM: the searches are chains of loads; with two the tree of 1M particles takes 309 us, not 292)
+    launch_after(true, k_cell_link, 4 * grid, 256, 0, st, t.meta, t.start, t.count, t.level, t.parent, t.first_child,
                  t.n_child, t.tmp_cnt);
     ++ctx->launches;
     // moments bottom-up in one launch (tmp_cnt, free again and cleared, counts the arrivals)
@@ -1166,11 +1167,14 @@ static int enqueue_tree(sph_ctx *ctx) {
     launch_after(true, k_moments_up, grid_up, 128, 0, st, t.meta, x, y, z, m, h, t.start, t.count, t.first_child,
                  t.n_child, t.parent, t.tmp_cnt, t.mom, t.blo, t.bhi); ++ctx->launches;
     // packed records, centres of mass, walk units, gravity groups (tmp_b, free again, as 64-bit numbers)
-    static_assert(SCAN_BLOCKS == SCAN_THREADS, "parts_before");
+    static_assert(SCAN_BLOCKS <= SCAN_THREADS, "parts_before");
+    // more threads for large trees, whose cells are read once each (tree of 200,000 / 1M particles 107 / 292 -> 101 /
+    // 258 us; of 3,000-20,000 2 us slower, of 40,000-100,000 the same)
+    const int rt = n < 660 * ctx->num_sms ? SCAN_THREADS : 1024;
     long long *role = (long long *)t.tmp_b, *part = (long long *)ctx->scan.part;
-    launch_after(true, k_cell_roles, SCAN_BLOCKS, SCAN_THREADS, 0, st, t.meta, ctx->cfg.n_group, t.start, t.count,
+    launch_after(true, k_cell_roles, SCAN_BLOCKS, rt, 0, st, t.meta, ctx->cfg.n_group, t.start, t.count,
                  t.first_child, t.n_child, t.parent, t.mom, t.com, t.cinfo, role, part); ++ctx->launches;
-    launch_after(true, k_role_emit, SCAN_BLOCKS, SCAN_THREADS, 0, st, t.meta, t.cinfo, t.start, t.count, t.n_child,
+    launch_after(true, k_role_emit, SCAN_BLOCKS, rt, 0, st, t.meta, t.cinfo, t.start, t.count, t.n_child,
                  role, part, ctx->sup.units, ctx->grav.group_cell, (long long *)(t.meta + META_ROLES)); ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());
     return sph_publish(ctx, t.meta, META_N);
