@@ -24,8 +24,8 @@ namespace {
 // blocks per SM (60 to 64 registers; three: 2.48 ms).  A pass of every functor over 100,003 particles, index
 // form: 3.12 -> 2.35 ms, host link and calls included.
 constexpr int LQ = 4;                  // lanes per i-particle
-constexpr int BT = 256;                // most threads per block
-constexpr int BI = BT / LQ;            // most i-particles per block
+constexpr int BT = 128;                // threads per block
+constexpr int BI = BT / LQ;            // i-particles per block
 constexpr int TJ = 32 * LQ;            // entries per tile
 constexpr int TP = 33 * LQ;            // its shared-memory slots: a slot of padding per 32 entries, so that the four
                                        // lanes' float4 reads fall into different banks
@@ -100,7 +100,7 @@ struct Walk {
 };
 
 // CalcDensity: rho = max(5, norm sum m_j W), h = 1.2 (m / rho)^(1/3)
-__global__ void __launch_bounds__(BT, 4) k_walk_dens32(const int64_t *meta, const sph_epi_dens *epi,
+__global__ void __launch_bounds__(BT, 8) k_walk_dens32(const int64_t *meta, const sph_epi_dens *epi,
                                                      JSrc<sph_epj_dens> epj, sph_result_dens *res) {
     __shared__ float4 sp[TP], sl[TP];   // position hi, mass; lo
     __shared__ float4 ip[BI], il[BI];   // of the i-particles: position hi, 1 / H; lo
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(BT, 4) k_walk_dens32(const int64_t *meta, cons
 }
 
 // CalcDerivative + grad-h factor: div v, rot v, grad_smth (force.h:89-106)
-__global__ void __launch_bounds__(BT, 4) k_walk_drvt32(const int64_t *meta, const sph_epi_drvt *epi,
+__global__ void __launch_bounds__(BT, 8) k_walk_drvt32(const int64_t *meta, const sph_epi_drvt *epi,
                                                      JSrc<sph_epj_drvt> epj, sph_result_drvt *res) {
     __shared__ float4 sp[TP], sl[TP], sv[TP], su[TP];   // position hi, mass; lo; velocity hi; lo
     // of the i-particles: position hi, 1 / H; lo, H; velocity hi, 1e-6 h; lo
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(BT, 4) k_walk_drvt32(const int64_t *meta, cons
 }
 
 // CalcHydroForce: acceleration, du/dt, dt (force.h:113-147)
-__global__ void __launch_bounds__(BT, 4) k_walk_hydro32(const int64_t *meta, const sph_epi_hydro *epi,
+__global__ void __launch_bounds__(BT, 8) k_walk_hydro32(const int64_t *meta, const sph_epi_hydro *epi,
                                                       JSrc<sph_epj_hydro> epj, sph_result_hydro *res) {
     // position hi, mass; lo, H; velocity hi, 1 / H; lo, rho; f P / rho^2, c_s, f, Bal
     __shared__ float4 sp[TP], sl[TP], sv[TP], su[TP], sa[TP];
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(BT, 4) k_walk_hydro32(const int64_t *meta, con
 }
 
 // CalcGravityForce<EPJ::Grav> then <SPJMonopole> (force.h:154-168): G m folded into the tile
-__global__ void __launch_bounds__(BT, 4) k_walk_grav32(const int64_t *meta, const sph_epi_grav *epi,
+__global__ void __launch_bounds__(BT, 8) k_walk_grav32(const int64_t *meta, const sph_epi_grav *epi,
                                                      JSrc<sph_epj_grav> epj, JSrc<sph_spj_monopole> spj,
                                                      sph_result_grav *res) {
     __shared__ float4 sp[TP], sl[TP];   // position hi, G m; lo
@@ -409,16 +409,17 @@ __global__ void __launch_bounds__(BT, 4) k_walk_grav32(const int64_t *meta, cons
     }
 }
 
-// 64 i-particles (256 threads) per block; with fewer walks than SMs (152) blocks of 32 i-particles, so that the few
-// walks spread over the chip
+// 32 i-particles (128 threads) per block.  Blocks of 64 leave more lanes without one (walks of 84 on average at 1M
+// particles: density / derivative / hydro / gravity dispatches of 244 walks 94 / 144 / 222 / 193 us, with 32 per block
+// 92 / 137 / 214 / 185; of 300,003 particles as long either way), blocks of 16 stage the j too often (225 / 203 for the
+// last two).
 struct Shape {
     dim3 grid;
     int threads;
     Shape(int n_walk, int max_i) {
-        const int ipb = n_walk < 152 ? 32 : BT / LQ;
-        const int chunks = (max_i + ipb - 1) / ipb;
+        const int chunks = (max_i + BI - 1) / BI;
         grid = dim3((unsigned)n_walk, (unsigned)(chunks < 1 ? 1 : (chunks > 4096 ? 4096 : chunks)));
-        threads = ipb * LQ;
+        threads = BT;
     }
 };
 
