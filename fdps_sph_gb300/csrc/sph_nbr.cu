@@ -547,7 +547,9 @@ __device__ __forceinline__ void filter_row(int i, int lane, int c, int K, int64_
     const float H2i = H2f[i], lo0 = H2i * BAND_LO, hi0 = H2i * BAND_HI;
     // two chunks ahead: entries; one chunk ahead: the h of their particles
     int jn = i, jm = i;
-    float rn = INFINITY, rm = INFINITY;   // past the end: no member of anything
+    // past the end: a NaN is below no threshold and inside no band, not even where 2.5 h squared overflows to infinity
+    const float none = __int_as_float(0x7fffffff);
+    float rn = none, rm = none;
     if (lane < c) {
         jn = *entry<SPILL>(row, row_s, K, lane);
         rn = *entry<SPILL>(rrow, rrow_s, K, lane);
@@ -563,7 +565,7 @@ __device__ __forceinline__ void filter_row(int i, int lane, int c, int K, int64_
         jn = jm;
         rn = rm;
         if (MODE != 0) hn = H2f[jn];
-        rm = INFINITY;
+        rm = none;
         if (kn < c) {
             jm = *entry<SPILL>(row, row_s, K, kn);
             rm = *entry<SPILL>(rrow, rrow_s, K, kn);
