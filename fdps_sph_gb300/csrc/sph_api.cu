@@ -8,7 +8,10 @@
 #include <fstream>
 #include <sstream>
 
+#include <cudaTypedefs.h>
+
 #include "sph_internal.cuh"
+#include "sph_pinned.h"
 
 using namespace sph;
 
@@ -190,19 +193,36 @@ __global__ void __launch_bounds__(512) k_gather_rows(uint64_t mask, int n, const
     for (; k < n; k += stride) out[k] = F[inv[k]];
 }
 
-// the device's address of a host block of doubles that is pinned from its first to its last byte, else null
-double *pinned_block(const double *p, size_t doubles) {
-    cudaPointerAttributes a, b;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, p + doubles - 1) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || ((uintptr_t)p & 7))
-        return nullptr;
-    // one mapping: the device addresses are as far apart as the host's
-    if ((const char *)b.devicePointer - (const char *)a.devicePointer != (const char *)(p + doubles - 1) - (const char *)p)
-        return nullptr;
-    return (double *)a.devicePointer;
+// the pinned host range (one allocation or registration) that holds p
+PinnedRange pinned_range(const char *p) {
+    static const PFN_cuPointerGetAttributes_v7000 get = []() -> PFN_cuPointerGetAttributes_v7000 {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &found) !=
+                cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        return (PFN_cuPointerGetAttributes_v7000)f;
+    }();
+    unsigned type = 0, managed = 0;
+    CUdeviceptr at = 0, first = 0;
+    size_t bytes = 0;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[5] = {&type, &managed, &at, &first, &bytes};   // an attribute that p does not have is left 0
+    if (!get || get(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed ||
+        !at || !first)
+        return {};
+    return {(const char *)(uintptr_t)first, bytes, (const char *)(uintptr_t)at};
+}
+
+// the device's address of a host block of doubles that kernels may read and write, else null (sph_pinned.h)
+double *pinned_block(const sph_ctx *ctx, const double *block, size_t doubles) {
+    return (double *)const_cast<char *>(
+        reachable_block((const char *)block, sizeof(double) * doubles, ctx->pageable, pinned_range));
 }
 
 // blocks per row: about two 512-thread blocks per SM over all rows saturate the link
@@ -477,7 +497,7 @@ int append_run(sph_ctx *ctx, int64_t n, const double *fields, int64_t ld, const 
     // others zeroed; from a pinned block by one kernel, else consecutive rows in one 2D copy
     const uint64_t all = (1ull << SPH_NFIELD) - 1;
     const uint64_t want = (flags & SPH_UPLOAD_STEP_INPUTS) ? (uint64_t)SPH_STEP_INPUT_FIELDS : all;
-    const double *pinned = pinned_block(fields, (size_t)ld * (SPH_NFIELD - 1) + n);
+    const double *pinned = pinned_block(ctx, fields, (size_t)ld * (SPH_NFIELD - 1) + n);
     if (pinned) {
         k_copy_rows<<<row_grid(ctx, want, n), 512, 0, ctx->stream>>>(want, n, pinned, ld, ctx->F + o, c);
         ++ctx->launches;
@@ -624,6 +644,12 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
         delete ctx;
         return SPH_ERR_CUDA;
     }
+    int pageable = 0;
+    if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        pageable = 0;
+    }
+    ctx->pageable = pageable == 1;
     for (int k = 0; k < MAX_MATERIALS; ++k) {
         std::memset(&ctx->mats_host[k], 0, sizeof(DevMaterial));
         ctx->mats_host[k].kind = -1;
@@ -1007,7 +1033,7 @@ int sph_download_run(sph_ctx *ctx, int64_t handle, double *fields, int64_t ld, i
     if (!fields || ld < n) return sph_fail(ctx, SPH_ERR_ARG, "bad output block");
     cudaSetDevice(ctx->device);
     const uint64_t all = (1ull << SPH_NFIELD) - 1;
-    double *pinned = ctx->sort.cap >= n ? pinned_block(fields, (size_t)ld * (SPH_NFIELD - 1) + n) : nullptr;
+    double *pinned = ctx->sort.cap >= n ? pinned_block(ctx, fields, (size_t)ld * (SPH_NFIELD - 1) + n) : nullptr;
     if (pinned) SPH_TRY(gather_to_host(ctx, all, (int)R.off[r], n, nullptr, pinned, ld));
     k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, pinned ? 0 : SPH_NFIELD, ctx->cap,
                                                              (int)R.off[r], n, ctx->slot, R.prun, nullptr, ctx->id,
@@ -1044,7 +1070,7 @@ int sph_download_fields(sph_ctx *ctx, double *fields, int64_t ld, uint64_t field
     field_mask &= (1ull << SPH_NFIELD) - 1;
     double *pinned = nullptr;
     if (field_mask && ctx->sort.cap >= n)   // (the scratch of the order: as many particles as were ever sorted)
-        pinned = pinned_block(fields, (size_t)ld * (63 - __builtin_clzll(field_mask)) + n);
+        pinned = pinned_block(ctx, fields, (size_t)ld * (63 - __builtin_clzll(field_mask)) + n);
     if (pinned) SPH_TRY(gather_to_host(ctx, field_mask, 0, n, ctx->runs.info, pinned, ld));
     if (!pinned || id || material) {
         k_unpermute<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(ctx->F, ctx->F2, pinned ? 0 : SPH_NFIELD, ctx->cap, 0,

@@ -343,6 +343,7 @@ struct sph_ctx {
     sph_config cfg;
     int device = 0;
     int num_sms = 0;
+    bool pageable = false;   // the device reads and writes pageable host memory
     cudaStream_t stream = nullptr;
     // sph_step_download: fields go to the host on their own stream as soon as the step has
     // finished writing them (unpermuted into dl_buf first)
