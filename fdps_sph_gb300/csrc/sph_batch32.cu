@@ -342,8 +342,10 @@ __global__ void __launch_bounds__(BT, 8) k_walk_grav32(const int64_t *meta, cons
     const Walk W(meta);
     if (W.ni <= 0) return;
     const double3 o = make_double3(epi[W.io].pos[0], epi[W.io].pos[1], epi[W.io].pos[2]);
-    // G m in units of the walk's first EPJ mass (or SPJ mass) keeps the FP32 products in range
-    const double gscale = W.nj > 0 ? G * epj[W.jo].mass : (W.ns > 0 ? G * spj[W.so].mass : G);
+    // G m in units of the walk's first EPJ mass (or SPJ mass) keeps the FP32 products in range; a mass that is no unit
+    // (0 x G m / 0 would be a NaN in every sum of the walk) leaves them as they are
+    const double m0 = W.nj > 0 ? epj[W.jo].mass : (W.ns > 0 ? spj[W.so].mass : 1.0);
+    const double gscale = G * (m0 != 0.0 && isfinite(m0) ? m0 : 1.0);
     const int64_t nl = W.nj + W.ns;
     for (int64_t i0 = (int64_t)blockIdx.y * W.ipb; i0 < W.ni; i0 += (int64_t)gridDim.y * W.ipb) {
         const int g = threadIdx.x / LQ;   // this lane's i-particle of the block's
