@@ -689,7 +689,7 @@ int sph_ctx_destroy(sph_ctx *ctx) {
                     ctx->grav.group_cell, ctx->grav.n_epj, ctx->grav.n_spj, ctx->grav.off_epj,
                     ctx->grav.off_spj, ctx->grav.epj, ctx->grav.spj, ctx->scan.part, ctx->scan.total,
                     ctx->sup.nbr, ctx->sup.cnt, ctx->sup.hsup, ctx->sup.pxh, ctx->sup.pxl, ctx->sup.H2f,
-                    ctx->sup.units, ctx->tree.cinfo, ctx->sup.r2, ctx->sup.m, ctx->sup.vR, ctx->sup.cvR,
+                    ctx->sup.units, ctx->tree.cinfo, ctx->sup.r2, ctx->sup.m, ctx->sup.H2s, ctx->sup.vR, ctx->sup.cvR,
                     ctx->sup.umark, ctx->sup.uoff, ctx->sup.uidx, ctx->runs.prun, ctx->runs.prun2,
                     ctx->runs.tiles, ctx->runs.info, ctx->runs.dt_dev, ctx->runs.part, ctx->runs.out,
                     ctx->runs.damp, ctx->runs.fixd, ctx->sup.soff, ctx->sup.need, ctx->sup.uover, ctx->sup.npass, ctx->dl_buf};

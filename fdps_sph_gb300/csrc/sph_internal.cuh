@@ -258,7 +258,8 @@ struct SphSuper {
     int *nbr = nullptr, *cnt = nullptr;   // superset, ELL
     float *r2 = nullptr;                  // FP32 r^2 of every superset entry
     float *m = nullptr;                   // neighbour mass x mscale of every superset entry
-    double *hsup = nullptr;               // h when the superset was built
+    double *hsup = nullptr;               // h the superset was built for
+    float *H2s = nullptr;                 // (2.5 hsup)^2 rounded up, for a repair's walk
     float4 *pxh = nullptr, *pxl = nullptr;  // double-float positions
     float *H2f = nullptr;                 // (2.5 h)^2 rounded up
     int2 *units = nullptr;                // (start, count) of the walk units
@@ -446,7 +447,7 @@ int sph_fail(sph_ctx *ctx, int code, const char *fmt, ...);
 // tree / sort (sph_tree.cu)
 int sph_tree_reserve(sph_ctx *ctx, int64_t n);
 int sph_sort_and_build(sph_ctx *ctx);          // root box, keys, sort, permute, octree, moments
-int sph_tree_refresh_hmax(sph_ctx *ctx);       // cell hmax after h changed
+int sph_tree_refresh_hmax(sph_ctx *ctx, const double *h);   // cell hmax of another h
 int sph_publish(sph_ctx *ctx, const int *src, int n);
 int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev, int len_host, int *total_dev);
 

@@ -99,7 +99,7 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
     const bool valid = lane < U.y;
     const int i = U.x + (valid ? lane : 0);
     const double xi = x[i], yi = y[i], zi = z[i];
-    if (valid) hsup[i] = h[i];   // the h this row is built for
+    if (hsup && valid) hsup[i] = h[i];   // the h this row is built for (a repair has set it: k_skin_raise)
     const float4 pih = xh[i], pil = xl[i];
     const float H2i = valid ? H2f[i] : 0.0f;
     double lo[3] = {valid ? xi : INFINITY, valid ? yi : INFINITY, valid ? zi : INFINITY};
@@ -341,21 +341,36 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
 // ---------------------------------------------------------------------------
 // incremental repair after h outgrew the skin
 //
-// A row built when particle j had smoothing length h_j(T) keeps every
-// neighbour as long as 2.5 h_j <= KAPPA * 2.5 h_j(T) for all j near it.  A
-// particle v that violates this (h_v > KAPPA * hsup_v) can be missing from
-// its own row and from the symmetric rows of particles within 2.5 h_v of it;
-// the rows of every unit within reach of a violator are walked again.
+// Every row i is built with the reach KAPPA max(2.5 hsup_i, 2.5 hsup_j), hsup
+// being the h recorded when all rows were walked, so it holds all neighbours
+// as long as h <= KAPPA hsup everywhere.  A particle v that violates this
+// gets hsup_v = h_v, and the rows of every unit within KAPPA 2.5 h_v of it
+// (its own among them) are walked again with that reach; hsup of all others
+// stays.  Where h of the moment were used for the others instead, rows inside and
+// outside the repaired units would hold different reaches for one
+// particle: a larger one recorded is missing outside (a later growth inside the
+// skin would not be seen there), a smaller one is missing inside.
 
+// vR: reach of the violators (0: none of them), counted in nviol
 __global__ void k_viol_mark(int n, const double *h, const double *hsup, float *vR, int *nviol) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool v = false;
     if (i < n) {
         v = h[i] > (double)KAPPA * hsup[i];
-        vR[i] = v ? __double2float_ru(SUPPORT * h[i] * 1.001) : 0.0f;
+        vR[i] = v ? __double2float_ru(SUPPORT * h[i] * (KAPPA * 1.001)) : 0.0f;
     }
     const unsigned b = __ballot_sync(FULLM, v);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nviol, __popc(b));
+}
+
+// what a repair's walk is built for: hsup raised to h for the violators, (2.5 hsup)^2 as k_h2f
+__global__ void k_skin_raise(int n, const double *h, const float *vR, double *hsup, float *H2s) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double s = vR[i] > 0.0f ? h[i] : hsup[i];
+    hsup[i] = s;
+    const double H = SUPPORT * s;
+    H2s[i] = __double2float_ru(H * H);
 }
 
 // after a density round: (2.5 h)^2 of the new h as k_h2f, and the count of k_viol_mark
@@ -899,6 +914,7 @@ int sph_nbr_prepare(sph_ctx *ctx) {
         SPH_TRY(dalloc_n(ctx, &S.pxh, pitch));
         SPH_TRY(dalloc_n(ctx, &S.pxl, pitch));
         SPH_TRY(dalloc_n(ctx, &S.H2f, pitch));
+        SPH_TRY(dalloc_n(ctx, &S.H2s, pitch));
         SPH_TRY(dalloc_n(ctx, &S.hsup, pitch));
         SPH_TRY(dalloc_n(ctx, &S.cnt, pitch));
         SPH_TRY(dalloc_n(ctx, &S.vR, pitch));
@@ -925,8 +941,9 @@ int sph_nbr_prepare(sph_ctx *ctx) {
     return SPH_OK;
 }
 
-// walks the units in uidx (or all units when uidx is null); grows the row capacity if needed
-static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
+// walks the units in uidx (or all units when uidx is null) for the current h, which hsup records, or (repair) for the
+// recorded hsup (k_skin_raise); grows the row capacity if needed
+static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk, bool repair) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
     const int64_t pitch = n;   // rows: particle i's entries at i * K .. i * K + K - 1
@@ -940,7 +957,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         SPH_CUDA(ctx, cudaMemsetAsync(S.uover, 0, sizeof(int) * S.cap_units, ctx->stream));
         S.cap_uover = S.cap_units;
     }
-    if (S.rebuilds_step > 0) SPH_TRY(sph_tree_refresh_hmax(ctx));   // cell hmax must follow the current h
+    // cell hmax must follow the h that is walked for
+    if (S.rebuilds_step > 0) SPH_TRY(sph_tree_refresh_hmax(ctx, repair ? S.hsup : FLD(ctx->F, SPH_SMTH, cap)));
     S.rebuilds_step += 1;
     for (int attempt = 0; attempt < 4; ++attempt) {
         if (!S.nbr || S.pitch < pitch || S.K_alloc != S.K || S.spill_alloc != S.spill_cap) {
@@ -979,7 +997,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
         if (blocks > 0) {
             auto walk = S.spill_on ? k_sup_walk<true> : k_sup_walk<false>;
             walk<<<blocks, NB_WARPS * 32, 0, ctx->stream>>>(n_walk, split, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
-                FLD(ctx->F, SPH_SMTH, cap), S.hsup, walk_xh(ctx), walk_xl(ctx), S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
+                FLD(ctx->F, SPH_SMTH, cap), repair ? nullptr : S.hsup, walk_xh(ctx), walk_xl(ctx),
+                repair ? S.H2s : S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
                 S.cnt, S.map(), S.uover, meta + META_ERR, meta + META_MAXCNT);
             ++ctx->launches;
         }
@@ -1049,7 +1068,7 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk) {
 // a full walk after a sort: the previous spill layout belongs to the previous order
 static int build_superset(sph_ctx *ctx) {
     ctx->sup.spill_on = false;
-    return walk_units(ctx, nullptr, ctx->sup.n_units);
+    return walk_units(ctx, nullptr, ctx->sup.n_units, false);
 }
 
 // makes the superset valid for the current h: full walk after a sort, otherwise a repair of
@@ -1073,6 +1092,8 @@ static int ensure_superset(sph_ctx *ctx) {
     if (nviol == 0) return SPH_OK;
     S.violators += nviol;
     if ((int64_t)nviol * 8 > n) return build_superset(ctx);   // widespread growth: walk everything
+    k_skin_raise<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_SMTH, cap), vR, S.hsup, S.H2s);
+    ++ctx->launches;
     // influence radius per cell, bottom-up
     const int grid = 2 * ctx->num_sms;
     for (int l = t.depth; l >= 0; --l) {
@@ -1089,7 +1110,7 @@ static int ensure_superset(sph_ctx *ctx) {
     SPH_TRY(sph_publish(ctx, ctx->scan.total, 1));
     SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int nmark = hs[0];
-    return walk_units(ctx, S.uidx, nmark);
+    return walk_units(ctx, S.uidx, nmark, true);
 }
 
 // exact list of `mode` (0 gather, 1 symmetric, 2 both) from a superset that is valid for the current h

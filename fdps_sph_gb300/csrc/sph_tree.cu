@@ -1306,9 +1306,8 @@ int sph_sort_and_build(sph_ctx *ctx) {
     return SPH_OK;
 }
 
-int sph_tree_refresh_hmax(sph_ctx *ctx) {
+int sph_tree_refresh_hmax(sph_ctx *ctx, const double *h) {
     Tree &t = ctx->tree;
-    const double *h = FLD(ctx->F, SPH_SMTH, ctx->cap);
     const int grid = 2 * ctx->num_sms;
     for (int l = t.depth; l >= 0; --l)
         k_hmax<<<grid, 128, 0, ctx->stream>>>(l, t.meta, h, t.start, t.count, t.first_child, t.n_child, t.bhi); ++ctx->launches;
