@@ -79,7 +79,45 @@ def parse():
                     help="skip the drop-in measurement through the MultiWalk dispatch / retrieve callbacks")
     ap.add_argument("--contact-steps", type=int, default=20,
                     help="mixed steps of the 1M contact state before its mixed-vs-FP64 comparison")
+    ap.add_argument("--detail", default=os.path.join(ROOT, "bench_detail.json"),
+                    help="file for everything measured; the printed line carries the headline's figures")
     return ap.parse_args()
+
+
+# Readers of the result keep the end of the output, a few thousand characters: the line stays below this many.
+LINE_MAX = 2500
+
+
+def result_line(out):
+    """The printed line of a run's results: the headline's keys whole, of the other sections what they measured in a
+    number or two.  Everything is in the --detail file."""
+    def short(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+
+    def pick(d, *keys):
+        return {k: short(d[k]) for k in keys if d.get(k) is not None}
+
+    # metric, value, unit, counts of the contract (strings and numbers), and its objects
+    line = {k: v for k, v in out.items() if not isinstance(v, (dict, list)) or k in ("config", "clocks", "e2e")}
+    if "roofline" in out:
+        line["roofline"] = pick(out["roofline"], "kernel", "bound", "achieved", "peak", "unit", "frac")
+    if "segments_ms_per_step" in out:
+        line["segments_ms_per_step"] = {k: float(f"{v:.3g}") for k, v in out["segments_ms_per_step"].items() if v > 0}
+    for k in ("fp64", "batch", "serving"):
+        if k in out:
+            line[k] = pick(out[k], "value", "unit", "ms_per_step", "vs_cpu_baseline")
+            if "step_latency_s" in out[k]:
+                line[k]["step_latency_p99_s"] = short(out[k]["step_latency_s"]["p99"])
+    if "multiwalk" in out:
+        m = out["multiwalk"]
+        line["multiwalk"] = pick(m, "value", "unit", "vs_cpu_baseline")
+        line["multiwalk"].update({k: short(m[k]["value"]) for k in ("index_form", "host_staging", "fp64") if k in m})
+    if "config_4m" in out:
+        line["config_4m"] = {k: {p: short(v[p]["ms_per_step"]) for p in ("mixed", "fp64") if p in v}
+                             for k, v in out["config_4m"].items() if k.startswith("theta_")}
+    if "cpu_baseline" in out:
+        line["cpu_baseline"] = pick(out["cpu_baseline"], "value", "unit", "cores", "kind", "sample")
+    return line
 
 
 class ClockSampler:
@@ -611,7 +649,12 @@ def main():
                 out[k]["vs_cpu_baseline"] = out[k]["value"] / v_cpu
         if "multiwalk" in out:
             out["multiwalk"]["index_form"]["vs_cpu_baseline"] = out["multiwalk"]["index_form"]["value"] / v_cpu
-    print(json.dumps(out))
+    try:
+        with open(a.detail, "w") as fh:
+            json.dump(out, fh)
+    except OSError as e:   # (a read-only place takes nothing from the line)
+        print(f"bench: cannot write {a.detail}: {e}", file=sys.stderr)
+    print(json.dumps(result_line(out)))
 
 
 def multiwalk(a, device, n_walk_limit=256, n_tags=4, steps=2):
