@@ -357,14 +357,15 @@ __global__ void __launch_bounds__(RS_THREADS) k_keys_hist(const double *x, const
     if (t < 256 && h[t]) atomicAdd(&hist[(int64_t)tile * 256 + t], h[t]);
 }
 
-// per run (blockIdx.y) and 32 digits (blockIdx.x): off[tile][digit] = keys of the digit in the run's earlier tiles,
-// tot[first tile][digit] = in all of them.  Warp w sums the w-th 32nd of the tiles, a digit per lane.
+// per run (blockIdx.x: only a grid's first extent goes beyond 65,535) and 32 digits (blockIdx.y): off[tile][digit] = keys
+// of the digit in the run's earlier tiles, tot[first tile][digit] = in all of them.  Warp w sums the w-th 32nd of the
+// tiles, a digit per lane.
 __global__ void __launch_bounds__(1024) k_rs_scan(const uint32_t *hist, const int4 *info, uint32_t *off,
                                                   uint32_t *tot) {
     after_previous();
     __shared__ uint32_t s[32][32];
-    const int4 r = info[blockIdx.y];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
+    const int4 r = info[blockIdx.x];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.y * 32 + lane;
     const int per = (r.w + 31) / 32, t0 = r.z + w * per, t1 = min(r.z + r.w, t0 + per);
     uint32_t v = 0;
 #pragma unroll 8
@@ -1127,7 +1128,7 @@ static int radix_sort(sph_ctx *ctx, int n) {
         uint32_t *next = last ? nullptr : s.hist + (pass + 1) % RS_HISTS * row;
         uint32_t *clear = last ? nullptr : s.hist + (pass + 2) % RS_HISTS * row;
         if (scan) {
-            launch_after(true, k_rs_scan, dim3(8, ctx->runs.R), 1024, 0, ctx->stream, hist, ctx->runs.info, s.hoff,
+            launch_after(true, k_rs_scan, dim3(ctx->runs.R, 8), 1024, 0, ctx->stream, hist, ctx->runs.info, s.hoff,
                          s.hoff + row);
             ++ctx->launches;
         }
