@@ -13,15 +13,16 @@
 // entry point is used.
 //
 // The array is shared by every call on a device and keeps the last call's
-// contents; each call rewrites all of it that it reads except the error
-// word, which it clears first.  Two calls whose work overlaps on the GPU
+// contents; each call rewrites all of it that it reads, the error word
+// among it.  Two calls whose work overlaps on the GPU
 // (different streams, no ordering between them) race on the array.  Called
 // eagerly, a call ends by reading the error word back to the host, so it
 // returns only after its work on `stream` has finished.  Called while
-// `stream` is being captured into a CUDA graph, it only records its work (the
-// memset, the launches and the device-to-device copies are all capturable)
-// and returns at once: a replay reports no status.
+// `stream` is being captured into a CUDA graph, it only records its work
+// (kernel launches and nothing else) and returns at once: a replay reports no
+// status.
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "sph_internal.cuh"
@@ -92,6 +93,18 @@ bool noalloc_ready(int dev) {
     return dev >= 0 && dev < 64 && g_na_ptr[dev] != nullptr;
 }
 
+// Where a call's status is written by a kernel.  Not the caller's frame: when the wait for the stream fails, the kernel may
+// still run after the call has returned.  A word is a call's own until then, and is never used again if the wait fails.
+constexpr int NA_WORDS = 256;
+int g_na_words[NA_WORDS];
+std::atomic<bool> g_na_taken[NA_WORDS];
+
+int take_word() {   // -1: all are taken
+    for (int k = 0; k < NA_WORDS; ++k)
+        if (!g_na_taken[k].exchange(true)) return k;
+    return -1;
+}
+
 }  // namespace
 
 extern "C" int sph_morton_order_noalloc(const double *x, const double *y, const double *z, int64_t n,
@@ -146,15 +159,20 @@ extern "C" int sph_morton_order_noalloc(const double *x, const double *y, const 
     }
     if (cudaGetLastError() != cudaSuccess) return SPH_ERR_CUDA;
     if (capturing) return SPH_OK;   // recorded; a replay's status is not read back
-    // the status: written to this frame by a kernel where the device reaches pageable memory (as the functor calls'
-    // results are), which saves the copy's detour (100,000 particles 138 -> 123 us; overlapped launches 140 -> 138)
+    // the status: written by a kernel where the device reaches pageable memory (as the functor calls' results are), which
+    // saves the copy's detour (100,000 particles 138 -> 123 us; overlapped launches 140 -> 138)
     int herr = 0;
-    if (pageable) launch_after(true, k_publish, 1, 64, 0, st, err, 1, &herr);
-    if ((pageable ? cudaGetLastError()
-                  : cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+    const int word = pageable ? take_word() : -1;
+    if (word >= 0) launch_after(true, k_publish, 1, 64, 0, st, err, 1, g_na_words + word);
+    if ((word >= 0 ? cudaGetLastError()
+                   : cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         cudaGetLastError();
         return SPH_ERR_CUDA;
+    }
+    if (word >= 0) {
+        herr = *(volatile int *)(g_na_words + word);
+        g_na_taken[word].store(false);
     }
     return (herr & ERR_NONFINITE) ? SPH_ERR_NONFINITE : SPH_OK;
 }

@@ -391,11 +391,10 @@ int sph_get_counters(sph_ctx *ctx, int64_t out[16]);
  * recorded).  Called eagerly, the call ends by reading its error word back
  * and synchronising `stream`, so it returns after its work is done.  Called
  * while `stream` is being captured into a CUDA graph, it records its work
- * (a memset, kernel launches, device-to-device copies) and returns SPH_OK at
- * once; a replay of the graph reports no status (a non-finite position then
- * leaves its key undefined).  Every call on a device shares the array: calls
- * (or replays) that overlap on the GPU race.  No device memory is allocated
- * or freed. */
+ * (kernel launches) and returns SPH_OK at once; a replay of the graph
+ * reports no status (a non-finite position then leaves its key undefined).
+ * Every call on a device shares the array: calls (or replays) that overlap on
+ * the GPU race.  No device memory is allocated or freed. */
 #define SPH_NOALLOC_MAX_N 131072
 int sph_morton_order_noalloc(const double *x, const double *y, const double *z, int64_t n, uint64_t *keys_out,
                              int32_t *order_out, void *stream);
