@@ -32,7 +32,7 @@ __device__ __forceinline__ double rcp64(double x) {
 // r = sqrt(x) and y = 1 / sqrt(x) (y = 0 at x = 0), within 2 units of 2^-53 each: seed y0, e = 1 - x y0^2,
 // both times (1 + e / 2 + 3 e^2 / 8)
 __device__ __forceinline__ void sqrt_rsqrt64(double x, double &r, double &y) {
-    const bool zero = (__double2hiint(x) | __double2loint(x)) == 0;
+    const bool zero = ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;   // (-0 too)
     if (!zero && !mid_range(x)) {
         r = sqrt(x);
         y = 1.0 / r;
