@@ -661,7 +661,7 @@ int sph_ctx_create(const sph_config *cfg, sph_ctx **out) {
     cudaEventCreate(&ctx->ev_end);
     if (cudaMalloc((void **)&ctx->mats_dev, sizeof(ctx->mats_host)) != cudaSuccess ||
         cudaMalloc((void **)&ctx->scratch_d, sizeof(double) * 8192) != cudaSuccess ||
-        cudaMallocHost((void **)&ctx->host_scalars, sizeof(double) * 512) != cudaSuccess) {
+        cudaMallocHost((void **)&ctx->host_scalars, sizeof(double) * HOST_SCALARS) != cudaSuccess) {
         cudaGetLastError();
         sph_ctx_destroy(ctx);
         return SPH_ERR_OOM;

@@ -340,6 +340,12 @@ struct TreeGraph {
 };
 }  // namespace sph
 
+namespace sph {
+// the context's pinned block: small results for the host, published words first (META_N ints), then each run's dt
+constexpr int HOST_SCALARS = 512, HOST_DT = 32;
+static_assert(META_N * sizeof(int) <= HOST_DT * sizeof(double), "the words end before the dt");
+}  // namespace sph
+
 struct sph_ctx {
     sph_config cfg;
     int device = 0;
@@ -365,7 +371,7 @@ struct sph_ctx {
     int32_t *mat = nullptr, *mat2 = nullptr;
     uint64_t *keys = nullptr;               // sorted keys of the current order
     double *scratch_d = nullptr;            // reductions [64]
-    double *host_scalars = nullptr;         // pinned [64]
+    double *host_scalars = nullptr;         // pinned [HOST_SCALARS]
 
     // mixed-precision packed copies (double-float hi/lo)
     float4 *xh = nullptr, *xl = nullptr, *vhf = nullptr, *vlf = nullptr;
@@ -455,9 +461,7 @@ int sph_scan_exclusive(sph_ctx *ctx, const int *in, int *out, const int *len_dev
 int sph_nbr_prepare(sph_ctx *ctx);       // after the sort (also packs the mixed path's records)
 int sph_nbr_refresh_h(sph_ctx *ctx);     // after h changed
 int sph_build_sph_lists(sph_ctx *ctx, int mode);
-int sph_density_from_superset(sph_ctx *ctx);
 int sph_density_fused(sph_ctx *ctx);     // mixed precision: all density passes of a step
-int sph_nbr_ensure_superset(sph_ctx *ctx);   // mixed precision: density pass without an exact list
 int time_mark(sph_ctx *ctx, int seg);
 int dl_milestone(sph_ctx *ctx, uint64_t final_fields);   // sph_step_download: send what is final      // event at the end of a timed segment (when timing is on)
 int sph_runs_layout(sph_ctx *ctx);        // offsets and tiles of the runs after a change of the run set

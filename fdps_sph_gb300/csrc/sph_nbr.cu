@@ -501,8 +501,6 @@ __global__ void k_unit_compact(int n_units, const int *umark, const int *off, in
 // ---------------------------------------------------------------------------
 // exact filter
 
-constexpr int ERR_SKIN = 16;
-
 // The FP32 r^2 stored by the walk is (x_j - x_i)^2 on double-float
 // coordinates, within 2^-21 of the exact value; outside a band of 2^-19
 // around the threshold it decides alone, inside it the oracle's FP64 test
@@ -634,67 +632,6 @@ k_filter(int n, const int *__restrict__ sup, const float *__restrict__ sup_r2, c
         if (MODE != 1) ocnt0[i] = k0;
         if (MODE != 0) ocnt1[i] = k1;
     }
-}
-
-// Mixed-precision density straight from the superset: the gather-set
-// decision of k_filter<0>, then CalcDensity's sum (force.h:9-23) in FP32
-// partial sums of 32 flushed to FP64, FLAG_GI floor and h update in FP64.
-__global__ void __launch_bounds__(128)
-k_density_sup32(int n, const int *__restrict__ sup, const float *__restrict__ sup_r2, const float *__restrict__ sup_m,
-                const int *__restrict__ scnt, RowMap rm, const double *__restrict__ x,
-                const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ m,
-                double *__restrict__ h, const double *__restrict__ hsup, double *__restrict__ dens, float dscale,
-                int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double hi = h[i];
-    const double Hi = __dmul_rn(SUPPORT, hi);
-    const double H2 = __dmul_rn(Hi, Hi);
-    const float H2i = (float)H2;
-    const float invH = 1.0f / (float)Hi;
-    const double xi = x[i], yi = y[i], zi = z[i];
-    const int c_all = scnt[i];
-    float acc_h = 0.0f, acc_l = 0.0f;
-    // the index row is read only for the rare entries whose FP32 distance is too close to the
-    // threshold to decide (exact_in's band); the stream is r^2 and m_j
-    for (int seg = 0; seg < 2; ++seg) {
-    int c;
-    const int64_t b = row_seg(rm, i, seg, c_all, &c);
-    if (c <= 0) break;
-    const int *row = sup + b;
-    const float *rrow = sup_r2 + b;
-    const float *mrow = sup_m + b;
-    // software-pipelined: the next chunk's four vector loads are in flight while this chunk is summed
-    float4 r0 = reinterpret_cast<const float4 *>(rrow)[0], r1 = reinterpret_cast<const float4 *>(rrow)[1];
-    float4 m0 = reinterpret_cast<const float4 *>(mrow)[0], m1 = reinterpret_cast<const float4 *>(mrow)[1];
-    for (int k = 0; k < c; k += 8) {
-        const float rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-        const float mj[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
-        const int m8 = min(8, c - k);
-        if (k + 8 < c) {
-            r0 = reinterpret_cast<const float4 *>(rrow + k + 8)[0];
-            r1 = reinterpret_cast<const float4 *>(rrow + k + 8)[1];
-            m0 = reinterpret_cast<const float4 *>(mrow + k + 8)[0];
-            m1 = reinterpret_cast<const float4 *>(mrow + k + 8)[1];
-        }
-        // every member goes straight into the compensated pair: the sum depends only on the
-        // sequence of members (the walk's order), not on where non-members sit in the row, so a
-        // row rebuilt with another skin (a repair, another run's violators) gives the same result
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (u >= m8) continue;
-            bool in = rr[u] < H2i * (1.0f - 1.9073486328125e-06f);
-            if (!in && !(rr[u] > H2i * (1.0f + 1.9073486328125e-06f)))
-                in = exact_in(rr[u], H2i, row[k + u], xi, yi, zi, H2, x, y, z, h, false);
-            if (!in) continue;
-            const float s_ = sqrt_a(rr[u]) * invH;
-            const float p = fmaxf(1.0f - s_, 0.0f);
-            const float p2 = p * p, p4 = p2 * p2;
-            df_add(acc_h, acc_l, mj[u] * ((1.0f + s_ * (8.0f + s_ * (25.0f + s_ * 32.0f))) * (p4 * p4)));
-        }
-    }
-    }
-    density_tail32(acc_h + acc_l, invH, dscale, m[i], dens + i, h + i);
 }
 
 // Every density pass of a step (CalcDensity, force.h:9-23, main.cpp:138-139) for a particle
@@ -832,12 +769,6 @@ k_density_fused32(int n, int n_pass, const int *__restrict__ sup, const float *_
         if (stopped) atomicAdd(n_stopped, 1);
     }
 }
-
-__global__ void k_skin_check(int n, const double *h, const double *hsup, int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && h[i] > (double)KAPPA * hsup[i]) atomicOr(err, ERR_SKIN);
-}
-
 
 // (2.5 h)^2 as float, rounded up so FP32 superset tests stay conservative
 __global__ void k_h2f(int n, const double *h, float *H2f) {
@@ -1142,25 +1073,6 @@ int sph_build_sph_lists(sph_ctx *ctx, int mode) {
     SPH_TRY(ensure_superset(ctx));
     return filter_lists(ctx, mode);
 }
-
-// mixed-precision density pass straight from the superset (no exact list)
-int sph_density_from_superset(sph_ctx *ctx) {
-    SphSuper &S = ctx->sup;
-    const int n = (int)ctx->n;
-    const int64_t cap = ctx->cap;
-    int *meta = ctx->tree.meta;
-    SPH_TRY(ensure_superset(ctx));
-    k_density_sup32<<<sph_div_up(n, 128), 128, 0, ctx->stream>>>(
-        n, S.nbr, S.r2, S.m, S.cnt, S.map(), FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap),
-        FLD(ctx->F, SPH_Z, cap), FLD(ctx->F, SPH_MASS, cap), FLD(ctx->F, SPH_SMTH, cap), S.hsup,
-        FLD(ctx->F, SPH_DENS, cap), (float)(1365.0 / 64.0 / (3.141592653589793 * ctx->mscale)), meta + META_ERR);
-    ++ctx->launches;
-    SPH_CUDA(ctx, cudaGetLastError());
-    ctx->lists[0].valid = false;
-    return sph_nbr_refresh_h(ctx);
-}
-
-int sph_nbr_ensure_superset(sph_ctx *ctx) { return ensure_superset(ctx); }
 
 // All density passes of the mixed path, the EoS and the exact lists of the final h: rounds of k_density_fused32, the
 // rows of the particles that left their skin walked again between rounds (each round takes every unfinished particle

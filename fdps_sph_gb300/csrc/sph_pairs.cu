@@ -926,23 +926,10 @@ struct GravShape<256> {
     static constexpr int MIN_BLOCKS = 4;
 };
 
-__device__ __forceinline__ void grav_acc(float px, float py, float pz, float e2, float4 q, float &a0, float &a1,
-                                         float &a2, float &a3) {
-    const float dx = px - q.x, dy = py - q.y, dz = pz - q.z;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, e2)));
-    const float ri = rsqrt_a(r2);
-    const float mri = q.w * ri;
-    const float mr3 = mri * ri * ri;
-    a0 = fmaf(-mr3, dx, a0);
-    a1 = fmaf(-mr3, dy, a1);
-    a2 = fmaf(-mr3, dz, a2);
-    a3 -= mri;
-}
-
-// grav_acc for two j at once (x, y, z, m: the pair's coordinates relative to the group origin and
-// masses), with the i-particle's negated coordinates and softening paired with themselves.  Per
-// interaction the same operations and roundings as grav_acc (q - p = -(p - q) exactly); the two j
-// accumulate in the two halves of a0..a3, and a3 sums +m / r (the potential's negative).
+// CalcGravityForce's pair (force.h:154-168) for two j at once (x, y, z, m: their coordinates relative
+// to the group origin and masses), with the i-particle's negated coordinates and softening paired with
+// themselves: d = x_j - x_i, a += m r^-3 d.  The two j accumulate in the two halves of a0..a3, and a3 sums
+// +m / r (the potential's negative).
 __device__ __forceinline__ void grav_acc2(f32x2 nx, f32x2 ny, f32x2 nz, f32x2 e2, f32x2 x, f32x2 y, f32x2 z,
                                           f32x2 m, f32x2 &a0, f32x2 &a1, f32x2 &a2, f32x2 &a3) {
     const f32x2 dx = f2_add(x, nx), dy = f2_add(y, ny), dz = f2_add(z, nz);
@@ -961,8 +948,9 @@ __device__ __forceinline__ void grav_acc2(f32x2 nx, f32x2 ny, f32x2 nz, f32x2 e2
 // NU: of a thread's two i-particles, both, or (small runs, whose groups do not fill the chip) one, the block's
 // blockIdx.y saying which: the partitions and so the bits are the same, the sums take half as long and the walk is done
 // twice.  Lists and sums, both against one: 137 -> 109 us at 3,000 particles, 152 -> 116 at 5,000, 189 -> 141 at 10,000,
-// 193 -> 175 at 40,000; 370 -> 339 at 100,000, but 278 -> 282 at 70,000 and from 150,000 on a loss (405 -> 432, 447 -> 514
-// at 200,000).  The line of 8 groups per SM (1,216; near 50,000 particles) lies where the gain ends for good or ill.
+// 193 -> 175 at 40,000, 278 -> 282 at 70,000, 370 -> 339 at 100,000 (1,075 groups), and from 150,000 on a loss (405 -> 432,
+// 447 -> 514 at 200,000).  The line of 8 groups per SM (1,216, some 113,000 particles) lies between the last gain and the
+// first real loss.
 template <int GF_T, int NU>
 __global__ void __launch_bounds__(GF_T, GravShape<GF_T>::MIN_BLOCKS)
 k_grav_fused32(const int *__restrict__ group_cell, const int4 *__restrict__ cinfo, const double4 *__restrict__ com,
@@ -1337,44 +1325,6 @@ __global__ void k_ext_force(int n, IntegArgs a, const double *dt, const unsigned
     a.az[i] += -a.vz[i] * 0.05 / d;
 }
 
-constexpr int RED_BLOCKS = 304;
-
-__global__ void k_min_partial(int n, const double *v, double *part) {
-    double r = 1.0e30;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double d = v[i];
-        r = (d < r) ? d : r;   // std::min(r, d) with r first, integral.h:16
-        if (d != d) r = d;     // a NaN dt propagates so the host sees it
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double t = __shfl_xor_sync(0xffffffffu, r, o);
-        r = (t < r || t != t) ? t : r;
-    }
-    __shared__ double s[32];
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = r;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) r = (s[w] < r || s[w] != s[w]) ? s[w] : r;
-        part[blockIdx.x] = r;
-    }
-}
-
-__global__ void k_min_final(const double *part, int nb, double *out) {
-    double r = 1.0e30;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) r = (part[b] < r || part[b] != part[b]) ? part[b] : r;
-    for (int o = 16; o > 0; o >>= 1) {
-        const double t = __shfl_xor_sync(0xffffffffu, r, o);
-        r = (t < r || t != t) ? t : r;
-    }
-    __shared__ double s[32];
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = r;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) r = (s[w] < r || s[w] != s[w]) ? s[w] : r;
-        *out = r;
-    }
-}
-
 // per run: one block per tile (tiles aligned to run starts), then one block per run over its tiles
 __device__ double block_min(double r) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -1414,38 +1364,7 @@ __global__ void k_min_runs(const double *part, const int4 *info, double *out, do
     }
 }
 
-// conserved quantities, fixed-order two-stage reduction in FP64
-__global__ void k_diag_partial(int n, const double *x, const double *y, const double *z, const double *vx,
-                               const double *vy, const double *vz, const double *m, const double *u,
-                               const double *pot, double *part) {
-    double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double mi = m[i];
-        const double v2 = vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i];
-        q[0] += mi * (u[i] + 0.5 * v2 + 0.5 * pot[i]);
-        q[1] += mi * vx[i];
-        q[2] += mi * vy[i];
-        q[3] += mi * vz[i];
-        q[4] += mi * (y[i] * vz[i] - z[i] * vy[i]);
-        q[5] += mi * (z[i] * vx[i] - x[i] * vz[i]);
-        q[6] += mi * (x[i] * vy[i] - y[i] * vx[i]);
-        q[7] += mi;
-    }
-    __shared__ double s[8][32];
-    for (int k = 0; k < 8; ++k) {
-        double v = q[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) s[k][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += s[threadIdx.x][w];
-        part[blockIdx.x * 8 + threadIdx.x] = v;
-    }
-}
-
-// per run: tiles (k_diag_partial over one tile's range), then each run's tiles in order
+// conserved quantities of every run, fixed-order reduction in FP64: a tile per block, then each run's tiles in order
 __global__ void k_diag_tiles(const double *x, const double *y, const double *z, const double *vx, const double *vy,
                              const double *vz, const double *m, const double *u, const double *pot, const int4 *tiles,
                              double *part) {
@@ -1484,14 +1403,6 @@ __global__ void k_diag_runs(const double *part, const int4 *info, int R, double 
         double v = 0.0;
         for (int b = q.z; b < q.z + q.w; ++b) v += part[b * 8 + c];
         out[k] = v;
-    }
-}
-
-__global__ void k_diag_final(const double *part, int nb, double *out) {
-    if (threadIdx.x < 8 && blockIdx.x == 0) {
-        double v = 0.0;
-        for (int b = 0; b < nb; ++b) v += part[b * 8 + threadIdx.x];
-        out[threadIdx.x] = v;
     }
 }
 
@@ -1721,8 +1632,8 @@ int sph_run_reduce_dt(sph_ctx *ctx) {
     Runs &R = ctx->runs;
     launch_after(true, k_min_tiles, R.T, 256, 0, ctx->stream, CF(SPH_DT), R.tiles, R.part); ++ctx->launches;
     // the host's values straight into the pinned block (behind the words of sph_publish) where they fit it
-    double *h = ctx->host_scalars + 32;
-    const bool fits = R.R <= 480;
+    double *h = ctx->host_scalars + HOST_DT;
+    const bool fits = R.R <= HOST_SCALARS - HOST_DT;
     launch_after(true, k_min_runs, R.R, 256, 0, ctx->stream, R.part, R.info, R.dt_dev, fits ? h : nullptr);
     ++ctx->launches;
     SPH_CUDA(ctx, cudaGetLastError());

@@ -695,8 +695,8 @@ __global__ void __launch_bounds__(OT_B) k_cell_levels(int n, int n_leaf, const u
 }
 
 // the cells: cell id = the exclusive scan of the block-and-level counts (level-major) plus the
-// rank of the particle among its block's starts at that level; start, count (the end found by
-// a binary search over the run's keys), level.  Also the level offsets in meta; more cells than
+// rank of the particle among its block's starts at that level; start, count (to the end of the
+// run of keys that share its digits), level.  Also the level offsets in meta; more cells than
 // the capacity sets ERR_CELL_OVERFLOW and leaves no cells.
 __global__ void __launch_bounds__(OT_B) k_cell_emit(int n, int64_t cap, const uint64_t *keys,
                                                     const int *prun, const int4 *info,
@@ -1284,7 +1284,7 @@ int sph_sort_and_build(sph_ctx *ctx) {
     SPH_TRY(sph_tree_reserve(ctx, n));
     cudaStream_t st = ctx->stream;
     // With event timing on the work is launched directly (its segments are timed); otherwise the
-    // ~170 launches of the sort and the level loop replay as one CUDA graph.
+    // 14 to 29 launches of the sort and the octree (by the sort's route) replay as one CUDA graph.
     if (ctx->timing || !ctx->use_graphs) SPH_TRY(enqueue_sort_tree(ctx));
     else SPH_TRY(sort_tree_graph(ctx));
     SPH_TRY(time_mark(ctx, SEG_TREE));
