@@ -248,6 +248,7 @@ template <class T>
 int dalloc(sph_ctx *ctx, T **p, int64_t n) {
     if (*p) cudaFree(*p);
     *p = nullptr;
+    ctx->allocations += 1;
     cudaError_t e = cudaMalloc((void **)p, sizeof(T) * (size_t)std::max<int64_t>(n, 1));
     if (e != cudaSuccess) {
         *p = nullptr;

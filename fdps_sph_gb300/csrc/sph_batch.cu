@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(256) k_scatter_results(const int64_t *meta, co
                    (int64_t)s_res * m[1] / 8);
 }
 
-// blocks per walk of the two copies: eight where the walks alone would leave SMs (152) idle
-dim3 copy_grid(int n_walk) { return dim3((unsigned)n_walk, n_walk < 152 ? 8 : 1); }
+// blocks per walk of the two copies: eight where the walks alone would leave SMs idle
+dim3 copy_grid(int n_walk) { return dim3((unsigned)n_walk, n_walk < GB300_SMS ? 8 : 1); }
 
 // where a dispatch's sections sit in the tag's staging (bytes, 16-byte aligned sections)
 struct Layout {
@@ -411,7 +411,7 @@ int upload_array(Resident &R, char *dst, const void *src, size_t bytes) {
     if (R.pageable == 1 && g_batch_staging.load() != SPH_BATCH_STAGING_HOST && bytes % 8 == 0 &&
         ((uintptr_t)src & 7u) == 0) {
         const int64_t words = (int64_t)(bytes / 8);
-        const int grid = (int)std::min<int64_t>(152 * 8, (words + 255) / 256);
+        const int grid = (int)std::min<int64_t>(GB300_SMS * 8, (words + 255) / 256);
         k_copy_flat<<<grid, 256, 0, R.stream>>>((const unsigned long long *)src, (unsigned long long *)dst, words);
         if (cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(R.stream) == cudaSuccess) return SPH_OK;
         cudaGetLastError();

@@ -6,6 +6,8 @@
 
 namespace sph {
 
+constexpr int GB300_SMS = 152;   // (these entry points have no context to ask)
+
 // The j entries of one dispatch's walks, entry k of the walk starting at offset jo being
 // src[jo + k].  Payload form (calcForceAllAndWriteBackMultiWalk): idx == nullptr, the entries are
 // the staged payloads themselves, base[k].  Index form (calcForceAllAndWriteBackMultiWalkIndex):

@@ -430,14 +430,14 @@ __global__ void __launch_bounds__(W * 32) k_walk_grav64(const int64_t *meta, int
 }
 
 // Blocks of 8 warps with 32 i-particles (four per warp, one staging of the j-list for them) where that still
-// gives every SM two blocks (152 SMs), else with 8 (one per warp), so that a few walks spread over the chip, and for
+// gives every SM two blocks, else with 8 (one per warp), so that a few walks spread over the chip, and for
 // the smallest dispatches 4 warps with one i-particle each, so that every warp has an FP64 pipe (one per SM quarter)
 // to itself: a call of every functor on one walk of 180 particles 168 -> 152 us.
 struct Shape {
     int ic, threads;
     dim3 grid;
     Shape(int n_walk, int64_t n_i, int max_i) {
-        ic = n_i >= 152 * 64 ? IC_MAX : (n_i > 152 * 4 ? W : 4);
+        ic = n_i >= GB300_SMS * 64 ? IC_MAX : (n_i > GB300_SMS * 4 ? W : 4);
         threads = ic == 4 ? 128 : W * 32;
         const int chunks = (max_i + ic - 1) / ic;
         grid = dim3((unsigned)n_walk, (unsigned)(chunks > 0 ? (chunks < 4096 ? chunks : 4096) : 1));

@@ -331,7 +331,7 @@ struct Runs {
 }  // namespace sph
 
 namespace sph {
-constexpr int GRAPH_KEY_N = 25;
+constexpr int GRAPH_KEY_N = 26;
 // a captured sort + octree build and what it was captured for
 struct TreeGraph {
     cudaGraphExec_t exec = nullptr;
@@ -421,6 +421,7 @@ struct sph_ctx {
     // CUDA graphs of the sort + octree build: one per state-buffer parity and layout
     bool use_graphs = true;
     sph::TreeGraph tree_graphs[4];
+    uintptr_t allocations = 0;   // of particle, run, tree and sort buffers so far
     int graph_next = 0;
     int64_t graph_captures = 0, graph_replays = 0;
 };

@@ -1029,6 +1029,7 @@ template <class T>
 static int dalloc(sph_ctx *ctx, T **p, int64_t n) {
     if (*p) cudaFree(*p);
     *p = nullptr;
+    ctx->allocations += 1;
     if (n <= 0) n = 1;
     cudaError_t e = cudaMalloc((void **)p, sizeof(T) * (size_t)n);
     if (e != cudaSuccess) {
@@ -1213,8 +1214,9 @@ static int enqueue_sort_tree(sph_ctx *ctx) {
     return enqueue_tree(ctx);
 }
 
-// Everything the captured work depends on: sizes and every buffer it touches.  The permutation
-// swaps the state buffers, so a step alternates between two keys.
+// Everything the captured work depends on: sizes, the buffers that trade places (the permutation swaps the state
+// buffers, so a step alternates between two keys), and the number of allocations: a buffer that moved is told from the
+// one that was captured even where the others came to lie at their old addresses.
 static void graph_key(const sph_ctx *ctx, uintptr_t key[GRAPH_KEY_N]) {
     const Tree &t = ctx->tree;
     const uintptr_t k[GRAPH_KEY_N] = {
@@ -1225,7 +1227,7 @@ static void graph_key(const sph_ctx *ctx, uintptr_t key[GRAPH_KEY_N]) {
         (uintptr_t)ctx->runs.tiles, (uintptr_t)ctx->runs.part, (uintptr_t)ctx->scan.part, (uintptr_t)t.cinfo,
         (uintptr_t)ctx->cfg.n_leaf, (uintptr_t)(ctx->runs.max_tiles > RS_DIRECT) +
             (uintptr_t)(ctx->runs.max_tiles > RB_KEYS / RUN_TILE), (uintptr_t)ctx->cfg.n_group,
-        (uintptr_t)ctx->sup.units, (uintptr_t)ctx->grav.group_cell};
+        (uintptr_t)ctx->sup.units, (uintptr_t)ctx->grav.group_cell, ctx->allocations};
     for (int i = 0; i < GRAPH_KEY_N; ++i) key[i] = k[i];
 }
 
