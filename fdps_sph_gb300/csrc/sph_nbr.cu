@@ -99,7 +99,7 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
     const bool valid = lane < U.y;
     const int i = U.x + (valid ? lane : 0);
     const double xi = x[i], yi = y[i], zi = z[i];
-    if (hsup && valid) hsup[i] = h[i];   // the h this row is built for (a repair has set it: k_skin_raise)
+    if (hsup && valid) hsup[i] = h[i];   // the h this row is built for (null: it is built for the recorded one)
     const float4 pih = xh[i], pil = xl[i];
     const float H2i = valid ? H2f[i] : 0.0f;
     double lo[3] = {valid ? xi : INFINITY, valid ? yi : INFINITY, valid ? zi : INFINITY};
@@ -351,20 +351,28 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
 // one particle: a larger one recorded is missing outside (a later growth
 // inside the skin would not be seen there), a smaller one is missing inside.
 //
+// That is the FP64 passes' rule.  The mixed passes still repair by the h of the moment, within 2.5 h_v.  In a mixed step
+// only violators change their h after a repair, so what can be missing is a violator that grows on, inside its new skin,
+// from the row of a particle between 1 / KAPPA and 1 of its support away (found: one pair in 40 runs of 2,000 to 300,000
+// particles, a few in 8 steps of 1M; a caller of single passes can see the other two cases too).  Such a pair weighs less
+// than 1e-6 of the kernel's centre, but one entry more shifts the blocks of 32 that a row's FP32 partial sums are rounded
+// in: with the FP64 rule a third of the runs of 1M particles and more change in last bits (up to 2e-7 of a component's
+// rms; 4e-6 after 16 steps of a sweep), and a mixed run gives the same bits in every build so far.
+//
 // Between the FP64 density passes every h is still on its way, and a particle that has used most of its skin tends to
 // leave it a pass later; so a repair takes in all that grew by more than SKIN_64, for fewer repairs in a row (prologue
-// of 71,184 particles in contact 3 -> 2, of 10,000 2 -> 1; 53.1 -> 52.5 and 9.85 -> 9.76 ms with four steps).  The mixed
-// passes leave only violators unfinished, and more units for the others are a loss (1M particles from a host 10.3 -> 10.6
-// ms a step).
+// of 71,184 particles in contact 3 -> 2, of 10,000 2 -> 1; 53.1 -> 52.5 and 9.85 -> 9.76 ms with four steps).
 constexpr double SKIN_64 = 1.04;
 
-// vR: reach of the particles a repair takes in (h > grown hsup; 0: the others); nviol: the violators among them
-__global__ void k_viol_mark(int n, double grown, const double *h, const double *hsup, float *vR, int *nviol) {
+// vR: reach (`reach` times 2.5 h) of the particles a repair takes in (h > grown hsup; 0: the others); nviol: the violators
+// among them
+__global__ void k_viol_mark(int n, double grown, double reach, const double *h, const double *hsup, float *vR,
+                            int *nviol) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool v = false;
     if (i < n) {
         v = h[i] > (double)KAPPA * hsup[i];
-        vR[i] = h[i] > grown * hsup[i] ? __double2float_ru(SUPPORT * h[i] * (KAPPA * 1.001)) : 0.0f;
+        vR[i] = h[i] > grown * hsup[i] ? __double2float_ru(SUPPORT * h[i] * reach) : 0.0f;
     }
     const unsigned b = __ballot_sync(FULLM, v);
     if ((threadIdx.x & 31) == 0 && b) atomicAdd(nviol, __popc(b));
@@ -879,9 +887,9 @@ int sph_nbr_prepare(sph_ctx *ctx) {
     return SPH_OK;
 }
 
-// walks the units in uidx (or all units when uidx is null) for the current h, which hsup records, or (repair) for the
-// recorded hsup (k_skin_raise); grows the row capacity if needed
-static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk, bool repair) {
+// walks the units in uidx (or all units when uidx is null) for the current h, which hsup records, or (recorded) for the
+// hsup there is (k_skin_raise); grows the row capacity if needed
+static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk, bool recorded) {
     SphSuper &S = ctx->sup;
     const int n = (int)ctx->n;
     const int64_t pitch = n;   // rows: particle i's entries at i * K .. i * K + K - 1
@@ -896,7 +904,7 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk, bool repair) {
         S.cap_uover = S.cap_units;
     }
     // cell hmax must follow the h that is walked for
-    if (S.rebuilds_step > 0) SPH_TRY(sph_tree_refresh_hmax(ctx, repair ? S.hsup : FLD(ctx->F, SPH_SMTH, cap)));
+    if (S.rebuilds_step > 0) SPH_TRY(sph_tree_refresh_hmax(ctx, recorded ? S.hsup : FLD(ctx->F, SPH_SMTH, cap)));
     S.rebuilds_step += 1;
     for (int attempt = 0; attempt < 4; ++attempt) {
         if (!S.nbr || S.pitch < pitch || S.K_alloc != S.K || S.spill_alloc != S.spill_cap) {
@@ -935,8 +943,8 @@ static int walk_units(sph_ctx *ctx, const int *uidx, int n_walk, bool repair) {
         if (blocks > 0) {
             auto walk = S.spill_on ? k_sup_walk<true> : k_sup_walk<false>;
             walk<<<blocks, NB_WARPS * 32, 0, ctx->stream>>>(n_walk, split, S.units, uidx, FLD(ctx->F, SPH_X, cap), FLD(ctx->F, SPH_Y, cap), FLD(ctx->F, SPH_Z, cap),
-                FLD(ctx->F, SPH_SMTH, cap), repair ? nullptr : S.hsup, walk_xh(ctx), walk_xl(ctx),
-                repair ? S.H2s : S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
+                FLD(ctx->F, SPH_SMTH, cap), recorded ? nullptr : S.hsup, walk_xh(ctx), walk_xl(ctx),
+                recorded ? S.H2s : S.H2f, ctx->runs.prun, T, S.nbr, S.r2, S.m,
                 S.cnt, S.map(), S.uover, meta + META_ERR, meta + META_MAXCNT);
             ++ctx->launches;
         }
@@ -1020,8 +1028,9 @@ static int ensure_superset(sph_ctx *ctx) {
     Tree &t = ctx->tree;
     float *vR = S.vR;
     SPH_CUDA(ctx, cudaMemsetAsync(meta + META_ERR + 8, 0, sizeof(int), ctx->stream));
-    const double grown = ctx->cfg.precision == SPH_PREC_MIXED ? (double)KAPPA : SKIN_64;
-    k_viol_mark<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, grown, FLD(ctx->F, SPH_SMTH, cap), S.hsup, vR,
+    const bool exact = ctx->cfg.precision != SPH_PREC_MIXED;   // (see above)
+    const double grown = exact ? SKIN_64 : (double)KAPPA, reach = exact ? KAPPA * 1.001 : 1.001;
+    k_viol_mark<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, grown, reach, FLD(ctx->F, SPH_SMTH, cap), S.hsup, vR,
                                                               meta + META_ERR + 8);
     ++ctx->launches;
     int *hs = (int *)ctx->host_scalars;
@@ -1031,8 +1040,10 @@ static int ensure_superset(sph_ctx *ctx) {
     if (nviol == 0) return SPH_OK;
     S.violators += nviol;
     if ((int64_t)nviol * 8 > n) return build_superset(ctx);   // widespread growth: walk everything
-    k_skin_raise<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_SMTH, cap), vR, S.hsup, S.H2s);
-    ++ctx->launches;
+    if (exact) {
+        k_skin_raise<<<sph_div_up(n, 256), 256, 0, ctx->stream>>>(n, FLD(ctx->F, SPH_SMTH, cap), vR, S.hsup, S.H2s);
+        ++ctx->launches;
+    }
     // influence radius per cell, bottom-up
     const int grid = 2 * ctx->num_sms;
     for (int l = t.depth; l >= 0; --l) {
@@ -1049,7 +1060,7 @@ static int ensure_superset(sph_ctx *ctx) {
     SPH_TRY(sph_publish(ctx, ctx->scan.total, 1));
     SPH_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     const int nmark = hs[0];
-    return walk_units(ctx, S.uidx, nmark, true);
+    return walk_units(ctx, S.uidx, nmark, exact);
 }
 
 // exact list of `mode` (0 gather, 1 symmetric, 2 both) from a superset that is valid for the current h
