@@ -356,7 +356,7 @@ k_sup_walk(int n_units, int split, const int2 *__restrict__ units, const int *__
 // from the row of a particle between 1 / KAPPA and 1 of its support away (found: one pair in 40 runs of 2,000 to 300,000
 // particles, a few in 8 steps of 1M; a caller of single passes can see the other two cases too).  Such a pair weighs less
 // than 1e-6 of the kernel's centre, but one entry more shifts the blocks of 32 that a row's FP32 partial sums are rounded
-// in: with the FP64 rule a third of the runs of 1M particles and more change in last bits (up to 2e-7 of a component's
+// in: with the FP64 rule 6 of 18 runs of 1M and 4M particles changed in last bits (up to 2e-7 of a component's
 // rms; 4e-6 after 16 steps of a sweep), and a mixed run gives the same bits in every build so far.
 //
 // Between the FP64 density passes every h is still on its way, and a particle that has used most of its skin tends to
